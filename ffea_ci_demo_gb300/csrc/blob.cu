@@ -190,6 +190,14 @@ struct BlobImpl final : ffea_gpu_blob {
     double *cheb = nullptr;  // its lambda_max estimate and the Lanczos record that makes it (CHEB_STATE)
     int *nb_ptr = nullptr, *nb_list = nullptr;  // its blocks' neighbour blocks
     unsigned int *nb_flags = nullptr;           // and their publication counters
+    // staged owned-rows CG: halo lists, local columns, and the messages (with the phase timers, cleared per solve)
+    int *halo_ptr = nullptr, *halo_list = nullptr;
+    unsigned short *lcol = nullptr;
+    int nhalo = 0;
+    bool cg_reg = false;  // the single-reduction CG keeps each lane's first matrix blocks in registers
+    char *comm = nullptr;
+    size_t comm_bytes = 0;
+    Msg *msg = nullptr, *rmsg = nullptr;
     float4 *dpos = nullptr;  // mixed path: node offsets from the reference point
     MixedElements me;        // mixed path: the element phase's FP32 node data, block lists and block sums
     // measurements: densities, reference positions of vertices and midpoints (SoA), per-block sums
@@ -327,6 +335,52 @@ struct BlobImpl final : ffea_gpu_blob {
         return FFEA_GPU_OK;
     }
 
+    // The rows of other blocks that each block's rows reach through the pattern, and every slot's column as an index
+    // into the block's staged vector (own rows first, then, from npb, the halo in ascending row order). The pattern
+    // is symmetric (an element couples each pair of its unpinned nodes both ways; a pinned row keeps only its diagonal
+    // and no row has its column), so a block reads from exactly the blocks that read from it, which the exchange's
+    // buffer reuse relies on.
+    struct Halo {
+        std::vector<int> ptr, list;
+        std::vector<unsigned short> lcol;
+        int largest = 0;
+    };
+    void build_halo(int npb, int grid, Halo &o) const {
+        const int N = h.N;
+        o.ptr.assign(grid + 1, 0);
+        o.list.clear();
+        o.lcol.assign(h.nslots, 0);
+        std::vector<int> at(N, -1), got;
+        for (int b = 0; b < grid; ++b) {
+            const int a0 = std::min(N, b * npb), a1 = std::min(N, (b + 1) * npb);
+            got.clear();
+            for (int a = a0; a < a1; ++a) {
+                const int s0 = h.slice_ptr[a >> 5], ln = a & 31;
+                for (int k = 0; k < h.rowlen[a]; ++k) {
+                    const int c = h.bcol[s0 + 32 * k + ln];
+                    if ((c < a0 || c >= a1) && at[c] < 0) {
+                        at[c] = 0;
+                        got.push_back(c);
+                    }
+                }
+            }
+            std::sort(got.begin(), got.end());
+            for (size_t i = 0; i < got.size(); ++i) at[got[i]] = (int)i;
+            for (int a = a0; a < a1; ++a) {
+                const int s0 = h.slice_ptr[a >> 5], ln = a & 31;
+                for (int k = 0; k < h.rowlen[a]; ++k) {
+                    const int c = h.bcol[s0 + 32 * k + ln];
+                    o.lcol[s0 + 32 * k + ln] = (unsigned short)((c >= a0 && c < a1) ? c - a0 : npb + at[c]);
+                }
+            }
+            for (int c : got) at[c] = -1;
+            o.list.insert(o.list.end(), got.begin(), got.end());
+            o.ptr[b + 1] = (int)o.list.size();
+            o.largest = std::max(o.largest, (int)got.size());
+        }
+        if (o.list.empty()) o.list.push_back(0);
+    }
+
     int init() override {
         CK(cudaGetDevice(&device));
         int major = 0, minor = 0;
@@ -448,22 +502,36 @@ struct BlobImpl final : ffea_gpu_blob {
             g_last_error = "cg kernel cannot be made resident";
             return FFEA_GPU_ECUDA;
         }
-        // one block per SM (fewer for small meshes). A mixed blob of up to 2048 rows runs in a single block (its
-        // barrier is a block barrier); an FP64 one only up to 256 rows, since its SpMV is bound by the FP64
-        // units of the SMs it runs on. A single block has as few threads as give each row 8 lanes. Threads per
-        // SpMV row chosen so that every warp handles its rows in one pass: tpn = the largest power of two <= 8
-        // with N <= warps * 32 / tpn
-        if (N <= (mixed ? 2048 : 256)) {
-            cg_grid = 1;
-            cg_block = std::min(Launch<R>::cg_threads(), std::max(128, (N * 8 + 31) / 32 * 32));
-        } else {
-            cg_grid = std::max(1, std::min(maxg, (N + 255) / 256));
-            cg_block = Launch<R>::cg_threads();
-        }
-        const long long lanes = (long long)cg_grid * cg_block;
-        tpn = 8;
-        while (tpn > 1 && (long long)N * tpn > lanes) tpn >>= 1;
-        partial_stride = cg_grid;
+        // The mixed CG_nomass solve (cg_mixed_sr_kernel) spreads small meshes further: its blocks exchange rows and sums
+        // as tagged messages, so a block more costs little, and up to SR_REG_ROWS rows its lanes hold the whole matrix
+        // in registers (four lanes of six blocks to a row). us per step at 64 / 128 / 192 / 256 / 320 rows a block:
+        // 10^3 cells 499 / 455 / 508 / 509 / 567, 20^3 976 / 879 / 930 / 968 / 1078, 24^3 - / 1117 / 1124 / 1166 / 1321.
+        // Above SR_REG_THREADS rows a block (N > 73,000) the form without register blocks takes over.
+        const bool sr_able = mixed && p.solver == FFEA_GPU_NOMASS_CG && 40.0 * (double)h.nslots <= L2_MATRIX_BYTES;
+        auto pick_grid = [&](bool sr) {
+            if (sr) {
+                cg_grid = std::max(1, std::min(maxg, (N + SR_REG_ROWS - 1) / SR_REG_ROWS));
+                const int rows = (N + cg_grid - 1) / cg_grid;
+                cg_block = (rows + 31) / 32 * 32 <= SR_REG_THREADS ? SR_REG_THREADS : Launch<R>::cg_threads();
+            } else if (N <= (mixed ? 2048 : 256)) {
+                cg_grid = 1;
+                cg_block = std::min(Launch<R>::cg_threads(), std::max(128, (N * 8 + 31) / 32 * 32));
+            } else {
+                cg_grid = std::max(1, std::min(maxg, (N + 255) / 256));
+                cg_block = Launch<R>::cg_threads();
+            }
+            // every block's rows in one pass (the staged kernel), or every row of the grid
+            auto one_pass = [&](int t) {
+                const int align = 32 / t, rows = (N + cg_grid - 1) / cg_grid;
+                return sr ? (long long)((rows + align - 1) / align * align) * t <= cg_block
+                          : (long long)N * t <= (long long)cg_grid * cg_block;
+            };
+            tpn = 8;
+            while (tpn > 1 && !one_pass(tpn)) tpn >>= 1;
+            const int align = 32 / tpn, rows = (N + cg_grid - 1) / cg_grid;
+            return (rows + align - 1) / align * align;  // rows per block
+        };
+        int npb = pick_grid(sr_able);
         // The CG kernel follows from the blob's size alone (no other input selects it):
         //  - each block keeps a run of rows in shared memory when they fit (cg_own_kernel, cg_mixed_own_kernel);
         //    the run is a multiple of a warp's rows so that a warp's rows share a SELL slice; else the grid-strided
@@ -472,37 +540,46 @@ struct BlobImpl final : ffea_gpu_blob {
         //    its FP32 matrix stays in L2
         {
             const int maxrows = Launch<R>::cg_own_max_rows(device);
-            const int align = 32 / tpn, rows = (N + cg_grid - 1) / cg_grid;
-            const int npb = (rows + align - 1) / align * align;
-            cg_npb = (maxrows > 0 && npb <= maxrows) ? npb : 0;
             // ... while its FP32 matrix (40 B per 3x3 block) stays in L2: once the SpMV streams the matrix from HBM
             // the two-reduction kernel's iterations are the shorter ones (64^3 cells: 38.7 against 43.5 us)
-            const bool l2_resident = 40.0 * (double)h.nslots <= L2_MATRIX_BYTES;
-            if (mixed && p.solver == FFEA_GPU_NOMASS_CG && maxrows > 0 && l2_resident) {
+            if (sr_able) {
                 // the polynomial preconditioner's two extra vectors per row must fit as well; else Jacobi
                 const int poly = p.cg_poly == 0 ? FFEA_GPU_CG_POLY_DEFAULT : std::max(p.cg_poly, 0);
+                Halo hl;
+                build_halo(npb, cg_grid, hl);
+                const size_t limit = (size_t)std::max(Launch<R>::cg_sr_smem_limit(device), 0);
                 for (int deg : {poly, 0}) {
-                    const int srrows = Launch<R>::cg_sr_max_rows(device, deg);
-                    if (srrows > 0 && npb <= srrows) {
+                    if ((long long)npb * tpn <= cg_block && npb + hl.largest < 65536 &&
+                        sr_smem_bytes(npb, hl.largest, deg) <= limit) {
                         cg_sr = true;
                         cg_poly = deg;
                         break;
                     }
                 }
-                if (cg_sr) cg_npb = npb;
+                if (cg_sr) {
+                    cg_npb = npb;
+                    cg_reg = cg_block == SR_REG_THREADS;
+                    nhalo = hl.largest;
+                    CK(mem.upload(&halo_ptr, hl.ptr));
+                    CK(mem.upload(&halo_list, hl.list));
+                    CK(mem.upload(&lcol, hl.lcol));
+                }
             }
+            if (!cg_sr) {
+                if (sr_able) npb = pick_grid(false);
+                cg_npb = (maxrows > 0 && npb <= maxrows) ? npb : 0;
+            }
+            partial_stride = cg_grid;
             if (cg_sr) {
-                // the first blocks of each owned row kept in shared memory for the solve, as many as the rest of
-                // the block's shared memory holds (ffea_gpu_params::cg_smem_blocks caps them: n > 0 at most n, -1
-                // none; the results do not depend on it)
-                // The block's shared memory stops at 168 KB so that L1 (the rest of the SM's 256 KB) keeps the
-                // neighbours' exchanged vectors: on the 40^3 cube 6 cached blocks per row (167 KB) gave 20.8 us per
-                // iteration, the 9 that fit (223 KB) 21.4 us, none 22.3 us.
-                const long long avail = std::min<long long>(Launch<R>::cg_sr_smem_limit(device), 168 * 1024) -
-                                        (long long)sr_smem_bytes(cg_npb, cg_poly);
+                // the first blocks of each owned row kept on chip for the solve: SR_REG_BLOCKS of each lane in registers
+                // (cg_reg), then as many as the rest of the block's shared memory holds
+                // (ffea_gpu_params::cg_smem_blocks caps those: n > 0 at most n, -1 none; the results do not depend on it)
+                const long long avail = (long long)Launch<R>::cg_sr_smem_limit(device) -
+                                        (long long)sr_smem_bytes(cg_npb, nhalo, cg_poly);
                 const long long S = sr_cache_stride(cg_npb, tpn);
                 int maxlen = 0;
                 for (int a = 0; a < N; ++a) maxlen = std::max(maxlen, h.rowlen[a]);
+                maxlen = std::max(0, maxlen - (cg_reg ? SR_REG_BLOCKS * tpn : 0));
                 cg_kc = avail <= 0 ? 0 : (int)std::min<long long>(maxlen, avail / (SR_CACHE_BYTES_PER_BLOCK * S));
                 if (p.cg_smem_blocks != 0) cg_kc = std::min(cg_kc, std::max(0, p.cg_smem_blocks));
             }
@@ -511,7 +588,7 @@ struct BlobImpl final : ffea_gpu_blob {
                 CK(cudaMemset(cheb, 0, CHEB_STATE * sizeof(double)));
             }
             // the FP64 owned-rows CG publishes its search direction the same way (CG_nomass's 3x3 pattern)
-            if (cg_sr || (!mixed && cg_npb > 0 && p.solver == FFEA_GPU_NOMASS_CG)) {
+            if (!mixed && cg_npb > 0 && p.solver == FFEA_GPU_NOMASS_CG) {
                 // the blocks each block's SpMV reads z (p) from: owners of the columns of its rows. The pattern is
                 // symmetric (an element couples each pair of its unpinned nodes both ways; a pinned row keeps only
                 // its diagonal and no row has its column), so these are also the blocks that read from it, which
@@ -542,7 +619,14 @@ struct BlobImpl final : ffea_gpu_blob {
         CK(mem.alloc(&st, 1));
         hist_cap = std::min(std::max(p.max_iterations_cg, 1), 1 << 20);
         CK(mem.alloc(&history, (size_t)hist_cap));
-        CK(mem.alloc(&phase_ns, (size_t)FFEA_GPU_CG_PHASES));
+        {
+            const size_t head = 256, rows = cg_sr ? 2 * (size_t)N : 0, red = cg_sr ? 2 * (size_t)MIXED_SR_NP * partial_stride : 0;
+            comm_bytes = head + (rows + red) * sizeof(Msg);
+            CK(mem.alloc(&comm, comm_bytes));
+            phase_ns = reinterpret_cast<unsigned long long *>(comm);
+            msg = reinterpret_cast<Msg *>(comm + head);
+            rmsg = msg + rows;
+        }
         CK(mem.alloc(&gb, 1));
         // RNG jump tables: draws of element e start 7e after the step's state; a step consumes 7T
         const int nchunks = (T + 31) / 32;
@@ -669,7 +753,10 @@ struct BlobImpl final : ffea_gpu_blob {
         ca.eps2 = p.epsilon2;
         ca.limit_ns = 2000000000ull;
         ca.history = history; ca.hist_cap = hist_cap; ca.tpn = tpn; ca.phase_ns = phase_ns;
-        CK(cudaMemsetAsync(phase_ns, 0, FFEA_GPU_CG_PHASES * sizeof(unsigned long long), stream));
+        CK(cudaMemsetAsync(comm, 0, comm_bytes, stream));
+        ca.halo_ptr = halo_ptr; ca.halo_list = halo_list; ca.lcol = lcol; ca.nhalo = nhalo;
+        ca.msg = msg; ca.rmsg = rmsg;
+        ca.reg = cg_reg;
         ca.dpos = dpos; ca.nmodes = nomass ? nmodes : 0;
         for (int i = 0; i < 36; ++i) ca.modes[i] = modes[i];
         ca.npb = cg_npb;

@@ -138,6 +138,53 @@ __device__ __forceinline__ bool grid_sync_ep(GridBarrier *gb, DevStatus *st, uns
     return barrier_ep(gb, gridDim.x, st, limit_ns, epoch);
 }
 
+// ---------------------------------------------------------------------------
+// Tagged messages between the blocks of a cooperative CG kernel. A message is one 16-byte word, three payload words
+// and the epoch it belongs to, written and read as a single 128-bit access of the GPU scope (so a reader sees all
+// of it or none), and its reader polls the message itself: the data travels with its own "ready" flag, one L2 round
+// trip after the store, where a counter and an acquire before the data's own load cost two and a fence. The words are
+// zeroed before the launch and epochs start at 1. Two buffers alternate by epoch: a block publishes epoch e + 2 only
+// after it has read what its readers published for e + 1, which they do only after they have read epoch e.
+// ---------------------------------------------------------------------------
+struct alignas(16) Msg {
+    uint32_t x, y, z, tag;
+};
+
+__device__ __forceinline__ void msg_put(Msg *p, uint32_t x, uint32_t y, uint32_t z, uint32_t tag) {
+    const unsigned long long lo = (unsigned long long)x | ((unsigned long long)y << 32),
+                             hi = (unsigned long long)z | ((unsigned long long)tag << 32);
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+                 "l"(lo), "l"(hi)
+                 : "memory");
+}
+
+__device__ __forceinline__ Msg msg_get(const Msg *p) {
+    unsigned long long lo, hi;
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(p)
+                 : "memory");
+    return {(uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32)};
+}
+
+// A poll is an L2 round trip (0.6 to 1 us), so the wait below is bounded to about two seconds.
+constexpr int MSG_POLLS = 1 << 21;
+
+// m = *p, read again until it carries `tag`: false once MSG_POLLS reads have not (recorded in st) or another block
+// has recorded that.
+__device__ __forceinline__ bool msg_wait(const Msg *p, uint32_t tag, Msg &m, DevStatus *st) {
+    for (int polls = 0; m.tag != tag; ++polls) {
+        if ((polls & 255) == 255 && *((volatile int *)&st->timeout)) return false;
+        if (polls >= MSG_POLLS) {
+            atomicExch(&st->timeout, 1);
+            atomicExch(&st->abort, 1);
+            return false;
+        }
+        m = msg_get(p);
+    }
+    return true;
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -203,6 +250,29 @@ __device__ __forceinline__ df32 df_add(df32 a, df32 b) {
 }
 
 __device__ __forceinline__ df32 df_add_f(df32 a, float b) { return df_add(a, df32{b, 0.f}); }
+
+// the product of two pairs (the low parts' product dropped: below the pair's precision), normalised
+__device__ __forceinline__ df32 df_mul(df32 a, df32 b) {
+    const float p = a.hi * b.hi;
+    float e = fmaf(a.hi, b.hi, -p);
+    e = fmaf(a.hi, b.lo, e);
+    e = fmaf(a.lo, b.hi, e);
+    const float hi = p + e;
+    return {hi, e - (hi - p)};
+}
+
+__device__ __forceinline__ df32 df_of(double v) {
+    const float hi = (float)v;
+    return {hi, (float)(v - (double)hi)};
+}
+
+__device__ __forceinline__ double df_double(df32 v) { return (double)v.hi + (double)v.lo; }
+
+__device__ __forceinline__ bool df_less(df32 a, df32 b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); }
+
+__device__ __forceinline__ df32 df_shfl_xor(df32 v, int o) {
+    return {__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
+}
 
 __device__ __forceinline__ df32 warp_sum_df(df32 v) {
 #pragma unroll

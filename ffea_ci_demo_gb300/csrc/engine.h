@@ -27,8 +27,6 @@ struct Launch {
     // mixed path: the most rows per block cg_mixed_own_kernel can keep in shared memory on `device`
     // (0: not available); a.npb > 0 selects that kernel in cg()
     static int cg_own_max_rows(int device);
-    // the same for cg_mixed_sr_kernel (a.sr selects it) with a Chebyshev preconditioner of degree poly; 0 for FP64
-    static int cg_sr_max_rows(int device, int poly);
     // the dynamic shared memory one cg_mixed_sr_kernel block may take on `device` (0 for FP64)
     static int cg_sr_smem_limit(int device);
     static cudaError_t euler(const EulerArgs<R> &a, cudaStream_t s);

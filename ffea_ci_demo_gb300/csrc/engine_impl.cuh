@@ -2,6 +2,7 @@
 // translation unit per arithmetic type (engine_fp64.cu, engine_mixed.cu).
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
 #include "engine.h"
@@ -125,26 +126,21 @@ int Launch<R>::cg_own_max_rows(int device) {
 }
 
 template <class R>
-int Launch<R>::cg_sr_max_rows(int device, int poly) {
-    if constexpr (std::is_same<R, float>::value)
-        return own_max_rows(cg_mixed_sr_kernel<R>, device, (int)sr_smem_bytes(1, poly));
-    else
-        return (void)device, (void)poly, 0;
-}
-
-template <class R>
 int Launch<R>::cg_sr_smem_limit(int device) {
     if constexpr (std::is_same<R, float>::value) {
-        int optin = 0;
-        cudaFuncAttributes fa{};
-        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess ||
-            cudaFuncGetAttributes(&fa, cg_mixed_sr_kernel<R>) != cudaSuccess)
-            return 0;
-        const int dyn = optin - (int)fa.sharedSizeBytes;
-        if (dyn <= 0 ||
-            cudaFuncSetAttribute(cg_mixed_sr_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
-            return 0;
-        return dyn;
+        int optin = 0, limit = 0;
+        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return 0;
+        const void *fns[2] = {(const void *)cg_mixed_sr_kernel<R, SR_REG_THREADS, SR_REG_BLOCKS>,
+                              (const void *)cg_mixed_sr_kernel<R, CG_THREADS, 0>};
+        for (int i = 0; i < 2; ++i) {
+            cudaFuncAttributes fa{};
+            if (cudaFuncGetAttributes(&fa, fns[i]) != cudaSuccess) return 0;
+            const int dyn = optin - (int)fa.sharedSizeBytes;
+            if (dyn <= 0 || cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
+                return 0;
+            limit = i == 0 ? dyn : std::min(limit, dyn);
+        }
+        return limit;
     } else {
         return (void)device, 0;
     }
@@ -159,8 +155,9 @@ cudaError_t Launch<R>::cg(const CgArgs<R> &a, int grid, int threads, cudaStream_
     if constexpr (std::is_same<R, float>::value) {
         fn = (const void *)cg_mixed_kernel<R>;
         if (a.npb > 0 && a.sr) {
-            fn = (const void *)cg_mixed_sr_kernel<R>;
-            smem = sr_smem_bytes(a.npb, a.poly) +
+            fn = a.reg ? (const void *)cg_mixed_sr_kernel<R, SR_REG_THREADS, SR_REG_BLOCKS>
+                       : (const void *)cg_mixed_sr_kernel<R, CG_THREADS, 0>;
+            smem = sr_smem_bytes(a.npb, a.nhalo, a.poly) +
                    (a.kc > 0 ? sr_cache_bytes(a.kc, sr_cache_stride(a.npb, a.tpn)) : 0);
         } else if (a.npb > 0) {
             fn = (const void *)cg_mixed_own_kernel<R>;

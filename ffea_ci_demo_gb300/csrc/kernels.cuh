@@ -759,6 +759,15 @@ struct CgArgs {
     double *cheb;
     float cheb_cost;
     int kc;               // cg_mixed_sr_kernel: 3x3 blocks per owned row kept in shared memory (0: none)
+    // owned-rows kernels that stage the vector their SpMV reads: the rows of other blocks that block b's rows
+    // reach (halo_list[halo_ptr[b] .. halo_ptr[b + 1])), every matrix slot's column as an index into the block's
+    // staged vector (own rows at 0 .. npb - 1, its halo from npb on), the rows' messages (two buffers of N) and
+    // the blocks' partial sums as messages (two buffers, rows of `stride`)
+    const int *halo_ptr, *halo_list;
+    const unsigned short *lcol;
+    Msg *msg, *rmsg;
+    int nhalo;            // the largest halo of any block
+    int reg;              // cg_mixed_sr_kernel: the form with the first blocks of each lane in registers
 };
 
 // p at node b for this iteration: p_new = beta p_old + D^{-1} r (vec3_scale_and_add with the
@@ -879,28 +888,36 @@ constexpr int CG_MAX_THREADS = 1024;
 
 constexpr int CG_PHASES = 10;  // the phase timers' slots (FFEA_GPU_CG_PHASES of the C ABI)
 
-// Phase timers of block 0, thread 0: the time since the previous mark is added to a shared-memory slot k during
-// the solve (a read-modify-write of phase_ns in global memory at every mark would hold block 0 for an L2 round
-// trip each time) and the slots are added to phase_ns when the solve ends.
+// Phase timers of one block (the middle one: the first and last own the mesh's corners), thread 0: the SM clock since
+// the previous mark is added to a shared-memory slot k during the solve, and the slots, as nanoseconds by the solve's
+// own ratio of global timer to SM clock, are added to phase_ns when it ends. (A mark on the global timer costs
+// 0.12 us, 2.3 us per iteration of the 6^3-cell solve; one on the clock register hides behind the barriers.)
+#define FFEA_TIMED_BLOCK (blockIdx.x == gridDim.x / 2 && threadIdx.x == 0)
 #define FFEA_PHASES_BEGIN(t_prev)                                                  \
-    __shared__ unsigned long long s_phase_[CG_PHASES];                    \
-    unsigned long long t_prev = 0ull;                                              \
-    if (blockIdx.x == 0 && threadIdx.x == 0) {                                     \
-        for (int k_ = 0; k_ < CG_PHASES; ++k_) s_phase_[k_] = 0ull;       \
-        t_prev = globaltimer_ns();                                                 \
+    __shared__ long long s_phase_[CG_PHASES];                                      \
+    __shared__ unsigned long long s_gt0_;                                          \
+    __shared__ long long s_ck0_, t_prev; /* in shared memory: no registers */     \
+    if (FFEA_TIMED_BLOCK) {                                                        \
+        for (int k_ = 0; k_ < CG_PHASES; ++k_) s_phase_[k_] = 0ll;                 \
+        s_gt0_ = globaltimer_ns();                                                 \
+        t_prev = s_ck0_ = clock64();                                               \
     }
 #define FFEA_MARK(g, t_prev, k)                                                   \
     do {                                                                          \
-        if (blockIdx.x == 0 && threadIdx.x == 0) {                                \
-            const unsigned long long t_now_ = globaltimer_ns();                   \
+        if (FFEA_TIMED_BLOCK) {                                                   \
+            const long long t_now_ = clock64();                                   \
             s_phase_[k] += t_now_ - (t_prev);                                     \
             (t_prev) = t_now_;                                                    \
         }                                                                         \
     } while (0)
 #define FFEA_PHASES_END(g)                                                        \
     do {                                                                          \
-        if (blockIdx.x == 0 && threadIdx.x == 0)                                  \
-            for (int k_ = 0; k_ < CG_PHASES; ++k_) (g).phase_ns[k_] += s_phase_[k_]; \
+        if (FFEA_TIMED_BLOCK) {                                                   \
+            const double c_ = (double)max(clock64() - s_ck0_, 1ll);               \
+            const double n_ = (double)(globaltimer_ns() - s_gt0_);                \
+            for (int k_ = 0; k_ < CG_PHASES; ++k_)                                \
+                (g).phase_ns[k_] += (unsigned long long)((double)s_phase_[k_] * (n_ / c_)); \
+        }                                                                         \
     } while (0)
 
 // FP64 CG: three phases (SpMV, residual update, direction update) with a grid barrier after each;

@@ -839,20 +839,135 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_own_kernel(const __grid_cons
     }
 }
 
-// The first kc 3x3 blocks of each owned row of cg_mixed_sr_kernel, kept in shared memory for the whole solve:
-// values at cv[(9 k + c) S + l], block columns at cc[k S + l] (l the row's index in the block). S is the
-// block's row count padded to S = 32 / tpn (mod 32), so that the tpn lanes of a row, which read blocks k, k + 1,
-// ..., k + tpn - 1 of the rows of one warp, fall on distinct banks.
+// The vector a staged SpMV reads, in shared memory: this block's rows at v[0, npb), then its halo. A thread's own
+// published row waits in its registers until the block's reads of the previous vector have ended.
+struct Staged {
+    float4 *v;
+    int npb;
+    int row;  // the row this thread has published but not yet staged (-1: none), and its value
+    float4 own;
+};
+
+// The halo of this block for publication `tag`: every thread reads its messages (two of them in flight) and puts
+// them, and its own published row, into the staged vector. The first barrier ends the reads of the previous vector.
+template <class A>
+__device__ __forceinline__ bool halo_exchange(const A &g, Staged &z, const int (&hx)[2], int h0, int nh,
+                                              unsigned int tag, DevStatus *st) {
+    __syncthreads();
+    if (z.row >= 0) z.v[z.row] = z.own;
+    z.row = -1;
+    int bad = 0;
+    if (nh > 0) {
+        const Msg *m = g.msg + (size_t)(tag & 1u) * g.N;
+        float4 *zh = z.v + z.npb;
+        for (int h = threadIdx.x, t = 0; h < nh; h += 2 * (int)blockDim.x, ++t) {
+            const int h2 = h + (int)blockDim.x;
+            const bool two = h2 < nh;
+            const Msg *pa = m + (t == 0 ? hx[0] : __ldg(g.halo_list + h0 + h));
+            const Msg *pb = two ? m + (t == 0 ? hx[1] : __ldg(g.halo_list + h0 + h2)) : pa;
+            Msg a = msg_get(pa), b = a;
+            if (two) b = msg_get(pb);
+            if (!msg_wait(pa, tag, a, st)) { bad = 1; break; }
+            zh[h] = make_float4(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z), 0.f);
+            if (two) {
+                if (!msg_wait(pb, tag, b, st)) { bad = 1; break; }
+                zh[h2] = make_float4(__uint_as_float(b.x), __uint_as_float(b.y), __uint_as_float(b.z), 0.f);
+            }
+        }
+    }
+    return __syncthreads_or(bad) == 0;
+}
+
+// The warp's sums of NV values (NV <= 16) over its lanes, one value left to each pair of lanes: each round halves
+// the lanes a value is spread over and the values a lane holds, so 11 values take 13 shuffles instead of 55. Returns
+// the sum and its index (-1 in lanes that hold none).
+template <int NV>
+__device__ __forceinline__ float warp_sum_spread(const float (&v)[NV], int &index) {
+    constexpr int n1 = (NV + 1) / 2, n2 = (n1 + 1) / 2, n3 = (n2 + 1) / 2, n4 = (n3 + 1) / 2;
+    static_assert(n4 == 1, "up to 16 values");
+    const int lane = threadIdx.x & 31;
+    float a[n1];
+    int at = 0, valid = NV;
+    auto round = [&](auto &dst, const auto &src, int n, int h, int o) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const float lo = src[i], hi = i + h < n ? src[i + h < n ? i + h : 0] : 0.f;
+            dst[i] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, o);
+        }
+        at += up ? h : 0;
+        valid = up ? valid - h : min(valid, h);  // how many of this lane's values are real
+    };
+    round(a, v, NV, n1, 16);
+    float b[n2], c[n3], d[1];
+    round(b, a, n1, n2, 8);
+    round(c, b, n2, n3, 4);
+    round(d, c, n3, n4, 2);
+    const float t = d[0] + __shfl_xor_sync(0xffffffffu, d[0], 1);
+    index = (valid > 0 && (lane & 1) == 0) ? at : -1;
+    return t;
+}
+
+// The grid's sums of NV per-thread FP32 values, as double-float pairs in s_out for the whole block: FP32 within each
+// warp, double-float over the block's warps, published as one message per value, and every block adds the blocks'
+// messages in the same order. `tag` counts the launch's reductions from 1. The caller must pass a __syncthreads()
+// before smem (NV x 32 floats) is written again.
+template <int NV, class A>
+__device__ __forceinline__ bool grid_reduce_msg(const A &g, const float (&v)[NV], float *smem, unsigned int tag,
+                                                df32 *s_out, DevStatus *st) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, nb = gridDim.x;
+    int idx;
+    const float ws = warp_sum_spread<NV>(v, idx);
+    if (idx >= 0) smem[idx * 32 + wid] = ws;
+    __syncthreads();
+    int bad = 0;
+    for (int i = wid; i < NV; i += nw) {
+        df32 t = {lane < nw ? smem[i * 32 + lane] : 0.f, 0.f};
+        t = warp_sum_df(t);
+        if (nb > 1) {
+            Msg *row = g.rmsg + ((size_t)(tag & 1u) * NV + i) * g.stride;
+            if (lane == 0) msg_put(row + blockIdx.x, __float_as_uint(t.hi), __float_as_uint(t.lo), 0u, tag);
+            t = df32{0.f, 0.f};
+            for (int b0 = 0; b0 < nb; b0 += 160) {
+                Msg m[5];
+#pragma unroll
+                for (int j = 0; j < 5; ++j) {
+                    const int b = b0 + lane + 32 * j;
+                    if (b < nb) m[j] = msg_get(row + b);
+                }
+#pragma unroll
+                for (int j = 0; j < 5; ++j) {
+                    const int b = b0 + lane + 32 * j;
+                    if (b < nb && !bad) {
+                        if (msg_wait(row + b, tag, m[j], st))
+                            t = df_add(t, df32{__uint_as_float(m[j].x), __uint_as_float(m[j].y)});
+                        else
+                            bad = 1;
+                    }
+                }
+            }
+            __syncwarp();
+            t = warp_sum_df(t);
+        }
+        if (lane == 0) s_out[i] = t;
+    }
+    return __syncthreads_or(bad) == 0;
+}
+
+// 3x3 blocks of each owned row of cg_mixed_sr_kernel kept in shared memory for the whole solve, kc of them after
+// those in registers (RowRegs): values 0-3, 4-7 and 8 of block k of row l at a[k S + l], b[k S + l], c[k S + l], its
+// local column at col[k S + l]. S is the block's row count padded to S = 8 / tpn (mod 8), so that the quarter warps'
+// 16-byte reads (8 / tpn rows x the row's tpn lanes, on blocks k, k + 1, ...) fall on distinct banks.
 struct SrCache {
-    const float *cv;
-    const int *cc;
+    const float4 *a, *b;
+    const float *c;
+    const unsigned short *col;
     int kc, S;
 };
 
 __host__ __device__ inline int sr_cache_stride(int npb, int tpn) {
-    const int r = tpn > 1 ? 32 / tpn : 0;
     int S = npb;
-    while ((S & 31) != r) ++S;
+    while (tpn > 1 && (S & 7) != 8 / tpn) ++S;
     return S;
 }
 
@@ -861,33 +976,49 @@ __host__ __device__ inline int sr_cache_stride(int npb, int tpn) {
     w1 = fmaf(WV[3], ZV.x, w1); w1 = fmaf(WV[4], ZV.y, w1); w1 = fmaf(WV[5], ZV.z, w1);        \
     w2 = fmaf(WV[6], ZV.x, w2); w2 = fmaf(WV[7], ZV.y, w2); w2 = fmaf(WV[8], ZV.z, w2)
 
-// Row a of w = V z for cg_mixed_sr_kernel: the preconditioned residual of neighbour b read as one float4.
-// Each lane takes blocks k = sub, sub + tpn, ... in order: first those held in shared memory (k < kc), then
-// the rest from the matrix in global memory, two per trip; the products are summed in block order either way,
-// so the row does not depend on kc.
-template <class A>
-__device__ __forceinline__ void spmv_row_w(const A &g, const SrCache &c, const float4 *z4, int a, int l, int sub,
-                                           bool valid, float &w0, float &w1, float &w2) {
+// The first RB 3x3 blocks of each lane of cg_mixed_sr_kernel (blocks sub, sub + tpn, ... of its row), kept in
+// registers for the whole solve, with their local columns two to a word. RB = 0: none.
+template <int RB>
+struct RowRegs {
+    float v[RB > 0 ? RB : 1][9];
+    unsigned int c[RB > 0 ? (RB + 1) / 2 : 1];
+};
+
+// Row l (of its block; SELL base and length given) of w = V z for cg_mixed_sr_kernel, z staged in shared memory.
+// Each lane takes blocks k = sub, sub + tpn, ... in order: first those in its
+// registers, then those held in shared memory (RB tpn <= k < RB tpn + kc), then the rest from the matrix in global
+// memory (two per trip where registers allow); the products are summed in block order either way, so the row does not depend on where its
+// blocks are.
+template <int RB, class A>
+__device__ __forceinline__ void spmv_row_w(const A &g, const SrCache &c, const RowRegs<RB> &rr, const float4 *zs,
+                                           int base, int len, int lane, int l, int sub, float &w0, float &w1,
+                                           float &w2) {
     w0 = 0.f; w1 = 0.f; w2 = 0.f;
     const int tpn = g.tpn;
-    if (valid) {
-        const int s = a >> 5, lane = a & 31;
-        const int base = __ldg(g.slice_ptr + s);
-        const int len = __ldg(g.rowlen + a);
-        const int kcl = min(c.kc, len);
+    if (len > 0) {
         int k = sub;
+        if constexpr (RB > 0) {
+#pragma unroll
+            for (int j = 0; j < RB; ++j, k += tpn) {
+                if (k < len) {
+                    const float4 z = zs[(j & 1) ? rr.c[j >> 1] >> 16 : rr.c[j >> 1] & 0xffffu];
+                    FFEA_W_FMA(rr.v[j], z);
+                }
+            }
+        }
+        const int k0 = RB * tpn, kcl = min(k0 + c.kc, len);
 #pragma unroll 1
         for (; k < kcl; k += tpn) {
-            float wk[9];
-#pragma unroll
-            for (int i = 0; i < 9; ++i) wk[i] = c.cv[(9 * k + i) * c.S + l];
-            const float4 z = z4[c.cc[k * c.S + l]];
+            const int at = (k - k0) * c.S + l;
+            const float4 va = c.a[at], vb = c.b[at];
+            const float wk[9] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w, c.c[at]};
+            const float4 z = zs[c.col[at]];
             FFEA_W_FMA(wk, z);
         }
         const float *v = g.val + 9 * (size_t)base + lane;
 #pragma unroll 1
-        for (; k + tpn < len; k += 2 * tpn) {
-            const int ba = __ldg(g.bcol + base + 32 * k + lane), bb = __ldg(g.bcol + base + 32 * (k + tpn) + lane);
+        for (; RB == 0 && k + tpn < len; k += 2 * tpn) {
+            const int ba = __ldg(g.lcol + base + 32 * k + lane), bb = __ldg(g.lcol + base + 32 * (k + tpn) + lane);
             const float *va = v + (size_t)32 * 9 * k, *vb = v + (size_t)32 * 9 * (k + tpn);
             float wa[9], wb[9];
 #pragma unroll
@@ -895,17 +1026,18 @@ __device__ __forceinline__ void spmv_row_w(const A &g, const SrCache &c, const f
                 wa[i] = __ldg(va + 32 * i);
                 wb[i] = __ldg(vb + 32 * i);
             }
-            const float4 za = z4[ba], zb = z4[bb];
+            const float4 za = zs[ba], zb = zs[bb];
             FFEA_W_FMA(wa, za);
             FFEA_W_FMA(wb, zb);
         }
-        if (k < len) {
-            const int b = __ldg(g.bcol + base + 32 * k + lane);
+#pragma unroll 1
+        for (; k < len; k += tpn) {
+            const int b = __ldg(g.lcol + base + 32 * k + lane);
             const float *vk = v + (size_t)32 * 9 * k;
             float wk[9];
 #pragma unroll
             for (int i = 0; i < 9; ++i) wk[i] = __ldg(vk + 32 * i);
-            const float4 z = z4[b];
+            const float4 z = zs[b];
             FFEA_W_FMA(wk, z);
         }
     }
@@ -917,15 +1049,23 @@ __device__ __forceinline__ void spmv_row_w(const A &g, const SrCache &c, const f
 }
 #undef FFEA_W_FMA
 
-// Bytes of dynamic shared memory cg_mixed_sr_kernel needs for npb owned rows: x, r, p, q, w, D^{-1}, D, d, and
-// with a polynomial preconditioner u (the preconditioned residual) and the Chebyshev correction.
+// cg_mixed_sr_kernel's two forms: up to SR_REG_THREADS lanes a block with SR_REG_BLOCKS 3x3 blocks of each lane in
+// registers, or 1024 threads without
+constexpr int SR_REG_THREADS = 512;
+constexpr int SR_REG_BLOCKS = 6;
+constexpr int SR_REG_ROWS = 128;  // rows a block is given while the mesh leaves SMs free
+
+// Bytes of dynamic shared memory cg_mixed_sr_kernel needs for npb owned rows and a halo of nhalo: the staged vector,
+// x, r, p, q, w, D^{-1}, D, d, and with a polynomial preconditioner u (the preconditioned
+// residual) and the Chebyshev correction.
 constexpr int SR_FIELDS = 24;
 constexpr int SR_FIELDS_POLY = 30;
-__host__ __device__ constexpr size_t sr_smem_bytes(int npb, int poly) {
-    return (size_t)(poly > 0 ? SR_FIELDS_POLY : SR_FIELDS) * npb * sizeof(float);
+__host__ __device__ constexpr size_t sr_smem_bytes(int npb, int nhalo, int poly) {
+    return (size_t)(poly > 0 ? SR_FIELDS_POLY : SR_FIELDS) * npb * sizeof(float) +
+           ((size_t)npb + nhalo) * sizeof(float4);
 }
-// ... plus the matrix cache of kc blocks per row at stride S: nine values and a column each
-constexpr int SR_CACHE_BYTES_PER_BLOCK = 10 * 4;
+// ... plus the matrix cache of kc blocks per row at stride S: nine values and a local column each
+constexpr int SR_CACHE_BYTES_PER_BLOCK = 9 * 4 + 2;
 __host__ __device__ constexpr size_t sr_cache_bytes(int kc, int S) {
     return (size_t)SR_CACHE_BYTES_PER_BLOCK * kc * S;
 }
@@ -978,10 +1118,16 @@ static __device__ __noinline__ double lanczos_lambda_max(const double *al, const
 // SpMV. One sweep computes w and all the dot products the step needs (r.z, r.r, z.w, z.q_old, p_old.w and the
 // rigid-mode moments of D z); p.q is then formed from them in FP64:
 //     p.q = z.w~ + beta (z.q_old + p_old.w~) + beta^2 p_old.q_old,    w~ = w + D Z A6 Z^T D z.
-// Per iteration: one grid barrier with a reduction, and one without (the new z must be visible before the
-// SpMV). Rows are owned as in cg_mixed_own_kernel. With M = D (Jacobi) the iterates are, in exact arithmetic,
-// those of the other mixed CG kernels; in FP32 they agree to rounding and converge in the same number of
-// iterations.
+// Rows are owned as in cg_mixed_own_kernel. With M = D (Jacobi) the iterates are, in exact arithmetic, those of the
+// other mixed CG kernels; in FP32 they agree to rounding and converge in the same number of iterations.
+// What bounds it is latency: a matrix pass waits for its neighbours' rows and a grid-wide sum for every block, each an
+// L2 round trip or two, around little arithmetic. So the exchange and the sums travel as tagged messages (Msg: one
+// round trip, no fence, no counter), the vector a pass reads is staged in shared memory (one gather of the halo
+// instead of an L2 read per block), and the matrix stays on chip: RB blocks of each lane in registers, the next kc of
+// each row in shared memory, what is left read from L2. 512 threads with 128 registers hold 6 blocks a lane without
+// spilling (8 spilled: the reloads missed the L1 that shared memory leaves, 3.51 against 3.09 ms per 40^3 step).
+// us per step, counters and L2 reads before -> now: 6^3 cells 590 -> 351, 20^3 1553 -> 879, 24^3 1859 -> 1117,
+// 40^3 3805 -> 3090, 45^3 (without register blocks) 4624 -> 4141.
 // Polynomial preconditioning (g.poly = d > 0, once lambda_max of D^{-1} V is known): M^{-1} = P_d(D^{-1} V) D^{-1},
 // with 1 - lambda P_d(lambda) the Chebyshev polynomial of degree d + 1 on [lambda_max / cheb_ratio(d),
 // lambda_max], scaled to 1 at 0. z is built by d steps of the Chebyshev iteration for V z = r from z = 0 (d SpMVs,
@@ -993,15 +1139,18 @@ static __device__ __noinline__ double lanczos_lambda_max(const double *al, const
 // cluster of the others (unscaled they sit at P_d(0), 15.7 for d = 4 on the 40^3 cube, which then needed 132
 // iterations a step instead of 110). The scale changes the shifted operator only on the rigid modes, where the
 // projected right-hand side has no component, so the solution is the same: the one with Z^T D x = 0.
-template <class R>
-__global__ void __launch_bounds__(1024, 1) cg_mixed_sr_kernel(const __grid_constant__ CgArgs<R> g) {
+template <class R, int NT, int RB>
+__global__ void __launch_bounds__(NT, 1) cg_mixed_sr_kernel(const __grid_constant__ CgArgs<R> g) {
     static_assert(sizeof(R) == sizeof(float), "the single-reduction CG is the mixed path's");
-    extern __shared__ float sn[];
+    extern __shared__ __align__(16) float4 sn_raw[];
     __shared__ float smemf[MIXED_SR_NP * 32];
     __shared__ double s_sc[MIXED_GATHER_NP];
     __shared__ double s_A6[36];
-    __shared__ double s_mp[6];        // moments of D p for the current direction
-    __shared__ double s_g, s_pq;      // r.z and p.q~ of the previous iteration
+    __shared__ df32 s_scf[MIXED_SR_NP];  // the iteration's sums
+    __shared__ df32 s_A6f[36];        // A6 times the shift's scale
+    __shared__ df32 s_mp[6];          // moments of D p for the current direction
+    __shared__ df32 s_pq;             // p.q~ of the previous iteration
+    __shared__ float s_g;             // and its r.z
     __shared__ float s_alpha, s_beta, s_tau[3], s_Om[3], s_dummy;
     __shared__ float s_c1[CHEB_MAX], s_c2[CHEB_MAX], s_ith;
     __shared__ double s_shift;        // scale of the rigid-mode shift: 1 / P_d(0) with the polynomial, else 1
@@ -1010,35 +1159,48 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_sr_kernel(const __grid_const
     if (st->abort) return;
     const bool defl = g.nmodes > 0;
     FFEA_PHASES_BEGIN(tm);
-    float2 *partials = reinterpret_cast<float2 *>(g.partials);
     const int npb = g.npb, a0 = blockIdx.x * npb;
     const int nloc = max(0, min(npb, g.N - a0));
+    // the staged vector first (16-byte aligned), then the row fields
+    Staged zs;
+    zs.v = reinterpret_cast<float4 *>(sn_raw);
+    zs.npb = npb;
+    zs.row = -1;
+    zs.own = make_float4(0.f, 0.f, 0.f, 0.f);
+    // then the matrix blocks in shared memory, then the row fields (see sr_smem_bytes, sr_cache_bytes)
+    SrCache mc;
+    mc.kc = g.kc;
+    mc.S = g.kc > 0 ? sr_cache_stride(npb, g.tpn) : 0;
+    const int ncache = mc.kc * mc.S;
+    float4 *const ca = zs.v + npb + g.nhalo, *const cb = ca + ncache;
+    float *const cc = reinterpret_cast<float *>(cb + ncache);
+    float *const sn = cc + ncache;
     float *sx = sn, *sr = sn + 3 * npb, *sp = sn + 6 * npb, *sq = sn + 9 * npb, *sw = sn + 12 * npb,
           *sdi = sn + 15 * npb, *sdg = sn + 18 * npb, *sd = sn + 21 * npb;
     // polynomial preconditioner: u = M^{-1} r and the Chebyshev correction dd (the residual of the Chebyshev
     // iteration shares w's storage: w is dead between the update and the next SpMV)
     float *su = sn + 24 * npb, *sdd = sn + 27 * npb;
-    // the matrix cache after the row fields, filled once for the solve
-    SrCache mc;
-    mc.kc = g.kc;
-    mc.S = g.kc > 0 ? sr_cache_stride(npb, g.tpn) : 0;
     {
-        float *cv = sn + (g.poly > 0 ? SR_FIELDS_POLY : SR_FIELDS) * npb;
-        int *cc = reinterpret_cast<int *>(cv + 9 * (size_t)mc.kc * mc.S);
+        // the matrix blocks in shared memory, filled once for the solve; their columns after the row fields
+        unsigned short *const col = reinterpret_cast<unsigned short *>(sn + (g.poly > 0 ? SR_FIELDS_POLY : SR_FIELDS) * npb);
+        const int k0 = RB * g.tpn;
         for (int t = threadIdx.x; t < mc.kc * nloc; t += blockDim.x) {
-            const int k = t / nloc, l = t - k * nloc, a = a0 + l;
+            const int kl = t / nloc, l = t - kl * nloc, a = a0 + l, k = k0 + kl;
             if (k >= __ldg(g.rowlen + a)) continue;
-            const int base = __ldg(g.slice_ptr + (a >> 5)), lane = a & 31;
+            const int base = __ldg(g.slice_ptr + (a >> 5)), lane = a & 31, at = kl * mc.S + l;
             const float *vk = g.val + 9 * (size_t)base + lane + (size_t)32 * 9 * k;
-#pragma unroll
-            for (int i = 0; i < 9; ++i) cv[(9 * k + i) * mc.S + l] = __ldg(vk + 32 * i);
-            cc[k * mc.S + l] = __ldg(g.bcol + base + 32 * k + lane);
+            ca[at] = make_float4(__ldg(vk), __ldg(vk + 32), __ldg(vk + 64), __ldg(vk + 96));
+            cb[at] = make_float4(__ldg(vk + 128), __ldg(vk + 160), __ldg(vk + 192), __ldg(vk + 224));
+            cc[at] = __ldg(vk + 256);
+            col[at] = __ldg(g.lcol + base + 32 * k + lane);
         }
-        mc.cv = cv;
-        mc.cc = cc;
+        mc.a = ca; mc.b = cb; mc.c = cc; mc.col = col;
     }
-    float4 *z4 = reinterpret_cast<float4 *>(g.q);
-    float4 *const y4a = reinterpret_cast<float4 *>(g.pbuf0), *const y4b = reinterpret_cast<float4 *>(g.pbuf1);
+    // this block's halo; a thread's first two entries in registers
+    const int h0 = __ldg(g.halo_ptr + blockIdx.x), nh = __ldg(g.halo_ptr + blockIdx.x + 1) - h0;
+    int hx[2];
+    hx[0] = (int)threadIdx.x < nh ? __ldg(g.halo_list + h0 + threadIdx.x) : 0;
+    hx[1] = (int)(threadIdx.x + blockDim.x) < nh ? __ldg(g.halo_list + h0 + threadIdx.x + blockDim.x) : 0;
     const int poly = g.poly;
     const double lmax = poly > 0 ? g.cheb[0] : 0.0;
     const bool cheb = lmax > 0.0;              // Chebyshev this solve
@@ -1065,24 +1227,55 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_sr_kernel(const __grid_const
     mixed_setup(g, s_sc, s_A6, s_tau, s_Om, &s_dummy, &s_conv);
     __syncthreads();
     const float ith = cheb ? s_ith : 0.f;
-    const int tpn = g.tpn, gpb = blockDim.x / tpn, grp = threadIdx.x / tpn, sub = threadIdx.x % tpn;
-    const int npass = (nloc + gpb - 1) / gpb;
-    unsigned int ep = 0;      // publication epochs of the neighbour exchanges
-    unsigned int bar_ep = 0;  // grid barriers passed
-    // Chebyshev steps 1..d after step 0 published y0 = D^{-1} r / theta (in y4a) and left D^{-1} r in sw:
-    // res -= D^{-1} V y, dd = c1 dd + c2 res, u += dd; each step publishes dd for the next one's SpMV (y4a and
-    // y4b alternate; a neighbour has read one before it publishes the next), the last one publishes u as z
+    // tpn lanes to a row, every row of the block at once (npb tpn <= NT)
+    const int tpn = g.tpn, l = threadIdx.x / tpn, sub = threadIdx.x % tpn;
+    const bool valid = l < nloc;
+    RowRegs<RB> rr;
+    int rbase = 0, rlen = 0;
+    if constexpr (RB > 0) {
+        if (valid) {
+            const int a = a0 + l, lane = a & 31;
+            rbase = __ldg(g.slice_ptr + (a >> 5));
+            rlen = __ldg(g.rowlen + a);
+#pragma unroll
+            for (int j = 0; j < RB; ++j) {
+                const int k = sub + j * tpn;
+                const bool in = k < rlen;
+#pragma unroll
+                for (int i = 0; i < 9; ++i)
+                    rr.v[j][i] = in ? __ldg(g.val + 9 * (size_t)rbase + lane + (size_t)32 * (9 * k + i)) : 0.f;
+                const unsigned int lc = in ? __ldg(g.lcol + rbase + 32 * k + lane) : 0u;
+                rr.c[j >> 1] = (j & 1) ? rr.c[j >> 1] | lc << 16 : lc;
+            }
+        }
+    }
+    // row l of w = V z over the staged vector
+    auto spmv = [&](float &w0, float &w1, float &w2) {
+        int base = rbase, len = rlen;
+        if constexpr (RB == 0) {
+            base = valid ? __ldg(g.slice_ptr + ((a0 + l) >> 5)) : 0;
+            len = valid ? __ldg(g.rowlen + a0 + l) : 0;
+        }
+        spmv_row_w<RB>(g, mc, rr, zs.v, base, len, (a0 + l) & 31, l, sub, w0, w1, w2);
+    };
+    unsigned int ep = 0;      // epochs of the published vectors
+    unsigned int red_ep = 0;  // epochs of the grid-wide sums
+    // row l of the vector published as epoch `tag`: to the block's staged vector and to the other blocks
+    auto publish = [&](unsigned int tag, int row, float v0, float v1, float v2) {
+        zs.row = row;
+        zs.own = make_float4(v0, v1, v2, 0.f);
+        msg_put(g.msg + (size_t)(tag & 1u) * g.N + a0 + row, __float_as_uint(v0), __float_as_uint(v1), __float_as_uint(v2),
+                tag);
+    };
+    // Chebyshev steps 1..d after step 0 published y0 = D^{-1} r / theta and left D^{-1} r in sw:
+    // res -= D^{-1} V y, dd = c1 dd + c2 res, u += dd; each step publishes dd for the next one's SpMV, the last one
+    // publishes u as z
     auto cheb_steps = [&]() -> bool {
         for (int j = 1; j <= poly; ++j) {
-            const float4 *yin = (j & 1) ? y4a : y4b;
-            float4 *yout = j == poly ? z4 : ((j & 1) ? y4b : y4a);
             const float c1 = s_c1[j - 1], c2 = s_c2[j - 1];
-            for (int ps = 0; ps < npass; ++ps) {
-                const int l = ps * gpb + grp;
-                const bool valid = l < nloc;
-                float t[3];
-                spmv_row_w(g, mc, yin, a0 + l, l, sub, valid, t[0], t[1], t[2]);
-                if (!valid || sub != 0) continue;
+            float t[3];
+            spmv(t[0], t[1], t[2]);
+            if (valid && sub == 0) {
                 float o[3];
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
@@ -1094,9 +1287,12 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_sr_kernel(const __grid_const
                     su[c * npb + l] = u;
                     o[c] = j < poly ? dd : u;
                 }
-                yout[a0 + l] = make_float4(o[0], o[1], o[2], 0.f);
+                publish(ep + 1, l, o[0], o[1], o[2]);
             }
-            if (!neighbour_sync(g, ++ep, st)) return false;
+            ++ep;
+            FFEA_MARK(g, tm, 6);
+            if (!halo_exchange(g, zs, hx, h0, nh, ep, st)) return false;
+            FFEA_MARK(g, tm, 7);
         }
         return true;
     };
@@ -1131,15 +1327,16 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_sr_kernel(const __grid_const
                 su[c * npb + l] = y[c];
                 sdd[c * npb + l] = y[c];
             }
-            y4a[a] = make_float4(y[0], y[1], y[2], 0.f);
+            publish(1u, l, y[0], y[1], y[2]);
         } else {
-            z4[a] = make_float4(z0, z1, z2, 0.f);
+            publish(1u, l, z0, z1, z2);
         }
     }
-    if (threadIdx.x < 6) s_mp[threadIdx.x] = 0.0;
-    if (threadIdx.x == 0) { s_g = 0.0; s_pq = 0.0; s_stop = 0; }
-    // the SpMV reads z only at neighbouring blocks' rows: wait for those blocks, not the whole grid
-    bool ok = neighbour_sync(g, ++ep, st);
+    if (threadIdx.x < 6) s_mp[threadIdx.x] = df32{0.f, 0.f};
+    if (threadIdx.x < 36) s_A6f[threadIdx.x] = df_of(s_A6[threadIdx.x] * s_shift);
+    if (threadIdx.x == 0) { s_g = 0.f; s_pq = df32{0.f, 0.f}; s_stop = 0; }
+    const df32 tol = df_of(g.eps2 * f2);
+    bool ok = halo_exchange(g, zs, hx, h0, nh, ++ep, st);
     if (ok && cheb) ok = cheb_steps();
     FFEA_MARK(g, tm, 0);
     int k = 0;  // updates applied so far
@@ -1149,12 +1346,9 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_sr_kernel(const __grid_const
         float acc[MIXED_SR_NP];
 #pragma unroll
         for (int i = 0; i < MIXED_SR_NP; ++i) acc[i] = 0.f;
-        for (int ps = 0; ps < npass; ++ps) {
-            const int l = ps * gpb + grp;
-            const bool valid = l < nloc;
-            float w0, w1, w2;
-            spmv_row_w(g, mc, z4, a0 + l, l, sub, valid, w0, w1, w2);
-            if (!valid || sub != 0) continue;
+        float w0, w1, w2;
+        spmv(w0, w1, w2);
+        if (valid && sub == 0) {
             sw[l] = w0; sw[npb + l] = w1; sw[2 * npb + l] = w2;
             const float r0 = sr[l], r1 = sr[npb + l], r2 = sr[2 * npb + l];
             float z0, z1, z2;
@@ -1178,53 +1372,52 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_sr_kernel(const __grid_const
             }
         }
         FFEA_MARK(g, tm, 1);
-        block_reduce_store<MIXED_SR_NP>(acc, smemf, partials, g.stride, 0);
-        FFEA_MARK(g, tm, 2);
-        if (!(ok = grid_sync_ep(g.gb, st, g.limit_ns, bar_ep))) break;
+        if (!(ok = grid_reduce_msg<MIXED_SR_NP>(g, acc, smemf, ++red_ep, s_scf, st))) break;
         FFEA_MARK(g, tm, 3);
-        grid_sum_df8<MIXED_SR_NP>(partials, g.stride, gridDim.x, s_sc);
         if (threadIdx.x < 32) {
+            // The iteration's scalars, in double-float as the sums arrive: this chain is on every block's critical path
+            // and FP64 runs at 1/64 of the FP32 rate (4.0 us per iteration; see below for the pairs').
             const int ln = threadIdx.x;
             // c = s A6 m(z): the rigid-mode coefficients of s D Z A6 Z^T D z, over six lanes
-            double c = 0.0;
+            df32 c = {0.f, 0.f}, mz = c, mp = c;
             if (defl && ln < 6) {
+                c = df_mul(s_A6f[6 * ln], s_scf[5]);
 #pragma unroll
-                for (int qq = 0; qq < 6; ++qq) c += s_A6[6 * ln + qq] * s_sc[5 + qq];
-                c *= s_shift;
+                for (int qq = 1; qq < 6; ++qq) c = df_add(c, df_mul(s_A6f[6 * ln + qq], s_scf[5 + qq]));
+                mz = s_scf[5 + ln];
+                mp = s_mp[ln];
             }
-            double mzc = (ln < 6) ? s_sc[5 + ln] * c : 0.0;   // m(z).c
-            double mpc = (ln < 6) ? s_mp[ln] * c : 0.0;       // m(p_old).c
+            df32 mzc = df_mul(mz, c), mpc = df_mul(mp, c);  // m(z).c, m(p_old).c
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) {
-                mzc += __shfl_xor_sync(0xffffffffu, mzc, o);
-                mpc += __shfl_xor_sync(0xffffffffu, mpc, o);
+                mzc = df_add(mzc, df_shfl_xor(mzc, o));
+                mpc = df_add(mpc, df_shfl_xor(mpc, o));
             }
-            const double gam = s_sc[0], rr = s_sc[1];
+            const df32 gam = s_scf[0], rr2 = s_scf[1];
             // |r|^2/|f|^2 < epsilon2 after an update, as NoMassCGSolver::solve tests it (a zero force: x = 0 at once)
-            const bool conv = f2 == 0.0 || (k > 0 && (g.check_last || k < g.imax) && rr < g.eps2 * f2);
-            if (ln == 0 && blockIdx.x == 0 && k > 0 && k - 1 < g.hist_cap) g.history[k - 1] = (f2 == 0.0) ? 0.0 : rr / f2;
+            const bool conv = f2 == 0.0 || (k > 0 && (g.check_last || k < g.imax) && df_less(rr2, tol));
+            if (ln == 0 && blockIdx.x == 0 && k > 0 && k - 1 < g.hist_cap)
+                reinterpret_cast<float2 *>(g.history)[k - 1] = make_float2(rr2.hi, rr2.lo);
             const bool stop = conv || k >= g.imax;
-            // the step lengths in FP32 (as cg_mixed_kernel forms them): FP64 division is slow on this GPU
-            const float beta_f = (k == 0) ? 0.f : (float)gam / (float)s_g;
-            const double beta = beta_f;
-            const double zw = s_sc[2] + mzc, pw = s_sc[4] + mpc;
-            const double pq = zw + beta * (s_sc[3] + pw) + beta * beta * s_pq;
+            const float beta = (k == 0) ? 0.f : gam.hi / s_g;
+            const df32 zw = df_add(s_scf[2], mzc), pw = df_add(s_scf[4], mpc), b1 = {beta, 0.f};
+            const df32 pq = df_add(df_add(zw, df_mul(b1, df_add(s_scf[3], pw))), df_mul(df_mul(b1, b1), s_pq));
+            const float alpha = gam.hi / pq.hi;
             if (rec && ln == 0 && blockIdx.x == 0 && !stop && k < CHEB_REC) {
-                g.cheb[1 + k] = gam / pq;
+                g.cheb[1 + k] = df_double(gam) / df_double(pq);
                 g.cheb[1 + CHEB_REC + k] = beta;
             }
             __syncwarp();
             if (ln < 6) {
-                const float cf = (float)c;
-                if (ln < 3) s_tau[ln] = cf; else s_Om[ln - 3] = cf;
-                s_mp[ln] = s_sc[5 + ln] + beta * s_mp[ln];
+                if (ln < 3) s_tau[ln] = c.hi; else s_Om[ln - 3] = c.hi;
+                s_mp[ln] = df_add(mz, df_mul(b1, mp));
             }
             if (ln == 0) {
                 s_conv = conv;
                 s_stop = stop;
-                s_beta = beta_f;
-                s_alpha = (float)gam / (float)pq;
-                s_g = gam;
+                s_beta = beta;
+                s_alpha = alpha;
+                s_g = gam.hi;
                 s_pq = pq;
             }
         }
@@ -1236,7 +1429,6 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_sr_kernel(const __grid_const
         // p = z + beta p ; q = w~ + beta q ; x += alpha p ; r -= alpha q ; z = M^{-1} r published (Jacobi), or
         // the Chebyshev iteration's first step (polynomial)
         for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
-            const int a = a0 + l;
             float wv[3] = {sw[l], sw[npb + l], sw[2 * npb + l]};
             if (defl) {
                 const float dx = sd[l], dy = sd[npb + l], dz = sd[2 * npb + l];
@@ -1265,13 +1457,13 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_sr_kernel(const __grid_const
                     zn[c] = y;
                 }
             }
-            (cheb ? y4a : z4)[a] = make_float4(zn[0], zn[1], zn[2], 0.f);
+            publish(ep + 1, l, zn[0], zn[1], zn[2]);
         }
         FFEA_MARK(g, tm, 5);
-        if (!(ok = neighbour_sync(g, ++ep, st))) break;
+        ++ep;
+        if (!(ok = halo_exchange(g, zs, hx, h0, nh, ep, st))) break;
         FFEA_MARK(g, tm, 7);
         if (cheb && !(ok = cheb_steps())) break;
-        FFEA_MARK(g, tm, 6);
     }
     for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
         const int a = a0 + l;
@@ -1282,6 +1474,11 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_sr_kernel(const __grid_const
         }
     }
     FFEA_PHASES_END(g);
+    if (blockIdx.x == 0)  // the history's |r|^2, kept as pairs, become |r|^2 / |f|^2
+        for (int i = threadIdx.x; i < min(k, g.hist_cap); i += blockDim.x) {
+            const float2 h = reinterpret_cast<const float2 *>(g.history)[i];
+            g.history[i] = f2 == 0.0 ? 0.0 : df_double(df32{h.x, h.y}) / f2;
+        }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (!ok) {
             st->abort = 1;
