@@ -184,6 +184,7 @@ struct BlobImpl final : ffea_gpu_blob {
     int cg_grid = 0, gather_blocks = 0, partial_stride = 0, tpn = 4;
     int cg_npb = 0;  // rows per block of the owned-rows CG kernels (0: cg_kernel / cg_mixed_kernel)
     int cg_block = 1024;  // threads per CG block
+    int ss_grid = 0, ss_block = 0, ss_tpn = 1;  // FP64: the same for the allocation-free solve's cg_kernel
     bool cg_sr = false;   // the mixed CG_nomass solve uses cg_mixed_sr_kernel
     int cg_poly = 0;      // with a Chebyshev preconditioner of this degree (0: Jacobi)
     int cg_kc = 0;        // and this many 3x3 blocks of each owned row in shared memory
@@ -194,7 +195,8 @@ struct BlobImpl final : ffea_gpu_blob {
     int *halo_ptr = nullptr, *halo_list = nullptr;
     unsigned short *lcol = nullptr;
     int nhalo = 0;
-    bool cg_reg = false;  // the single-reduction CG keeps each lane's first matrix blocks in registers
+    int cg_unit = 0;      // FP64: components per unit of cg_own_unit_kernel (0: another kernel)
+    int cg_reg = 0;  // the single-reduction CG's form: matrix blocks of each lane in registers
     char *comm = nullptr;
     size_t comm_bytes = 0;
     Msg *msg = nullptr, *rmsg = nullptr;
@@ -381,6 +383,50 @@ struct BlobImpl final : ffea_gpu_blob {
         if (o.list.empty()) o.list.push_back(0);
     }
 
+    // The FP64 CG's launch: rows per block, units and lanes per unit of cg_own_unit_kernel, by the FP64 instructions on
+    // the fullest sub-partition of a block (see there); left alone (cg_unit = 0) when no form holds the blob's rows.
+    int pick_units(int maxg) {
+        const bool b3 = p.solver == FFEA_GPU_NOMASS_CG;
+        if (p.solver == FFEA_GPU_MASSLUMPED) return FFEA_GPU_OK;
+        const int N = h.N;
+        int maxlen = 1;
+        for (int a = 0; a < N; ++a) maxlen = std::max(maxlen, h.rowlen[a]);
+        // Rows a block is given while the mesh leaves SMs free: more blocks share the FP64 work but lengthen the sums. us per
+        // step at 8 / 16 / 32 / 64 rows: 343 nodes CG_nomass 772 / 689 / 785 / 844, 2197 nodes 1820 / 1726 / 1803 / 1934;
+        // a mass matrix has a third of the products, and 64 nodes are best in one block (CG 127 / 108 / 120 / 96).
+        const int want = !b3 && N <= 64 ? 64 : 16;
+        const int grid = std::max(1, std::min(maxg, (N + want - 1) / want)), npb = (N + grid - 1) / grid;
+        int best = 0, best_nc = 0, best_tpu = 0;
+        for (int nc : {1, 3})
+            for (int t = 1; t <= (nc == 1 ? 8 : 1); t *= 2) {
+                const int lanes = own_unit_count(npb, nc) * t;
+                if (lanes > OWN_UNIT_THREADS) continue;
+                const int warps = (lanes + 127) / 128;  // on the fullest sub-partition
+                int lg = 0;
+                while ((1 << lg) < t) ++lg;
+                const int c = warps * ((b3 ? 3 * nc : nc) * ((maxlen + t - 1) / t) + nc * (lg + 7));
+                if (!best || c < best) { best = c; best_nc = nc; best_tpu = t; }
+            }
+        if (!best) return FFEA_GPU_OK;
+        Halo hl;
+        build_halo(npb, grid, hl);
+        const int vals = b3 ? 9 : 1;
+        const size_t limit = (size_t)std::max(Launch<R>::cg_unit_smem_limit(device, best_nc, b3), 0);
+        const size_t need = own_unit_smem(npb, hl.largest, best_nc, vals, 0);
+        if (npb + hl.largest >= 65536 || need > limit) return FFEA_GPU_OK;
+        cg_unit = best_nc;
+        tpn = best_tpu;
+        cg_grid = grid;
+        cg_npb = npb;
+        cg_block = std::min(OWN_UNIT_THREADS, std::max(256, (own_unit_count(npb, best_nc) * tpn + 31) / 32 * 32));
+        nhalo = hl.largest;
+        cg_kc = best_nc == 3 ? (int)std::min<size_t>(maxlen, (limit - need) / ((size_t)npb * (vals * sizeof(double) + 2))) : 0;
+        CK(mem.upload(&halo_ptr, hl.ptr));
+        CK(mem.upload(&halo_list, hl.list));
+        CK(mem.upload(&lcol, hl.lcol));
+        return FFEA_GPU_OK;
+    }
+
     int init() override {
         CK(cudaGetDevice(&device));
         int major = 0, minor = 0;
@@ -504,7 +550,7 @@ struct BlobImpl final : ffea_gpu_blob {
         }
         // The mixed CG_nomass solve (cg_mixed_sr_kernel) spreads small meshes further: its blocks exchange rows and sums
         // as tagged messages, so a block more costs little, and up to SR_REG_ROWS rows its lanes hold the whole matrix
-        // in registers (four lanes of six blocks to a row). us per step at 64 / 128 / 192 / 256 / 320 rows a block:
+        // in registers (four lanes of four blocks to a row). us per step at 64 / 128 / 192 / 256 / 320 rows a block:
         // 10^3 cells 499 / 455 / 508 / 509 / 567, 20^3 976 / 879 / 930 / 968 / 1078, 24^3 - / 1117 / 1124 / 1166 / 1321.
         // Above SR_REG_THREADS rows a block (N > 73,000) the form without register blocks takes over.
         const bool sr_able = mixed && p.solver == FFEA_GPU_NOMASS_CG && 40.0 * (double)h.nslots <= L2_MATRIX_BYTES;
@@ -532,6 +578,7 @@ struct BlobImpl final : ffea_gpu_blob {
             return (rows + align - 1) / align * align;  // rows per block
         };
         int npb = pick_grid(sr_able);
+        ss_grid = cg_grid; ss_block = cg_block; ss_tpn = tpn;
         // The CG kernel follows from the blob's size alone (no other input selects it):
         //  - each block keeps a run of rows in shared memory when they fit (cg_own_kernel, cg_mixed_own_kernel);
         //    the run is a multiple of a warp's rows so that a warp's rows share a SELL slice; else the grid-strided
@@ -558,20 +605,24 @@ struct BlobImpl final : ffea_gpu_blob {
                 }
                 if (cg_sr) {
                     cg_npb = npb;
-                    cg_reg = cg_block == SR_REG_THREADS;
+                    cg_reg = cg_block != SR_REG_THREADS ? 0 : tpn >= 4 ? 4 : 6;
                     nhalo = hl.largest;
                     CK(mem.upload(&halo_ptr, hl.ptr));
                     CK(mem.upload(&halo_list, hl.list));
                     CK(mem.upload(&lcol, hl.lcol));
                 }
             }
-            if (!cg_sr) {
+            if (!mixed) {
+                const int unit_rc = pick_units(maxg);
+                if (unit_rc) return unit_rc;
+            }
+            if (!cg_sr && !cg_unit) {
                 if (sr_able) npb = pick_grid(false);
                 cg_npb = (maxrows > 0 && npb <= maxrows) ? npb : 0;
             }
             partial_stride = cg_grid;
             if (cg_sr) {
-                // the first blocks of each owned row kept on chip for the solve: SR_REG_BLOCKS of each lane in registers
+                // the first blocks of each owned row kept on chip for the solve: some of each lane in registers
                 // (cg_reg), then as many as the rest of the block's shared memory holds
                 // (ffea_gpu_params::cg_smem_blocks caps those: n > 0 at most n, -1 none; the results do not depend on it)
                 const long long avail = (long long)Launch<R>::cg_sr_smem_limit(device) -
@@ -579,7 +630,7 @@ struct BlobImpl final : ffea_gpu_blob {
                 const long long S = sr_cache_stride(cg_npb, tpn);
                 int maxlen = 0;
                 for (int a = 0; a < N; ++a) maxlen = std::max(maxlen, h.rowlen[a]);
-                maxlen = std::max(0, maxlen - (cg_reg ? SR_REG_BLOCKS * tpn : 0));
+                maxlen = std::max(0, maxlen - cg_reg * tpn);
                 cg_kc = avail <= 0 ? 0 : (int)std::min<long long>(maxlen, avail / (SR_CACHE_BYTES_PER_BLOCK * S));
                 if (p.cg_smem_blocks != 0) cg_kc = std::min(cg_kc, std::max(0, p.cg_smem_blocks));
             }
@@ -588,7 +639,7 @@ struct BlobImpl final : ffea_gpu_blob {
                 CK(cudaMemset(cheb, 0, CHEB_STATE * sizeof(double)));
             }
             // the FP64 owned-rows CG publishes its search direction the same way (CG_nomass's 3x3 pattern)
-            if (!mixed && cg_npb > 0 && p.solver == FFEA_GPU_NOMASS_CG) {
+            if (!mixed && !cg_unit && cg_npb > 0 && p.solver == FFEA_GPU_NOMASS_CG) {
                 // the blocks each block's SpMV reads z (p) from: owners of the columns of its rows. The pattern is
                 // symmetric (an element couples each pair of its unpinned nodes both ways; a pinned row keeps only
                 // its diagonal and no row has its column), so these are also the blocks that read from it, which
@@ -620,7 +671,8 @@ struct BlobImpl final : ffea_gpu_blob {
         hist_cap = std::min(std::max(p.max_iterations_cg, 1), 1 << 20);
         CK(mem.alloc(&history, (size_t)hist_cap));
         {
-            const size_t head = 256, rows = cg_sr ? 2 * (size_t)N : 0, red = cg_sr ? 2 * (size_t)MIXED_SR_NP * partial_stride : 0;
+            const size_t head = 256, rows = cg_sr ? 2 * (size_t)N : cg_unit ? 6 * (size_t)N : 0,
+                         red = (cg_sr ? 2 * (size_t)MIXED_SR_NP : cg_unit ? 4 : 0) * MSG_COPIES * partial_stride;
             comm_bytes = head + (rows + red) * sizeof(Msg);
             CK(mem.alloc(&comm, comm_bytes));
             phase_ns = reinterpret_cast<unsigned long long *>(comm);
@@ -668,7 +720,7 @@ struct BlobImpl final : ffea_gpu_blob {
         if (fused_prep()) CK(mem.alloc(&rng_bufs[1], 6));
         // a blob that the allocation-free solve accepts gets the static scratch placed now, and that solve's
         // kernels loaded (cg_kernel by the occupancy query above), so that its first solve allocates nothing
-        if (!mixed && p.solver != FFEA_GPU_MASSLUMPED && N <= SOLVE_STATIC_MAX_NODES && cg_grid <= SOLVE_MAX_BLOCKS) {
+        if (!mixed && p.solver != FFEA_GPU_MASSLUMPED && N <= SOLVE_STATIC_MAX_NODES && ss_grid <= SOLVE_MAX_BLOCKS) {
             double *ss = nullptr;
             const int src = solve_scratch(device, &ss);
             if (src) return src;
@@ -762,7 +814,8 @@ struct BlobImpl final : ffea_gpu_blob {
         ca.npb = cg_npb;
         ca.sr = cg_sr && nomass;
         ca.poly = ca.sr ? cg_poly : 0;
-        ca.kc = ca.sr ? cg_kc : 0;
+        ca.kc = ca.sr || cg_unit ? cg_kc : 0;
+        ca.unit = cg_unit;
         ca.cheb = cheb;
         // a Chebyshev step (SpMV + neighbour exchange) against a whole iteration (SpMV, exchange, grid-wide
         // reduction): about half while the FP32 matrix (40 B per 3x3 block) stays in L2, more once it streams
@@ -1154,7 +1207,7 @@ struct BlobImpl final : ffea_gpu_blob {
                 return FFEA_GPU_EINPUT;
             }
             const int N = h.N;
-            if (N > SOLVE_STATIC_MAX_NODES || cg_grid > SOLVE_MAX_BLOCKS) {
+            if (N > SOLVE_STATIC_MAX_NODES || ss_grid > SOLVE_MAX_BLOCKS) {
                 g_last_error = "ffea_gpu_blob_solve_static: " + std::to_string(N) +
                                " vertex nodes exceed the static scratch limit of " +
                                std::to_string(SOLVE_STATIC_MAX_NODES);
@@ -1202,8 +1255,8 @@ struct BlobImpl final : ffea_gpu_blob {
             ca.imax = p.max_iterations_cg;
             ca.eps2 = p.epsilon2;
             ca.limit_ns = 2000000000ull;
-            ca.history = nullptr; ca.hist_cap = 0; ca.tpn = tpn; ca.phase_ns = sphase;
-            CK(Launch<R>::cg(ca, cg_grid, cg_block, stream));
+            ca.history = nullptr; ca.hist_cap = 0; ca.tpn = ss_tpn; ca.phase_ns = sphase;
+            CK(Launch<R>::cg(ca, ss_grid, ss_block, stream));
             DevStatus ds{};
             CK(cudaMemcpy2DAsync(staging, 3 * sizeof(double), s + SS_X, 4 * sizeof(double), 3 * sizeof(double), N,
                                  cudaMemcpyDeviceToHost, stream));

@@ -170,20 +170,72 @@ __device__ __forceinline__ Msg msg_get(const Msg *p) {
 // A poll is an L2 round trip (0.6 to 1 us), so the wait below is bounded to about two seconds.
 constexpr int MSG_POLLS = 1 << 21;
 
-// m = *p, read again until it carries `tag`: false once MSG_POLLS reads have not (recorded in st) or another block
-// has recorded that.
-__device__ __forceinline__ bool msg_wait(const Msg *p, uint32_t tag, Msg &m, DevStatus *st) {
-    for (int polls = 0; m.tag != tag; ++polls) {
+// m[j] = *p[j] for the K messages with use[j], read again until every one carries `tag`: those still missing are read
+// together, so the wait ends one round trip after the last of them arrives (waited for one after another, each costs
+// its own: 4.1 against 2.6 us per grid-wide sum of 137 blocks). False once MSG_POLLS rounds have passed (recorded in
+// st) or another block has recorded that.
+template <int K>
+__device__ __forceinline__ bool msg_wait_all(const Msg *const (&p)[K], const bool (&use)[K], uint32_t tag, Msg (&m)[K],
+                                             DevStatus *st) {
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+        if (use[j]) m[j] = msg_get(p[j]);
+    for (int polls = 0;; ++polls) {
+        bool missing = false;
+#pragma unroll
+        for (int j = 0; j < K; ++j) missing = missing || (use[j] && m[j].tag != tag);
+        if (!missing) return true;
         if ((polls & 255) == 255 && *((volatile int *)&st->timeout)) return false;
         if (polls >= MSG_POLLS) {
             atomicExch(&st->timeout, 1);
             atomicExch(&st->abort, 1);
             return false;
         }
-        m = msg_get(p);
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+            if (use[j] && m[j].tag != tag) m[j] = msg_get(p[j]);
+    }
+}
+
+// A grid-wide sum's messages are polled by every block: they are published in MSG_COPIES copies on lines of their own
+// (one per lane of the publishing warp), block b reading copy b mod MSG_COPIES, or the polls of all 152 SMs on the
+// same twenty lines hold up the messages themselves.
+constexpr int MSG_COPIES = 16;
+
+// add(message of block b) for every block b = lane, lane + 32, ... < nb, in that order, once each carries `tag`: one
+// message a lane for up to 32 blocks, else K at a time. False on a timeout.
+template <int K, class F>
+__device__ __forceinline__ bool msg_collect(const Msg *row, int nb, uint32_t tag, DevStatus *st, F add) {
+    const int lane = threadIdx.x & 31;
+    if (nb <= 32) {
+        const Msg *const at[1] = {row + lane};
+        const bool use[1] = {lane < nb};
+        Msg m[1];
+        if (!msg_wait_all<1>(at, use, tag, m, st)) return false;
+        if (use[0]) add(m[0]);
+        return true;
+    }
+    for (int b0 = lane; b0 - lane < nb; b0 += 32 * K) {
+        const Msg *at[K];
+        bool use[K];
+        Msg m[K];
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            at[j] = row + b0 + 32 * j;
+            use[j] = b0 + 32 * j < nb;
+        }
+        if (!msg_wait_all<K>(at, use, tag, m, st)) return false;
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+            if (use[j]) add(m[j]);
     }
     return true;
 }
+
+// This thread's warp in its block, as a value that the compiler knows to be the same in all 32 lanes: a branch on it
+// keeps the warp together, and a shuffle inside it is one instruction (behind a branch on threadIdx.x each was a call:
+// 1.5 us for twelve).
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll

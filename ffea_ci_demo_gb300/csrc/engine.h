@@ -27,6 +27,9 @@ struct Launch {
     // mixed path: the most rows per block cg_mixed_own_kernel can keep in shared memory on `device`
     // (0: not available); a.npb > 0 selects that kernel in cg()
     static int cg_own_max_rows(int device);
+    // the dynamic shared memory a block of cg_own_unit_kernel's form may take on `device` (0 for the mixed path);
+    // a.unit selects it in cg()
+    static int cg_unit_smem_limit(int device, int nc, int block3);
     // the dynamic shared memory one cg_mixed_sr_kernel block may take on `device` (0 for FP64)
     static int cg_sr_smem_limit(int device);
     static cudaError_t euler(const EulerArgs<R> &a, cudaStream_t s);

@@ -125,14 +125,40 @@ int Launch<R>::cg_own_max_rows(int device) {
         return own_max_rows(cg_own_kernel<R>, device, (int)own_smem_bytes_d(1));
 }
 
+// cg_own_unit_kernel's form for units of nc components (1 or 3) and 3x3 blocks or scalar entries
+template <class R>
+static const void *own_unit_kernel(int nc, int block3) {
+    if (nc == 3)
+        return block3 ? (const void *)cg_own_unit_kernel<R, 3, true> : (const void *)cg_own_unit_kernel<R, 3, false>;
+    return block3 ? (const void *)cg_own_unit_kernel<R, 1, true> : (const void *)cg_own_unit_kernel<R, 1, false>;
+}
+
+template <class R>
+int Launch<R>::cg_unit_smem_limit(int device, int nc, int block3) {
+    if constexpr (std::is_same<R, float>::value) {
+        return (void)device, (void)nc, (void)block3, 0;
+    } else {
+        int optin = 0;
+        cudaFuncAttributes fa{};
+        const void *fn = own_unit_kernel<R>(nc, block3);
+        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess ||
+            cudaFuncGetAttributes(&fa, fn) != cudaSuccess)
+            return 0;
+        const int dyn = optin - (int)fa.sharedSizeBytes;
+        if (dyn <= 0 || cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
+            return 0;
+        return dyn;
+    }
+}
+
 template <class R>
 int Launch<R>::cg_sr_smem_limit(int device) {
     if constexpr (std::is_same<R, float>::value) {
         int optin = 0, limit = 0;
         if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return 0;
-        const void *fns[2] = {(const void *)cg_mixed_sr_kernel<R, SR_REG_THREADS, SR_REG_BLOCKS>,
-                              (const void *)cg_mixed_sr_kernel<R, CG_THREADS, 0>};
-        for (int i = 0; i < 2; ++i) {
+        const void *fns[3] = {(const void *)cg_mixed_sr_kernel<R, 4>, (const void *)cg_mixed_sr_kernel<R, 6>,
+                              (const void *)cg_mixed_sr_kernel<R, 0>};
+        for (int i = 0; i < 3; ++i) {
             cudaFuncAttributes fa{};
             if (cudaFuncGetAttributes(&fa, fns[i]) != cudaSuccess) return 0;
             const int dyn = optin - (int)fa.sharedSizeBytes;
@@ -155,8 +181,9 @@ cudaError_t Launch<R>::cg(const CgArgs<R> &a, int grid, int threads, cudaStream_
     if constexpr (std::is_same<R, float>::value) {
         fn = (const void *)cg_mixed_kernel<R>;
         if (a.npb > 0 && a.sr) {
-            fn = a.reg ? (const void *)cg_mixed_sr_kernel<R, SR_REG_THREADS, SR_REG_BLOCKS>
-                       : (const void *)cg_mixed_sr_kernel<R, CG_THREADS, 0>;
+            fn = a.reg == 4   ? (const void *)cg_mixed_sr_kernel<R, 4>
+                 : a.reg == 6 ? (const void *)cg_mixed_sr_kernel<R, 6>
+                              : (const void *)cg_mixed_sr_kernel<R, 0>;
             smem = sr_smem_bytes(a.npb, a.nhalo, a.poly) +
                    (a.kc > 0 ? sr_cache_bytes(a.kc, sr_cache_stride(a.npb, a.tpn)) : 0);
         } else if (a.npb > 0) {
@@ -165,7 +192,10 @@ cudaError_t Launch<R>::cg(const CgArgs<R> &a, int grid, int threads, cudaStream_
         }
     } else {
         fn = (const void *)cg_kernel<R>;
-        if (a.npb > 0) {
+        if (a.npb > 0 && a.unit) {
+            fn = own_unit_kernel<R>(a.unit, a.block3);
+            smem = own_unit_smem(a.npb, a.nhalo, a.unit, a.block3 ? 9 : 1, a.kc);
+        } else if (a.npb > 0) {
             fn = (const void *)cg_own_kernel<R>;
             smem = own_smem_bytes_d(a.npb);
         }

@@ -762,12 +762,13 @@ struct CgArgs {
     // owned-rows kernels that stage the vector their SpMV reads: the rows of other blocks that block b's rows
     // reach (halo_list[halo_ptr[b] .. halo_ptr[b + 1])), every matrix slot's column as an index into the block's
     // staged vector (own rows at 0 .. npb - 1, its halo from npb on), the rows' messages (two buffers of N) and
-    // the blocks' partial sums as messages (two buffers, rows of `stride`)
+    // the blocks' partial sums as messages (two buffers, MSG_COPIES rows of `stride` per value)
     const int *halo_ptr, *halo_list;
     const unsigned short *lcol;
     Msg *msg, *rmsg;
     int nhalo;            // the largest halo of any block
-    int reg;              // cg_mixed_sr_kernel: the form with the first blocks of each lane in registers
+    int unit;             // FP64: components per unit of cg_own_unit_kernel (1 or 3; 0: another kernel)
+    int reg;              // cg_mixed_sr_kernel: blocks of each lane in registers (its form: 0, 4 or 6)
 };
 
 // p at node b for this iteration: p_new = beta p_old + D^{-1} r (vec3_scale_and_add with the
@@ -1118,6 +1119,379 @@ __device__ __forceinline__ void spmv_row_pd(const CgArgs<R> &g, const double2 *p
         q0 += __shfl_xor_sync(0xffffffffu, q0, o);
         q1 += __shfl_xor_sync(0xffffffffu, q1, o);
         q2 += __shfl_xor_sync(0xffffffffu, q2, o);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The FP64 CG with each block owning a run of npb rows, at most OWN_UNIT_THREADS units (below) a block: everything a
+// row needs stays in its thread's registers, the direction is staged in shared memory, and rows and sums travel as
+// tagged messages.
+//
+// GB300 issues an FP64 instruction for a warp once in about 64 cycles per SM sub-partition, so a block's time is the
+// number of FP64 instructions on its fullest sub-partition, and a chain of them costs as much as their issue. What
+// follows from that:
+//  - small meshes take one unit per scalar row (NC = 1): three times the lanes, each with a third of the products and
+//    a third of the shuffle adds, and tpu lanes to a unit, chosen by counting the instructions of the fullest
+//    sub-partition; larger ones one unit per row (NC = 3), whose dot products fuse over the components;
+//  - a block's partial sums are added over full warps (block_sum_units), not 32 in sequence by one warp;
+//  - the step length's division is the only one left between a sum and what waits for it: 1/delta for beta is formed
+//    while the sums travel, the convergence test multiplies, and the history is divided at the end;
+//  - x is updated while the residual's sums travel.
+// us per step before (barriers on counters, 256 rows a block, shared-memory state) -> now: 64 nodes consistent mass
+// 288 -> 168, 343 nodes 1905 -> 695, 9261 nodes consistent mass 670 -> 440, 40^3 cells 18.7 -> 16.3 ms (there the SpMV
+// issues for 14.2 of its 16.4 us per iteration).
+// Every value is computed from the same products as in cg_kernel, fused in the same way per component; only the
+// grouping of sums changes.
+// ---------------------------------------------------------------------------
+constexpr int OWN_UNIT_THREADS = 512;
+
+// values per matrix block that a unit multiplies, and blocks of each lane in registers
+template <int NC, bool B3>
+struct UnitBlock {
+    static constexpr int V = B3 ? 3 * NC : 1;
+    static constexpr int RB = NC == 1 ? (B3 ? 6 : 12) : 0;
+};
+
+// Bytes of dynamic shared memory: the staged direction (3 per row of the block and its halo), the units' addends of
+// two sums, and kc matrix blocks per row (values, then local columns; NC = 3 only)
+__host__ __device__ inline int own_unit_count(int npb, int nc) { return nc == 3 ? npb : 3 * npb; }
+__host__ __device__ inline size_t own_unit_smem(int npb, int nhalo, int nc, int vals, int kc) {
+    return (3 * ((size_t)npb + nhalo) + 2 * (size_t)own_unit_count(npb, nc)) * sizeof(double) +
+           (size_t)kc * npb * (vals * sizeof(double) + sizeof(unsigned short));
+}
+
+// The sum over u < U of NV addends per unit, s[i U + u], in s_out[i] for warp i's lane 0 (other threads: not
+// defined): four warps (one per sub-partition) per value add strided runs, one warp their 128 partials.
+template <int NV>
+__device__ __forceinline__ double block_sum_units(double *s, int U, int i) {
+    const int lane = threadIdx.x & 31, wid = warp_index();
+    __syncthreads();
+    if (U > 64) {
+        double t = 0.0;
+        const int v = wid >> 2, at = threadIdx.x & 127;
+        if (v < NV) {
+            if (at < U) t = s[v * U + at];
+            for (int u = at + 128; u < U; u += 128) t += s[v * U + u];
+        }
+        __syncthreads();
+        if (v < NV && at < U) s[v * U + at] = t;
+        __syncthreads();
+    }
+    double t = 0.0;
+    if (i < NV) {
+        if (U > 64) {
+            const int n = U < 128 ? U : 128;
+            t = lane < n ? s[i * U + lane] : 0.0;
+            double t2 = lane + 32 < n ? s[i * U + lane + 32] : 0.0;
+            if (n > 64) {
+                const double t3 = lane + 64 < n ? s[i * U + lane + 64] : 0.0, t4 = lane + 96 < n ? s[i * U + lane + 96] : 0.0;
+                t += t3;
+                t2 += t4;
+            }
+            t += t2;
+        } else {
+            t = lane < U ? s[i * U + lane] : 0.0;
+            if (lane + 32 < U) t += s[i * U + lane + 32];
+        }
+        t = warp_sum(t);
+    }
+    return t;
+}
+
+// The grid's sums of NV addends per unit (s[i U + u], written by the caller): warp i
+// publishes and collects value i and its lane 0 passes it to `finish` before the block's closing barrier. `tag` counts
+// the launch's reductions from 1. While the messages travel the block runs `meanwhile`.
+template <int NV, class A, class F, class G>
+__device__ __forceinline__ bool grid_reduce_units(const A &g, double *s, int U, unsigned int tag, DevStatus *st,
+                                                  F meanwhile, G finish) {
+    const int lane = threadIdx.x & 31, wid = warp_index(), nb = gridDim.x;
+    double t = block_sum_units<NV>(s, U, wid);
+    int bad = 0;
+    Msg *const rows = g.rmsg + ((size_t)(tag & 1u) * 2 + wid) * MSG_COPIES * g.stride;
+    const Msg *const row = rows + (size_t)(blockIdx.x % MSG_COPIES) * g.stride;
+    if (wid < NV && nb > 1 && lane < MSG_COPIES)
+        msg_put(rows + (size_t)lane * g.stride + blockIdx.x, (uint32_t)__double2loint(t), (uint32_t)__double2hiint(t), 0u,
+                tag);
+    meanwhile();
+    if (wid < NV) {
+        if (nb > 1) {
+            t = 0.0;
+            if (!msg_collect<5>(row, nb, tag, st,
+                             [&](const Msg &m) { t += __hiloint2double((int)m.y, (int)m.x); }))
+                bad = 1;
+            __syncwarp();
+            t = warp_sum(t);
+        }
+        if (lane == 0 && !bad) finish(wid, t);
+    }
+    return __syncthreads_or(bad) == 0;
+}
+
+template <class R, int NC, bool B3>
+__global__ void __launch_bounds__(OWN_UNIT_THREADS, 1) cg_own_unit_kernel(const __grid_constant__ CgArgs<R> g) {
+    static_assert(sizeof(R) == sizeof(double), "the FP64 owned-rows CG");
+    constexpr int V = UnitBlock<NC, B3>::V, RB = UnitBlock<NC, B3>::RB;
+    extern __shared__ __align__(16) double snd_u[];
+    __shared__ double s_sc[2];
+    __shared__ double s_alpha, s_beta, s_idelta, s_delta;
+    __shared__ int s_conv;
+    DevStatus *st = g.st;
+    if (st->abort) return;
+    FFEA_PHASES_BEGIN(tm);
+    const int npb = g.npb, a0 = blockIdx.x * npb, nloc = max(0, min(npb, g.N - a0)), N = g.N;
+    const int S = npb + g.nhalo, U = own_unit_count(npb, NC);
+    double *const zp = snd_u, *const red = zp + 3 * S, *const cv = red + 2 * U;
+    const int ncache = g.kc * npb;
+    unsigned short *const ccol = reinterpret_cast<unsigned short *>(cv + (size_t)V * ncache);
+    // this thread's unit: row l (component c0 of it, or all three), lane `sub` of the unit's tpu
+    const int tpu = g.tpn, u = threadIdx.x / tpu, sub = threadIdx.x % tpu;
+    const int c0 = NC == 3 ? 0 : u / npb, l = NC == 3 ? u : u - c0 * npb;
+    const bool valid = l < nloc && c0 < 3, owner = valid && sub == 0;
+    const int a = a0 + (valid ? l : 0), lane_a = a & 31;
+    const int base = valid ? __ldg(g.slice_ptr + (a >> 5)) : 0, len = valid ? __ldg(g.rowlen + a) : 0;
+    // value j of block k that this unit multiplies
+    auto value = [&](int k, int j) -> const R * {
+        if constexpr (B3) return g.val + 9 * (size_t)base + lane_a + (size_t)32 * (9 * k + 3 * c0 + j);
+        else return g.val + base + lane_a + (size_t)32 * k;
+    };
+    R rv[RB > 0 ? RB * V : 1];
+    unsigned int rc[RB > 0 ? (RB + 1) / 2 : 1];
+    if constexpr (RB > 0) {
+#pragma unroll
+        for (int j = 0; j < RB; ++j) {
+            const int k = sub + j * tpu;
+            const bool in = k < len;
+#pragma unroll
+            for (int i = 0; i < V; ++i) rv[j * V + i] = in ? __ldg(value(k, i)) : 0.0;
+            const unsigned int lc = in ? __ldg(g.lcol + base + 32 * k + lane_a) : 0u;
+            rc[j >> 1] = (j & 1) ? rc[j >> 1] | lc << 16 : lc;
+        }
+    } else {
+        for (int t = threadIdx.x; t < g.kc * nloc; t += blockDim.x) {
+            const int k = t / nloc, lr = t - k * nloc, ar = a0 + lr;
+            if (k >= __ldg(g.rowlen + ar)) continue;
+            const int br = __ldg(g.slice_ptr + (ar >> 5)), ln = ar & 31;
+#pragma unroll
+            for (int i = 0; i < V; ++i)
+                cv[(size_t)i * ncache + k * npb + lr] =
+                    __ldg(g.val + (B3 ? 9 * (size_t)br + ln + (size_t)32 * (9 * k + i) : (size_t)br + ln + 32 * k));
+            ccol[k * npb + lr] = __ldg(g.lcol + br + 32 * k + ln);
+        }
+    }
+    const int h0 = __ldg(g.halo_ptr + blockIdx.x), nh = __ldg(g.halo_ptr + blockIdx.x + 1) - h0;
+    R x[NC], r[NC], p[NC], di[NC];
+    // p = z = D^{-1} r  (conjugate_gradient_residual_assume_x_zero, src/NoMassCGSolver.cpp:196-220)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        x[c] = 0.0;
+        r[c] = valid ? g.r[4 * a + c0 + c] : 0.0;
+        di[c] = valid ? __ldg(g.dinv + 4 * a + c0 + c) : 0.0;
+        p[c] = di[c] * r[c];
+    }
+    unsigned int ep = 0, red_ep = 0;  // epochs of the published directions and of the grid-wide sums
+    // the direction to the other blocks and, with the halo's, into the staged vector
+    auto exchange = [&]() -> bool {
+        ++ep;
+        Msg *const m = g.msg + (size_t)(ep & 1u) * 3 * N;
+        if (owner)
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+                msg_put(m + (size_t)(c0 + c) * N + a, (uint32_t)__double2loint(p[c]), (uint32_t)__double2hiint(p[c]), 0u,
+                        ep);
+        __syncthreads();  // the SpMV of the previous direction has ended
+        if (owner)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) zp[(c0 + c) * S + l] = p[c];
+        int bad = 0;
+        for (int t = threadIdx.x; t < 3 * nh; t += 2 * (int)blockDim.x) {
+            const int t2 = t + (int)blockDim.x;
+            const bool use[2] = {true, t2 < 3 * nh};
+            const int ca = (t >= nh) + (t >= 2 * nh), cb = (t2 >= nh) + (t2 >= 2 * nh);
+            const int ha = t - ca * nh, hb = t2 - cb * nh;
+            const Msg *const at[2] = {m + (size_t)ca * N + __ldg(g.halo_list + h0 + ha),
+                                      m + (use[1] ? (size_t)cb * N + __ldg(g.halo_list + h0 + hb) : 0)};
+            Msg v[2];
+            if (!msg_wait_all<2>(at, use, ep, v, st)) { bad = 1; break; }
+            zp[ca * S + npb + ha] = __hiloint2double((int)v[0].y, (int)v[0].x);
+            if (use[1]) zp[cb * S + npb + hb] = __hiloint2double((int)v[1].y, (int)v[1].x);
+        }
+        return __syncthreads_or(bad) == 0;
+    };
+    grid_sum_d<2>(g.init_partials, g.init_stride, g.n_init, s_sc);
+    const double f2 = s_sc[0], tol = g.eps2 * f2;
+    if (threadIdx.x == 0) s_delta = s_sc[1];
+    bool ok = exchange(), conv = false;
+    FFEA_MARK(g, tm, 0);
+    int it = 0;
+    for (; ok && it < g.imax; ++it) {
+        // q = V p ; pTq   (get_alpha_denominator :253-266)
+        R q[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) q[c] = 0.0;
+        if (len > 0) {
+            if constexpr (RB > 0) {
+#pragma unroll
+                for (int j = 0; j < RB; ++j) {
+                    if (sub + j * tpu < len) {
+                        const int col = (j & 1) ? rc[j >> 1] >> 16 : rc[j >> 1] & 0xffffu;
+                        if constexpr (B3) {
+#pragma unroll
+                            for (int i = 0; i < 3; ++i) q[0] = fma(rv[j * V + i], zp[i * S + col], q[0]);
+                        } else {
+                            q[0] = fma(rv[j], zp[c0 * S + col], q[0]);
+                        }
+                    }
+                }
+#pragma unroll 1
+                for (int k = sub + RB * tpu; k < len; k += tpu) {
+                    const int col = __ldg(g.lcol + base + 32 * k + lane_a);
+                    if constexpr (B3) {
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) q[0] = fma(__ldg(value(k, i)), zp[i * S + col], q[0]);
+                    } else {
+                        q[0] = fma(__ldg(value(k, 0)), zp[c0 * S + col], q[0]);
+                    }
+                }
+            } else {
+                int k = 0;
+                const int kcl = min(g.kc, len);
+#pragma unroll 1
+                for (; k < kcl; ++k) {
+                    const int at = k * npb + l, col = ccol[at];
+                    const R p0 = zp[col], p1 = zp[S + col], p2 = zp[2 * S + col];
+                    if constexpr (B3) {
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) {
+                            q[c] = fma(cv[(size_t)(3 * c) * ncache + at], p0, q[c]);
+                            q[c] = fma(cv[(size_t)(3 * c + 1) * ncache + at], p1, q[c]);
+                            q[c] = fma(cv[(size_t)(3 * c + 2) * ncache + at], p2, q[c]);
+                        }
+                    } else {
+                        const R m = cv[at];
+                        q[0] = fma(m, p0, q[0]);
+                        if constexpr (NC == 3) {
+                            q[1] = fma(m, p1, q[1]);
+                            q[2] = fma(m, p2, q[2]);
+                        }
+                    }
+                }
+#pragma unroll 2
+                for (; k < len; ++k) {
+                    const int col = __ldg(g.lcol + base + 32 * k + lane_a);
+                    const R p0 = zp[col], p1 = zp[S + col], p2 = zp[2 * S + col];
+                    if constexpr (B3) {
+                        R v[9];
+#pragma unroll
+                        for (int i = 0; i < 9; ++i) v[i] = __ldg(value(k, i));
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) {
+                            q[c] = fma(v[3 * c], p0, q[c]);
+                            q[c] = fma(v[3 * c + 1], p1, q[c]);
+                            q[c] = fma(v[3 * c + 2], p2, q[c]);
+                        }
+                    } else {
+                        const R m = __ldg(value(k, 0));
+                        q[0] = fma(m, p0, q[0]);
+                        if constexpr (NC == 3) {
+                            q[1] = fma(m, p1, q[1]);
+                            q[2] = fma(m, p2, q[2]);
+                        }
+                    }
+                }
+            }
+        }
+        if (u - (int)(threadIdx.x & 31) / tpu < U)  // the warp holds a unit
+            for (int o = 1; o < tpu; o <<= 1)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) q[c] += __shfl_xor_sync(0xffffffffu, q[c], o);
+        if (u < U) {
+            double pq = p[0] * q[0];
+#pragma unroll
+            for (int c = 1; c < NC; ++c) pq = fma(p[c], q[c], pq);
+            if (sub == 0) red[u] = pq;
+        }
+        FFEA_MARK(g, tm, 1);
+        ok = grid_reduce_units<1>(
+            g, red, U, ++red_ep, st,
+            [&] {
+                if (threadIdx.x == blockDim.x - 32) s_idelta = 1.0 / s_delta;  // for beta
+            },
+            [&](int, double t) { s_alpha = s_delta / t; });
+        if (!ok) break;
+        FFEA_MARK(g, tm, 3);
+        const double alpha = s_alpha;
+        // x += alpha p ; r += (-alpha) q ; |r|^2 ; r.z   (vec3_add_to_scaled, residual2, apply_preconditioner)
+        R z[NC];
+        if (u < U) {
+            double rr = 0.0, rz = 0.0;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                r[c] = fma(-alpha, q[c], r[c]);
+                z[c] = di[c] * r[c];
+                rr = c == 0 ? r[c] * r[c] : fma(r[c], r[c], rr);
+                rz = c == 0 ? r[c] * z[c] : fma(r[c], z[c], rz);
+            }
+            if (sub == 0) {
+                red[u] = rr;
+                red[U + u] = rz;
+            }
+        }
+        FFEA_MARK(g, tm, 5);
+        ok = grid_reduce_units<2>(
+            g, red, U, ++red_ep, st,
+            [&] {
+                if (u < U)
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) x[c] = fma(alpha, p[c], x[c]);
+            },
+            [&](int i, double t) {
+                if (i == 0) {
+                    s_conv = (g.check_last || it + 1 < g.imax) && (f2 == 0.0 || t < tol);
+                    if (blockIdx.x == 0 && it < g.hist_cap) g.history[it] = t;
+                } else {
+                    s_beta = t * s_idelta;
+                    s_delta = t;
+                }
+            });
+        if (!ok) break;
+        FFEA_MARK(g, tm, 7);
+        if ((conv = s_conv != 0)) {
+            ++it;
+            break;
+        }
+        const R beta = s_beta;
+        // p = beta p + z   (vec3_scale_and_add :202-212)
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+            if (u < U) p[c] = fma(beta, p[c], z[c]);
+        FFEA_MARK(g, tm, 8);
+        if (!(ok = exchange())) break;
+        FFEA_MARK(g, tm, 9);
+    }
+    if (owner)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            g.x[4 * a + c0 + c] = x[c];
+            g.r[4 * a + c0 + c] = r[c];
+        }
+    FFEA_PHASES_END(g);
+    if (blockIdx.x == 0) {  // the history's |r|^2 becomes |r|^2 / |f|^2
+        __syncthreads();
+        for (int i = threadIdx.x; i < min(it, g.hist_cap); i += blockDim.x)
+            g.history[i] = f2 == 0.0 ? 0.0 : g.history[i] / f2;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (!ok) {
+            st->abort = 1;
+        } else if (!conv) {
+            st->cg_fail = 1;
+            st->abort = 1;
+            st->last_iters = g.imax;
+            st->total_iters += g.imax;
+        } else {
+            st->last_iters = it;
+            st->total_iters += it;
+        }
     }
 }
 

@@ -862,17 +862,14 @@ __device__ __forceinline__ bool halo_exchange(const A &g, Staged &z, const int (
         float4 *zh = z.v + z.npb;
         for (int h = threadIdx.x, t = 0; h < nh; h += 2 * (int)blockDim.x, ++t) {
             const int h2 = h + (int)blockDim.x;
-            const bool two = h2 < nh;
-            const Msg *pa = m + (t == 0 ? hx[0] : __ldg(g.halo_list + h0 + h));
-            const Msg *pb = two ? m + (t == 0 ? hx[1] : __ldg(g.halo_list + h0 + h2)) : pa;
-            Msg a = msg_get(pa), b = a;
-            if (two) b = msg_get(pb);
-            if (!msg_wait(pa, tag, a, st)) { bad = 1; break; }
-            zh[h] = make_float4(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z), 0.f);
-            if (two) {
-                if (!msg_wait(pb, tag, b, st)) { bad = 1; break; }
-                zh[h2] = make_float4(__uint_as_float(b.x), __uint_as_float(b.y), __uint_as_float(b.z), 0.f);
-            }
+            const bool use[2] = {true, h2 < nh};
+            const Msg *const at[2] = {m + (t == 0 ? hx[0] : __ldg(g.halo_list + h0 + h)),
+                                      m + (!use[1] ? 0 : t == 0 ? hx[1] : __ldg(g.halo_list + h0 + h2))};
+            Msg v[2];
+            if (!msg_wait_all<2>(at, use, tag, v, st)) { bad = 1; break; }
+            zh[h] = make_float4(__uint_as_float(v[0].x), __uint_as_float(v[0].y), __uint_as_float(v[0].z), 0.f);
+            if (use[1])
+                zh[h2] = make_float4(__uint_as_float(v[1].x), __uint_as_float(v[1].y), __uint_as_float(v[1].z), 0.f);
         }
     }
     return __syncthreads_or(bad) == 0;
@@ -912,10 +909,10 @@ __device__ __forceinline__ float warp_sum_spread(const float (&v)[NV], int &inde
 // warp, double-float over the block's warps, published as one message per value, and every block adds the blocks'
 // messages in the same order. `tag` counts the launch's reductions from 1. The caller must pass a __syncthreads()
 // before smem (NV x 32 floats) is written again.
-template <int NV, class A>
+template <int NV, int K, class A>
 __device__ __forceinline__ bool grid_reduce_msg(const A &g, const float (&v)[NV], float *smem, unsigned int tag,
                                                 df32 *s_out, DevStatus *st) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, nb = gridDim.x;
+    const int lane = threadIdx.x & 31, wid = warp_index(), nw = blockDim.x >> 5, nb = gridDim.x;
     int idx;
     const float ws = warp_sum_spread<NV>(v, idx);
     if (idx >= 0) smem[idx * 32 + wid] = ws;
@@ -925,27 +922,15 @@ __device__ __forceinline__ bool grid_reduce_msg(const A &g, const float (&v)[NV]
         df32 t = {lane < nw ? smem[i * 32 + lane] : 0.f, 0.f};
         t = warp_sum_df(t);
         if (nb > 1) {
-            Msg *row = g.rmsg + ((size_t)(tag & 1u) * NV + i) * g.stride;
-            if (lane == 0) msg_put(row + blockIdx.x, __float_as_uint(t.hi), __float_as_uint(t.lo), 0u, tag);
+            Msg *const rows = g.rmsg + ((size_t)(tag & 1u) * NV + i) * MSG_COPIES * g.stride;
+            const Msg *const row = rows + (size_t)(blockIdx.x % MSG_COPIES) * g.stride;
+            if (lane < MSG_COPIES)
+                msg_put(rows + (size_t)lane * g.stride + blockIdx.x, __float_as_uint(t.hi), __float_as_uint(t.lo), 0u, tag);
             t = df32{0.f, 0.f};
-            for (int b0 = 0; b0 < nb; b0 += 160) {
-                Msg m[5];
-#pragma unroll
-                for (int j = 0; j < 5; ++j) {
-                    const int b = b0 + lane + 32 * j;
-                    if (b < nb) m[j] = msg_get(row + b);
-                }
-#pragma unroll
-                for (int j = 0; j < 5; ++j) {
-                    const int b = b0 + lane + 32 * j;
-                    if (b < nb && !bad) {
-                        if (msg_wait(row + b, tag, m[j], st))
-                            t = df_add(t, df32{__uint_as_float(m[j].x), __uint_as_float(m[j].y)});
-                        else
-                            bad = 1;
-                    }
-                }
-            }
+            if (!msg_collect<K>(row, nb, tag, st, [&](const Msg &m) {
+                    t = df_add(t, df32{__uint_as_float(m.x), __uint_as_float(m.y)});
+                }))
+                bad = 1;
             __syncwarp();
             t = warp_sum_df(t);
         }
@@ -1049,10 +1034,14 @@ __device__ __forceinline__ void spmv_row_w(const A &g, const SrCache &c, const R
 }
 #undef FFEA_W_FMA
 
-// cg_mixed_sr_kernel's two forms: up to SR_REG_THREADS lanes a block with SR_REG_BLOCKS 3x3 blocks of each lane in
-// registers, or 1024 threads without
+// cg_mixed_sr_kernel's forms: up to SR_REG_THREADS lanes a block with RB 3x3 blocks of each lane in registers (4 where a
+// row has four lanes or more, so that they hold all of a usual row; else 6), or 1024 threads without (RB = 0). K is
+// how many of a sum's messages a lane waits for at once: as many as the registers hold without spilling.
 constexpr int SR_REG_THREADS = 512;
-constexpr int SR_REG_BLOCKS = 6;
+template <int RB>
+struct SrForm {
+    static constexpr int THREADS = RB > 0 ? SR_REG_THREADS : 1024, K = RB == 4 ? 5 : RB == 6 ? 3 : 2;
+};
 constexpr int SR_REG_ROWS = 128;  // rows a block is given while the mesh leaves SMs free
 
 // Bytes of dynamic shared memory cg_mixed_sr_kernel needs for npb owned rows and a halo of nhalo: the staged vector,
@@ -1124,10 +1113,10 @@ static __device__ __noinline__ double lanczos_lambda_max(const double *al, const
 // L2 round trip or two, around little arithmetic. So the exchange and the sums travel as tagged messages (Msg: one
 // round trip, no fence, no counter), the vector a pass reads is staged in shared memory (one gather of the halo
 // instead of an L2 read per block), and the matrix stays on chip: RB blocks of each lane in registers, the next kc of
-// each row in shared memory, what is left read from L2. 512 threads with 128 registers hold 6 blocks a lane without
-// spilling (8 spilled: the reloads missed the L1 that shared memory leaves, 3.51 against 3.09 ms per 40^3 step).
-// us per step, counters and L2 reads before -> now: 6^3 cells 590 -> 351, 20^3 1553 -> 879, 24^3 1859 -> 1117,
-// 40^3 3805 -> 3090, 45^3 (without register blocks) 4624 -> 4141.
+// each row in shared memory, what is left read from L2. 512 threads with 128 registers hold 6 blocks a lane
+// (8 spilled, and the reloads missed the L1 that shared memory leaves: 3.51 against 3.09 ms per 40^3 step).
+// us per step, counters and L2 reads before -> now: 6^3 cells 590 -> 317, 10^3 - -> 404, 20^3 1553 -> 780,
+// 30^3 - -> 1380, 40^3 3805 -> 2745, 45^3 (without register blocks) 4624 -> 4018.
 // Polynomial preconditioning (g.poly = d > 0, once lambda_max of D^{-1} V is known): M^{-1} = P_d(D^{-1} V) D^{-1},
 // with 1 - lambda P_d(lambda) the Chebyshev polynomial of degree d + 1 on [lambda_max / cheb_ratio(d),
 // lambda_max], scaled to 1 at 0. z is built by d steps of the Chebyshev iteration for V z = r from z = 0 (d SpMVs,
@@ -1139,8 +1128,8 @@ static __device__ __noinline__ double lanczos_lambda_max(const double *al, const
 // cluster of the others (unscaled they sit at P_d(0), 15.7 for d = 4 on the 40^3 cube, which then needed 132
 // iterations a step instead of 110). The scale changes the shifted operator only on the rigid modes, where the
 // projected right-hand side has no component, so the solution is the same: the one with Z^T D x = 0.
-template <class R, int NT, int RB>
-__global__ void __launch_bounds__(NT, 1) cg_mixed_sr_kernel(const __grid_constant__ CgArgs<R> g) {
+template <class R, int RB>
+__global__ void __launch_bounds__(SrForm<RB>::THREADS, 1) cg_mixed_sr_kernel(const __grid_constant__ CgArgs<R> g) {
     static_assert(sizeof(R) == sizeof(float), "the single-reduction CG is the mixed path's");
     extern __shared__ __align__(16) float4 sn_raw[];
     __shared__ float smemf[MIXED_SR_NP * 32];
@@ -1227,7 +1216,7 @@ __global__ void __launch_bounds__(NT, 1) cg_mixed_sr_kernel(const __grid_constan
     mixed_setup(g, s_sc, s_A6, s_tau, s_Om, &s_dummy, &s_conv);
     __syncthreads();
     const float ith = cheb ? s_ith : 0.f;
-    // tpn lanes to a row, every row of the block at once (npb tpn <= NT)
+    // tpn lanes to a row, every row of the block at once (npb tpn <= blockDim)
     const int tpn = g.tpn, l = threadIdx.x / tpn, sub = threadIdx.x % tpn;
     const bool valid = l < nloc;
     RowRegs<RB> rr;
@@ -1372,9 +1361,9 @@ __global__ void __launch_bounds__(NT, 1) cg_mixed_sr_kernel(const __grid_constan
             }
         }
         FFEA_MARK(g, tm, 1);
-        if (!(ok = grid_reduce_msg<MIXED_SR_NP>(g, acc, smemf, ++red_ep, s_scf, st))) break;
+        if (!(ok = grid_reduce_msg<MIXED_SR_NP, SrForm<RB>::K>(g, acc, smemf, ++red_ep, s_scf, st))) break;
         FFEA_MARK(g, tm, 3);
-        if (threadIdx.x < 32) {
+        if (warp_index() == 0) {
             // The iteration's scalars, in double-float as the sums arrive: this chain is on every block's critical path
             // and FP64 runs at 1/64 of the FP32 rate (4.0 us per iteration; see below for the pairs').
             const int ln = threadIdx.x;

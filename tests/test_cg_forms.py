@@ -1,9 +1,21 @@
-"""The mixed CG_nomass solve (cg_mixed_sr_kernel) at the edges of its launch forms, against the FP64 path."""
+"""The CG kernels at the edges of their launch forms: the mixed CG_nomass solve (cg_mixed_sr_kernel) against the FP64
+path, the FP64 solve against the oracle."""
 import numpy as np
 import pytest
 
+import pyoracle
 from ffea_ci_demo_gb300 import lib
 from ffea_ci_demo_gb300.mesh import apply_shear, kuhn_box
+
+
+def renumbered(m, shuffle):
+    """The same blob with its vertices numbered at random (a block's halo is then most of the mesh)."""
+    if shuffle:
+        new = np.concatenate([np.random.default_rng(9).permutation(m.n_linear), np.arange(m.n_linear, m.n_nodes)])
+        pos = np.empty_like(m.pos)
+        pos[new] = m.pos
+        m.pos, m.tets = pos, new[m.tets].astype(np.int32)
+    return m
 
 
 # rows per block of the single-reduction CG at the edges of its forms: one block (8 and 128 rows), two blocks,
@@ -14,13 +26,7 @@ from ffea_ci_demo_gb300.mesh import apply_shear, kuhn_box
                                            ((33, 9, 7), True), ((20, 20, 20), True), ((30, 29, 31), False),
                                            ((42, 42, 42), False)])
 def test_single_reduction_cg_forms(cells, shuffle):
-    m = kuhn_box(*cells, 5.0, seed=4)
-    if shuffle:  # vertices renumbered at random: the same blob in another node order
-        rng = np.random.default_rng(9)
-        new = np.concatenate([rng.permutation(m.n_linear), np.arange(m.n_linear, m.n_nodes)])
-        pos = np.empty_like(m.pos)
-        pos[new] = m.pos
-        m.pos, m.tets = pos, new[m.tets].astype(np.int32)
+    m = renumbered(kuhn_box(*cells, 5.0, seed=4), shuffle)
     kw = dict(solver="CG_nomass", dt=1e-13, kT=4.11e-21, calc_noise=1)
     p0 = apply_shear(m, 0.001) * (m.scale / 1.7e-10)
     out = {}
@@ -34,3 +40,29 @@ def test_single_reduction_cg_forms(cells, shuffle):
     move = np.abs(out["fp64", False] - p0).max()
     assert np.abs(out["mixed", False] - out["fp64", False]).max() < 1e-5 * move  # the mixed path's bound
     assert np.array_equal(out["mixed", False], out["mixed", True])  # where the matrix is read from does not matter
+
+
+# the FP64 solve (cg_own_unit_kernel) at the edges of its forms, against the oracle's CG: one block, several, a halo
+# of most of the mesh, one unit per component up to 170 rows a block, per row from there, and (44^3 cells, 600 rows a
+# block) beyond the kernel
+@pytest.mark.gpu
+@pytest.mark.parametrize("cells,solver,shuffle", [((1, 1, 1), "CG", False), ((3, 3, 3), "CG", False),
+                                                  ((4, 3, 3), "CG_nomass", False), ((12, 12, 12), "CG_nomass", True),
+                                                  ((28, 28, 29), "CG", False), ((29, 28, 29), "CG_nomass", False),
+                                                  ((31, 31, 31), "CG", True), ((31, 31, 31), "CG_nomass", False),
+                                                  ((44, 44, 44), "CG", False)])
+def test_fp64_cg_forms(cells, solver, shuffle):
+    m = renumbered(kuhn_box(*cells, 5.0, seed=4), shuffle)
+    kw = dict(solver=solver, dt=1e-13 if solver == "CG_nomass" else 1e-14, kT=4.11e-21, calc_noise=1)
+    p0 = apply_shear(m, 0.001) * (m.scale / 1.7e-10)
+    b = lib.Blob(m, **kw)
+    o = pyoracle.OracleBlob(m, threads=1, fast=True, **kw)
+    b.set_state(pos=p0)
+    o.set_pos(p0)
+    b.update(2)
+    assert o.step(2) == 0
+    assert b.cg_kernel() == "cg_own_kernel"
+    moved = np.abs(o.pos() - p0).max()
+    assert np.abs(b.pos() - o.pos()).max() < 1e-8 * moved + 1e-15 * np.abs(p0).max()  # and the positions' rounding
+    h = b.cg_history()
+    assert len(h) == b.cg_iterations()[0] and h[-1] < 1e-20 <= h[-2]  # the stopping test's own quantity
