@@ -532,7 +532,7 @@ struct BlobImpl final : ffea_gpu_blob {
         CK(mem.alloc(&pbuf0, 4 * (size_t)N));
         CK(mem.alloc(&pbuf1, 4 * (size_t)N));
         CK(mem.alloc(&q, 4 * (size_t)N));
-        const int gthreads = Launch<R>::gather_threads();
+        const int gthreads = Launch<R>::gather_threads(h.N);
         gather_blocks = (N + gthreads - 1) / gthreads;
         constexpr bool mixed = std::is_same<R, float>::value;
         CK(mem.alloc(&init_partials, (mixed ? MIXED_GATHER_NP : 2) * (size_t)gather_blocks));
@@ -839,6 +839,7 @@ struct BlobImpl final : ffea_gpu_blob {
         if ((rc = mark(2))) return rc;
         GatherArgs<R> ga{};
         ga.N = h.N;
+        ga.threads = Launch<R>::gather_threads(h.N);
         ga.mode = p.solver == FFEA_GPU_MASSLUMPED ? 1 : 0;
         ga.inc_ptr = inc_ptr; ga.inc = inc; ga.ef = ef; ga.pinned = pinned;
         ga.parts = me.parts; ga.part_ptr = me.part_ptr;
@@ -849,8 +850,8 @@ struct BlobImpl final : ffea_gpu_blob {
         ga.partials = init_partials; ga.stride = gather_blocks; ga.st = st; ga.gb = gb;
         ga.dpos = dpos; ga.px = px; ga.py = py; ga.pz = pz; ga.diag = diag;
         ga.xc[0] = xc[0]; ga.xc[1] = xc[1]; ga.xc[2] = xc[2];
-        // the mixed mass-lumped step updates positions in the gather (no solve between them)
-        ga.fuse_euler = std::is_same<R, float>::value && p.solver == FFEA_GPU_MASSLUMPED;
+        // the mass-lumped step updates positions in the gather (no solve between them)
+        ga.fuse_euler = p.solver == FFEA_GPU_MASSLUMPED;
         ga.upx = px; ga.upy = py; ga.upz = pz; ga.uvx = vx; ga.uvy = vy; ga.uvz = vz; ga.dt = p.dt;
         if (ga.fuse_euler && fused_prep()) {
             ga.nu = me.u;
@@ -878,6 +879,11 @@ struct BlobImpl final : ffea_gpu_blob {
             sn.lin_ev = sn_lin_ev;
             sn.on = sn.noise || sn.lin_ptr != nullptr;
         }
+        if (ga.fuse_euler && !fused_prep() && !ga.sn.noise) {
+            // the FP64 gather closes the step where none of its threads draws from the stream
+            ga.fin_jump = step_jump;
+            ga.fin_next = rng_state();
+        }
         CK(ctf.launch(stream));
         // midpoints that carry force: each computed once (the vertices' linearise replay reads it up to ~20 times)
         const int M = (int)h.mid_nodes.size();
@@ -891,7 +897,7 @@ struct BlobImpl final : ffea_gpu_blob {
             ga.nrng = rng_state();
             ga.nchunk_state = me.chunk_state;
             ga.nnchunks = me.nchunks;
-            gblocks = std::max(gblocks, (me.nchunks + Launch<R>::gather_threads() - 1) / Launch<R>::gather_threads());
+            gblocks = std::max(gblocks, (me.nchunks + Launch<R>::gather_threads(h.N) - 1) / Launch<R>::gather_threads(h.N));
         }
         CK(Launch<R>::gather(ga, gblocks, stream));
         if ((rc = mark(3))) return rc;
@@ -902,9 +908,12 @@ struct BlobImpl final : ffea_gpu_blob {
             eu.N = h.N; eu.nomass = nomass; eu.dt = p.dt; eu.x = x;
             eu.px = px; eu.py = py; eu.pz = pz; eu.vx = vx; eu.vy = vy; eu.vz = vz;
             eu.st = st;
+            eu.rng_state = rng_state();
+            eu.step_jump = step_jump;
             CK(Launch<R>::euler(eu, stream));
+        } else if (!ga.fin_next) {
+            CK(launch_finish_step(rng_state(), step_jump, st, stream));
         }
-        if (!ga.fin_next) CK(launch_finish_step(rng_state(), step_jump, st, stream));
         return mark(5);
     }
 

@@ -18,7 +18,7 @@ struct Launch {
     static cudaError_t gather(const GatherArgs<R> &a, int blocks, cudaStream_t s);
     // the step's midpoint forces (M midpoints) into out, for the gather's linearise replay
     static cudaError_t mid_force(const NodeForces &sn, int M, R *out, const DevStatus *st, cudaStream_t s);
-    static int gather_threads();
+    static int gather_threads(int N);
     // persistent cooperative CG of `grid` blocks of `threads` threads (128 <= threads <= cg_threads(),
     // a multiple of 32)
     static cudaError_t cg(const CgArgs<R> &a, int grid, int threads, cudaStream_t s);

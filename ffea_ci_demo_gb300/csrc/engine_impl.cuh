@@ -23,7 +23,13 @@ cudaError_t Launch<R>::element(const ElemArgs<R> &a, cudaStream_t s) {
         return (void)a, (void)s, cudaErrorNotSupported;
     } else {
         if (a.T <= 0) return cudaSuccess;
-        element_kernel<R><<<(a.T + ELEM_THREADS - 1) / ELEM_THREADS, ELEM_THREADS, 0, s>>>(a);
+        // four lanes to an element while that leaves a sub-partition (608 of them) two warps at most; us at 1296 / 6000 /
+        // 10,368 elements, four lanes against one: inertial 25 / 40 / 56 against 49 / 49 / 50, CG_nomass 14 / 20 / 25
+        // against 23 / 23 / 24
+        if (a.T <= 608 * 2 * 8)
+            element_split_kernel<R><<<(4 * a.T + ELEM_THREADS - 1) / ELEM_THREADS, ELEM_THREADS, 0, s>>>(a);
+        else
+            element_kernel<R><<<(a.T + ELEM_THREADS - 1) / ELEM_THREADS, ELEM_THREADS, 0, s>>>(a);
         count_launch();
         return cudaGetLastError();
     }
@@ -47,13 +53,18 @@ cudaError_t Launch<R>::assemble(const AsmArgs<R> &a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+// threads per block of the gather of N nodes: an FP64 blob that leaves SMs free takes small blocks (its adds share the
+// SM's FP64 units)
 template <class R>
-int Launch<R>::gather_threads() { return GATHER_THREADS; }
+int Launch<R>::gather_threads(int N) {
+    return !std::is_same<R, float>::value && N <= 152 * 128 ? 64 : GATHER_THREADS;
+}
 
 template <class R>
 cudaError_t Launch<R>::gather(const GatherArgs<R> &a, int blocks, cudaStream_t s) {
-    // modes 0 and 1 reduce over blocks of GATHER_THREADS; the batch's mode 2 takes any of 64, 128, 256
-    const int bt = (a.mode == 2 && a.threads > 0) ? a.threads : GATHER_THREADS;
+    // the mixed modes 0 and 1 reduce over blocks of GATHER_THREADS; FP64 and the batch's mode 2 take any of 64, 128, 256
+    const bool fp64 = !std::is_same<R, float>::value;
+    const int bt = ((a.mode == 2 || fp64) && a.threads > 0) ? a.threads : GATHER_THREADS;
     if (!(bt == 64 || bt == 128 || bt == 256)) return cudaErrorInvalidValue;
     if constexpr (std::is_same<R, float>::value) {
         const bool nf = a.sn.on || a.sn.node_ctf || a.sn.vface_ptr || a.drag;

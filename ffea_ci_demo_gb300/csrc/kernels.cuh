@@ -238,6 +238,182 @@ __global__ void __launch_bounds__(128) element_kernel(ElemArgs<R> g) {
     gm[12] = vol;
 }
 
+// The same element phase with four lanes to an element, lane v working for vertex v (and, for v < 3, row v of the
+// stress). An FP64 instruction holds a sub-partition for 64 cycles whatever lanes it has, and one thread's element is a
+// chain of 750 of them (1,560 with the viscous term of the inertial solvers: 49 us however few elements there are), so
+// the vertices' gradients, the stress rows, the five divisions, the four square roots, the draws' conversions and the
+// viscous rows are each spread over the four lanes: 180 (470) instructions. Every value is formed by element_kernel's
+// expression in its order (products commute exactly), so the results are bit-identical.
+template <class R>
+__global__ void __launch_bounds__(128) element_split_kernel(ElemArgs<R> g) {
+    static_assert(sizeof(R) == sizeof(double), "the FP64 path's");
+    constexpr unsigned FULL = 0xffffffffu;
+    if (g.st->abort) return;
+    const int e_ = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, v = threadIdx.x & 3;
+    const bool live = e_ < g.T;
+    const int e = live ? e_ : g.T - 1;
+    const int4 t = g.tet[e];
+    const int node = v == 0 ? t.x : v == 1 ? t.y : v == 2 ? t.z : t.w;
+    auto lane = [&](double x, int s) { return __shfl_sync(FULL, x, s, 4); };
+    // calculate_jacobian :191-203
+    const double x[3] = {g.px[node], g.py[node], g.pz[node]};
+    double Jv[3], J[3][3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) Jv[c] = x[c] - lane(x[c], 0);
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) J[r][c] = lane(Jv[c], r + 1);
+    // calc_shape_function_derivatives_and_volume :222-292: vertex v's gradient is the cross product of two edges
+    double q[3], p[3], gv[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        q[c] = v == 1 ? J[2][c] : v == 2 ? J[0][c] : J[1][c];
+        p[c] = v == 1 ? J[1][c] : v == 2 ? J[2][c] : J[0][c];
+    }
+    gv[0] = q[2] * p[1] - q[1] * p[2];
+    gv[1] = q[0] * p[2] - q[2] * p[0];
+    gv[2] = q[1] * p[0] - q[0] * p[1];
+    const double part = Jv[0] * gv[0];
+    double det = lane(part, 1) + lane(part, 2) + lane(part, 3);
+    const double last = g.recompute ? det : g.last_det[e];
+    const bool inverted = last * det < 0;  // the step is void
+    if (live && v == 0) {
+        if (inverted) {
+            atomicAdd(&g.st->inversions, 1);
+            atomicExch(&g.st->abort, 1);
+        } else if (!g.recompute) {
+            g.last_det[e] = det;
+        }
+    }
+    const double vol = (1.0 / 6.0) * fabs(det);
+    det = 1.0 / det;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) gv[c] *= det;
+    double grad[4][3];  // every vertex's gradient
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        grad[1][c] = lane(gv[c], 1);
+        grad[2][c] = lane(gv[c], 2);
+        grad[3][c] = lane(gv[c], 3);
+        grad[0][c] = -(grad[1][c] + grad[2][c] + grad[3][c]);
+        if (v == 0) gv[c] = grad[0][c];
+    }
+    const double G = g.G[e], E = g.E[e], A = g.A[e], B = g.B[e], vol0 = g.vol0[e];
+    // add_shear_elastic_stress :375-392, row v of F and S (lane 3 repeats row 2)
+    double Fv[3], S[3];
+    {
+        double Jc[3];  // column v of J
+#pragma unroll
+        for (int k = 0; k < 3; ++k) Jc[k] = v == 0 ? J[k][0] : v == 1 ? J[k][1] : J[k][2];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            double s = 0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) s += Jc[k] * g.jinv[(size_t)(3 * j + k) * g.T + e];
+            Fv[j] = s;
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            double s = 0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) s += Fv[k] * lane(Fv[k], j);
+            S[j] = s;
+        }
+    }
+    // G vol0 / vol, vol0 / vol, vol / vol0, G 2 / 3, one to a lane
+    const double quot = (v == 0 ? G * vol0 : v == 1 ? vol0 : v == 2 ? vol : G * 2.0) /
+                        (v == 2 ? vol0 : v == 3 ? 3.0 : vol);
+    const double sc = lane(quot, 0), v0v = lane(quot, 1), vv0 = lane(quot, 2), c_2 = E - lane(quot, 3);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) S[j] *= sc;
+    // the diagonal of the row: shear, then add_bulk_elastic_stress :397-403
+    const double cb = G * (1.0 - v0v) + 0.5 * c_2 * (vv0 - v0v);
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+        if (j == min(v, 2)) {
+            S[j] -= G;
+            S[j] += cb;
+        }
+    // add_fluctuating_stress :412-431
+    if (g.calc_noise == 1) {
+        uint32_t base[6], s6[6], k6[7];
+        const uint32_t *rs = g.rng_state;
+        int le = e;
+        if (g.elem_blob) {
+            const int b = g.elem_blob[e];
+            le = e - g.elem_off[b];
+            rs += 6 * (size_t)b;
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) s6[k] = rs[k];
+        mrg_apply(g.chunk_jump[le >> 5], s6, base);
+        mrg_apply(g.lane_jump[le & 31], base, s6);
+#pragma unroll
+        for (int k = 0; k < 7; ++k) k6[k] = mrg_step(s6);
+        const double X = (24 * g.kT) / (vol * g.dt);
+        const double root = sqrt(v == 0 ? X : v == 1 ? B : v == 2 ? 2 * A : A);
+        const double c = lane(root, 0), sB = lane(root, 1), s2A = lane(root, 2), sA = lane(root, 3);
+        const double norm = 1.0 / (4294967087.0 + 1.0);
+        auto half = [&](uint32_t k) { return (-.5) + ((.5) - (-.5)) * ((double)k * norm); };  // mrg_rand_half
+        const double bf = sB * half(k6[0]);
+        const double nd = c * (s2A * half(v == 0 ? k6[1] : v == 1 ? k6[2] : k6[3]) + bf);
+        // off the diagonal, (0, 1) takes draw 4, (0, 2) draw 5, (1, 2) draw 6
+        const double n1 = c * sA * half(v == 2 || v == 3 ? k6[5] : k6[4]);  // row 0: (0,1); row 1: (1,0); row 2: (2,0)
+        const double n2 = c * sA * half(v == 0 ? k6[5] : k6[6]);            // row 0: (0,2); row 1: (1,2); row 2: (2,1)
+        S[0] += v == 0 ? nd : n1;
+        S[1] += v == 0 ? n1 : v == 1 ? nd : n2;
+        S[2] += v < 2 ? n2 : nd;
+    }
+    double du[3] = {0, 0, 0};  // vertex v
+    if (!g.nomass) {
+        // get_element_velocity_vector :448-463 + mat12_apply (src/mat_vec_fns.cpp:28-36): rows 4 c + v of the viscosity
+        // matrix (visc_entry), in its column order
+        const double w[3] = {g.vx[node], g.vy[node], g.vz[node]};
+        const double AB = A + B;
+        double diag[4], d2A[4], sp[3];
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            d2A[b] = (gv[0] * grad[b][0] + gv[1] * grad[b][1] + gv[2] * grad[b][2]) * A;
+        sp[0] = (B + A) * (gv[0] * gv[1]) * vol;
+        sp[1] = (B + A) * (gv[0] * gv[2]) * vol;
+        sp[2] = (B + A) * (gv[1] * gv[2]) * vol;
+#pragma unroll
+        for (int Jn = 0; Jn < 3; ++Jn) {
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                diag[b] = (gv[Jn] * grad[b][Jn] * AB + d2A[b]) * vol;
+                const double wb = lane(w[Jn], b);
+#pragma unroll
+                for (int I = 0; I < 3; ++I) {
+                    double entry;
+                    if (I == Jn) {
+                        entry = diag[b];
+                    } else {
+                        entry = (B * (gv[I] * grad[b][Jn]) + A * (grad[b][I] * gv[Jn])) * vol;
+                        if (b == v) entry = sp[I + Jn - 1];
+                    }
+                    du[I] += entry * wb;
+                }
+            }
+        }
+    }
+    // apply_stress_tensor :436-443
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        du[i] += vol * (gv[0] * lane(S[0], i) + gv[1] * lane(S[1], i) + gv[2] * lane(S[2], i));
+    if (!live || inverted) return;
+    // add_element_force_vector :468-483 (node_force starts at zero every step)
+    R *ef = g.ef + 12 * (size_t)e + 3 * v;
+    R *gm = g.geom + 16 * (size_t)e;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        ef[c] = 0 - du[c];
+        gm[4 * c + v] = gv[c];
+    }
+    if (v == 0) gm[12] = vol;
+}
+
 // ---------------------------------------------------------------------------
 // matrix assembly: CSR values = sum of element sources in element order
 // (SparseMatrixFixedPattern::build + sparse_entry_sources::sum_all_sources)
@@ -648,11 +824,25 @@ struct GatherArgs {
     uint32_t *fin_next;
 };
 
+// closes a step: the stream state advances by the step's draws and the step is counted
+__device__ __forceinline__ void finish_step(uint32_t *rng_state, const MrgJump *step_jump, DevStatus *st) {
+    uint32_t s[6], o[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) s[k] = rng_state[k];
+    mrg_apply(*step_jump, s, o);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) rng_state[k] = o[k];
+    st->steps_done += 1;
+}
+
 template <class R>
 __global__ void __launch_bounds__(256) gather_kernel(GatherArgs<R> g) {
     __shared__ double smem[64];
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a == 0 && g.gb) g.gb->count = 0u;
+    if (a == 0 && g.fin_next && !g.st->abort) {  // no thread of this launch reads the stream state
+        finish_step(g.fin_next, g.fin_jump, g.st);
+    }
     double acc[2] = {0.0, 0.0};
     const bool live = a < g.N && !g.st->abort;
     if (live) {
@@ -662,12 +852,25 @@ __global__ void __launch_bounds__(256) gather_kernel(GatherArgs<R> g) {
             F1 = (R)g.sn.node_ctf[3 * (size_t)a + 1];
             F2 = (R)g.sn.node_ctf[3 * (size_t)a + 2];
         }
-        for (int m = g.inc_ptr[a]; m < g.inc_ptr[a + 1]; ++m) {
-            const int es = g.inc[m];
-            const R *c = g.ef + 12 * (size_t)(es >> 2) + 3 * (es & 3);
-            F0 += c[0];
-            F1 += c[1];
-            F2 += c[2];
+        // eight contributions in flight (each is two dependent loads), added in order
+        const int m1 = g.inc_ptr[a + 1];
+        for (int m = g.inc_ptr[a]; m < m1; m += 8) {
+            R c[8][3];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int es = g.inc[min(m + j, m1 - 1)];
+                const R *f = g.ef + 12 * (size_t)(es >> 2) + 3 * (es & 3);
+                c[j][0] = f[0];
+                c[j][1] = f[1];
+                c[j][2] = f[2];
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (m + j < m1) {
+                    F0 += c[j][0];
+                    F1 += c[j][1];
+                    F2 += c[j][2];
+                }
         }
         if (g.sn.vface_ptr) {
             R F[3] = {F0, F1, F2};
@@ -691,9 +894,16 @@ __global__ void __launch_bounds__(256) gather_kernel(GatherArgs<R> g) {
         g.f[4 * a + 1] = (double)F1;
         g.f[4 * a + 2] = (double)F2;
         if (g.mode == 1) {  // MassLumpedSolver::solve, src/MassLumpedSolver.cpp:65-72
-            g.x[4 * a] = F0 * g.dinv[4 * a];
-            g.x[4 * a + 1] = F1 * g.dinv[4 * a + 1];
-            g.x[4 * a + 2] = F2 * g.dinv[4 * a + 2];
+            const R x0 = F0 * g.dinv[4 * a], x1 = F1 * g.dinv[4 * a + 1], x2 = F2 * g.dinv[4 * a + 2];
+            g.x[4 * a] = x0;
+            g.x[4 * a + 1] = x1;
+            g.x[4 * a + 2] = x2;
+            if (g.fuse_euler) {  // nothing lies between the mass-lumped solve and euler_integrate (euler_kernel)
+                if (!(isfinite(x0) && isfinite(x1) && isfinite(x2))) atomicExch(&g.st->nonfinite, 1);
+                const double v0 = g.uvx[a] + x0 * g.dt, v1 = g.uvy[a] + x1 * g.dt, v2 = g.uvz[a] + x2 * g.dt;
+                g.uvx[a] = v0; g.uvy[a] = v1; g.uvz[a] = v2;
+                g.upx[a] += v0 * g.dt; g.upy[a] += v1 * g.dt; g.upz[a] += v2 * g.dt;
+            }
         } else {  // conjugate_gradient_residual_assume_x_zero (src/NoMassCGSolver.cpp:196-220)
             const R z0 = g.dinv[4 * a] * F0, z1 = g.dinv[4 * a + 1] * F1, z2 = g.dinv[4 * a + 2] * F2;
             g.r[4 * a] = F0; g.r[4 * a + 1] = F1; g.r[4 * a + 2] = F2;
@@ -1663,7 +1873,7 @@ struct EulerArgs {
     double dt;
     const R *x;
     double *px, *py, *pz, *vx, *vy, *vz;
-    uint32_t *rng_state;     // advanced by step_jump once per step
+    uint32_t *rng_state;     // advanced by step_jump, which closes the step (or null)
     const MrgJump *step_jump;
     DevStatus *st;
 };
@@ -1672,6 +1882,7 @@ template <class R>
 __global__ void __launch_bounds__(256) euler_kernel(EulerArgs<R> g) {
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (g.st->abort || g.st->cg_fail) return;
+    if (a == 0 && g.rng_state) finish_step(g.rng_state, g.step_jump, g.st);
     if (a < g.N) {
         const double x0 = (double)g.x[4 * a], x1 = (double)g.x[4 * a + 1], x2 = (double)g.x[4 * a + 2];
         if (!(isfinite(x0) && isfinite(x1) && isfinite(x2))) atomicExch(&g.st->nonfinite, 1);

@@ -66,3 +66,24 @@ def test_fp64_cg_forms(cells, solver, shuffle):
     assert np.abs(b.pos() - o.pos()).max() < 1e-8 * moved + 1e-15 * np.abs(p0).max()  # and the positions' rounding
     h = b.cg_history()
     assert len(h) == b.cg_iterations()[0] and h[-1] < 1e-20 <= h[-2]  # the stopping test's own quantity
+
+
+# the FP64 element phase's two forms (four lanes to an element up to 9,728 elements) at their edges, against the
+# oracle: forces, volumes and positions bit for bit, the inertial solvers' viscous term and the noise included
+@pytest.mark.gpu
+@pytest.mark.parametrize("cells,solver,noise", [((1, 1, 1), "masslumped", 1), ((3, 5, 7), "masslumped", 0),
+                                                ((3, 5, 7), "CG_nomass", 1), ((11, 11, 13), "masslumped", 1),
+                                                ((12, 11, 13), "masslumped", 1)])
+def test_fp64_element_forms(cells, solver, noise):
+    m = kuhn_box(*cells, 3.0, seed=4)
+    kw = dict(solver=solver, dt=1e-14, kT=4.11e-21, calc_noise=noise)
+    p0 = apply_shear(m, 0.01, seed=5) * (m.scale / 1.7e-10)
+    b, o = lib.Blob(m, **kw), pyoracle.OracleBlob(m, threads=1, **kw)
+    b.set_state(pos=p0)
+    o.set_pos(p0)
+    n = 1 if solver == "CG_nomass" else 3
+    b.update(n)
+    assert o.step(n) == 0
+    assert np.array_equal(b.rhs(), o.rhs()) and np.array_equal(b.rng_state(), o.rng_state())
+    if solver == "masslumped":
+        assert np.array_equal(b.pos(), o.pos()) and np.array_equal(b.vel(), o.vel())
