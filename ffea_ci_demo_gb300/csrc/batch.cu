@@ -80,6 +80,18 @@ struct ffea_gpu_batch {
     int *d_node_of = nullptr;
     int2 *ref_src = nullptr;
     int max_rows = 0, max_elems = 0;
+    // the solve on chip (sr_batch_kernel), when plan_solve found room for every blob: arguments per blob, the blocks'
+    // tasks and the messages; on_chip says which kernel the steps launch
+    bool sr_ok = false, on_chip = false;
+    int sr_grid = 0, sr_tpn = 1;
+    size_t sr_smem = 0, sr_msg_bytes = 0;
+    std::vector<SrBlob> sr_host;
+    SrBlob *sr_args = nullptr;
+    SrTask *sr_tasks = nullptr;
+    int *sr_task_ptr = nullptr, *sr_halo_ptr = nullptr, *sr_halo_list = nullptr;
+    unsigned short *sr_lcol = nullptr;
+    Msg *sr_msg = nullptr;
+    double *sr_cheb = nullptr;
     // launch configuration (ffea_gpu_batch_tune)
     int cg_threads = 256, tpn = 4, ncta = 0, ncta_cap = 0;
     // launch shapes of the force phase (ffea_gpu_batch_set_shapes): elements per block of the element kernel,
@@ -108,6 +120,7 @@ struct ffea_gpu_batch {
     }
 
     int init();
+    int plan_solve();
     int configure(int threads, int tpn_);
     int set_shapes(int em, int at, int as, int gt);
     int time_forces(int reps, double &ms);
@@ -142,6 +155,15 @@ struct ffea_gpu_batch {
     int upload_desc(int only = -1) {
         const size_t b0 = only < 0 ? 0 : (size_t)only, nb = only < 0 ? hdesc.size() : 1;
         CK(cudaMemcpyAsync(desc + b0, hdesc.data() + b0, nb * sizeof(BlobCgDesc), cudaMemcpyHostToDevice, stream));
+        for (size_t b = b0; sr_ok && b < b0 + nb; ++b) {
+            SrBlob &a = sr_host[b];
+            a.nmodes = hdesc[b].nmodes;
+            for (int i = 0; i < 36; ++i) a.modes[i] = hdesc[b].modes[i];
+            for (int c = 0; c < 3; ++c) a.xc[c] = hdesc[b].xc[c];
+        }
+        if (sr_ok)
+            CK(cudaMemcpyAsync(sr_args + b0, sr_host.data() + b0, nb * sizeof(SrBlob), cudaMemcpyHostToDevice,
+                               stream));
         CK(cudaStreamSynchronize(stream));
         return FFEA_GPU_OK;
     }
@@ -330,7 +352,8 @@ int ffea_gpu_batch::init() {
     }
     CK(mem.alloc(&desc, (size_t)nblobs));
     CK(mem.upload(&blob_iters, it0));
-    int rc = upload_desc();
+    int rc = plan_solve();
+    if (!rc) rc = upload_desc();
     if (rc) return rc;
     // the grid of the largest configuration the tuner may pick bounds the per-CTA arrays
     ncta_cap = 0;
@@ -344,7 +367,13 @@ int ffea_gpu_batch::init() {
     CK(cudaDeviceSynchronize());
     // default: 256-thread CTAs (the largest size whose grid still has a CTA per blob if not), 4 lanes per row
     for (int t : {256, 128}) {
-        if (BatchLaunch::cg_max_grid(device, t) >= nblobs) return configure(t, 4);
+        const int grid = BatchLaunch::cg_max_grid(device, t);
+        if (grid < nblobs) continue;
+        if (!on_chip) return configure(t, 4);
+        cg_threads = t;
+        tpn = 4;
+        ncta = grid;
+        return capture();
     }
     g_last_error = "no CTA size gives one CTA per blob";
     return FFEA_GPU_EINPUT;
@@ -360,7 +389,125 @@ int ffea_gpu_batch::configure(int threads, int tpn_) {
     cg_threads = threads;
     tpn = tpn_;
     ncta = grid;
+    on_chip = false;
     return capture();
+}
+
+// The solve on chip: rows per block, the blocks' tasks and the kernel's arguments. A blob of n rows takes
+// ceil(n / rows) blocks, one if it fits; the blobs, longest first, each go to the blocks that are free soonest, in that order on every
+// block. `rows` is the candidate with the shortest schedule by the measured time of an iteration, 11 + 0.047 rows us
+// (10^3 to 40^3 cells; its latencies do not shrink with the rows, so full blocks win as soon as there is work for
+// them all), times 0.17 iterations per row along a side (2 per cell) with the polynomial. Blobs of one block keep the
+// Jacobi preconditioner (3 us an iteration, which the polynomial's passes would cost as well). Left out (sr_ok false:
+// cg_batch_kernel) when a blob's rows do not fit, or when there are so many tiny blobs that a block would run more
+// than four one after another while cg_batch_kernel runs up to eight on an SM at once.
+int ffea_gpu_batch::plan_solve() {
+    int sms = 0;
+    const size_t limit = BatchLaunch::sr_smem_limit(device, sms);
+    if (limit == 0 || sms <= 0 || nblobs > 4 * sms) return FFEA_GPU_OK;
+    const int N = h.N;
+    const int want_poly = p.cg_poly == 0 ? FFEA_GPU_CG_POLY_DEFAULT : std::max(p.cg_poly, 0);
+    std::vector<int> order(nblobs);
+    std::vector<double> free_at, cost(nblobs);
+    std::vector<std::vector<int>> where(nblobs);
+    auto blocks_of = [&](int n, int rows) { return n <= SR_REG_THREADS ? 1 : (n + rows - 1) / rows; };
+    // blocks per blob and the schedule for `rows`; returns its length in us
+    auto schedule = [&](int rows) {
+        for (int b = 0; b < nblobs; ++b) {
+            order[b] = b;
+            const int n = row_off[b + 1] - row_off[b], blocks = blocks_of(n, rows);
+            const double side = std::cbrt((double)n);
+            if (blocks > sms) return 1e300;
+            const double per = (n + blocks - 1) / blocks;
+            cost[b] = blocks > 1 && want_poly > 0 ? 2.0 * side * (11.0 + 0.047 * per)
+                                                  : 12.5 * side * (blocks > 1 ? 5.0 + 0.012 * per : 3.0);
+        }
+        std::sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y] || (cost[x] == cost[y] && x < y); });
+        free_at.assign(sms, 0.0);
+        std::vector<int> by(sms);
+        for (int c = 0; c < sms; ++c) by[c] = c;
+        double end = 0.0;
+        for (int b : order) {
+            const int n = row_off[b + 1] - row_off[b], blocks = blocks_of(n, rows);
+            std::sort(by.begin(), by.end(), [&](int x, int y) { return free_at[x] < free_at[y] || (free_at[x] == free_at[y] && x < y); });
+            where[b].assign(by.begin(), by.begin() + blocks);
+            const double t = free_at[by[blocks - 1]] + cost[b];
+            for (int c : where[b]) free_at[c] = t;
+            end = std::max(end, t);
+        }
+        return end;
+    };
+    int rows = 0;
+    double best = 1e300;
+    for (int r : {128, 160, 192, 224, 256, 320, 384, 448, 512}) {
+        const double t = schedule(r);
+        if (t < best) { best = t; rows = r; }
+    }
+    if (rows == 0) return FFEA_GPU_OK;
+    schedule(rows);
+    sr_host.assign(nblobs, SrBlob{});
+    Halo hl;
+    std::vector<int> first_ptr(nblobs);
+    std::vector<long long> msg_off(nblobs);
+    long long msgs = 2 * (long long)N;
+    sr_smem = 0;
+    for (int b = 0; b < nblobs; ++b) {
+        SrBlob &a = sr_host[b];
+        const int n = row_off[b + 1] - row_off[b], blocks = (int)where[b].size(), npb = (n + blocks - 1) / blocks;
+        int t = 8;
+        while (t > 1 && npb * t > SR_REG_THREADS) t >>= 1;
+        if (b == 0) first_ptr[b] = 0;
+        else first_ptr[b] = (int)hl.ptr.size() - 1;
+        build_halo(h, row_off[b], n, npb, blocks, hl);
+        const int poly = blocks > 1 ? want_poly : 0;
+        const size_t need = sr_smem_bytes(npb, hl.largest, poly);
+        if (npb > SR_REG_THREADS || npb + hl.largest >= 65536 || need > limit) return FFEA_GPU_OK;
+        int maxlen = 0;
+        for (int r = row_off[b]; r < row_off[b + 1]; ++r) maxlen = std::max(maxlen, h.rowlen[r]);
+        const int S = sr_cache_stride(npb, t);
+        a.N = n;
+        a.row0 = row_off[b];
+        a.npb = npb;
+        a.tpn = t;
+        a.nhalo = hl.largest;
+        a.poly = poly;
+        a.kc = (int)std::min<size_t>(std::max(0, maxlen - 6 * t), (limit - need) / ((size_t)SR_CACHE_BYTES_PER_BLOCK * S));
+        if (p.cg_smem_blocks != 0) a.kc = std::min(a.kc, std::max(0, p.cg_smem_blocks));
+        sr_smem = std::max(sr_smem, need + (a.kc > 0 ? sr_cache_bytes(a.kc, S) : 0));
+        a.stride = blocks;
+        msg_off[b] = msgs;
+        if (blocks > 1) msgs += 2ll * MSG_VALUES * MSG_COPIES * blocks;
+        if (b == 0) sr_tpn = t;
+    }
+    std::vector<int> tptr(sms + 1, 0);
+    std::vector<std::vector<SrTask>> per(sms);
+    for (int b : order)
+        for (int k = 0; k < (int)where[b].size(); ++k) per[where[b][k]].push_back({b, k, (int)where[b].size()});
+    std::vector<SrTask> tasks;
+    for (int c = 0; c < sms; ++c) {
+        tasks.insert(tasks.end(), per[c].begin(), per[c].end());
+        tptr[c + 1] = (int)tasks.size();
+    }
+    if (hl.list.empty()) hl.list.push_back(0);
+    CK(mem.upload(&sr_tasks, tasks));
+    CK(mem.upload(&sr_task_ptr, tptr));
+    CK(mem.upload(&sr_halo_ptr, hl.ptr));
+    CK(mem.upload(&sr_halo_list, hl.list));
+    CK(mem.upload(&sr_lcol, hl.lcol));
+    sr_msg_bytes = (size_t)msgs * sizeof(Msg);
+    CK(mem.alloc(&sr_msg, (size_t)msgs));
+    CK(mem.alloc(&sr_cheb, (size_t)CHEB_STATE * nblobs));
+    CK(mem.alloc(&sr_args, (size_t)nblobs));
+    for (int b = 0; b < nblobs; ++b) {
+        SrBlob &a = sr_host[b];
+        a.cheb = sr_cheb + (size_t)CHEB_STATE * b;
+        a.halo_ptr = sr_halo_ptr + first_ptr[b];
+        a.rmsg = sr_msg + msg_off[b];
+        a.blob_iters = blob_iters + b;
+    }
+    sr_grid = sms;
+    sr_ok = on_chip = true;
+    return FFEA_GPU_OK;
 }
 
 // the force phase's launch shapes; the step graph is captured again
@@ -401,7 +548,7 @@ int ffea_gpu_batch::time_forces(int reps, double &ms) {
 
 // one step of every blob, as launched into `stream` (captured by capture())
 int ffea_gpu_batch::record_step() {
-    CK(BatchLaunch::schedule(desc, blob_iters, nblobs, ncta, cta_blob, st, stream));
+    if (!on_chip) CK(BatchLaunch::schedule(desc, blob_iters, nblobs, ncta, cta_blob, st, stream));
     int rc = launch_forces();
     if (!rc) rc = launch_gather();
     if (rc) return rc;
@@ -501,6 +648,29 @@ int ffea_gpu_batch::launch_gather() {
 
 // barrier reset + the persistent CG over every blob
 int ffea_gpu_batch::launch_cg_only() {
+    if (on_chip) {
+        CK(cudaMemsetAsync(sr_msg, 0, sr_msg_bytes, stream));
+        SrBatchArgs a{};
+        CgArgs<float> &ca = a.common;
+        ca.block3 = ca.check_last = 1;
+        ca.slice_ptr = slice_ptr; ca.rowlen = rowlen; ca.bcol = bcol;
+        ca.val = val; ca.dinv = dinv; ca.diag = diag;
+        ca.x = x; ca.r = r;
+        ca.px = px; ca.py = py; ca.pz = pz;
+        ca.mstride = h.N;
+        ca.st = st;
+        ca.imax = p.max_iterations_cg;
+        ca.eps2 = p.epsilon2;
+        ca.cheb_cost = 0.5f;
+        ca.halo_list = sr_halo_list;
+        ca.lcol = sr_lcol;
+        ca.msg = sr_msg;
+        a.blobs = sr_args;
+        a.task_ptr = sr_task_ptr;
+        a.tasks = sr_tasks;
+        CK(BatchLaunch::sr(a, sr_grid, sr_smem, stream));
+        return FFEA_GPU_OK;
+    }
     CK(cudaMemsetAsync(gbs, 0, (size_t)nblobs * sizeof(GridBarrier), stream));
     BatchCgArgs ca{};
     ca.nblobs = nblobs;
@@ -927,9 +1097,9 @@ int ffea_gpu_batch_cg_iterations(ffea_gpu_batch *bt, int *last_per_blob, long lo
 
 int ffea_gpu_batch_config(ffea_gpu_batch *bt, int *cg_threads, int *threads_per_row, int *ctas) {
     if (!bt) return FFEA_GPU_EINPUT;
-    if (cg_threads) *cg_threads = bt->cg_threads;
-    if (threads_per_row) *threads_per_row = bt->tpn;
-    if (ctas) *ctas = bt->ncta;
+    if (cg_threads) *cg_threads = bt->on_chip ? ffea::SR_REG_THREADS : bt->cg_threads;
+    if (threads_per_row) *threads_per_row = bt->on_chip ? bt->sr_tpn : bt->tpn;
+    if (ctas) *ctas = bt->on_chip ? bt->sr_grid : bt->ncta;
     return FFEA_GPU_OK;
 }
 
@@ -963,6 +1133,7 @@ int ffea_gpu_batch_tune(ffea_gpu_batch *bt, int solves, double *best_ms) {
     // the force phase's launch shapes, one at a time (coordinate search): elements per block, then the
     // assembly's threads per block and slot split, then the gather's threads per block
     const int keep_threads = bt->cg_threads, keep_tpn = bt->tpn;
+    const bool keep_chip = bt->on_chip;
     const int keep_em = bt->me.threads, keep_at = bt->asm_threads, keep_as = bt->asm_split,
               keep_gt = bt->gather_threads;
     auto restore = [&]() {
@@ -1017,6 +1188,10 @@ int ffea_gpu_batch_tune(ffea_gpu_batch *bt, int solves, double *best_ms) {
         if (rc) {
             restore();
             bt->configure(keep_threads, keep_tpn);
+            if (keep_chip) {
+                bt->on_chip = true;
+                bt->capture();
+            }
             return rc;
         }
     }
@@ -1030,50 +1205,66 @@ int ffea_gpu_batch_tune(ffea_gpu_batch *bt, int solves, double *best_ms) {
     };
     int best_t = keep_threads, best_p = keep_tpn;
     double best = 1e300;
+    // mean time of `solves` solves by the configuration set, after `warm` untimed ones
+    auto time_solves = [&](int warm, double &mean) -> int {
+        double tot = 0.0;
+        for (int k = -warm; k < solves; ++k) {
+            int r2 = prepare();
+            if (r2) return r2;
+            cudaError_t e = cudaEventRecord(bt->ev0, bt->stream);
+            if (e == cudaSuccess && (r2 = bt->launch_cg_only())) return r2;
+            if (e == cudaSuccess) e = cudaEventRecord(bt->ev1, bt->stream);
+            if (e == cudaSuccess) e = cudaEventSynchronize(bt->ev1);
+            float ms = 0.f;
+            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, bt->ev0, bt->ev1);
+            if (e != cudaSuccess) return cuda_fail(e, "batch tune");
+            if (k >= 0) tot += ms;
+        }
+        DevStatus s{};
+        int r2 = bt->read_status(s);
+        if (!r2) r2 = ffea_gpu_batch::status_code(s);
+        mean = tot / solves;
+        return r2;
+    };
+    bool best_chip = false;
+    if (bt->sr_ok) {
+        // the solve on chip: its first solve estimates the preconditioner's interval, its second is the trial
+        bt->on_chip = true;
+        rc = time_solves(2, best);
+        best_chip = true;
+        bt->on_chip = false;
+    }
     for (int t : {128, 256, 512, 1024}) {
         const int grid = BatchLaunch::cg_max_grid(bt->device, t);
+        if (rc) break;
         if (grid < bt->nblobs || grid > bt->ncta_cap) continue;
         for (int p : {1, 2, 4, 8}) {
             bt->cg_threads = t;
             bt->tpn = p;
             bt->ncta = grid;
-            double tot = 0.0;
-            for (int k = 0; k <= solves && rc == FFEA_GPU_OK; ++k) {
-                if ((rc = prepare())) break;
-                cudaError_t e = cudaEventRecord(bt->ev0, bt->stream);
-                if (e == cudaSuccess) rc = bt->launch_cg_only();
-                if (rc) break;
-                if (e == cudaSuccess) e = cudaEventRecord(bt->ev1, bt->stream);
-                if (e == cudaSuccess) e = cudaEventSynchronize(bt->ev1);
-                float ms = 0.f;
-                if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, bt->ev0, bt->ev1);
-                if (e != cudaSuccess) rc = cuda_fail(e, "batch tune");
-                if (k > 0) tot += ms;  // the first solve of each configuration is a warm-up
-            }
-            if (rc) break;
-            DevStatus s{};
-            if ((rc = bt->read_status(s))) break;
-            if ((rc = ffea_gpu_batch::status_code(s))) break;
-            if (tot / solves < best) {
-                best = tot / solves;
+            double mean = 0.0;
+            if ((rc = time_solves(1, mean))) break;  // the first solve of each configuration is a warm-up
+            if (mean < best) {
+                best = mean;
                 best_t = t;
                 best_p = p;
+                best_chip = false;
             }
         }
-        if (rc) break;
     }
     // the tuning solves are not steps: put the status counters back
     if (!rc) {
         CK(cudaMemcpyAsync(bt->st, &s0, sizeof(DevStatus), cudaMemcpyHostToDevice, bt->stream));
         CK(cudaStreamSynchronize(bt->stream));
     }
-    if (rc) {
-        restore();
-        bt->configure(keep_threads, keep_tpn);
-        return rc;
-    }
-    if (best_ms) *best_ms = best;
-    return bt->configure(best_t, best_p);
+    const bool chip = rc ? keep_chip : best_chip;
+    if (rc) restore();
+    else if (best_ms) *best_ms = best;
+    const int rc2 = rc ? bt->configure(keep_threads, keep_tpn) : bt->configure(best_t, best_p);
+    if (rc2 || !chip) return rc ? rc : rc2;
+    bt->on_chip = true;
+    const int rc3 = bt->capture();
+    return rc ? rc : rc3;
 }
 
 }  // extern "C"

@@ -37,4 +37,25 @@ struct BatchCgArgs {
     unsigned long long limit_ns;
 };
 
+// The batch's solve on chip (sr_batch_kernel): per blob its solve's arguments, and per block of the launch the blobs it
+// works for, task_ptr[c] .. task_ptr[c + 1), in one order common to all blocks
+struct SrTask {
+    int blob, rank, nblocks;
+};
+// what differs from blob to blob in the solve's arguments (the fields of CgArgs by the same names)
+struct SrBlob {
+    int N, row0, npb, tpn, kc, nhalo, poly, nmodes, stride, pad;
+    const int *halo_ptr;
+    Msg *rmsg;
+    double *cheb;
+    int *blob_iters;
+    double xc[3], modes[36];
+};
+struct SrBatchArgs {
+    CgArgs<float> common;
+    const SrBlob *blobs;
+    const int *task_ptr;
+    const SrTask *tasks;
+};
+
 }  // namespace ffea

@@ -337,52 +337,6 @@ struct BlobImpl final : ffea_gpu_blob {
         return FFEA_GPU_OK;
     }
 
-    // The rows of other blocks that each block's rows reach through the pattern, and every slot's column as an index
-    // into the block's staged vector (own rows first, then, from npb, the halo in ascending row order). The pattern
-    // is symmetric (an element couples each pair of its unpinned nodes both ways; a pinned row keeps only its diagonal
-    // and no row has its column), so a block reads from exactly the blocks that read from it, which the exchange's
-    // buffer reuse relies on.
-    struct Halo {
-        std::vector<int> ptr, list;
-        std::vector<unsigned short> lcol;
-        int largest = 0;
-    };
-    void build_halo(int npb, int grid, Halo &o) const {
-        const int N = h.N;
-        o.ptr.assign(grid + 1, 0);
-        o.list.clear();
-        o.lcol.assign(h.nslots, 0);
-        std::vector<int> at(N, -1), got;
-        for (int b = 0; b < grid; ++b) {
-            const int a0 = std::min(N, b * npb), a1 = std::min(N, (b + 1) * npb);
-            got.clear();
-            for (int a = a0; a < a1; ++a) {
-                const int s0 = h.slice_ptr[a >> 5], ln = a & 31;
-                for (int k = 0; k < h.rowlen[a]; ++k) {
-                    const int c = h.bcol[s0 + 32 * k + ln];
-                    if ((c < a0 || c >= a1) && at[c] < 0) {
-                        at[c] = 0;
-                        got.push_back(c);
-                    }
-                }
-            }
-            std::sort(got.begin(), got.end());
-            for (size_t i = 0; i < got.size(); ++i) at[got[i]] = (int)i;
-            for (int a = a0; a < a1; ++a) {
-                const int s0 = h.slice_ptr[a >> 5], ln = a & 31;
-                for (int k = 0; k < h.rowlen[a]; ++k) {
-                    const int c = h.bcol[s0 + 32 * k + ln];
-                    o.lcol[s0 + 32 * k + ln] = (unsigned short)((c >= a0 && c < a1) ? c - a0 : npb + at[c]);
-                }
-            }
-            for (int c : got) at[c] = -1;
-            o.list.insert(o.list.end(), got.begin(), got.end());
-            o.ptr[b + 1] = (int)o.list.size();
-            o.largest = std::max(o.largest, (int)got.size());
-        }
-        if (o.list.empty()) o.list.push_back(0);
-    }
-
     // The FP64 CG's launch: rows per block, units and lanes per unit of cg_own_unit_kernel, by the FP64 instructions on
     // the fullest sub-partition of a block (see there); left alone (cg_unit = 0) when no form holds the blob's rows.
     int pick_units(int maxg) {
@@ -408,8 +362,8 @@ struct BlobImpl final : ffea_gpu_blob {
                 if (!best || c < best) { best = c; best_nc = nc; best_tpu = t; }
             }
         if (!best) return FFEA_GPU_OK;
-        Halo hl;
-        build_halo(npb, grid, hl);
+        host::Halo hl;
+        host::build_halo(h, 0, N, npb, grid, hl);
         const int vals = b3 ? 9 : 1;
         const size_t limit = (size_t)std::max(Launch<R>::cg_unit_smem_limit(device, best_nc, b3), 0);
         const size_t need = own_unit_smem(npb, hl.largest, best_nc, vals, 0);
@@ -592,8 +546,8 @@ struct BlobImpl final : ffea_gpu_blob {
             if (sr_able) {
                 // the polynomial preconditioner's two extra vectors per row must fit as well; else Jacobi
                 const int poly = p.cg_poly == 0 ? FFEA_GPU_CG_POLY_DEFAULT : std::max(p.cg_poly, 0);
-                Halo hl;
-                build_halo(npb, cg_grid, hl);
+                host::Halo hl;
+                host::build_halo(h, 0, N, npb, cg_grid, hl);
                 const size_t limit = (size_t)std::max(Launch<R>::cg_sr_smem_limit(device), 0);
                 for (int deg : {poly, 0}) {
                     if ((long long)npb * tpn <= cg_block && npb + hl.largest < 65536 &&
@@ -672,7 +626,7 @@ struct BlobImpl final : ffea_gpu_blob {
         CK(mem.alloc(&history, (size_t)hist_cap));
         {
             const size_t head = 256, rows = cg_sr ? 2 * (size_t)N : cg_unit ? 6 * (size_t)N : 0,
-                         red = (cg_sr ? 2 * (size_t)MIXED_SR_NP : cg_unit ? 4 : 0) * MSG_COPIES * partial_stride;
+                         red = (cg_sr || cg_unit ? 2 * (size_t)MSG_VALUES : 0) * MSG_COPIES * partial_stride;
             comm_bytes = head + (rows + red) * sizeof(Msg);
             CK(mem.alloc(&comm, comm_bytes));
             phase_ns = reinterpret_cast<unsigned long long *>(comm);
@@ -792,7 +746,7 @@ struct BlobImpl final : ffea_gpu_blob {
     int launch_cg(const double *init, int n_init) {
         const bool nomass = p.solver == FFEA_GPU_NOMASS_CG;
         CgArgs<R> ca{};
-        ca.N = h.N;
+        ca.N = ca.mstride = h.N;
         ca.block3 = nomass;
         ca.check_last = nomass;
         ca.slice_ptr = slice_ptr; ca.rowlen = rowlen; ca.bcol = bcol;

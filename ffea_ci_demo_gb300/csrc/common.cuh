@@ -201,6 +201,7 @@ __device__ __forceinline__ bool msg_wait_all(const Msg *const (&p)[K], const boo
 // (one per lane of the publishing warp), block b reading copy b mod MSG_COPIES, or the polls of all 152 SMs on the
 // same twenty lines hold up the messages themselves.
 constexpr int MSG_COPIES = 16;
+constexpr int MSG_VALUES = 16;  // values a reduction's buffer holds
 
 // add(message of block b) for every block b = lane, lane + 32, ... < nb, in that order, once each carries `tag`: one
 // message a lane for up to 32 blocks, else K at a time. False on a timeout.

@@ -84,6 +84,9 @@ struct BatchLaunch {
     static cudaError_t cg(const BatchCgArgs &a, int grid, int threads, cudaStream_t s);
     // CTAs of `threads` threads that can be resident at once on `device`
     static int cg_max_grid(int device, int threads);
+    // cooperative launch of sr_batch_kernel on `grid` blocks; the dynamic shared memory a block may take and the SMs
+    static cudaError_t sr(const SrBatchArgs &a, int grid, size_t smem, cudaStream_t s);
+    static size_t sr_smem_limit(int device, int &sms);
     static cudaError_t finish(uint32_t *rng_states, const MrgJump *step_jumps, int nblobs, DevStatus *st,
                               cudaStream_t s);
     // every blob's strain energy (batch_strain_kernel) into out[nblobs]

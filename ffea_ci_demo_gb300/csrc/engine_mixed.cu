@@ -109,6 +109,39 @@ cudaError_t BatchLaunch::cg(const BatchCgArgs &a, int grid, int threads, cudaStr
     return e;
 }
 
+cudaError_t BatchLaunch::sr(const SrBatchArgs &a, int grid, size_t smem, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(SR_REG_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, sr_batch_kernel, a);
+    count_launch();
+    return e;
+}
+
+size_t BatchLaunch::sr_smem_limit(int device, int &sms) {
+    int optin = 0, per_sm = 0;
+    cudaFuncAttributes fa{};
+    sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess ||
+        cudaFuncGetAttributes(&fa, sr_batch_kernel) != cudaSuccess)
+        return 0;
+    const int dyn = optin - (int)fa.sharedSizeBytes;
+    if (dyn <= 0 ||
+        cudaFuncSetAttribute(sr_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sr_batch_kernel, SR_REG_THREADS, dyn) != cudaSuccess ||
+        per_sm < 1)
+        return 0;
+    return (size_t)dyn;
+}
+
 int BatchLaunch::cg_max_grid(int device, int threads) {
     int nsm = 0, per_sm = 0;
     cudaFuncAttributes fa{};

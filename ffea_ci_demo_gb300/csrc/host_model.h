@@ -489,6 +489,53 @@ inline int build_model(const ffea_gpu_mesh *mesh, const ffea_gpu_params *p, Host
     return FFEA_GPU_OK;
 }
 
+// Rows [row0, row0 + nrows) split into `grid` blocks of npb rows: the rows of other blocks that each block's rows reach
+// through the pattern (appended to list, in ascending row order; ptr[b] .. ptr[b + 1]), and every slot's column as an
+// index into its block's staged vector (own rows first, then, from npb, the halo; written to lcol). The pattern is
+// symmetric (an element couples each pair of its unpinned nodes both ways; a pinned row keeps only its diagonal and no
+// row has its column), so a block reads from exactly the blocks that read from it, which the exchange's buffer reuse
+// relies on.
+struct Halo {
+    std::vector<int> ptr, list;
+    std::vector<unsigned short> lcol;
+    int largest = 0;  // of the blocks added last
+};
+
+inline void build_halo(const HostModel &h, int row0, int nrows, int npb, int grid, Halo &o) {
+    const int row1 = row0 + nrows;
+    if (o.ptr.empty()) o.ptr.push_back(0);
+    if (o.lcol.empty()) o.lcol.assign(std::max<long long>(h.nslots, 1), 0);
+    o.largest = 0;
+    std::vector<int> at(nrows, -1), got;
+    for (int b = 0; b < grid; ++b) {
+        const int a0 = std::min(row1, row0 + b * npb), a1 = std::min(row1, row0 + (b + 1) * npb);
+        got.clear();
+        for (int a = a0; a < a1; ++a) {
+            const int s0 = h.slice_ptr[a >> 5], ln = a & 31;
+            for (int k = 0; k < h.rowlen[a]; ++k) {
+                const int c = h.bcol[s0 + 32 * k + ln];
+                if ((c < a0 || c >= a1) && at[c - row0] < 0) {
+                    at[c - row0] = 0;
+                    got.push_back(c);
+                }
+            }
+        }
+        std::sort(got.begin(), got.end());
+        for (size_t i = 0; i < got.size(); ++i) at[got[i] - row0] = (int)i;
+        for (int a = a0; a < a1; ++a) {
+            const int s0 = h.slice_ptr[a >> 5], ln = a & 31;
+            for (int k = 0; k < h.rowlen[a]; ++k) {
+                const int c = h.bcol[s0 + 32 * k + ln];
+                o.lcol[s0 + 32 * k + ln] = (unsigned short)((c >= a0 && c < a1) ? c - a0 : npb + at[c - row0]);
+            }
+        }
+        for (int c : got) at[c - row0] = -1;
+        o.list.insert(o.list.end(), got.begin(), got.end());
+        o.ptr.push_back((int)o.list.size());
+        o.largest = std::max(o.largest, (int)got.size());
+    }
+}
+
 template <class R>
 std::vector<R> cast_vec(const std::vector<double> &v) {
     return std::vector<R>(v.begin(), v.end());

@@ -972,12 +972,18 @@ struct CgArgs {
     // owned-rows kernels that stage the vector their SpMV reads: the rows of other blocks that block b's rows
     // reach (halo_list[halo_ptr[b] .. halo_ptr[b + 1])), every matrix slot's column as an index into the block's
     // staged vector (own rows at 0 .. npb - 1, its halo from npb on), the rows' messages (two buffers of N) and
-    // the blocks' partial sums as messages (two buffers, MSG_COPIES rows of `stride` per value)
+    // the blocks' partial sums as messages (two buffers of MSG_VALUES values, MSG_COPIES rows of `stride` each)
     const int *halo_ptr, *halo_list;
     const unsigned short *lcol;
     Msg *msg, *rmsg;
     int nhalo;            // the largest halo of any block
     int unit;             // FP64: components per unit of cg_own_unit_kernel (1 or 3; 0: another kernel)
+    // the rows solved, [row0, row0 + N), and the stride of the two message buffers (a batch solves one blob's rows of the
+    // concatenation; one blob: 0 and N)
+    int row0, mstride;
+    const double *px, *py, *pz;  // a batch's solve forms its blob's node offsets and moments itself, about xc
+    double xc[3];
+    int *blob_iters;      // and leaves its iteration count here (see SrBlob)
     int reg;              // cg_mixed_sr_kernel: blocks of each lane in registers (its form: 0, 4 or 6)
 };
 
@@ -1103,19 +1109,19 @@ constexpr int CG_PHASES = 10;  // the phase timers' slots (FFEA_GPU_CG_PHASES of
 // the previous mark is added to a shared-memory slot k during the solve, and the slots, as nanoseconds by the solve's
 // own ratio of global timer to SM clock, are added to phase_ns when it ends. (A mark on the global timer costs
 // 0.12 us, 2.3 us per iteration of the 6^3-cell solve; one on the clock register hides behind the barriers.)
-#define FFEA_TIMED_BLOCK (blockIdx.x == gridDim.x / 2 && threadIdx.x == 0)
-#define FFEA_PHASES_BEGIN(t_prev)                                                  \
+#define FFEA_TIMED_BLOCK(g) ((g).phase_ns && blockIdx.x == gridDim.x / 2 && threadIdx.x == 0)
+#define FFEA_PHASES_BEGIN(g, t_prev)                                               \
     __shared__ long long s_phase_[CG_PHASES];                                      \
     __shared__ unsigned long long s_gt0_;                                          \
     __shared__ long long s_ck0_, t_prev; /* in shared memory: no registers */     \
-    if (FFEA_TIMED_BLOCK) {                                                        \
+    if (FFEA_TIMED_BLOCK(g)) {                                                        \
         for (int k_ = 0; k_ < CG_PHASES; ++k_) s_phase_[k_] = 0ll;                 \
         s_gt0_ = globaltimer_ns();                                                 \
         t_prev = s_ck0_ = clock64();                                               \
     }
 #define FFEA_MARK(g, t_prev, k)                                                   \
     do {                                                                          \
-        if (FFEA_TIMED_BLOCK) {                                                   \
+        if (FFEA_TIMED_BLOCK(g)) {                                                   \
             const long long t_now_ = clock64();                                   \
             s_phase_[k] += t_now_ - (t_prev);                                     \
             (t_prev) = t_now_;                                                    \
@@ -1123,7 +1129,7 @@ constexpr int CG_PHASES = 10;  // the phase timers' slots (FFEA_GPU_CG_PHASES of
     } while (0)
 #define FFEA_PHASES_END(g)                                                        \
     do {                                                                          \
-        if (FFEA_TIMED_BLOCK) {                                                   \
+        if (FFEA_TIMED_BLOCK(g)) {                                                   \
             const double c_ = (double)max(clock64() - s_ck0_, 1ll);               \
             const double n_ = (double)(globaltimer_ns() - s_gt0_);                \
             for (int k_ = 0; k_ < CG_PHASES; ++k_)                                \
@@ -1143,7 +1149,7 @@ __global__ void __launch_bounds__(1024, 1) cg_kernel(const __grid_constant__ CgA
     __shared__ int s_conv;
     DevStatus *st = g.st;
     if (st->abort) return;
-    FFEA_PHASES_BEGIN(tm);
+    FFEA_PHASES_BEGIN(g, tm);
     R *p = g.pbuf0;
     // p = z = D^{-1} r  (conjugate_gradient_residual_assume_x_zero, src/NoMassCGSolver.cpp:196-220)
     FFEA_NODE_LOOP(g, a) {
@@ -1417,7 +1423,7 @@ __device__ __forceinline__ bool grid_reduce_units(const A &g, double *s, int U, 
     const int lane = threadIdx.x & 31, wid = warp_index(), nb = gridDim.x;
     double t = block_sum_units<NV>(s, U, wid);
     int bad = 0;
-    Msg *const rows = g.rmsg + ((size_t)(tag & 1u) * 2 + wid) * MSG_COPIES * g.stride;
+    Msg *const rows = g.rmsg + ((size_t)(tag & 1u) * MSG_VALUES + wid) * MSG_COPIES * g.stride;
     const Msg *const row = rows + (size_t)(blockIdx.x % MSG_COPIES) * g.stride;
     if (wid < NV && nb > 1 && lane < MSG_COPIES)
         msg_put(rows + (size_t)lane * g.stride + blockIdx.x, (uint32_t)__double2loint(t), (uint32_t)__double2hiint(t), 0u,
@@ -1447,7 +1453,7 @@ __global__ void __launch_bounds__(OWN_UNIT_THREADS, 1) cg_own_unit_kernel(const 
     __shared__ int s_conv;
     DevStatus *st = g.st;
     if (st->abort) return;
-    FFEA_PHASES_BEGIN(tm);
+    FFEA_PHASES_BEGIN(g, tm);
     const int npb = g.npb, a0 = blockIdx.x * npb, nloc = max(0, min(npb, g.N - a0)), N = g.N;
     const int S = npb + g.nhalo, U = own_unit_count(npb, NC);
     double *const zp = snd_u, *const red = zp + 3 * S, *const cv = red + 2 * U;
@@ -1724,7 +1730,7 @@ __global__ void __launch_bounds__(1024, 1) cg_own_kernel(const __grid_constant__
     __shared__ int s_conv;
     DevStatus *st = g.st;
     if (st->abort) return;
-    FFEA_PHASES_BEGIN(tm);
+    FFEA_PHASES_BEGIN(g, tm);
     const int npb = g.npb, a0 = blockIdx.x * npb;
     const int nloc = max(0, min(npb, g.N - a0));
     double *sx = snd, *sr = snd + 3 * npb, *sq = snd + 6 * npb, *sp = snd + 9 * npb;

@@ -10,8 +10,9 @@
 // substream per blob) and the CG: every blob has its own right-hand side,
 // rigid modes, step lengths and stopping test.
 //
-// cg_batch_kernel is one persistent cooperative launch for the whole batch.
-// The scheduler (schedule_kernel, run at the head of every step) splits the
+// The CG is one persistent cooperative launch for the whole batch:
+// sr_batch_kernel wherever the host finds room for every blob on chip, else
+// cg_batch_kernel. For that one the scheduler (schedule_kernel, run at the head of every step) splits the
 // grid's CTAs into one group per blob, sized in proportion to the blob's
 // rows x CG iterations of the previous step, so that all groups finish
 // together. Each group runs the mixed-precision deflated Jacobi-PCG of
@@ -247,6 +248,31 @@ __global__ void __launch_bounds__(BATCH_MAX_THREADS) cg_batch_kernel(const __gri
             atomicMax(&st->last_iters, it);
             atomicAdd(reinterpret_cast<unsigned long long *>(&st->total_iters), (unsigned long long)it);
         }
+    }
+}
+
+// The batch's solve on chip. Each block of the launch (one per SM) works through its tasks: one blob's solve together
+// with that blob's other blocks (sr_solve: matrix in registers and shared memory, rows and sums as tagged messages,
+// Chebyshev preconditioner for blobs of more than one block). Every block takes its tasks in the same global order of
+// blobs, so the first blob not yet finished always has all its blocks, and none waits for ever.
+// cg_batch_kernel streams every blob's matrix from HBM each iteration, all blobs at once (0.64 of the copy rate, which
+// bounds it); here a blob's matrix is read once per solve and what bounds the solve is its exchanges' latency, so the
+// host gives a block as many rows as the chip holds (plan_solve). 32 blobs of 8 to 32 cells a side, 219,234 nodes:
+// 18.0 -> 6.0 ms per solve (15.8 by the best of cg_batch_kernel's shapes); 8 such blobs 10.1 -> 2.2, 64 34.4 -> 12.7,
+// 40 blobs of 2 to 8 cells 1.71 -> 0.63, 200 of 3 to 6 cells 1.35 -> 0.47.
+__global__ void __launch_bounds__(SR_REG_THREADS, 1) sr_batch_kernel(const __grid_constant__ SrBatchArgs b) {
+    __shared__ SrBlob s_bl;
+    if (b.common.st->abort) return;
+    const int t1 = b.task_ptr[blockIdx.x + 1];
+    for (int t = b.task_ptr[blockIdx.x]; t < t1; ++t) {
+        const SrTask task = b.tasks[t];
+        __syncthreads();  // the previous solve's reads of its arguments have ended
+        static_assert(sizeof(SrBlob) % 4 == 0, "copied by words");
+        const int *src = reinterpret_cast<const int *>(b.blobs + task.blob);
+        for (int i = threadIdx.x; i < (int)(sizeof(SrBlob) / 4); i += blockDim.x)
+            reinterpret_cast<int *>(&s_bl)[i] = src[i];
+        __syncthreads();
+        if (!sr_solve<6, true>(b.common, s_bl, task.rank, task.nblocks)) return;
     }
 }
 

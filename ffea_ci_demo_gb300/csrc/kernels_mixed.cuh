@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_kernel(const __grid_constant
     DevStatus *st = g.st;
     if (st->abort) return;
     const bool defl = g.nmodes > 0;
-    FFEA_PHASES_BEGIN(tm);
+    FFEA_PHASES_BEGIN(g, tm);
     float2 *partials = reinterpret_cast<float2 *>(g.partials);
     // set-up: G = Z^T D Z from the moments M, projected right-hand side
     grid_sum_df<MIXED_GATHER_NP>(reinterpret_cast<const float2 *>(g.init_partials), g.init_stride, g.n_init, s_sc);
@@ -661,7 +661,7 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_own_kernel(const __grid_cons
     DevStatus *st = g.st;
     if (st->abort) return;
     const bool defl = g.nmodes > 0;
-    FFEA_PHASES_BEGIN(tm);
+    FFEA_PHASES_BEGIN(g, tm);
     float2 *partials = reinterpret_cast<float2 *>(g.partials);
     const int npb = g.npb, a0 = blockIdx.x * npb;
     const int nloc = max(0, min(npb, g.N - a0));
@@ -858,7 +858,7 @@ __device__ __forceinline__ bool halo_exchange(const A &g, Staged &z, const int (
     z.row = -1;
     int bad = 0;
     if (nh > 0) {
-        const Msg *m = g.msg + (size_t)(tag & 1u) * g.N;
+        const Msg *m = g.msg + (size_t)(tag & 1u) * g.mstride;
         float4 *zh = z.v + z.npb;
         for (int h = threadIdx.x, t = 0; h < nh; h += 2 * (int)blockDim.x, ++t) {
             const int h2 = h + (int)blockDim.x;
@@ -905,14 +905,14 @@ __device__ __forceinline__ float warp_sum_spread(const float (&v)[NV], int &inde
     return t;
 }
 
-// The grid's sums of NV per-thread FP32 values, as double-float pairs in s_out for the whole block: FP32 within each
+// The sums over nb blocks (this one of rank `rank`) of NV per-thread FP32 values, as double-float pairs in s_out for the whole block: FP32 within each
 // warp, double-float over the block's warps, published as one message per value, and every block adds the blocks'
 // messages in the same order. `tag` counts the launch's reductions from 1. The caller must pass a __syncthreads()
 // before smem (NV x 32 floats) is written again.
 template <int NV, int K, class A>
-__device__ __forceinline__ bool grid_reduce_msg(const A &g, const float (&v)[NV], float *smem, unsigned int tag,
-                                                df32 *s_out, DevStatus *st) {
-    const int lane = threadIdx.x & 31, wid = warp_index(), nw = blockDim.x >> 5, nb = gridDim.x;
+__device__ __forceinline__ bool grid_reduce_msg(const A &g, int rank, int nb, const float (&v)[NV], float *smem,
+                                                unsigned int tag, df32 *s_out, DevStatus *st) {
+    const int lane = threadIdx.x & 31, wid = warp_index(), nw = blockDim.x >> 5;
     int idx;
     const float ws = warp_sum_spread<NV>(v, idx);
     if (idx >= 0) smem[idx * 32 + wid] = ws;
@@ -922,10 +922,10 @@ __device__ __forceinline__ bool grid_reduce_msg(const A &g, const float (&v)[NV]
         df32 t = {lane < nw ? smem[i * 32 + lane] : 0.f, 0.f};
         t = warp_sum_df(t);
         if (nb > 1) {
-            Msg *const rows = g.rmsg + ((size_t)(tag & 1u) * NV + i) * MSG_COPIES * g.stride;
-            const Msg *const row = rows + (size_t)(blockIdx.x % MSG_COPIES) * g.stride;
+            Msg *const rows = g.rmsg + ((size_t)(tag & 1u) * MSG_VALUES + i) * MSG_COPIES * g.stride;
+            const Msg *const row = rows + (size_t)(rank % MSG_COPIES) * g.stride;
             if (lane < MSG_COPIES)
-                msg_put(rows + (size_t)lane * g.stride + blockIdx.x, __float_as_uint(t.hi), __float_as_uint(t.lo), 0u, tag);
+                msg_put(rows + (size_t)lane * g.stride + rank, __float_as_uint(t.hi), __float_as_uint(t.lo), 0u, tag);
             t = df32{0.f, 0.f};
             if (!msg_collect<K>(row, nb, tag, st, [&](const Msg &m) {
                     t = df_add(t, df32{__uint_as_float(m.x), __uint_as_float(m.y)});
@@ -975,11 +975,10 @@ struct RowRegs {
 // memory (two per trip where registers allow); the products are summed in block order either way, so the row does not depend on where its
 // blocks are.
 template <int RB, class A>
-__device__ __forceinline__ void spmv_row_w(const A &g, const SrCache &c, const RowRegs<RB> &rr, const float4 *zs,
+__device__ __forceinline__ void spmv_row_w(const A &g, int tpn, const SrCache &c, const RowRegs<RB> &rr, const float4 *zs,
                                            int base, int len, int lane, int l, int sub, float &w0, float &w1,
                                            float &w2) {
     w0 = 0.f; w1 = 0.f; w2 = 0.f;
-    const int tpn = g.tpn;
     if (len > 0) {
         int k = sub;
         if constexpr (RB > 0) {
@@ -1128,14 +1127,56 @@ static __device__ __noinline__ double lanczos_lambda_max(const double *al, const
 // cluster of the others (unscaled they sit at P_d(0), 15.7 for d = 4 on the 40^3 cube, which then needed 132
 // iterations a step instead of 110). The scale changes the shifted operator only on the rigid modes, where the
 // projected right-hand side has no component, so the solution is the same: the one with Z^T D x = 0.
-template <class R, int RB>
-__global__ void __launch_bounds__(SrForm<RB>::THREADS, 1) cg_mixed_sr_kernel(const __grid_constant__ CgArgs<R> g) {
-    static_assert(sizeof(R) == sizeof(float), "the single-reduction CG is the mixed path's");
+// A batch's set-up moments of the blob's rows (sums 1 and 2 of the solve), in s_sc for the whole block; a call of its
+// own, so that its 28 values share no registers with the solve.
+template <int K, class A, class B>
+__device__ __noinline__ bool sr_moments(const A &g, const B &bl, int a0, int nloc, int rank, int nb, float *smemf,
+                                        df32 *s_scf, double *s_sc) {
+    // f.f, S1_f, S2_f and M = sum Phi^T D Phi (cf. gather_mixed_kernel), half of them per sum
+    static_assert(MIXED_GATHER_NP == 28, "two sums of 14");
+    float m[MIXED_GATHER_NP];
+#pragma unroll
+    for (int i = 0; i < MIXED_GATHER_NP; ++i) m[i] = 0.f;
+    for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
+        const int a = a0 + l;
+        const float4 d = make_float4((float)(g.px[a] - bl.xc[0]), (float)(g.py[a] - bl.xc[1]),
+                                     (float)(g.pz[a] - bl.xc[2]), 0.f);
+        const float F0 = g.r[4 * a], F1 = g.r[4 * a + 1], F2 = g.r[4 * a + 2];
+        m[0] += F0 * F0 + F1 * F1 + F2 * F2;
+        m[1] += F0; m[2] += F1; m[3] += F2;
+        m[4] += d.y * F2 - d.z * F1; m[5] += d.z * F0 - d.x * F2; m[6] += d.x * F1 - d.y * F0;
+        float phi[6][3];
+        phi_cols(d.x, d.y, d.z, phi);
+        const float D[3] = {g.diag[4 * a], g.diag[4 * a + 1], g.diag[4 * a + 2]};
+        int k = 7;
+#pragma unroll
+        for (int i = 0; i < 6; ++i)
+#pragma unroll
+            for (int j = i; j < 6; ++j, ++k)
+                m[k] += phi[i][0] * D[0] * phi[j][0] + phi[i][1] * D[1] * phi[j][1] + phi[i][2] * D[2] * phi[j][2];
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        float v[14];
+#pragma unroll
+        for (int i = 0; i < 14; ++i) v[i] = m[14 * half + i];
+        if (!grid_reduce_msg<14, K>(bl, rank, nb, v, smemf, (unsigned)half + 1u, s_scf, g.st)) return false;
+        if (threadIdx.x < 14) s_sc[14 * half + threadIdx.x] = df_double(s_scf[threadIdx.x]);
+        __syncthreads();
+    }
+    return true;
+}
+
+// One solve by nb blocks, this one of rank `rank`, with the launch's arguments g and the blob's own bl: the whole grid for a blob (cg_mixed_sr_kernel), or one blob's
+// blocks of a batch (BATCH: kernels_batch.cuh), which also forms the moments that the single blob's gather leaves in
+// g.init_partials. Returns false on a timeout.
+template <int RB, bool BATCH, class A, class B>
+__device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int nb) {
     extern __shared__ __align__(16) float4 sn_raw[];
-    __shared__ float smemf[MIXED_SR_NP * 32];
+    __shared__ float smemf[14 * 32];
     __shared__ double s_sc[MIXED_GATHER_NP];
     __shared__ double s_A6[36];
-    __shared__ df32 s_scf[MIXED_SR_NP];  // the iteration's sums
+    __shared__ df32 s_scf[14];  // the iteration's sums
     __shared__ df32 s_A6f[36];        // A6 times the shift's scale
     __shared__ df32 s_mp[6];          // moments of D p for the current direction
     __shared__ df32 s_pq;             // p.q~ of the previous iteration
@@ -1145,11 +1186,10 @@ __global__ void __launch_bounds__(SrForm<RB>::THREADS, 1) cg_mixed_sr_kernel(con
     __shared__ double s_shift;        // scale of the rigid-mode shift: 1 / P_d(0) with the polynomial, else 1
     __shared__ int s_conv, s_stop;
     DevStatus *st = g.st;
-    if (st->abort) return;
-    const bool defl = g.nmodes > 0;
-    FFEA_PHASES_BEGIN(tm);
-    const int npb = g.npb, a0 = blockIdx.x * npb;
-    const int nloc = max(0, min(npb, g.N - a0));
+    const bool defl = bl.nmodes > 0;
+    FFEA_PHASES_BEGIN(g, tm);
+    const int npb = bl.npb, a0 = bl.row0 + rank * npb;
+    const int nloc = max(0, min(npb, bl.N - rank * npb));
     // the staged vector first (16-byte aligned), then the row fields
     Staged zs;
     zs.v = reinterpret_cast<float4 *>(sn_raw);
@@ -1158,10 +1198,10 @@ __global__ void __launch_bounds__(SrForm<RB>::THREADS, 1) cg_mixed_sr_kernel(con
     zs.own = make_float4(0.f, 0.f, 0.f, 0.f);
     // then the matrix blocks in shared memory, then the row fields (see sr_smem_bytes, sr_cache_bytes)
     SrCache mc;
-    mc.kc = g.kc;
-    mc.S = g.kc > 0 ? sr_cache_stride(npb, g.tpn) : 0;
+    mc.kc = bl.kc;
+    mc.S = bl.kc > 0 ? sr_cache_stride(npb, bl.tpn) : 0;
     const int ncache = mc.kc * mc.S;
-    float4 *const ca = zs.v + npb + g.nhalo, *const cb = ca + ncache;
+    float4 *const ca = zs.v + npb + bl.nhalo, *const cb = ca + ncache;
     float *const cc = reinterpret_cast<float *>(cb + ncache);
     float *const sn = cc + ncache;
     float *sx = sn, *sr = sn + 3 * npb, *sp = sn + 6 * npb, *sq = sn + 9 * npb, *sw = sn + 12 * npb,
@@ -1171,8 +1211,8 @@ __global__ void __launch_bounds__(SrForm<RB>::THREADS, 1) cg_mixed_sr_kernel(con
     float *su = sn + 24 * npb, *sdd = sn + 27 * npb;
     {
         // the matrix blocks in shared memory, filled once for the solve; their columns after the row fields
-        unsigned short *const col = reinterpret_cast<unsigned short *>(sn + (g.poly > 0 ? SR_FIELDS_POLY : SR_FIELDS) * npb);
-        const int k0 = RB * g.tpn;
+        unsigned short *const col = reinterpret_cast<unsigned short *>(sn + (bl.poly > 0 ? SR_FIELDS_POLY : SR_FIELDS) * npb);
+        const int k0 = RB * bl.tpn;
         for (int t = threadIdx.x; t < mc.kc * nloc; t += blockDim.x) {
             const int kl = t / nloc, l = t - kl * nloc, a = a0 + l, k = k0 + kl;
             if (k >= __ldg(g.rowlen + a)) continue;
@@ -1186,12 +1226,12 @@ __global__ void __launch_bounds__(SrForm<RB>::THREADS, 1) cg_mixed_sr_kernel(con
         mc.a = ca; mc.b = cb; mc.c = cc; mc.col = col;
     }
     // this block's halo; a thread's first two entries in registers
-    const int h0 = __ldg(g.halo_ptr + blockIdx.x), nh = __ldg(g.halo_ptr + blockIdx.x + 1) - h0;
+    const int h0 = __ldg(bl.halo_ptr + rank), nh = __ldg(bl.halo_ptr + rank + 1) - h0;
     int hx[2];
     hx[0] = (int)threadIdx.x < nh ? __ldg(g.halo_list + h0 + threadIdx.x) : 0;
     hx[1] = (int)(threadIdx.x + blockDim.x) < nh ? __ldg(g.halo_list + h0 + threadIdx.x + blockDim.x) : 0;
-    const int poly = g.poly;
-    const double lmax = poly > 0 ? g.cheb[0] : 0.0;
+    const int poly = bl.poly;
+    const double lmax = poly > 0 ? bl.cheb[0] : 0.0;
     const bool cheb = lmax > 0.0;              // Chebyshev this solve
     const bool rec = poly > 0 && lmax == 0.0;  // Jacobi this solve, recording the Lanczos coefficients
     if (cheb && threadIdx.x == 0) {
@@ -1211,13 +1251,25 @@ __global__ void __launch_bounds__(SrForm<RB>::THREADS, 1) cg_mixed_sr_kernel(con
         s_shift = 1.0 / p0;
     }
     if (!cheb && threadIdx.x == 0) s_shift = 1.0;
-    grid_sum_df8<MIXED_GATHER_NP>(reinterpret_cast<const float2 *>(g.init_partials), g.init_stride, g.n_init, s_sc);
+    unsigned int red_ep = 0;  // epochs of the sums over the blocks
+    auto offset = [&](int a) {
+        if constexpr (BATCH)
+            return make_float4((float)(g.px[a] - bl.xc[0]), (float)(g.py[a] - bl.xc[1]), (float)(g.pz[a] - bl.xc[2]), 0.f);
+        else
+            return g.dpos[a];
+    };
+    if constexpr (BATCH) {
+        if (!sr_moments<SrForm<RB>::K>(g, bl, a0, nloc, rank, nb, smemf, s_scf, s_sc)) return false;
+        red_ep = 2;
+    } else {
+        grid_sum_df8<MIXED_GATHER_NP>(reinterpret_cast<const float2 *>(g.init_partials), g.init_stride, g.n_init, s_sc);
+    }
     const double f2 = s_sc[0];
-    mixed_setup(g, s_sc, s_A6, s_tau, s_Om, &s_dummy, &s_conv);
+    mixed_setup(bl, s_sc, s_A6, s_tau, s_Om, &s_dummy, &s_conv);
     __syncthreads();
     const float ith = cheb ? s_ith : 0.f;
     // tpn lanes to a row, every row of the block at once (npb tpn <= blockDim)
-    const int tpn = g.tpn, l = threadIdx.x / tpn, sub = threadIdx.x % tpn;
+    const int tpn = bl.tpn, l = threadIdx.x / tpn, sub = threadIdx.x % tpn;
     const bool valid = l < nloc;
     RowRegs<RB> rr;
     int rbase = 0, rlen = 0;
@@ -1245,15 +1297,14 @@ __global__ void __launch_bounds__(SrForm<RB>::THREADS, 1) cg_mixed_sr_kernel(con
             base = valid ? __ldg(g.slice_ptr + ((a0 + l) >> 5)) : 0;
             len = valid ? __ldg(g.rowlen + a0 + l) : 0;
         }
-        spmv_row_w<RB>(g, mc, rr, zs.v, base, len, (a0 + l) & 31, l, sub, w0, w1, w2);
+        spmv_row_w<RB>(g, tpn, mc, rr, zs.v, base, len, (a0 + l) & 31, l, sub, w0, w1, w2);
     };
     unsigned int ep = 0;      // epochs of the published vectors
-    unsigned int red_ep = 0;  // epochs of the grid-wide sums
     // row l of the vector published as epoch `tag`: to the block's staged vector and to the other blocks
     auto publish = [&](unsigned int tag, int row, float v0, float v1, float v2) {
         zs.row = row;
         zs.own = make_float4(v0, v1, v2, 0.f);
-        msg_put(g.msg + (size_t)(tag & 1u) * g.N + a0 + row, __float_as_uint(v0), __float_as_uint(v1), __float_as_uint(v2),
+        msg_put(g.msg + (size_t)(tag & 1u) * g.mstride + a0 + row, __float_as_uint(v0), __float_as_uint(v1), __float_as_uint(v2),
                 tag);
     };
     // Chebyshev steps 1..d after step 0 published y0 = D^{-1} r / theta and left D^{-1} r in sw:
@@ -1291,7 +1342,7 @@ __global__ void __launch_bounds__(SrForm<RB>::THREADS, 1) cg_mixed_sr_kernel(con
         float r0 = g.r[4 * a], r1 = g.r[4 * a + 1], r2 = g.r[4 * a + 2];
         const float i0 = g.dinv[4 * a], i1 = g.dinv[4 * a + 1], i2 = g.dinv[4 * a + 2];
         if (defl) {
-            const float4 d = g.dpos[a];
+            const float4 d = offset(a);
             const float D0 = g.diag[4 * a], D1 = g.diag[4 * a + 1], D2 = g.diag[4 * a + 2];
             r0 -= D0 * (s_tau[0] + (s_Om[1] * d.z - s_Om[2] * d.y));
             r1 -= D1 * (s_tau[1] + (s_Om[2] * d.x - s_Om[0] * d.z));
@@ -1361,7 +1412,7 @@ __global__ void __launch_bounds__(SrForm<RB>::THREADS, 1) cg_mixed_sr_kernel(con
             }
         }
         FFEA_MARK(g, tm, 1);
-        if (!(ok = grid_reduce_msg<MIXED_SR_NP, SrForm<RB>::K>(g, acc, smemf, ++red_ep, s_scf, st))) break;
+        if (!(ok = grid_reduce_msg<MIXED_SR_NP, SrForm<RB>::K>(bl, rank, nb, acc, smemf, ++red_ep, s_scf, st))) break;
         FFEA_MARK(g, tm, 3);
         if (warp_index() == 0) {
             // The iteration's scalars, in double-float as the sums arrive: this chain is on every block's critical path
@@ -1385,16 +1436,16 @@ __global__ void __launch_bounds__(SrForm<RB>::THREADS, 1) cg_mixed_sr_kernel(con
             const df32 gam = s_scf[0], rr2 = s_scf[1];
             // |r|^2/|f|^2 < epsilon2 after an update, as NoMassCGSolver::solve tests it (a zero force: x = 0 at once)
             const bool conv = f2 == 0.0 || (k > 0 && (g.check_last || k < g.imax) && df_less(rr2, tol));
-            if (ln == 0 && blockIdx.x == 0 && k > 0 && k - 1 < g.hist_cap)
+            if (ln == 0 && rank == 0 && k > 0 && k - 1 < g.hist_cap)
                 reinterpret_cast<float2 *>(g.history)[k - 1] = make_float2(rr2.hi, rr2.lo);
             const bool stop = conv || k >= g.imax;
             const float beta = (k == 0) ? 0.f : gam.hi / s_g;
             const df32 zw = df_add(s_scf[2], mzc), pw = df_add(s_scf[4], mpc), b1 = {beta, 0.f};
             const df32 pq = df_add(df_add(zw, df_mul(b1, df_add(s_scf[3], pw))), df_mul(df_mul(b1, b1), s_pq));
             const float alpha = gam.hi / pq.hi;
-            if (rec && ln == 0 && blockIdx.x == 0 && !stop && k < CHEB_REC) {
-                g.cheb[1 + k] = df_double(gam) / df_double(pq);
-                g.cheb[1 + CHEB_REC + k] = beta;
+            if (rec && ln == 0 && rank == 0 && !stop && k < CHEB_REC) {
+                bl.cheb[1 + k] = df_double(gam) / df_double(pq);
+                bl.cheb[1 + CHEB_REC + k] = beta;
             }
             __syncwarp();
             if (ln < 6) {
@@ -1463,38 +1514,58 @@ __global__ void __launch_bounds__(SrForm<RB>::THREADS, 1) cg_mixed_sr_kernel(con
         }
     }
     FFEA_PHASES_END(g);
-    if (blockIdx.x == 0)  // the history's |r|^2, kept as pairs, become |r|^2 / |f|^2
+    if (rank == 0)  // the history's |r|^2, kept as pairs, become |r|^2 / |f|^2
         for (int i = threadIdx.x; i < min(k, g.hist_cap); i += blockDim.x) {
             const float2 h = reinterpret_cast<const float2 *>(g.history)[i];
             g.history[i] = f2 == 0.0 ? 0.0 : df_double(df32{h.x, h.y}) / f2;
         }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (rank == 0 && threadIdx.x == 0) {
         if (!ok) {
-            st->abort = 1;
+            atomicExch(&st->abort, 1);
         } else if (!s_conv) {
-            st->cg_fail = 1;
-            st->abort = 1;
-            st->last_iters = g.imax;
-            st->total_iters += g.imax;
+            atomicExch(&st->cg_fail, 1);
+            if constexpr (BATCH) {
+                // cg_fail alone: `abort` raised now could stop a block that another blob's blocks wait for;
+                // batch_finish_kernel raises it
+                *bl.blob_iters = g.imax;
+            } else {
+                st->abort = 1;
+                st->last_iters = g.imax;
+                st->total_iters += g.imax;
+            }
         } else {
-            st->last_iters = k;
-            st->total_iters += k;
+            if constexpr (BATCH) {
+                *bl.blob_iters = k;
+                atomicMax(&st->last_iters, k);
+                atomicAdd(reinterpret_cast<unsigned long long *>(&st->total_iters), (unsigned long long)k);
+            } else {
+                st->last_iters = k;
+                st->total_iters += k;
+            }
             if (rec && k >= 2) {
                 // the estimate of lambda_max(D^-1 V) for the next solves, from this Jacobi solve's Lanczos matrix
-                const double lm = lanczos_lambda_max(g.cheb + 1, g.cheb + 1 + CHEB_REC, min(k, CHEB_REC));
+                const double lm = lanczos_lambda_max(bl.cheb + 1, bl.cheb + 1 + CHEB_REC, min(k, CHEB_REC));
                 if (isfinite(lm) && lm > 0.0) {
-                    g.cheb[0] = CHEB_MARGIN * lm;
-                    g.cheb[CHEB_KJ] = (double)k;
+                    bl.cheb[0] = CHEB_MARGIN * lm;
+                    bl.cheb[CHEB_KJ] = (double)k;
                 }
-            } else if (cheb && g.cheb[CHEB_KJ] > 0.0) {
+            } else if (cheb && bl.cheb[CHEB_KJ] > 0.0) {
                 // the trial: the polynomial is kept when its iterations, each costing 1 + poly * cheb_cost Jacobi
                 // iterations, took less than the Jacobi solve (a well-conditioned matrix, e.g. with a large
                 // Stokes drag on its diagonal, converges in a few Jacobi iterations and keeps Jacobi)
-                if ((double)k * (1.0 + poly * (double)g.cheb_cost) >= g.cheb[CHEB_KJ]) g.cheb[0] = -1.0;
-                g.cheb[CHEB_KJ] = 0.0;
+                if ((double)k * (1.0 + poly * (double)g.cheb_cost) >= bl.cheb[CHEB_KJ]) bl.cheb[0] = -1.0;
+                bl.cheb[CHEB_KJ] = 0.0;
             }
         }
     }
+    return ok;
+}
+
+template <class R, int RB>
+__global__ void __launch_bounds__(SrForm<RB>::THREADS, 1) cg_mixed_sr_kernel(const __grid_constant__ CgArgs<R> g) {
+    static_assert(sizeof(R) == sizeof(float), "the single-reduction CG is the mixed path's");
+    if (g.st->abort) return;
+    sr_solve<RB, false>(g, g, (int)blockIdx.x, (int)gridDim.x);
 }
 
 }  // namespace ffea

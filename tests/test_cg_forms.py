@@ -87,3 +87,28 @@ def test_fp64_element_forms(cells, solver, noise):
     assert np.array_equal(b.rhs(), o.rhs()) and np.array_equal(b.rng_state(), o.rng_state())
     if solver == "masslumped":
         assert np.array_equal(b.pos(), o.pos()) and np.array_equal(b.vel(), o.vel())
+
+
+# the batch's solve on chip at its edges: blobs of one block and of many, more tasks than SMs, and (610 blobs, four
+# times the SMs and two) beyond it; each blob as the single mixed blob from the same state, and the same bits again
+@pytest.mark.gpu
+@pytest.mark.parametrize("cells", [[(7, 7, 7), (8, 7, 7)], [(12, 12, 12), (2, 2, 2), (20, 19, 21), (1, 1, 1)],
+                                   [(3, 3, 3)] * 200 + [(9, 9, 9)], [(33, 33, 33), (31, 30, 32)], [(2, 2, 1)] * 610])
+def test_batch_solve_forms(cells):
+    box = {c: kuhn_box(*c, 5.0, seed=4) for c in set(cells)}
+    meshes = [box[c] for c in cells]
+    kw = dict(dt=1e-13, kT=4.11e-21, calc_noise=1)
+    x0 = [apply_shear(m, 0.001) * (m.scale / 1.7e-10) for m in meshes]
+    runs = []
+    for _ in range(2):
+        bt = lib.Batch(meshes, **kw)
+        bt.set_positions(np.concatenate(x0))
+        bt.update(4)
+        runs.append(bt.positions())
+    assert np.array_equal(*runs)
+    for b in sorted({0, 1, len(meshes) // 2, len(meshes) - 1}):
+        s = lib.Blob(meshes[b], precision="mixed", rng_state=lib.Batch(meshes[:b + 1], **kw).rng_state(b), **kw)
+        s.set_state(pos=x0[b])
+        s.update(4)
+        assert np.abs(bt.pos(b) - s.pos()).max() < 1e-5 * np.abs(s.pos() - x0[b]).max(), b
+        assert np.array_equal(bt.rng_state(b), s.rng_state()), b
