@@ -476,7 +476,8 @@ int ffea_gpu_batch::plan_solve() {
         sr_smem = std::max(sr_smem, need + (a.kc > 0 ? sr_cache_bytes(a.kc, S) : 0));
         a.stride = blocks;
         msg_off[b] = msgs;
-        if (blocks > 1) msgs += 2ll * MSG_VALUES * MSG_COPIES * blocks;
+        // its barrier, then its sums' messages
+        msgs += sizeof(GridBarrier) / sizeof(Msg) + (blocks > 1 ? 2ll * MSG_VALUES * MSG_COPIES * blocks : 0ll);
         if (b == 0) sr_tpn = t;
     }
     std::vector<int> tptr(sms + 1, 0);
@@ -502,7 +503,8 @@ int ffea_gpu_batch::plan_solve() {
         SrBlob &a = sr_host[b];
         a.cheb = sr_cheb + (size_t)CHEB_STATE * b;
         a.halo_ptr = sr_halo_ptr + first_ptr[b];
-        a.rmsg = sr_msg + msg_off[b];
+        a.gb = reinterpret_cast<GridBarrier *>(sr_msg + msg_off[b]);
+        a.rmsg = sr_msg + msg_off[b] + sizeof(GridBarrier) / sizeof(Msg);
         a.blob_iters = blob_iters + b;
     }
     sr_grid = sms;
@@ -661,7 +663,7 @@ int ffea_gpu_batch::launch_cg_only() {
         ca.st = st;
         ca.imax = p.max_iterations_cg;
         ca.eps2 = p.epsilon2;
-        ca.cheb_cost = 0.5f;
+        ca.cheb_cost = 0.35f;
         ca.halo_list = sr_halo_list;
         ca.lcol = sr_lcol;
         ca.msg = sr_msg;

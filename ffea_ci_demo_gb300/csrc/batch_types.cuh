@@ -47,6 +47,7 @@ struct SrBlob {
     int N, row0, npb, tpn, kc, nhalo, poly, nmodes, stride, pad;
     const int *halo_ptr;
     Msg *rmsg;
+    GridBarrier *gb;
     double *cheb;
     int *blob_iters;
     double xc[3], modes[36];

@@ -148,9 +148,14 @@ __global__ void __launch_bounds__(SOLVE_PREP_THREADS)
 
 namespace {
 
-// FP32 matrix bytes up to which the mixed CG_nomass matrix is taken to stay in the GPU's L2 (129 MB, shared with
-// the vectors and the exchange buffers)
-constexpr double L2_MATRIX_BYTES = 64e6;
+// FP32 matrix bytes up to which the mixed CG_nomass matrix is taken to stay in the GPU's L2 (129 MB, shared with the
+// vectors and the messages) for the passes of cg_mixed_sr_kernel; ms per step with that kernel against
+// cg_mixed_own_kernel's Jacobi iterations: 48^3 cells (70 MB) 4.6 / 8.2, 52^3 (90 MB) 6.1 / 10.7
+constexpr double L2_MATRIX_BYTES = 100e6;
+// how much of a larger matrix cg_mixed_own_kernel asks L2 to keep while the rest streams past it: 64^3 cells (161 MB),
+// ms per step at 0 / 2 / 3 / 4 / 5 eighths 26.0 / 23.8 / 23.3 / 26.0 / 29.5, and 29.8 without the hints (L2 holds about
+// half its size of lines that both dies read)
+constexpr double L2_KEEP_BYTES = 62e6;
 
 template <class R>
 struct BlobImpl final : ffea_gpu_blob {
@@ -513,11 +518,11 @@ struct BlobImpl final : ffea_gpu_blob {
                 cg_grid = std::max(1, std::min(maxg, (N + SR_REG_ROWS - 1) / SR_REG_ROWS));
                 const int rows = (N + cg_grid - 1) / cg_grid;
                 cg_block = (rows + 31) / 32 * 32 <= SR_REG_THREADS ? SR_REG_THREADS : Launch<R>::cg_threads();
-            } else if (N <= (mixed ? 2048 : 256)) {
+            } else if (N <= (mixed ? 512 : 256)) {
                 cg_grid = 1;
                 cg_block = std::min(Launch<R>::cg_threads(), std::max(128, (N * 8 + 31) / 32 * 32));
             } else {
-                cg_grid = std::max(1, std::min(maxg, (N + 255) / 256));
+                cg_grid = std::max(1, std::min(maxg, mixed ? (N + 63) / 64 : (N + 255) / 256));
                 cg_block = Launch<R>::cg_threads();
             }
             // every block's rows in one pass (the staged kernel), or every row of the grid
@@ -763,6 +768,7 @@ struct BlobImpl final : ffea_gpu_blob {
         ca.halo_ptr = halo_ptr; ca.halo_list = halo_list; ca.lcol = lcol; ca.nhalo = nhalo;
         ca.msg = msg; ca.rmsg = rmsg;
         ca.reg = cg_reg;
+        ca.l2_keep = (int)std::min(8.0, 8.0 * L2_KEEP_BYTES / std::max(40.0 * (double)h.nslots, 1.0));
         ca.dpos = dpos; ca.nmodes = nomass ? nmodes : 0;
         for (int i = 0; i < 36; ++i) ca.modes[i] = modes[i];
         ca.npb = cg_npb;
@@ -771,10 +777,9 @@ struct BlobImpl final : ffea_gpu_blob {
         ca.kc = ca.sr || cg_unit ? cg_kc : 0;
         ca.unit = cg_unit;
         ca.cheb = cheb;
-        // a Chebyshev step (SpMV + neighbour exchange) against a whole iteration (SpMV, exchange, grid-wide
-        // reduction): about half while the FP32 matrix (40 B per 3x3 block) stays in L2, more once it streams
-        // from HBM
-        ca.cheb_cost = 40.0 * (double)h.nslots <= L2_MATRIX_BYTES ? 0.5f : 0.9f;
+        // a Chebyshev step (SpMV + neighbour exchange) against a whole Jacobi iteration: 0.26 to 0.35 measured from 20^3
+        // to 48^3 cells
+        ca.cheb_cost = 0.35f;
         if (nb_flags) {
             ca.nb_ptr = nb_ptr; ca.nb_list = nb_list; ca.flags = nb_flags;
             CK(cudaMemsetAsync(nb_flags, 0, (size_t)FLAG_STRIDE * cg_grid * sizeof(unsigned int), stream));

@@ -172,7 +172,7 @@ constexpr int MSG_POLLS = 1 << 21;
 
 // m[j] = *p[j] for the K messages with use[j], read again until every one carries `tag`: those still missing are read
 // together, so the wait ends one round trip after the last of them arrives (waited for one after another, each costs
-// its own: 4.1 against 2.6 us per grid-wide sum of 137 blocks). False once MSG_POLLS rounds have passed (recorded in
+// its own). False once MSG_POLLS rounds have passed (recorded in
 // st) or another block has recorded that.
 template <int K>
 __device__ __forceinline__ bool msg_wait_all(const Msg *const (&p)[K], const bool (&use)[K], uint32_t tag, Msg (&m)[K],
@@ -198,10 +198,14 @@ __device__ __forceinline__ bool msg_wait_all(const Msg *const (&p)[K], const boo
 }
 
 // A grid-wide sum's messages are polled by every block: they are published in MSG_COPIES copies on lines of their own
-// (one per lane of the publishing warp), block b reading copy b mod MSG_COPIES, or the polls of all 152 SMs on the
-// same twenty lines hold up the messages themselves.
+// (one per lane of the publishing warp), block b reading copy b mod MSG_COPIES, or the polls of all blocks on the same
+// few lines hold up the messages themselves (22 blocks: 213 against 199 us per step).
 constexpr int MSG_COPIES = 16;
 constexpr int MSG_VALUES = 16;  // values a reduction's buffer holds
+// Sums over more blocks than this go through a counter barrier instead: one poller to a block, where all blocks polling
+// all messages hold one another up (us per step, messages against the barrier: 137 blocks FP64 1728 / 1486, 145 blocks
+// FP64 3588 / 3087, 152 blocks mixed 40^3 2755 / 2575; 22 blocks FP64 646 / 767).
+constexpr int MSG_SUM_BLOCKS = 32;
 
 // add(message of block b) for every block b = lane, lane + 32, ... < nb, in that order, once each carries `tag`: one
 // message a lane for up to 32 blocks, else K at a time. False on a timeout.

@@ -977,6 +977,7 @@ struct CgArgs {
     const unsigned short *lcol;
     Msg *msg, *rmsg;
     int nhalo;            // the largest halo of any block
+    int l2_keep;          // cg_mixed_own_kernel: of every eight matrix slices, how many are kept in L2
     int unit;             // FP64: components per unit of cg_own_unit_kernel (1 or 3; 0: another kernel)
     // the rows solved, [row0, row0 + N), and the stride of the two message buffers (a batch solves one blob's rows of the
     // concatenation; one blob: 0 and N)
@@ -1422,6 +1423,23 @@ __device__ __forceinline__ bool grid_reduce_units(const A &g, double *s, int U, 
                                                   F meanwhile, G finish) {
     const int lane = threadIdx.x & 31, wid = warp_index(), nb = gridDim.x;
     double t = block_sum_units<NV>(s, U, wid);
+    if (nb > MSG_SUM_BLOCKS) {
+        double *const rowd = reinterpret_cast<double *>(g.rmsg) + (size_t)(tag & 1u) * MSG_VALUES * g.stride;
+        if (wid < NV && lane == 0) rowd[wid * g.stride + blockIdx.x] = t;
+        meanwhile();
+        unsigned int epoch = tag - 1u;
+        if (!barrier_ep(g.gb, (unsigned)nb, st, g.limit_ns, epoch)) return false;
+        if (wid < NV) {
+            double q[5];
+#pragma unroll
+            for (int j = 0; j < 5; ++j) q[j] = lane + 32 * j < nb ? __ldcg(rowd + wid * g.stride + lane + 32 * j) : 0.0;
+            t = (q[0] + q[1]) + (q[2] + q[3]) + q[4];
+            t = warp_sum(t);
+            if (lane == 0) finish(wid, t);
+        }
+        __syncthreads();
+        return true;
+    }
     int bad = 0;
     Msg *const rows = g.rmsg + ((size_t)(tag & 1u) * MSG_VALUES + wid) * MSG_COPIES * g.stride;
     const Msg *const row = rows + (size_t)(blockIdx.x % MSG_COPIES) * g.stride;

@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(256, (MODE == 1 && !NF) ? 8 : 1) gather_mixed_
 template <class A>
 __device__ __noinline__ void mixed_setup(const A &g, const double *s_sc, double *s_A6, float *s_tau, float *s_Om, float *s_beta,
                             int *s_conv) {
-    __shared__ double sM[36], sAug[6][12], sF[6], sV[6], sC[6], sPiv;
+    __shared__ double sM[36], sT[36], sAug[6][12], sF[6], sV[6], sC[6], sPiv;
     const int t = threadIdx.x, k = g.nmodes;
     if (t < 36) {
         const int i = t / 6, j = t % 6, lo = i < j ? i : j, hi = i < j ? j : i;
@@ -199,12 +199,20 @@ __device__ __noinline__ void mixed_setup(const A &g, const double *s_sc, double 
         sM[t] = s_sc[7 + lo * 6 - (lo * (lo - 1)) / 2 + (hi - lo)];
     }
     __syncthreads();
+    // G = modes M modes^T and, after the inversion, A6 = modes^T G^{-1} modes, each in two products of six terms
+    if (t < 36) {
+        const int i = t / 6, j = t % 6;
+        double sum = 0.0;
+        if (j < k)
+            for (int q = 0; q < 6; ++q) sum += sM[6 * i + q] * g.modes[6 * j + q];
+        sT[t] = sum;
+    }
+    __syncthreads();
     if (t < 36) {
         const int i = t / 6, j = t % 6;
         double sum = 0.0;
         if (i < k && j < k)
-            for (int p = 0; p < 6; ++p)
-                for (int q = 0; q < 6; ++q) sum += g.modes[6 * i + p] * sM[6 * p + q] * g.modes[6 * j + q];
+            for (int p = 0; p < 6; ++p) sum += g.modes[6 * i + p] * sT[6 * p + j];
         sAug[i][j] = sum;
         sAug[i][6 + j] = (i == j) ? 1.0 : 0.0;
     }
@@ -223,10 +231,17 @@ __device__ __noinline__ void mixed_setup(const A &g, const double *s_sc, double 
         __syncthreads();
     }
     if (t < 36) {
+        const int i = t / 6, q = t % 6;
+        double sum = 0.0;
+        if (i < k)
+            for (int j = 0; j < k; ++j) sum += sAug[i][6 + j] * g.modes[6 * j + q];
+        sT[t] = sum;
+    }
+    __syncthreads();
+    if (t < 36) {
         const int p = t / 6, q = t % 6;
         double sum = 0.0;
-        for (int i = 0; i < k; ++i)
-            for (int j = 0; j < k; ++j) sum += g.modes[6 * i + p] * sAug[i][6 + j] * g.modes[6 * j + q];
+        for (int i = 0; i < k; ++i) sum += g.modes[6 * i + p] * sT[6 * i + q];
         s_A6[t] = sum;
     }
     if (t < 6) {
@@ -429,7 +444,7 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_kernel(const __grid_constant
 template <int NV>
 __device__ __forceinline__ void block_reduce_store(const float (&v)[NV], float *smem, float2 *partials, int stride,
                                                    int row0) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, wid = warp_index(), nw = blockDim.x >> 5;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const float w = warp_sum_f(v[i]);
@@ -445,9 +460,12 @@ __device__ __forceinline__ void block_reduce_store(const float (&v)[NV], float *
 
 // grid_sum_df with each lane's loads issued eight at a time before their sums: the same fixed order, the
 // partials' L2 latency paid once per 256 blocks.
-template <int NV>
-__device__ __forceinline__ void grid_sum_df8(const float2 *partials, int stride, int nb, double *s_out) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+__device__ __forceinline__ void put_sum(double *s, df32 t) { *s = (double)t.hi + (double)t.lo; }
+__device__ __forceinline__ void put_sum(df32 *s, df32 t) { *s = t; }
+
+template <int NV, class T>
+__device__ __forceinline__ void grid_sum_df8(const float2 *partials, int stride, int nb, T *s_out) {
+    const int lane = threadIdx.x & 31, wid = warp_index(), nw = blockDim.x >> 5;
     for (int i = wid; i < NV; i += nw) {
         df32 t = {0.f, 0.f};
         for (int b0 = 0; b0 < nb; b0 += 256) {
@@ -461,7 +479,7 @@ __device__ __forceinline__ void grid_sum_df8(const float2 *partials, int stride,
             for (int j = 0; j < 8; ++j) t = df_add(t, df32{q[j].x, q[j].y});
         }
         t = warp_sum_df(t);
-        if (lane == 0) s_out[i] = (double)t.hi + (double)t.lo;
+        if (lane == 0) put_sum(s_out + i, t);
     }
     __syncthreads();
 }
@@ -525,9 +543,16 @@ __device__ __forceinline__ void spmv_row_zu(const A &g, const float4 *z4, const 
 // The same row with two blocks per trip: both blocks' loads (values, columns, z and p) issue before
 // either block's products, halving the chain of dependent L2 round trips per lane. The products are
 // accumulated in the same order as spmv_row_z, so the result is identical.
+// a read-only load with an L2 eviction policy (createpolicy)
+__device__ __forceinline__ float ldg_l2(const float *p, uint64_t policy) {
+    float v;
+    asm("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(policy));
+    return v;
+}
+
 template <class A>
 __device__ __forceinline__ void spmv_row_z2(const A &g, const float4 *z4, const float4 *p4, float beta, bool first,
-                                            int a, int sub, bool valid, float &q0, float &q1, float &q2) {
+                                            int a, int sub, bool valid, uint64_t policy, float &q0, float &q1, float &q2) {
     q0 = 0.f; q1 = 0.f; q2 = 0.f;
     const int tpn = g.tpn;
     if (valid) {
@@ -543,8 +568,8 @@ __device__ __forceinline__ void spmv_row_z2(const A &g, const float4 *z4, const 
             float wa[9], wb[9];
 #pragma unroll
             for (int i = 0; i < 9; ++i) {
-                wa[i] = __ldg(va + 32 * i);
-                wb[i] = __ldg(vb + 32 * i);
+                wa[i] = ldg_l2(va + 32 * i, policy);
+                wb[i] = ldg_l2(vb + 32 * i, policy);
             }
             const float4 za = z4[ba], zb = z4[bb];
             float pa0 = za.x, pa1 = za.y, pa2 = za.z, pb0 = zb.x, pb1 = zb.y, pb2 = zb.z;
@@ -565,7 +590,7 @@ __device__ __forceinline__ void spmv_row_z2(const A &g, const float4 *z4, const 
             const float *vk = v + (size_t)32 * 9 * k;
             float w[9];
 #pragma unroll
-            for (int i = 0; i < 9; ++i) w[i] = __ldg(vk + 32 * i);
+            for (int i = 0; i < 9; ++i) w[i] = ldg_l2(vk + 32 * i, policy);
             const float4 z = z4[b];
             float p0 = z.x, p1 = z.y, p2 = z.z;
             if (!first) {
@@ -636,206 +661,6 @@ __device__ __forceinline__ void spmv_row_z(const A &g, const float4 *z4, const f
         q0 += __shfl_xor_sync(0xffffffffu, q0, o);
         q1 += __shfl_xor_sync(0xffffffffu, q1, o);
         q2 += __shfl_xor_sync(0xffffffffu, q2, o);
-    }
-}
-
-// Bytes of dynamic shared memory cg_mixed_own_kernel needs for npb owned rows: x, r, q, p, D^{-1}, D, d.
-constexpr int OWN_FIELDS = 21;
-__host__ __device__ constexpr size_t own_smem_bytes(int npb) { return (size_t)OWN_FIELDS * npb * sizeof(float); }
-
-// The mixed CG of cg_mixed_kernel with each block owning a fixed run of npb rows: the rows' x, r, q, p,
-// D^{-1}, D and offsets stay in shared memory for the whole solve, the block computes its own rows' SpMV,
-// and only what other blocks read goes to global memory: z = D^{-1} r (in the q buffer) and the search
-// direction (double-buffered). The arithmetic is the same as cg_mixed_kernel's: p = z + beta p_old is
-// formed identically by the owner and by every block that reads row b as a neighbour.
-template <class R>
-__global__ void __launch_bounds__(1024, 1) cg_mixed_own_kernel(const __grid_constant__ CgArgs<R> g) {
-    static_assert(sizeof(R) == sizeof(float), "the owned-rows CG is the mixed path's");
-    extern __shared__ float sn[];
-    __shared__ float smemf[MIXED_A_NP * 32];
-    __shared__ double s_sc[MIXED_GATHER_NP];
-    __shared__ double s_A6[36];
-    __shared__ float s_alpha, s_beta, s_tau[3], s_Om[3];
-    __shared__ double s_delta;
-    __shared__ int s_conv;
-    DevStatus *st = g.st;
-    if (st->abort) return;
-    const bool defl = g.nmodes > 0;
-    FFEA_PHASES_BEGIN(g, tm);
-    float2 *partials = reinterpret_cast<float2 *>(g.partials);
-    const int npb = g.npb, a0 = blockIdx.x * npb;
-    const int nloc = max(0, min(npb, g.N - a0));
-    float *sx = sn, *sr = sn + 3 * npb, *sq = sn + 6 * npb, *sp = sn + 9 * npb, *sdi = sn + 12 * npb,
-          *sdg = sn + 15 * npb, *sd = sn + 18 * npb;
-    float4 *z4 = reinterpret_cast<float4 *>(g.q);
-    grid_sum_df8<MIXED_GATHER_NP>(reinterpret_cast<const float2 *>(g.init_partials), g.init_stride, g.n_init, s_sc);
-    const double f2 = s_sc[0];
-    mixed_setup(g, s_sc, s_A6, s_tau, s_Om, &s_beta, &s_conv);
-    float acc0[1] = {0.f};
-    for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
-        const int a = a0 + l;
-        float r0 = g.r[4 * a], r1 = g.r[4 * a + 1], r2 = g.r[4 * a + 2];
-        const float i0 = g.dinv[4 * a], i1 = g.dinv[4 * a + 1], i2 = g.dinv[4 * a + 2];
-        if (defl) {
-            const float4 d = g.dpos[a];
-            const float D0 = g.diag[4 * a], D1 = g.diag[4 * a + 1], D2 = g.diag[4 * a + 2];
-            r0 -= D0 * (s_tau[0] + (s_Om[1] * d.z - s_Om[2] * d.y));
-            r1 -= D1 * (s_tau[1] + (s_Om[2] * d.x - s_Om[0] * d.z));
-            r2 -= D2 * (s_tau[2] + (s_Om[0] * d.y - s_Om[1] * d.x));
-            sdg[l] = D0; sdg[npb + l] = D1; sdg[2 * npb + l] = D2;
-            sd[l] = d.x; sd[npb + l] = d.y; sd[2 * npb + l] = d.z;
-        }
-        sr[l] = r0; sr[npb + l] = r1; sr[2 * npb + l] = r2;
-        sdi[l] = i0; sdi[npb + l] = i1; sdi[2 * npb + l] = i2;
-        sx[l] = 0.f; sx[npb + l] = 0.f; sx[2 * npb + l] = 0.f;
-        const float z0 = i0 * r0, z1 = i1 * r1, z2 = i2 * r2;
-        z4[a] = make_float4(z0, z1, z2, 0.f);
-        acc0[0] += r0 * z0 + r1 * z1 + r2 * z2;
-    }
-    const int row0 = MIXED_A_NP + MIXED_B_NP;
-    block_reduce_store<1>(acc0, smemf, partials, g.stride, row0);
-    unsigned int bar_ep = 0;  // grid barriers passed
-    bool ok = grid_sync_ep(g.gb, st, g.limit_ns, bar_ep);
-    if (ok) {
-        grid_sum_df8<1>(partials + row0 * g.stride, 0, gridDim.x, s_sc);
-        if (threadIdx.x == 0) s_delta = s_sc[0];
-        __syncthreads();
-    }
-    const float4 *pold = reinterpret_cast<const float4 *>(g.pbuf0);
-    float4 *pnew = reinterpret_cast<float4 *>(g.pbuf1);
-    const int tpn = g.tpn, gpb = blockDim.x / tpn, grp = threadIdx.x / tpn, sub = threadIdx.x % tpn;
-    const int npass = (nloc + gpb - 1) / gpb;
-    FFEA_MARK(g, tm, 0);
-    int it = 0;
-    // a zero force (a blob exactly at rest without noise) has the solution x = 0: no iteration
-    if (f2 == 0.0 && threadIdx.x == 0) s_conv = 1;
-    for (; ok && it < g.imax && f2 != 0.0; ++it) {
-        const bool first = it == 0;
-        const float beta = s_beta;
-        // phase A: q = V p over the block's rows (p formed on the fly); p.q; moments of D p
-        float acc[MIXED_A_NP];
-#pragma unroll
-        for (int i = 0; i < MIXED_A_NP; ++i) acc[i] = 0.f;
-        for (int ps = 0; ps < npass; ++ps) {
-            const int l = ps * gpb + grp;
-            const bool valid = l < nloc;
-            float q0, q1, q2;
-            if (g.block3) spmv_row_z2(g, z4, pold, beta, first, a0 + l, sub, valid, q0, q1, q2);
-            else spmv_row_z(g, z4, pold, beta, first, a0 + l, sub, valid, q0, q1, q2);
-            if (!valid || sub != 0) continue;
-            const float z0 = sdi[l] * sr[l], z1 = sdi[npb + l] * sr[npb + l], z2 = sdi[2 * npb + l] * sr[2 * npb + l];
-            float p0 = z0, p1 = z1, p2 = z2;
-            if (!first) {
-                p0 = fmaf(beta, sp[l], z0); p1 = fmaf(beta, sp[npb + l], z1); p2 = fmaf(beta, sp[2 * npb + l], z2);
-            }
-            sp[l] = p0; sp[npb + l] = p1; sp[2 * npb + l] = p2;
-            sq[l] = q0; sq[npb + l] = q1; sq[2 * npb + l] = q2;
-            pnew[a0 + l] = make_float4(p0, p1, p2, 0.f);
-            acc[0] += p0 * q0 + p1 * q1 + p2 * q2;
-            if (defl) {
-                const float dx = sd[l], dy = sd[npb + l], dz = sd[2 * npb + l];
-                const float e0 = sdg[l] * p0, e1 = sdg[npb + l] * p1, e2 = sdg[2 * npb + l] * p2;
-                acc[1] += e0; acc[2] += e1; acc[3] += e2;
-                acc[4] += dy * e2 - dz * e1;
-                acc[5] += dz * e0 - dx * e2;
-                acc[6] += dx * e1 - dy * e0;
-            }
-        }
-        FFEA_MARK(g, tm, 1);
-        block_reduce_store<MIXED_A_NP>(acc, smemf, partials, g.stride, 0);
-        FFEA_MARK(g, tm, 2);
-        if (!(ok = grid_sync_ep(g.gb, st, g.limit_ns, bar_ep))) break;
-        FFEA_MARK(g, tm, 3);
-        grid_sum_df8<MIXED_A_NP>(partials, g.stride, gridDim.x, s_sc);
-        if (threadIdx.x < 32) {
-            const int ln = threadIdx.x;
-            double tO = 0.0;
-            if (defl && ln < 6) {
-#pragma unroll
-                for (int qq = 0; qq < 6; ++qq) tO += s_A6[6 * ln + qq] * s_sc[1 + qq];
-            }
-            double prod = (ln < 6) ? tO * s_sc[1 + ln] : 0.0;
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1) prod += __shfl_xor_sync(0xffffffffu, prod, o);
-            if (ln < 6) {
-                if (ln < 3) s_tau[ln] = (float)tO; else s_Om[ln - 3] = (float)tO;
-            }
-            if (ln == 0) s_alpha = (float)s_delta / (float)(s_sc[0] + prod);
-        }
-        __syncthreads();
-        FFEA_MARK(g, tm, 4);
-        const float alpha = s_alpha;
-        const float t0 = s_tau[0], t1 = s_tau[1], t2 = s_tau[2], O0 = s_Om[0], O1 = s_Om[1], O2 = s_Om[2];
-        // phase B: x += alpha p ; r -= alpha (q + D (tau + Omega x d)) ; z = D^{-1} r ; r.r ; r.z
-        float acc2[MIXED_B_NP] = {0.f, 0.f};
-        for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
-            float p[3], qv[3], rv[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                p[c] = sp[c * npb + l];
-                qv[c] = sq[c * npb + l];
-                sx[c * npb + l] += alpha * p[c];
-            }
-            if (defl) {
-                const float dx = sd[l], dy = sd[npb + l], dz = sd[2 * npb + l];
-                qv[0] += sdg[l] * (t0 + (O1 * dz - O2 * dy));
-                qv[1] += sdg[npb + l] * (t1 + (O2 * dx - O0 * dz));
-                qv[2] += sdg[2 * npb + l] * (t2 + (O0 * dy - O1 * dx));
-            }
-            float z[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                rv[c] = sr[c * npb + l] - alpha * qv[c];
-                sr[c * npb + l] = rv[c];
-                z[c] = sdi[c * npb + l] * rv[c];
-            }
-            z4[a0 + l] = make_float4(z[0], z[1], z[2], 0.f);
-            acc2[0] += rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
-            acc2[1] += rv[0] * z[0] + rv[1] * z[1] + rv[2] * z[2];
-        }
-        FFEA_MARK(g, tm, 5);
-        block_reduce_store<MIXED_B_NP>(acc2, smemf, partials, g.stride, MIXED_A_NP);
-        FFEA_MARK(g, tm, 6);
-        if (!(ok = grid_sync_ep(g.gb, st, g.limit_ns, bar_ep))) break;
-        FFEA_MARK(g, tm, 7);
-        grid_sum_df8<MIXED_B_NP>(partials + MIXED_A_NP * g.stride, g.stride, gridDim.x, s_sc);
-        if (threadIdx.x == 0) {
-            s_conv = (g.check_last || it + 1 < g.imax) && (f2 == 0.0 || s_sc[0] < g.eps2 * f2);
-            if (blockIdx.x == 0 && it < g.hist_cap) g.history[it] = (f2 == 0.0) ? 0.0 : s_sc[0] / f2;
-            const double delta_old = s_delta;
-            s_delta = s_sc[1];
-            s_beta = (float)s_delta / (float)delta_old;
-        }
-        __syncthreads();
-        FFEA_MARK(g, tm, 8);
-        if (s_conv) {
-            ++it;
-            break;
-        }
-        const float4 *t = pold; pold = pnew; pnew = const_cast<float4 *>(t);
-    }
-    // the solution (and residual) back to global memory
-    for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
-        const int a = a0 + l;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            g.x[4 * a + c] = sx[c * npb + l];
-            g.r[4 * a + c] = sr[c * npb + l];
-        }
-    }
-    FFEA_PHASES_END(g);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        if (!ok) {
-            st->abort = 1;
-        } else if (!s_conv) {
-            st->cg_fail = 1;
-            st->abort = 1;
-            st->last_iters = g.imax;
-            st->total_iters += g.imax;
-        } else {
-            st->last_iters = it;
-            st->total_iters += it;
-        }
     }
 }
 
@@ -911,12 +736,24 @@ __device__ __forceinline__ float warp_sum_spread(const float (&v)[NV], int &inde
 // before smem (NV x 32 floats) is written again.
 template <int NV, int K, class A>
 __device__ __forceinline__ bool grid_reduce_msg(const A &g, int rank, int nb, const float (&v)[NV], float *smem,
-                                                unsigned int tag, df32 *s_out, DevStatus *st) {
+                                                unsigned int tag, df32 *s_out, DevStatus *st, GridBarrier *gb) {
     const int lane = threadIdx.x & 31, wid = warp_index(), nw = blockDim.x >> 5;
     int idx;
     const float ws = warp_sum_spread<NV>(v, idx);
     if (idx >= 0) smem[idx * 32 + wid] = ws;
     __syncthreads();
+    if (gb && nb > MSG_SUM_BLOCKS) {
+        float2 *const rows = reinterpret_cast<float2 *>(g.rmsg) + (size_t)(tag & 1u) * MSG_VALUES * g.stride;
+        for (int i = wid; i < NV; i += nw) {
+            df32 t = {lane < nw ? smem[i * 32 + lane] : 0.f, 0.f};
+            t = warp_sum_df(t);
+            if (lane == 0) rows[i * g.stride + rank] = make_float2(t.hi, t.lo);
+        }
+        unsigned int epoch = tag - 1u;
+        if (!barrier_ep(gb, (unsigned)nb, st, 2000000000ull, epoch)) return false;
+        grid_sum_df8<NV>(rows, g.stride, nb, s_out);
+        return true;
+    }
     int bad = 0;
     for (int i = wid; i < NV; i += nw) {
         df32 t = {lane < nw ? smem[i * 32 + lane] : 0.f, 0.f};
@@ -937,6 +774,222 @@ __device__ __forceinline__ bool grid_reduce_msg(const A &g, int rank, int nb, co
         if (lane == 0) s_out[i] = t;
     }
     return __syncthreads_or(bad) == 0;
+}
+
+// Bytes of dynamic shared memory cg_mixed_own_kernel needs for npb owned rows: x, r, q, p, D^{-1}, D, d.
+constexpr int OWN_FIELDS = 21;
+__host__ __device__ constexpr size_t own_smem_bytes(int npb) { return (size_t)OWN_FIELDS * npb * sizeof(float); }
+
+// The mixed CG of cg_mixed_kernel with each block owning a fixed run of npb rows: the rows' x, r, q, p,
+// D^{-1}, D and offsets stay in shared memory for the whole solve, the block computes its own rows' SpMV,
+// and only what other blocks read goes to global memory: z = D^{-1} r (in the q buffer) and the search
+// direction (double-buffered). The arithmetic is the same as cg_mixed_kernel's: p = z + beta p_old is
+// formed identically by the owner and by every block that reads row b as a neighbour.
+template <class R>
+__global__ void __launch_bounds__(1024, 1) cg_mixed_own_kernel(const __grid_constant__ CgArgs<R> g) {
+    static_assert(sizeof(R) == sizeof(float), "the owned-rows CG is the mixed path's");
+    extern __shared__ float sn[];
+    __shared__ float smemf[MIXED_A_NP * 32];
+    __shared__ double s_sc[MIXED_GATHER_NP];
+    __shared__ double s_A6[36];
+    __shared__ df32 s_A6f[36], s_scf[MIXED_A_NP];
+    __shared__ float s_alpha, s_beta, s_tau[3], s_Om[3];
+    __shared__ df32 s_delta;
+    __shared__ int s_conv;
+    DevStatus *st = g.st;
+    if (st->abort) return;
+    const bool defl = g.nmodes > 0;
+    FFEA_PHASES_BEGIN(g, tm);
+    float2 *partials = reinterpret_cast<float2 *>(g.partials);
+    const int npb = g.npb, a0 = blockIdx.x * npb;
+    const int nloc = max(0, min(npb, g.N - a0));
+    float *sx = sn, *sr = sn + 3 * npb, *sq = sn + 6 * npb, *sp = sn + 9 * npb, *sdi = sn + 12 * npb,
+          *sdg = sn + 15 * npb, *sd = sn + 18 * npb;
+    float4 *z4 = reinterpret_cast<float4 *>(g.q);
+    grid_sum_df8<MIXED_GATHER_NP>(reinterpret_cast<const float2 *>(g.init_partials), g.init_stride, g.n_init, s_sc);
+    const double f2 = s_sc[0];
+    mixed_setup(g, s_sc, s_A6, s_tau, s_Om, &s_beta, &s_conv);
+    float acc0[1] = {0.f};
+    for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
+        const int a = a0 + l;
+        float r0 = g.r[4 * a], r1 = g.r[4 * a + 1], r2 = g.r[4 * a + 2];
+        const float i0 = g.dinv[4 * a], i1 = g.dinv[4 * a + 1], i2 = g.dinv[4 * a + 2];
+        if (defl) {
+            const float4 d = g.dpos[a];
+            const float D0 = g.diag[4 * a], D1 = g.diag[4 * a + 1], D2 = g.diag[4 * a + 2];
+            r0 -= D0 * (s_tau[0] + (s_Om[1] * d.z - s_Om[2] * d.y));
+            r1 -= D1 * (s_tau[1] + (s_Om[2] * d.x - s_Om[0] * d.z));
+            r2 -= D2 * (s_tau[2] + (s_Om[0] * d.y - s_Om[1] * d.x));
+            sdg[l] = D0; sdg[npb + l] = D1; sdg[2 * npb + l] = D2;
+            sd[l] = d.x; sd[npb + l] = d.y; sd[2 * npb + l] = d.z;
+        }
+        sr[l] = r0; sr[npb + l] = r1; sr[2 * npb + l] = r2;
+        sdi[l] = i0; sdi[npb + l] = i1; sdi[2 * npb + l] = i2;
+        sx[l] = 0.f; sx[npb + l] = 0.f; sx[2 * npb + l] = 0.f;
+        const float z0 = i0 * r0, z1 = i1 * r1, z2 = i2 * r2;
+        z4[a] = make_float4(z0, z1, z2, 0.f);
+        acc0[0] += r0 * z0 + r1 * z1 + r2 * z2;
+    }
+    if (threadIdx.x < 36) s_A6f[threadIdx.x] = df_of(s_A6[threadIdx.x]);
+    const df32 tol = df_of(g.eps2 * f2);
+    const int row0 = MIXED_A_NP + MIXED_B_NP;
+    block_reduce_store<1>(acc0, smemf, partials, g.stride, row0);
+    unsigned int bar_ep = 0;  // grid barriers passed
+    bool ok = grid_sync_ep(g.gb, st, g.limit_ns, bar_ep);
+    if (ok) {
+        grid_sum_df8<1>(partials + row0 * g.stride, 0, gridDim.x, s_scf);
+        if (threadIdx.x == 0) s_delta = s_scf[0];
+        __syncthreads();
+    }
+    const float4 *pold = reinterpret_cast<const float4 *>(g.pbuf0);
+    float4 *pnew = reinterpret_cast<float4 *>(g.pbuf1);
+    uint64_t keep, stream;
+    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(keep));
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(stream));
+    const int tpn = g.tpn, gpb = blockDim.x / tpn, grp = threadIdx.x / tpn, sub = threadIdx.x % tpn;
+    const int npass = (nloc + gpb - 1) / gpb;
+    FFEA_MARK(g, tm, 0);
+    int it = 0;
+    // a zero force (a blob exactly at rest without noise) has the solution x = 0: no iteration
+    if (f2 == 0.0 && threadIdx.x == 0) s_conv = 1;
+    for (; ok && it < g.imax && f2 != 0.0; ++it) {
+        const bool first = it == 0;
+        const float beta = s_beta;
+        // phase A: q = V p over the block's rows (p formed on the fly); p.q; moments of D p
+        float acc[MIXED_A_NP];
+#pragma unroll
+        for (int i = 0; i < MIXED_A_NP; ++i) acc[i] = 0.f;
+        for (int ps = 0; ps < npass; ++ps) {
+            const int l = ps * gpb + grp;
+            const bool valid = l < nloc;
+            float q0, q1, q2;
+            if (g.block3)
+                spmv_row_z2(g, z4, pold, beta, first, a0 + l, sub, valid, ((a0 + l) >> 5 & 7) < g.l2_keep ? keep : stream, q0,
+                            q1, q2);
+            else spmv_row_z(g, z4, pold, beta, first, a0 + l, sub, valid, q0, q1, q2);
+            if (!valid || sub != 0) continue;
+            const float z0 = sdi[l] * sr[l], z1 = sdi[npb + l] * sr[npb + l], z2 = sdi[2 * npb + l] * sr[2 * npb + l];
+            float p0 = z0, p1 = z1, p2 = z2;
+            if (!first) {
+                p0 = fmaf(beta, sp[l], z0); p1 = fmaf(beta, sp[npb + l], z1); p2 = fmaf(beta, sp[2 * npb + l], z2);
+            }
+            sp[l] = p0; sp[npb + l] = p1; sp[2 * npb + l] = p2;
+            sq[l] = q0; sq[npb + l] = q1; sq[2 * npb + l] = q2;
+            pnew[a0 + l] = make_float4(p0, p1, p2, 0.f);
+            acc[0] += p0 * q0 + p1 * q1 + p2 * q2;
+            if (defl) {
+                const float dx = sd[l], dy = sd[npb + l], dz = sd[2 * npb + l];
+                const float e0 = sdg[l] * p0, e1 = sdg[npb + l] * p1, e2 = sdg[2 * npb + l] * p2;
+                acc[1] += e0; acc[2] += e1; acc[3] += e2;
+                acc[4] += dy * e2 - dz * e1;
+                acc[5] += dz * e0 - dx * e2;
+                acc[6] += dx * e1 - dy * e0;
+            }
+        }
+        FFEA_MARK(g, tm, 1);
+        block_reduce_store<MIXED_A_NP>(acc, smemf, partials, g.stride, 0);
+        FFEA_MARK(g, tm, 2);
+        if (!(ok = grid_sync_ep(g.gb, st, g.limit_ns, bar_ep))) break;
+        FFEA_MARK(g, tm, 3);
+        grid_sum_df8<MIXED_A_NP>(partials, g.stride, gridDim.x, s_scf);
+        if (warp_index() == 0) {
+            // (tau, Omega) = A6 S; p.V~p = p.q + S . (tau, Omega); alpha = delta / p.V~p
+            const int ln = threadIdx.x;
+            df32 tO = {0.f, 0.f}, sv = tO;
+            if (defl && ln < 6) {
+                tO = df_mul(s_A6f[6 * ln], s_scf[1]);
+#pragma unroll
+                for (int qq = 1; qq < 6; ++qq) tO = df_add(tO, df_mul(s_A6f[6 * ln + qq], s_scf[1 + qq]));
+                sv = s_scf[1 + ln];
+            }
+            df32 prod = df_mul(tO, sv);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) prod = df_add(prod, df_shfl_xor(prod, o));
+            if (ln < 6) {
+                if (ln < 3) s_tau[ln] = tO.hi; else s_Om[ln - 3] = tO.hi;
+            }
+            if (ln == 0) s_alpha = s_delta.hi / df_add(s_scf[0], prod).hi;
+        }
+        __syncthreads();
+        FFEA_MARK(g, tm, 4);
+        const float alpha = s_alpha;
+        const float t0 = s_tau[0], t1 = s_tau[1], t2 = s_tau[2], O0 = s_Om[0], O1 = s_Om[1], O2 = s_Om[2];
+        // phase B: x += alpha p ; r -= alpha (q + D (tau + Omega x d)) ; z = D^{-1} r ; r.r ; r.z
+        float acc2[MIXED_B_NP] = {0.f, 0.f};
+        for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
+            float p[3], qv[3], rv[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                p[c] = sp[c * npb + l];
+                qv[c] = sq[c * npb + l];
+                sx[c * npb + l] += alpha * p[c];
+            }
+            if (defl) {
+                const float dx = sd[l], dy = sd[npb + l], dz = sd[2 * npb + l];
+                qv[0] += sdg[l] * (t0 + (O1 * dz - O2 * dy));
+                qv[1] += sdg[npb + l] * (t1 + (O2 * dx - O0 * dz));
+                qv[2] += sdg[2 * npb + l] * (t2 + (O0 * dy - O1 * dx));
+            }
+            float z[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                rv[c] = sr[c * npb + l] - alpha * qv[c];
+                sr[c * npb + l] = rv[c];
+                z[c] = sdi[c * npb + l] * rv[c];
+            }
+            z4[a0 + l] = make_float4(z[0], z[1], z[2], 0.f);
+            acc2[0] += rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
+            acc2[1] += rv[0] * z[0] + rv[1] * z[1] + rv[2] * z[2];
+        }
+        FFEA_MARK(g, tm, 5);
+        block_reduce_store<MIXED_B_NP>(acc2, smemf, partials, g.stride, MIXED_A_NP);
+        FFEA_MARK(g, tm, 6);
+        if (!(ok = grid_sync_ep(g.gb, st, g.limit_ns, bar_ep))) break;
+        FFEA_MARK(g, tm, 7);
+        grid_sum_df8<MIXED_B_NP>(partials + MIXED_A_NP * g.stride, g.stride, gridDim.x, s_scf);
+        if (threadIdx.x == 0) {
+            s_conv = (g.check_last || it + 1 < g.imax) && (f2 == 0.0 || df_less(s_scf[0], tol));
+            if (blockIdx.x == 0 && it < g.hist_cap)  // divided by |f|^2 at the end
+                reinterpret_cast<float2 *>(g.history)[it] = make_float2(s_scf[0].hi, s_scf[0].lo);
+            s_beta = s_scf[1].hi / s_delta.hi;
+            s_delta = s_scf[1];
+        }
+        __syncthreads();
+        FFEA_MARK(g, tm, 8);
+        if (s_conv) {
+            ++it;
+            break;
+        }
+        const float4 *t = pold; pold = pnew; pnew = const_cast<float4 *>(t);
+    }
+    // the solution (and residual) back to global memory
+    for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
+        const int a = a0 + l;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            g.x[4 * a + c] = sx[c * npb + l];
+            g.r[4 * a + c] = sr[c * npb + l];
+        }
+    }
+    FFEA_PHASES_END(g);
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < min(it, g.hist_cap); i += blockDim.x) {
+            const float2 h = reinterpret_cast<const float2 *>(g.history)[i];
+            g.history[i] = f2 == 0.0 ? 0.0 : df_double(df32{h.x, h.y}) / f2;
+        }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (!ok) {
+            st->abort = 1;
+        } else if (!s_conv) {
+            st->cg_fail = 1;
+            st->abort = 1;
+            st->last_iters = g.imax;
+            st->total_iters += g.imax;
+        } else {
+            st->last_iters = it;
+            st->total_iters += it;
+        }
+    }
 }
 
 // 3x3 blocks of each owned row of cg_mixed_sr_kernel kept in shared memory for the whole solve, kc of them after
@@ -1063,7 +1116,7 @@ __host__ __device__ constexpr size_t sr_cache_bytes(int kc, int S) {
 // Lanczos matrix of the first CHEB_REC iterations of a Jacobi-preconditioned solve. State (CHEB_STATE doubles):
 // [0] the estimate (0: not yet known, -1: Jacobi kept), [1, 1 + CHEB_REC) step lengths, then as many direction
 // coefficients, then [CHEB_KJ] the iterations of the Jacobi solve while the first polynomial solve (the trial)
-// is pending.
+// is pending, then (CHEB_COEF) the recurrence's coefficients for the estimate.
 constexpr int CHEB_MAX = 8;
 constexpr int CHEB_REC = 64;
 // the interval's width: degrees 4 and up gain from a wider one (40^3 Kuhn cube, degree 4, CG per step: ratio 30
@@ -1071,33 +1124,68 @@ constexpr int CHEB_REC = 64;
 __host__ __device__ constexpr double cheb_ratio(int degree) { return degree > 2 ? 120.0 : 30.0; }
 constexpr double CHEB_MARGIN = 1.05;
 constexpr int CHEB_KJ = 1 + 2 * CHEB_REC;
-constexpr int CHEB_STATE = CHEB_KJ + 1;
+constexpr int CHEB_COEF = CHEB_KJ + 1;
+constexpr int CHEB_STATE = CHEB_COEF + 2 * CHEB_MAX + 2;
 
 // Largest eigenvalue of the Lanczos matrix of n preconditioned-CG iterations (step lengths al, direction
-// coefficients be, be[0] unused): T_ii = 1/al_i + be_i/al_{i-1}, T_i,i+1 = sqrt(be_{i+1})/al_i. Bisection on the
-// Sturm count of negative LDL^T pivots, between the largest diagonal entry and the Gershgorin bound. One thread.
-static __device__ __noinline__ double lanczos_lambda_max(const double *al, const double *be, int n) {
+// coefficients be, be[0] unused): T_ii = 1/al_i + be_i/al_{i-1}, T_i,i+1 = sqrt(be_{i+1})/al_i. The Sturm count of
+// negative LDL^T pivots at 32 points at once, one to a lane (an FP64 instruction costs the same for one lane as for
+// 32), narrows the interval between the largest diagonal entry and the Gershgorin bound 33-fold a round; by bisection
+// on one thread it took 2.6 ms, three quarters of a 20^3-cell blob's first step. One whole warp, all lanes with the
+// same arguments; w: scratch for 2 n doubles.
+static __device__ __noinline__ double lanczos_lambda_max(const double *al, const double *be, int n, double *w) {
+    const int lane = threadIdx.x & 31;
     double lo = 0.0, hi = 0.0;
-    for (int i = 0; i < n; ++i) {
-        const double d = 1.0 / al[i] + (i > 0 ? be[i] / al[i - 1] : 0.0);
-        const double el = i > 0 ? sqrt(be[i]) / al[i - 1] : 0.0, er = i + 1 < n ? sqrt(be[i + 1]) / al[i] : 0.0;
+    for (int i = lane; i < n; i += 32) {
+        const double ia = 1.0 / al[i], ip = i > 0 ? 1.0 / al[i - 1] : 0.0, b = i > 0 ? be[i] : 0.0;
+        const double d = ia + b * ip, er = i + 1 < n ? sqrt(be[i + 1]) * ia : 0.0;
+        w[i] = d;
+        w[n + i] = b * ip * ip;
         lo = fmax(lo, d);
-        hi = fmax(hi, d + el + er);
+        hi = fmax(hi, d + sqrt(b) * ip + er);
     }
-    for (int it = 0; it < 48 && hi - lo > 1e-6 * hi; ++it) {
-        const double x = 0.5 * (lo + hi);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fmax(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    __syncwarp();
+    for (int it = 0; it < 8 && hi - lo > 1e-6 * hi; ++it) {
+        const double h = (hi - lo) / 33.0, x = lo + (lane + 1) * h;
         int below = 0;
         double q = 1.0;
         for (int i = 0; i < n; ++i) {
-            const double d = 1.0 / al[i] + (i > 0 ? be[i] / al[i - 1] : 0.0);
-            const double e2 = i > 0 ? be[i] / (al[i - 1] * al[i - 1]) : 0.0;
-            q = (d - x) - (i > 0 ? e2 / q : 0.0);
+            q = (w[i] - x) - (i > 0 ? w[n + i] / q : 0.0);
             if (q == 0.0) q = -1e-300;
             below += q < 0.0;
         }
-        if (below == n) hi = x; else lo = x;
+        // the first point above every eigenvalue
+        const unsigned int above = __ballot_sync(0xffffffffu, below == n);
+        const int f = above ? __ffs(above) - 1 : 32;
+        if (f < 32) hi = lo + (f + 1) * h;
+        lo += f * h;
     }
     return hi;
+}
+
+// The Chebyshev recurrence's coefficients for an interval that ends at lmax, kept behind the estimate in the blob's
+// state (CHEB_COEF: c1, c2, 1/theta and the rigid-mode shift's scale 1/P_d(0)). One thread.
+static __device__ __noinline__ void cheb_coefficients(double *state, int degree) {
+    const double b = state[0], a = b / cheb_ratio(degree), theta = 0.5 * (b + a), delta = 0.5 * (b - a);
+    const double sigma = theta / delta;
+    double *c = state + CHEB_COEF;
+    // the same recurrence at lambda = 0, where the residual stays D^{-1} r, gives P_d(0)
+    double rho = 1.0 / sigma, p0 = 1.0 / theta, d0 = p0;
+    for (int j = 0; j < degree; ++j) {
+        const double rn = 1.0 / (2.0 * sigma - rho);
+        c[j] = rn * rho;
+        c[CHEB_MAX + j] = 2.0 * rn / delta;
+        d0 = rn * rho * d0 + 2.0 * rn / delta;
+        p0 += d0;
+        rho = rn;
+    }
+    c[2 * CHEB_MAX] = 1.0 / theta;
+    c[2 * CHEB_MAX + 1] = 1.0 / p0;
 }
 
 // The mixed CG with one reduction per iteration (the single-synchronisation rearrangement of Chronopoulos and
@@ -1160,7 +1248,7 @@ __device__ __noinline__ bool sr_moments(const A &g, const B &bl, int a0, int nlo
         float v[14];
 #pragma unroll
         for (int i = 0; i < 14; ++i) v[i] = m[14 * half + i];
-        if (!grid_reduce_msg<14, K>(bl, rank, nb, v, smemf, (unsigned)half + 1u, s_scf, g.st)) return false;
+        if (!grid_reduce_msg<14, K>(bl, rank, nb, v, smemf, (unsigned)half + 1u, s_scf, g.st, bl.gb)) return false;
         if (threadIdx.x < 14) s_sc[14 * half + threadIdx.x] = df_double(s_scf[threadIdx.x]);
         __syncthreads();
     }
@@ -1234,21 +1322,16 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
     const double lmax = poly > 0 ? bl.cheb[0] : 0.0;
     const bool cheb = lmax > 0.0;              // Chebyshev this solve
     const bool rec = poly > 0 && lmax == 0.0;  // Jacobi this solve, recording the Lanczos coefficients
-    if (cheb && threadIdx.x == 0) {
-        const double b = lmax, a = lmax / cheb_ratio(poly), theta = 0.5 * (b + a), delta = 0.5 * (b - a);
-        const double sigma = theta / delta;
-        // the same recurrence at lambda = 0, where the residual stays D^{-1} r, gives P_d(0)
-        double rho = 1.0 / sigma, p0 = 1.0 / theta, d0 = p0;
-        for (int j = 0; j < poly; ++j) {
-            const double rn = 1.0 / (2.0 * sigma - rho);
-            s_c1[j] = (float)(rn * rho);
-            s_c2[j] = (float)(2.0 * rn / delta);
-            d0 = rn * rho * d0 + 2.0 * rn / delta;
-            p0 += d0;
-            rho = rn;
+    if (cheb) {
+        const double *c = bl.cheb + CHEB_COEF;
+        if ((int)threadIdx.x < poly) {
+            s_c1[threadIdx.x] = (float)c[threadIdx.x];
+            s_c2[threadIdx.x] = (float)c[CHEB_MAX + threadIdx.x];
         }
-        s_ith = (float)(1.0 / theta);
-        s_shift = 1.0 / p0;
+        if (threadIdx.x == 0) {
+            s_ith = (float)c[2 * CHEB_MAX];
+            s_shift = c[2 * CHEB_MAX + 1];
+        }
     }
     if (!cheb && threadIdx.x == 0) s_shift = 1.0;
     unsigned int red_ep = 0;  // epochs of the sums over the blocks
@@ -1412,7 +1495,7 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
             }
         }
         FFEA_MARK(g, tm, 1);
-        if (!(ok = grid_reduce_msg<MIXED_SR_NP, SrForm<RB>::K>(bl, rank, nb, acc, smemf, ++red_ep, s_scf, st))) break;
+        if (!(ok = grid_reduce_msg<MIXED_SR_NP, SrForm<RB>::K>(bl, rank, nb, acc, smemf, ++red_ep, s_scf, st, bl.gb))) break;
         FFEA_MARK(g, tm, 3);
         if (warp_index() == 0) {
             // The iteration's scalars, in double-float as the sums arrive: this chain is on every block's critical path
@@ -1519,6 +1602,13 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
             const float2 h = reinterpret_cast<const float2 *>(g.history)[i];
             g.history[i] = f2 == 0.0 ? 0.0 : df_double(df32{h.x, h.y}) / f2;
         }
+    double lm = 0.0;
+    if (rank == 0 && rec && ok) {
+        __syncthreads();  // the staged vector is done with
+        if (warp_index() == 0 && s_conv && k >= 2)
+            lm = lanczos_lambda_max(bl.cheb + 1, bl.cheb + 1 + CHEB_REC, min(k, CHEB_REC),
+                                    reinterpret_cast<double *>(sn_raw));
+    }
     if (rank == 0 && threadIdx.x == 0) {
         if (!ok) {
             atomicExch(&st->abort, 1);
@@ -1544,10 +1634,10 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
             }
             if (rec && k >= 2) {
                 // the estimate of lambda_max(D^-1 V) for the next solves, from this Jacobi solve's Lanczos matrix
-                const double lm = lanczos_lambda_max(bl.cheb + 1, bl.cheb + 1 + CHEB_REC, min(k, CHEB_REC));
                 if (isfinite(lm) && lm > 0.0) {
                     bl.cheb[0] = CHEB_MARGIN * lm;
                     bl.cheb[CHEB_KJ] = (double)k;
+                    cheb_coefficients(bl.cheb, poly);
                 }
             } else if (cheb && bl.cheb[CHEB_KJ] > 0.0) {
                 // the trial: the polynomial is kept when its iterations, each costing 1 + poly * cheb_cost Jacobi

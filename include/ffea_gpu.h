@@ -199,7 +199,7 @@ int ffea_gpu_blob_cg_preconditioner(ffea_gpu_blob *blob, int *degree, double *la
 /* Name of the persistent CG kernel the blob's steps launch, fixed at creation by the blob's size and
  * precision alone (static string; "none" for masslumped, which solves no system):
  *   FP64: "cg_own_kernel" (each block keeps its rows on chip) or "cg_kernel" (grid-strided, larger blobs);
- *   mixed: "cg_mixed_sr_kernel" (CG_nomass, one reduction per iteration, FP32 matrix up to 64 MB so that it
+ *   mixed: "cg_mixed_sr_kernel" (CG_nomass, one reduction per iteration, FP32 matrix up to 100 MB so that it
  *   stays in L2), "cg_mixed_own_kernel" (two reductions, rows on chip) or "cg_mixed_kernel" (grid-strided). */
 const char *ffea_gpu_blob_cg_kernel(ffea_gpu_blob *blob);
 
