@@ -60,6 +60,7 @@ struct ffea_gpu_batch {
     Arena lin_mem;
     int *inc_ptr, *inc, *pinned, *slice_ptr, *rowlen, *bcol, *diagk, *src_ptr, *grp_slice;
     unsigned *src;
+    uchar4 *kpos = nullptr;  // the assembly by rows
     double *drag = nullptr;
     float *val, *dinv, *diag;
     float *x, *r, *q, *pbuf0, *pbuf1;
@@ -254,6 +255,13 @@ int ffea_gpu_batch::init() {
     CK(mem.upload(&grp_slice, h.grp_slice));
     CK(mem.upload(&src_ptr, h.src_ptr));
     CK(mem.upload(&src, h.src));
+    if (asm_row_fits<float>(h.width)) {
+        std::vector<uchar4> kp(h.inc.size());
+        for (size_t i = 0; i < kp.size(); ++i)
+            kp[i] = make_uchar4(h.kpos[4 * i], h.kpos[4 * i + 1], h.kpos[4 * i + 2], h.kpos[4 * i + 3]);
+        CK(mem.upload(&kpos, kp));
+        CK(Launch<float>::assemble_init());
+    }
     if (!h.drag.empty()) CK(mem.upload(&drag, h.drag));
     CK(mem.alloc(&val, 9 * (size_t)h.nslots));
     CK(mem.alloc(&dinv, 4 * (size_t)N));
@@ -597,6 +605,9 @@ int ffea_gpu_batch::launch_forces() {
     aa.slice_ptr = slice_ptr; aa.rowlen = rowlen; aa.bcol = bcol; aa.diagk = diagk;
     aa.src_ptr = src_ptr; aa.src = src;
     aa.geom = geom; aa.A = A; aa.B = B;
+        aa.inc_ptr = inc_ptr; aa.inc = inc; aa.pinned = pinned; aa.kpos = kpos;
+        aa.nslices = h.nslices;
+        aa.width = kpos ? h.width : 0;
     aa.drag = (p.calc_stokes == 1) ? drag : nullptr;
     aa.val = val; aa.dinv = dinv; aa.diag = diag; aa.st = st;
     aa.threads = asm_threads;

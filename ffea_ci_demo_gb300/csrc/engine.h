@@ -15,6 +15,8 @@ template <class R>
 struct Launch {
     static cudaError_t element(const ElemArgs<R> &a, cudaStream_t s);
     static cudaError_t assemble(const AsmArgs<R> &a, cudaStream_t s);
+    // the shared-memory limit of the assembly by rows, before the first launch (and outside stream capture)
+    static cudaError_t assemble_init();
     static cudaError_t gather(const GatherArgs<R> &a, int blocks, cudaStream_t s);
     // the step's midpoint forces (M midpoints) into out, for the gather's linearise replay
     static cudaError_t mid_force(const NodeForces &sn, int M, R *out, const DevStatus *st, cudaStream_t s);

@@ -154,6 +154,10 @@ struct HostModel {
     std::vector<std::vector<int>> nbr;  // sorted neighbours per vertex
     std::vector<int> src_ptr;
     std::vector<unsigned> src;
+    // per incidence entry (inc), the block index in the row of each of the element's four vertices (255: pinned, or a
+    // row of more blocks than that, `width` then being 0); width: the most blocks of any slice
+    std::vector<unsigned char> kpos;
+    int width = 0;
     // mass matrix values (solver CG), SELL scalar over the same pattern; lumped inverse masses
     std::vector<double> mass_sell, inv_mass;
     // Stokes noise: per vertex, the linearise events of its elements (element order), each holding up to
@@ -454,6 +458,21 @@ inline int build_model(const ffea_gpu_mesh *mesh, const ffea_gpu_params *p, Host
                     const long long k = slot_of(t[a], t[b]);
                     h.src[h.src_ptr[k] + fill[k]++] = ((unsigned)e << 4) | ((unsigned)a << 2) | (unsigned)b;
                 }
+            }
+        }
+    }
+    if (p->solver == FFEA_GPU_NOMASS_CG) {
+        for (int s = 0; s < h.nslices; ++s) h.width = std::max(h.width, (h.slice_ptr[s + 1] - h.slice_ptr[s]) / 32);
+        if (h.width >= 255) h.width = 0;
+        h.kpos.assign(h.width ? 4 * h.inc.size() : 0, 255);
+        for (int a = 0; a < N && h.width; ++a) {
+            if (h.pinned[a]) continue;
+            const auto &v = h.nbr[a];
+            for (int m = h.inc_ptr[a]; m < h.inc_ptr[a + 1]; ++m) {
+                const int *t = &h.tet4[4 * (size_t)(h.inc[m] >> 2)];
+                for (int b = 0; b < 4; ++b)
+                    if (!h.pinned[t[b]])
+                        h.kpos[4 * (size_t)m + b] = (unsigned char)(std::lower_bound(v.begin(), v.end(), t[b]) - v.begin());
             }
         }
     }

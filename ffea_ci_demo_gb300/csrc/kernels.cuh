@@ -434,6 +434,11 @@ struct AsmArgs {
     DevStatus *st;
     int threads;            // threads per block (0: the default); 64, 128 or 256
     int split;              // 0: three threads per slot while they fit on the GPU at once; 1: three; 2: one
+    // by rows (assemble_rows_kernel): each row's elements in order, element << 2 | vertex, and per element the row's block
+    // indices of its four vertices (255: pinned); width: the widest slice's blocks (0: no such lists)
+    const int *inc_ptr, *inc, *pinned;
+    const uchar4 *kpos;
+    int nslices, width;
 };
 
 constexpr unsigned SRC_IDENTITY = 0xffffffffu;
@@ -550,6 +555,92 @@ __global__ void __launch_bounds__(256) assemble_kernel(AsmArgs<R> g) {
     R *vp = g.val + 9 * (size_t)g.slice_ptr[s] + 32 * 9 * (size_t)k + lane + 32 * 3 * b0;
 #pragma unroll
     for (int c = 0; c < 3 * NB; ++c) vp[32 * c] = v[c];
+}
+
+// The assembly by rows: a block of 128 threads has one slice of 32 rows, four lanes to a row, lane b adding the 3x3 block
+// of (the row's vertex, vertex b) of each of the row's elements, in element order, into the row's blocks in shared
+// memory. An element's geometry is read once per row that holds it, as one 64-byte record, where a thread per slot
+// reads two gradients from scattered places for each of a slot's sources (16 an element): 40^3 cells 167 -> 103 us, 64^3
+// 618 -> 346 us (mixed; L1 requests bound it), 40^3 FP64 1114 -> 943 us (the FP64 pipe bounds it). The values leave as
+// they lie in the slice, whole lines at a time. Each slot's sum has the same terms in the same order as in
+// assemble_kernel, so the FP64 matrix is bit-identical. The shared rows are 33 apart, so that the four lanes of a row, on
+// blocks of the same row, fall on different banks.
+constexpr int ASM_ROW_THREADS = 128;
+template <class R>
+__host__ __device__ constexpr size_t asm_row_smem(int width) { return (size_t)9 * 33 * width * sizeof(R); }
+// Matrices whose widest slice leaves an SM three blocks in FP32, two in FP64. Measured at 40^3 cells with more shared
+// memory than its rows need: FP32 six blocks or more 103 us, three 125, two 164, one 258, by slots 166; FP64 942 us from
+// six blocks to two, by slots 1111.
+template <class R>
+constexpr size_t ASM_ROW_SMEM = (sizeof(R) == 4 ? 75 : 112) * (size_t)1024;
+template <class R>
+constexpr bool asm_row_fits(int width) { return width > 0 && asm_row_smem<R>(width) <= ASM_ROW_SMEM<R>; }
+
+template <class R>
+__global__ void __launch_bounds__(ASM_ROW_THREADS) assemble_rows_kernel(AsmArgs<R> g) {
+    extern __shared__ __align__(16) unsigned char asm_smem[];
+    R *const acc = reinterpret_cast<R *>(asm_smem);
+    if (g.st->abort) return;
+    const int s = blockIdx.x, r = threadIdx.x >> 2, b = threadIdx.x & 3, a = 32 * s + r;
+    const int base = g.slice_ptr[s], w = (g.slice_ptr[s + 1] - base) >> 5;
+    for (int i = threadIdx.x; i < 9 * 33 * w; i += ASM_ROW_THREADS) acc[i] = (R)0.0;
+    const bool row = a < g.N, fixed = row && g.pinned[a];
+    int m = row && !fixed ? g.inc_ptr[a] : 0;
+    const int m1 = row && !fixed ? g.inc_ptr[a + 1] : 0;
+    const int most = __reduce_max_sync(0xffffffffu, m1 - m);
+    // one element's record: the two gradients, the volume and the coefficients
+    struct Rec {
+        R ga[3], gb[3], vol, A, B;
+        int k;
+        bool same;
+    };
+    auto load = [&](int q, Rec &x) {
+        x.k = 255;
+        if (q >= m1) return;
+        const int es = g.inc[q], e = es >> 2, sa = es & 3;
+        const uchar4 kp = g.kpos[q];
+        x.k = b == 0 ? kp.x : b == 1 ? kp.y : b == 2 ? kp.z : kp.w;
+        x.same = sa == b;
+        const R *gm = g.geom + 16 * (size_t)e;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            x.ga[c] = gm[4 * c + sa];
+            x.gb[c] = gm[4 * c + b];
+        }
+        x.vol = gm[12];
+        x.A = g.A[e];
+        x.B = g.B[e];
+    };
+    __syncthreads();
+    Rec cur, next;
+    load(m, cur);
+    for (int i = 0; i < most; ++i) {
+        load(m + i + 1, next);
+        if (cur.k != 255) {
+            R *const v = acc + (size_t)9 * 33 * cur.k + r;
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                    v[33 * (3 * p + q)] += visc_block_entry<R>(cur.ga, cur.gb, cur.same, cur.A, cur.B, cur.vol, p, q);
+        }
+        __syncwarp();  // the next element of the row may add to the same blocks from other lanes
+        cur = next;
+    }
+    __syncthreads();
+    if (row && b < 3) {
+        R *const d = acc + (size_t)33 * (9 * g.diagk[a] + 4 * b) + r;
+        R x = *d;
+        if (fixed) x += (R)1;  // a pinned row is the identity
+        if (g.drag) x += (R)g.drag[a];
+        *d = x;
+        // calc_inverse_diagonal (src/SparseMatrixFixedPattern.cpp:305-312)
+        g.dinv[4 * a + b] = (R)1.0 / x;
+        if (g.diag) g.diag[4 * a + b] = x;
+    }
+    __syncthreads();
+    R *const out = g.val + 9 * (size_t)base;
+    for (int i = threadIdx.x; i < 9 * 32 * w; i += ASM_ROW_THREADS) out[i] = acc[33 * (i >> 5) + (i & 31)];
 }
 
 // ---------------------------------------------------------------------------

@@ -354,7 +354,8 @@ int ffea_gpu_batch_set_config(ffea_gpu_batch *batch, int cg_threads, int threads
 /* Launch shapes of the force phase: elements per thread block of the element kernel (64, 128, 256; the
  * block's vertices are staged in shared memory and its forces summed per vertex there), threads per
  * block of the assembly (64, 128, 256) and its slot split (0: three threads per matrix slot while they
- * fit on the GPU at once, 1: three, 2: one), threads per block of the node-force gather (64, 128, 256).
+ * fit on the GPU at once, 1: three, 2: one; both only for matrices with rows of very many blocks, others
+ * being assembled row by row), threads per block of the node-force gather (64, 128, 256).
  * Any shape gives the same trajectory to FP32 rounding (the block sums change grouping). */
 int ffea_gpu_batch_shapes(ffea_gpu_batch *batch, int *element_threads, int *assembly_threads, int *assembly_split,
                           int *gather_threads);

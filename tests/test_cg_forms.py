@@ -5,7 +5,7 @@ import pytest
 
 import pyoracle
 from ffea_ci_demo_gb300 import lib
-from ffea_ci_demo_gb300.mesh import apply_shear, kuhn_box
+from ffea_ci_demo_gb300.mesh import MID_EDGES, Mesh, apply_shear, kuhn_box
 
 
 def renumbered(m, shuffle):
@@ -112,3 +112,61 @@ def test_batch_solve_forms(cells):
         s.update(4)
         assert np.abs(bt.pos(b) - s.pos()).max() < 1e-5 * np.abs(s.pos() - x0[b]).max(), b
         assert np.array_equal(bt.rng_state(b), s.rng_state()), b
+
+
+# the FP64 assembly by rows (152 slices of 32 rows and more) beside the assembly by slots, against the oracle's matrix:
+# the last size by slots and the first by rows, pinned vertices and a Stokes drag on the diagonal
+@pytest.mark.gpu
+@pytest.mark.parametrize("cells", [(15, 15, 17), (16, 16, 16), (17, 17, 15)])
+def test_fp64_assembly_forms(cells):
+    m = kuhn_box(*cells, 5.0, seed=4)
+    m.pinned = np.nonzero(m.pos[:m.n_linear, 0] == 0.0)[0].astype(np.int32)
+    kw = dict(solver="CG_nomass", dt=1e-13, kT=4.11e-21, calc_noise=1, calc_stokes=1)
+    p0 = apply_shear(m, 0.001) * (m.scale / 1.7e-10)
+    p0[m.pinned] = m.pos[m.pinned] * (m.scale / 1.7e-10)
+    b, o = lib.Blob(m, **kw), pyoracle.OracleBlob(m, threads=1, **kw)
+    b.set_state(pos=p0)
+    o.set_pos(p0)
+    b.update(1)
+    assert o.step(1) == 0
+    g, c = b.pattern(), o.csr()
+    assert np.array_equal(g["key"], c["key"]) and np.array_equal(g["col"], c["col"])
+    assert np.array_equal(g["val"], c["val"])
+
+
+def fan(n, r=5.0, h=5.0):
+    """n elements around one edge, whose two vertices have rows of n + 2 blocks (pinned vertices have none)."""
+    th = 2 * np.pi * np.arange(n) / n
+    lin = np.vstack([[[0, 0, 0], [0, 0, h]], np.stack([r * np.cos(th), r * np.sin(th), np.full(n, 0.5 * h)], 1)])
+    i = np.arange(n)
+    t4 = np.stack([0 * i, 2 + i, 2 + (i + 1) % n, 1 + 0 * i], 1)
+    mid, tets = {}, []
+    for t in t4:
+        tets.append(list(t) + [mid.setdefault(tuple(sorted((t[a], t[b]))), n + 2 + len(mid)) for a, b in MID_EDGES])
+    pos = np.vstack([lin] + [0.5 * (lin[a] + lin[b])[None] for a, b in mid])
+    b = kuhn_box(1, 1, 1, h)
+    return Mesh(pos=pos, tets=np.array(tets, np.int32), material=np.tile(b.material[:1], (n, 1)),
+                stokes_radius=np.full(len(pos), 1.0), scale=b.scale, n_linear=n + 2)
+
+
+# the FP32 assembly: a ragged slice, whole slices and some rows more, three pins, and rows of 64 blocks (the widest by
+# rows) and 65 (by slots). An FP32 gradient is off by some 16 roundings, times 1 / sin of the narrowest angle through
+# the determinant; an entry has two gradients, a volume and two dozen additions: 128 roundings of the row's largest
+@pytest.mark.gpu
+@pytest.mark.parametrize("mesh,angle", [(lambda: kuhn_box(1, 1, 1, 5.0, seed=4), 0.5),
+                                        (lambda: kuhn_box(7, 1, 1, 5.0, seed=4), 0.5),
+                                        (lambda: kuhn_box(10, 2, 1, 5.0, seed=4), 0.5),
+                                        (lambda: kuhn_box(9, 9, 9, 5.0, seed=4), 0.5),
+                                        (lambda: fan(65), 2 * np.pi / 65), (lambda: fan(66), 2 * np.pi / 66)])
+def test_mixed_assembly_forms(mesh, angle):
+    m = mesh()
+    m.pinned = np.arange(2, 5, dtype=np.int32)
+    kw = dict(solver="CG_nomass", dt=1e-16, kT=4.11e-21, calc_noise=0, calc_stokes=1)
+    b, o = lib.Blob(m, precision="mixed", **kw), pyoracle.OracleBlob(m, threads=1, **kw)
+    b.update(1)
+    assert o.step(1) == 0
+    g, c = b.pattern(), o.csr()
+    assert np.array_equal(g["key"], c["key"]) and np.array_equal(g["col"], c["col"])
+    scale = np.maximum.reduceat(np.abs(c["val"]), c["key"][:-1])[np.repeat(np.arange(len(c["key"]) - 1),
+                                                                         np.diff(c["key"]))]
+    assert (np.abs(g["val"] - c["val"]) <= 128 * 2.0**-24 / np.sin(angle) * scale).all()
