@@ -418,6 +418,10 @@ def run_batch(args, ws, rank=0, ranks=None) -> dict:
     ms = t["ms"] / k
     cg_ms = t["cg_ms"] / k
     peak, peak_kind = measured_peak()
+    # the on-chip solve has one 512-thread block per SM; cg_batch_kernel's groups at that size have two
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    kernel = "sr_batch_kernel" if cfg["cg_threads"] == 512 and cfg["ctas"] <= sms else "cg_batch_kernel"
     out = {"workload": f"ensemble of {args.blobs} Kuhn cubes, cells per side log-uniform in [8,32] (seeded), "
                        f"G ~ U[1e8,1e9] Pa, K = 3.9 G; NoMassCG eps=1e-10, dt=1e-12 s, kT=4.11e-21 J, mixed",
            "blobs": len(meshes_all), "nodes": nodes_all, "tets": sum(m.n_elem for m in meshes_all),
@@ -428,19 +432,20 @@ def run_batch(args, ws, rank=0, ranks=None) -> dict:
            "cg_iters_per_blob": {"min": int(last.min()), "mean": float(last.mean()), "max": int(last.max())},
            "launch_config": cfg, "tuned_best_solve_ms": tuned_ms, "gpu_launches": launches,
            "clocks": clk.summary(),
-           "roofline": {"bound": "hbm", "kernel": "cg_batch_kernel",
+           "roofline": {"bound": "hbm", "kernel": kernel,
                         "achieved": fmt / (cg_ms / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                         "frac": fmt / (cg_ms / 1e3) / 1e9 / peak, "peak_source": peak_kind,
                         "ms_per_launch": cg_ms,
                         "frac_over_whole_step": fmt / (ms / 1e3) / 1e9 / peak,
                         "bytes": "SELL format per CG iteration of each blob x its iterations",
-                        "traffic": (fmt * ratio) if (ratio := profiled("cg_batch_kernel_ensemble64",
+                        "traffic": (fmt * ratio) if (ratio := profiled(f"{kernel}_ensemble64",
                                                                        "dram_bytes_per_format_byte")) else None,
                         "traffic_note": "DRAM bytes per step scaled by format bytes from the ncu capture of a timed "
-                                        "launch of the 64-blob ensemble (profiles/cg_batch_kernel_ensemble64.txt)",
+                                        f"launch of the 64-blob ensemble (profiles/{kernel}_ensemble64.txt)"
+                        if ratio else None,
                         # the captured launch's DRAM bytes over its duration, against the measured copy peak
-                        "dram_frac_cg_kernel": profiled("cg_batch_kernel_ensemble64", "dram_gbs") / peak
-                        if profiled("cg_batch_kernel_ensemble64", "dram_gbs") else None,
+                        "dram_frac_cg_kernel": profiled(f"{kernel}_ensemble64", "dram_gbs") / peak
+                        if profiled(f"{kernel}_ensemble64", "dram_gbs") else None,
                         "bytes_per_step_format_cg": fmt, "bytes_per_step_model_cg": model,
                         "model_equiv_gbs": model / (ms / 1e3) / 1e9}}
     if ws > 1:
