@@ -102,7 +102,8 @@ cudaError_t Launch<R>::gather(const GatherArgs<R> &a, int blocks, cudaStream_t s
 template <class R>
 cudaError_t Launch<R>::mid_force(const NodeForces &sn, int M, R *out, const DevStatus *st, cudaStream_t s) {
     if (M <= 0) return cudaSuccess;
-    mid_force_kernel<R><<<(M + 255) / 256, 256, 0, s>>>(sn, M, out, st);
+    // small blocks: the draws' scaling is FP64, and more SMs have more FP64 units
+    mid_force_kernel<R><<<(M + 63) / 64, 64, 0, s>>>(sn, M, out, st);
     count_launch();
     return cudaGetLastError();
 }

@@ -728,22 +728,45 @@ __device__ __forceinline__ void midpoint_force(const NodeForces &sn, int m, R (&
 // the vertex's share of Blob::linearise_force (src/Blob.cpp:781-799): for each element holding the vertex,
 // in element order, force += 0.5 * (f_m1 + f_m2 + f_m3) over that element's three midpoints at the vertex
 // that still carry force (a midpoint's force is moved by the first element holding it, then zeroed)
+// Where mid_force_kernel has formed the midpoints' forces, LIN_EVENTS events are in flight (each is two dependent loads,
+// whose latency sets the time) and are added in order; with the midpoints' draws in blocks of 64 the gather phase of
+// the 64-node FP64 blob goes 28.4 -> 24.3 us, of 2720 nodes mixed 24.5 -> 22.5, of 9261 nodes FP64 34.0 -> 30.6.
+constexpr int LIN_EVENTS = 4;
 template <class R>
 __device__ __forceinline__ void midpoint_linearise(const NodeForces &sn, int a, R (&F)[3]) {
-    for (int k = sn.lin_ptr[a]; k < sn.lin_ptr[a + 1]; ++k) {
+    const int k1 = sn.lin_ptr[a + 1];
+    int k = sn.lin_ptr[a];
+    if (sn.mid_f) {
+        const R *mid_f = static_cast<const R *>(sn.mid_f);
+        for (; k < k1; k += LIN_EVENTS) {
+            int4 ev[LIN_EVENTS];
+#pragma unroll
+            for (int i = 0; i < LIN_EVENTS; ++i) ev[i] = sn.lin_ev[min(k + i, k1 - 1)];
+            R fm[LIN_EVENTS][3][3];
+#pragma unroll
+            for (int i = 0; i < LIN_EVENTS; ++i) {
+                const int m[3] = {ev[i].x, ev[i].y, ev[i].z};
+#pragma unroll
+                for (int j = 0; j < 3; ++j)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) fm[i][j][c] = m[j] < 0 ? (R)0 : mid_f[3 * (size_t)m[j] + c];
+            }
+#pragma unroll
+            for (int i = 0; i < LIN_EVENTS; ++i)
+                if (k + i < k1)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) F[c] += (R)0.5 * (fm[i][0][c] + fm[i][1][c] + fm[i][2][c]);
+        }
+        return;
+    }
+    for (; k < k1; ++k) {
         const int4 ev = sn.lin_ev[k];
         const int m[3] = {ev.x, ev.y, ev.z};
         R fm[3][3];
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             fm[j][0] = fm[j][1] = fm[j][2] = (R)0;
-            if (m[j] < 0) continue;
-            if (sn.mid_f) {
-                const R *mf = static_cast<const R *>(sn.mid_f) + 3 * (size_t)m[j];
-                fm[j][0] = mf[0]; fm[j][1] = mf[1]; fm[j][2] = mf[2];
-            } else {
-                midpoint_force<R>(sn, m[j], fm[j]);
-            }
+            if (m[j] >= 0) midpoint_force<R>(sn, m[j], fm[j]);
         }
 #pragma unroll
         for (int c = 0; c < 3; ++c) F[c] += (R)0.5 * (fm[0][c] + fm[1][c] + fm[2][c]);

@@ -170,3 +170,17 @@ def test_mixed_assembly_forms(mesh, angle):
     scale = np.maximum.reduceat(np.abs(c["val"]), c["key"][:-1])[np.repeat(np.arange(len(c["key"]) - 1),
                                                                          np.diff(c["key"]))]
     assert (np.abs(g["val"] - c["val"]) <= 128 * 2.0**-24 / np.sin(angle) * scale).all()
+
+
+# the midpoints' Stokes noise on the vertices, four linearise events in flight: vertices with one event to 24 and (the
+# fan's axis) 69, so every remainder of four; the right-hand side bit for bit
+@pytest.mark.gpu
+@pytest.mark.parametrize("mesh", [lambda: kuhn_box(1, 1, 1, 5.0, seed=4), lambda: kuhn_box(3, 2, 4, 5.0, seed=4),
+                                  lambda: fan(69)])
+def test_midpoint_noise_forms(mesh):
+    m = mesh()
+    kw = dict(solver="CG", dt=1e-16, kT=4.11e-21, calc_noise=1, calc_stokes=1)
+    b, o = lib.Blob(m, **kw), pyoracle.OracleBlob(m, threads=1, **kw)
+    b.update(1)
+    assert o.step(1) == 0
+    assert np.array_equal(b.rhs()[:m.n_linear], o.rhs()[:m.n_linear])
