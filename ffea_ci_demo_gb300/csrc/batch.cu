@@ -58,9 +58,10 @@ struct ffea_gpu_batch {
     std::vector<CtfModel> ctf_models;
     CtfDevice ctf;
     Arena lin_mem;
-    int *inc_ptr, *inc, *pinned, *slice_ptr, *rowlen, *bcol, *diagk, *src_ptr, *grp_slice;
-    unsigned *src;
-    uchar4 *kpos = nullptr;  // the assembly by rows
+    int *inc_ptr, *inc, *pinned, *slice_ptr, *rowlen, *bcol, *diagk;
+    int *src_ptr = nullptr, *grp_slice = nullptr;  // the assembly by slots, or
+    unsigned *src = nullptr;
+    unsigned char *kpos = nullptr;  // by rows
     double *drag = nullptr;
     float *val, *dinv, *diag;
     float *x, *r, *q, *pbuf0, *pbuf1;
@@ -252,15 +253,13 @@ int ffea_gpu_batch::init() {
     CK(mem.upload(&rowlen, h.rowlen));
     CK(mem.upload(&bcol, h.bcol));
     CK(mem.upload(&diagk, h.diagk));
-    CK(mem.upload(&grp_slice, h.grp_slice));
-    CK(mem.upload(&src_ptr, h.src_ptr));
-    CK(mem.upload(&src, h.src));
-    if (asm_row_fits<float>(h.width)) {
-        std::vector<uchar4> kp(h.inc.size());
-        for (size_t i = 0; i < kp.size(); ++i)
-            kp[i] = make_uchar4(h.kpos[4 * i], h.kpos[4 * i + 1], h.kpos[4 * i + 2], h.kpos[4 * i + 3]);
-        CK(mem.upload(&kpos, kp));
+    if (asm_by_rows<float>(h.width, h.nslices)) {  // (CG_nomass alone has row lists)
+        CK(mem.upload(&kpos, h.kpos));
         CK(Launch<float>::assemble_init());
+    } else {
+        CK(mem.upload(&grp_slice, h.grp_slice));
+        CK(mem.upload(&src_ptr, h.src_ptr));
+        CK(mem.upload(&src, h.src));
     }
     if (!h.drag.empty()) CK(mem.upload(&drag, h.drag));
     CK(mem.alloc(&val, 9 * (size_t)h.nslots));
@@ -605,9 +604,10 @@ int ffea_gpu_batch::launch_forces() {
     aa.slice_ptr = slice_ptr; aa.rowlen = rowlen; aa.bcol = bcol; aa.diagk = diagk;
     aa.src_ptr = src_ptr; aa.src = src;
     aa.geom = geom; aa.A = A; aa.B = B;
-        aa.inc_ptr = inc_ptr; aa.inc = inc; aa.pinned = pinned; aa.kpos = kpos;
-        aa.nslices = h.nslices;
-        aa.width = kpos ? h.width : 0;
+    aa.inc_ptr = inc_ptr; aa.inc = inc; aa.pinned = pinned;
+    aa.kpos = reinterpret_cast<const uchar4 *>(kpos);
+    aa.nslices = h.nslices;
+    aa.width = kpos ? h.width : 0;
     aa.drag = (p.calc_stokes == 1) ? drag : nullptr;
     aa.val = val; aa.dinv = dinv; aa.diag = diag; aa.st = st;
     aa.threads = asm_threads;

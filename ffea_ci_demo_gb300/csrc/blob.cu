@@ -168,9 +168,10 @@ struct BlobImpl final : ffea_gpu_blob {
     R *jinv, *G, *E, *A, *B, *vol0, *ef = nullptr, *geom = nullptr;
     double *last_det;
     int *inc_ptr, *inc, *pinned;
-    int *slice_ptr, *rowlen, *bcol, *diagk, *src_ptr, *grp_slice;
-    unsigned *src;
-    uchar4 *kpos = nullptr;  // the assembly by rows
+    int *slice_ptr, *rowlen, *bcol, *diagk;
+    int *src_ptr = nullptr, *grp_slice = nullptr;  // the assembly by slots, or
+    unsigned *src = nullptr;
+    unsigned char *kpos = nullptr;  // by rows
     double *drag = nullptr;
     R *val, *dinv;
     double *f;
@@ -462,16 +463,14 @@ struct BlobImpl final : ffea_gpu_blob {
         CK(mem.upload(&rowlen, h.rowlen));
         CK(mem.upload(&bcol, h.bcol));
         CK(mem.upload(&diagk, h.diagk));
-        CK(mem.upload(&grp_slice, h.grp_slice));
-        CK(mem.upload(&src_ptr, h.src_ptr));
-        CK(mem.upload(&src, h.src));
-    if (asm_row_fits<R>(h.width)) {
-        std::vector<uchar4> kp(h.inc.size());
-        for (size_t i = 0; i < kp.size(); ++i)
-            kp[i] = make_uchar4(h.kpos[4 * i], h.kpos[4 * i + 1], h.kpos[4 * i + 2], h.kpos[4 * i + 3]);
-        CK(mem.upload(&kpos, kp));
-        CK(Launch<R>::assemble_init());
-    }
+        if (asm_by_rows<R>(h.width, h.nslices)) {  // (CG_nomass alone has row lists)
+            CK(mem.upload(&kpos, h.kpos));
+            CK(Launch<R>::assemble_init());
+        } else {
+            CK(mem.upload(&grp_slice, h.grp_slice));
+            CK(mem.upload(&src_ptr, h.src_ptr));
+            CK(mem.upload(&src, h.src));
+        }
         if (!h.drag.empty()) CK(mem.upload(&drag, h.drag));
         const bool block3 = p.solver == FFEA_GPU_NOMASS_CG;
         if (p.solver == FFEA_GPU_CG) {
@@ -749,7 +748,8 @@ struct BlobImpl final : ffea_gpu_blob {
         aa.slice_ptr = slice_ptr; aa.rowlen = rowlen; aa.bcol = bcol; aa.diagk = diagk;
         aa.src_ptr = src_ptr; aa.src = src;
         aa.geom = geom; aa.A = A; aa.B = B;
-        aa.inc_ptr = inc_ptr; aa.inc = inc; aa.pinned = pinned; aa.kpos = kpos;
+        aa.inc_ptr = inc_ptr; aa.inc = inc; aa.pinned = pinned;
+        aa.kpos = reinterpret_cast<const uchar4 *>(kpos);
         aa.nslices = h.nslices;
         aa.width = kpos ? h.width : 0;
         aa.drag = (p.calc_stokes == 1) ? drag : nullptr;

@@ -46,10 +46,7 @@ cudaError_t Launch<R>::assemble(const AsmArgs<R> &a, cudaStream_t s) {
     if (a.N <= 0 || a.nslots <= 0) return cudaSuccess;
     const int bt = a.threads > 0 ? a.threads : ASM_THREADS;
     if (!(bt == 64 || bt == 128 || bt == 256)) return cudaErrorInvalidValue;
-    // by rows, except FP64 blobs that leave SMs free, where three threads per slot shorten the chain of FP64 adds; us by
-    // rows against by slots: FP64 343 / 2197 / 9261 / 68,921 nodes 85 / 86 / 144 / 945 against 35 / 73 / 216 / 1114, mixed
-    // 2720 / 9261 / 68,921 / 274,625 nodes 24 / 27 / 103 / 346 against 36 / 35 / 167 / 618
-    if (a.width > 0 && (std::is_same<R, float>::value || a.nslices >= 152)) {
+    if (asm_by_rows<R>(a.width, a.nslices)) {
         assemble_rows_kernel<R><<<a.nslices, ASM_ROW_THREADS, asm_row_smem<R>(a.width), s>>>(a);
         count_launch();
         return cudaGetLastError();

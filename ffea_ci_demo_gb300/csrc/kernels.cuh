@@ -575,6 +575,13 @@ template <class R>
 constexpr size_t ASM_ROW_SMEM = (sizeof(R) == 4 ? 75 : 112) * (size_t)1024;
 template <class R>
 constexpr bool asm_row_fits(int width) { return width > 0 && asm_row_smem<R>(width) <= ASM_ROW_SMEM<R>; }
+// The rule: by rows wherever they fit, except FP64 blobs that leave SMs free, where three threads per slot shorten the
+// chain of FP64 adds; us by rows against by slots: FP64 343 / 2197 / 9261 / 68,921 nodes 85 / 86 / 144 / 945 against
+// 35 / 73 / 216 / 1114, mixed 2720 / 9261 / 68,921 / 274,625 nodes 24 / 27 / 103 / 346 against 36 / 35 / 167 / 618.
+template <class R>
+constexpr bool asm_by_rows(int width, int nslices) {
+    return asm_row_fits<R>(width) && (sizeof(R) == 4 || nslices >= 152);
+}
 
 template <class R>
 __global__ void __launch_bounds__(ASM_ROW_THREADS) assemble_rows_kernel(AsmArgs<R> g) {
