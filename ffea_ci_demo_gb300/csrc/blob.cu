@@ -463,10 +463,10 @@ struct BlobImpl final : ffea_gpu_blob {
         CK(mem.upload(&rowlen, h.rowlen));
         CK(mem.upload(&bcol, h.bcol));
         CK(mem.upload(&diagk, h.diagk));
-        if (asm_by_rows<R>(h.width, h.nslices)) {  // (CG_nomass alone has row lists)
+        if (asm_by_rows<R>(h.width, h.nslices)) {  // (the other solvers have no such matrix)
             CK(mem.upload(&kpos, h.kpos));
             CK(Launch<R>::assemble_init());
-        } else {
+        } else if (p.solver == FFEA_GPU_NOMASS_CG) {
             CK(mem.upload(&grp_slice, h.grp_slice));
             CK(mem.upload(&src_ptr, h.src_ptr));
             CK(mem.upload(&src, h.src));
