@@ -25,6 +25,7 @@
 // S2 = sum d_a x v_a; D Z c at node a is D_a (tau + Omega x d_a).
 #pragma once
 
+#include "cg_shapes.h"
 #include "kernels.cuh"
 #include "kernels_element_mixed.cuh"
 
@@ -1096,16 +1097,7 @@ struct SrForm {
 };
 constexpr int SR_REG_ROWS = 128;  // rows a block is given while the mesh leaves SMs free
 
-// Bytes of dynamic shared memory cg_mixed_sr_kernel needs for npb owned rows and a halo of nhalo: the staged vector,
-// x, r, p, q, w, D^{-1}, D, d, and with a polynomial preconditioner u (the preconditioned
-// residual) and the Chebyshev correction.
-constexpr int SR_FIELDS = 24;
-constexpr int SR_FIELDS_POLY = 30;
-__host__ __device__ constexpr size_t sr_smem_bytes(int npb, int nhalo, int poly) {
-    return (size_t)(poly > 0 ? SR_FIELDS_POLY : SR_FIELDS) * npb * sizeof(float) +
-           ((size_t)npb + nhalo) * sizeof(float4);
-}
-// ... plus the matrix cache of kc blocks per row at stride S: nine values and a local column each
+// sr_smem_bytes grows by the matrix cache of kc blocks per row at stride S: nine values and a local column each
 constexpr int SR_CACHE_BYTES_PER_BLOCK = 9 * 4 + 2;
 __host__ __device__ constexpr size_t sr_cache_bytes(int kc, int S) {
     return (size_t)SR_CACHE_BYTES_PER_BLOCK * kc * S;
@@ -1118,7 +1110,6 @@ __host__ __device__ constexpr size_t sr_cache_bytes(int kc, int S) {
 // coefficients, then [CHEB_KJ] the iterations of the Jacobi solve while the first polynomial solve (the trial)
 // is pending, then (CHEB_COEF) the recurrence's coefficients for the estimate.
 constexpr int CHEB_MAX = 8;
-constexpr int CHEB_REC = 64;
 // the interval's width: degrees 4 and up gain from a wider one (40^3 Kuhn cube, degree 4, CG per step: ratio 30
 // 4.24 ms, 60 4.10, 120 4.04, 250 4.06), degree 2 hardly (30 4.17, 60 4.14, 120 4.17 ms)
 __host__ __device__ constexpr double cheb_ratio(int degree) { return degree > 2 ? 120.0 : 30.0; }
