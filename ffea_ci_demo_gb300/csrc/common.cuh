@@ -325,6 +325,10 @@ __device__ __forceinline__ df32 df_of(double v) {
 
 __device__ __forceinline__ double df_double(df32 v) { return (double)v.hi + (double)v.lo; }
 
+// The smallest tolerance |r|^2 is tested against as a pair: below it a pair's low part leaves FP32's range, and from 1e-45
+// on the pair is zero and nothing is less, so the tests there are made in FP64 (|r|^2 may round to zero, which is less).
+constexpr float DF_TEST_MIN = 1e-30f;
+
 __device__ __forceinline__ bool df_less(df32 a, df32 b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); }
 
 __device__ __forceinline__ df32 df_shfl_xor(df32 v, int o) {

@@ -1,0 +1,47 @@
+"""The CG solves at the ends of their ranges: tiny forces, the smallest blobs."""
+import numpy as np
+import pytest
+
+from ffea_ci_demo_gb300 import lib
+from ffea_ci_demo_gb300.mesh import apply_shear, kuhn_box
+
+
+# |f|^2 of about 1e-25 and 1e-27: the tolerance 1e-20 |f|^2 (1e-45, 1e-47) is at and below FP32's smallest number, |r|^2
+# rounds to zero first and is less than it in FP64. Viscosity (and density) keep the diagonal below 1, so that r.z and p.q
+# outlast |r|^2. The mixed path's bound against FP64 (velocities: the moves are below the positions' rounding).
+@pytest.mark.gpu
+@pytest.mark.parametrize("solver,kernel", [("CG_nomass", "cg_mixed_sr_kernel"), ("CG", "cg_mixed_own_kernel")])
+@pytest.mark.parametrize("scale", [1e-10, 1e-11])
+def test_mixed_solve_of_a_tiny_force_converges(gpu, solver, kernel, scale):
+    m = kuhn_box(3, 3, 3, 5.0, seed=4)
+    m.material = m.material.copy()
+    m.material[:, 3:5] *= scale
+    m.material[:, 1:3] *= 1e-3 if solver == "CG_nomass" else 1e-6
+    m.material[:, 0] *= 1.0 if solver == "CG_nomass" else 1e-6
+    v = {}
+    for prec in ("fp64", "mixed"):
+        b = lib.Blob(m, solver=solver, precision=prec, dt=1e-16, kT=0.0, calc_noise=0)
+        b.set_state(pos=apply_shear(m, 1e-6) * (m.scale / 1.7e-10))
+        b.update(1)
+        v[prec] = b.vel()
+    assert b.cg_kernel() == kernel
+    assert 0 < (b.rhs() ** 2).sum() < 1e-24
+    assert np.abs(v["mixed"] - v["fp64"]).max() < 1e-5 * np.abs(v["fp64"]).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("solver", ["CG_nomass", "CG"])
+def test_one_element_blob(gpu, solver):
+    """A single tetrahedron: four rows, its first solve's Lanczos record and the polynomial's solves after it."""
+    from test_mixed_elements import one_tet
+
+    m = one_tet()
+    kw = dict(solver=solver, dt=1e-14, kT=4.11e-21, calc_noise=1)
+    p0 = apply_shear(m, 0.001) * (m.scale / 1.7e-10)
+    out = {}
+    for prec in ("fp64", "mixed"):
+        b = lib.Blob(m, precision=prec, **kw)
+        b.set_state(pos=p0)
+        b.update(4)
+        out[prec] = b.pos()
+    assert np.abs(out["mixed"] - out["fp64"]).max() < 1e-5 * np.abs(out["fp64"] - p0).max()
