@@ -114,7 +114,7 @@ int Launch<R>::cg_max_grid(int device) {
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
     cudaError_t e;
     if constexpr (std::is_same<R, float>::value)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cg_mixed_kernel<R>, CG_THREADS, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cg_mixed_kernel<R, true>, CG_THREADS, 0);
     else
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cg_kernel<R>, CG_THREADS, 0);
     if (e != cudaSuccess) return 0;
@@ -202,7 +202,7 @@ cudaError_t Launch<R>::cg(const CgArgs<R> &a, int grid, int threads, cudaStream_
     const void *fn;
     size_t smem = 0;
     if constexpr (std::is_same<R, float>::value) {
-        fn = (const void *)cg_mixed_kernel<R>;
+        fn = a.block3 ? (const void *)cg_mixed_kernel<R, true> : (const void *)cg_mixed_kernel<R, false>;
         if (a.npb > 0 && a.sr) {
             fn = a.reg == 4   ? (const void *)cg_mixed_sr_kernel<R, 4>
                  : a.reg == 6 ? (const void *)cg_mixed_sr_kernel<R, 6>

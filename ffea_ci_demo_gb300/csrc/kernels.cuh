@@ -1109,55 +1109,18 @@ struct CgArgs {
     int reg;              // cg_mixed_sr_kernel: blocks of each lane in registers (its form: 0, 4 or 6)
 };
 
-// p at node b for this iteration: p_new = beta p_old + D^{-1} r (vec3_scale_and_add with the
-// preconditioned residual, src/NoMassCGSolver.cpp:181-183), or z itself on the first iteration.
+// Row a of q = V p, summed by the tpn lanes of a node group over blocks k = sub, sub + tpn, ... and combined with
+// shuffles; every lane of the group returns the row. All 32 lanes of the warp call it together (rows past the end pass
+// valid = false).
 template <class A, class R>
-__device__ __forceinline__ void p_on_the_fly(const A &g, const R *pold, R beta, bool first, int b, R &p0, R &p1,
-                                              R &p2) {
-    const R z0 = g.dinv[4 * b] * g.r[4 * b], z1 = g.dinv[4 * b + 1] * g.r[4 * b + 1],
-            z2 = g.dinv[4 * b + 2] * g.r[4 * b + 2];
-    if (first) {
-        p0 = z0; p1 = z1; p2 = z2;
-    } else {
-        p0 = fma(beta, pold[4 * b], z0);
-        p1 = fma(beta, pold[4 * b + 1], z1);
-        p2 = fma(beta, pold[4 * b + 2], z2);
-    }
-}
-
-// Row a of q = V p, summed by the tpn lanes of a node group over blocks k = sub, sub + tpn, ... and
-// combined with shuffles; every lane of the group returns the row. All 32 lanes of the warp call it
-// together (rows past the end pass valid = false). ONTHEFLY: p is formed from p_old, r and D^{-1}
-// (mixed path); otherwise it is read from pold (FP64 path).
-template <bool ONTHEFLY, class A, class R>
-__device__ __forceinline__ void spmv_row(const A &g, const R *pold, R beta, bool first, int a, int sub, bool valid,
-                                         R &q0, R &q1, R &q2) {
+__device__ __forceinline__ void spmv_row(const A &g, const R *p, int a, int sub, bool valid, R &q0, R &q1, R &q2) {
     q0 = 0.0; q1 = 0.0; q2 = 0.0;
     const int tpn = g.tpn;
     if (valid) {
         const int s = a >> 5, lane = a & 31;
         const int base = g.slice_ptr[s];
         const int len = g.rowlen[a];
-        if (g.block3 && ONTHEFLY) {
-            // one block per trip, the next block's column index prefetched so that its dependent
-            // loads can issue as soon as the current trip's loads are out
-            const R *v = g.val + 9 * (size_t)base + lane;
-            int k = sub;
-            int bn = (k < len) ? g.bcol[base + 32 * k + lane] : 0;
-#pragma unroll 1
-            for (; k < len; k += tpn) {
-                const int b = bn;
-                if (k + tpn < len) bn = g.bcol[base + 32 * (k + tpn) + lane];
-                const R *vk = v + (size_t)32 * 9 * k;
-                const R v0 = vk[0], v1 = vk[32], v2 = vk[64], v3 = vk[96], v4 = vk[128], v5 = vk[160], v6 = vk[192],
-                        v7 = vk[224], v8 = vk[256];
-                R p0, p1, p2;
-                p_on_the_fly(g, pold, beta, first, b, p0, p1, p2);
-                q0 = fma(v0, p0, q0); q0 = fma(v1, p1, q0); q0 = fma(v2, p2, q0);
-                q1 = fma(v3, p0, q1); q1 = fma(v4, p1, q1); q1 = fma(v5, p2, q1);
-                q2 = fma(v6, p0, q2); q2 = fma(v7, p1, q2); q2 = fma(v8, p2, q2);
-            }
-        } else if (g.block3) {
+        if (g.block3) {
             const R *v = g.val + 9 * (size_t)base + lane;
 #pragma unroll 1
             for (int k = sub; k < len; k += tpn) {
@@ -1165,12 +1128,7 @@ __device__ __forceinline__ void spmv_row(const A &g, const R *pold, R beta, bool
                 const R *vk = v + (size_t)32 * 9 * k;
                 const R v0 = vk[0], v1 = vk[32], v2 = vk[64], v3 = vk[96], v4 = vk[128], v5 = vk[160], v6 = vk[192],
                         v7 = vk[224], v8 = vk[256];
-                R p0, p1, p2;
-                if (ONTHEFLY) {
-                    p_on_the_fly(g, pold, beta, first, b, p0, p1, p2);
-                } else {
-                    p0 = pold[4 * b]; p1 = pold[4 * b + 1]; p2 = pold[4 * b + 2];
-                }
+                const R p0 = p[4 * b], p1 = p[4 * b + 1], p2 = p[4 * b + 2];
                 q0 = fma(v0, p0, q0); q0 = fma(v1, p1, q0); q0 = fma(v2, p2, q0);
                 q1 = fma(v3, p0, q1); q1 = fma(v4, p1, q1); q1 = fma(v5, p2, q1);
                 q2 = fma(v6, p0, q2); q2 = fma(v7, p1, q2); q2 = fma(v8, p2, q2);
@@ -1180,15 +1138,9 @@ __device__ __forceinline__ void spmv_row(const A &g, const R *pold, R beta, bool
             for (int k = sub; k < len; k += tpn) {
                 const int b = g.bcol[base + 32 * k + lane];
                 const R m = v[32 * k];
-                R p0, p1, p2;
-                if (ONTHEFLY) {
-                    p_on_the_fly(g, pold, beta, first, b, p0, p1, p2);
-                } else {
-                    p0 = pold[4 * b]; p1 = pold[4 * b + 1]; p2 = pold[4 * b + 2];
-                }
-                q0 = fma(m, p0, q0);
-                q1 = fma(m, p1, q1);
-                q2 = fma(m, p2, q2);
+                q0 = fma(m, p[4 * b], q0);
+                q1 = fma(m, p[4 * b + 1], q1);
+                q2 = fma(m, p[4 * b + 2], q2);
             }
         }
     }
@@ -1291,7 +1243,7 @@ __global__ void __launch_bounds__(1024, 1) cg_kernel(const __grid_constant__ CgA
         {
             FFEA_SPMV_LOOP(g, a, sub, valid) {
                 R q0, q1, q2;
-                spmv_row<false>(g, p, (R)0, false, a, sub, valid, q0, q1, q2);
+                spmv_row(g, p, a, sub, valid, q0, q1, q2);
                 if (valid && sub == 0) {
                     g.q[4 * a] = q0; g.q[4 * a + 1] = q1; g.q[4 * a + 2] = q2;
                     acc1[0] += (double)fma(p[4 * a + 2], q2, fma(p[4 * a + 1], q1, p[4 * a] * q0));

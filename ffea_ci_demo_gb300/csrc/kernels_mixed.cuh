@@ -270,7 +270,93 @@ __device__ __noinline__ void mixed_setup(const A &g, const double *s_sc, double 
     __syncthreads();
 }
 
-template <class R>
+// p at node b for this iteration: p_new = beta p_old + D^{-1} r (vec3_scale_and_add with the
+// preconditioned residual, src/NoMassCGSolver.cpp:181-183), or z itself on the first iteration.
+template <class A>
+__device__ __forceinline__ void p_on_the_fly(const A &g, const float *pold, float beta, bool first, int b, float &p0,
+                                             float &p1, float &p2) {
+    const float4 di = *reinterpret_cast<const float4 *>(g.dinv + 4 * (size_t)b),
+                 r = *reinterpret_cast<const float4 *>(g.r + 4 * (size_t)b);
+    p0 = di.x * r.x;
+    p1 = di.y * r.y;
+    p2 = di.z * r.z;
+    if (!first) {
+        const float4 po = *reinterpret_cast<const float4 *>(pold + 4 * (size_t)b);
+        p0 = fmaf(beta, po.x, p0);
+        p1 = fmaf(beta, po.y, p1);
+        p2 = fmaf(beta, po.z, p2);
+    }
+}
+
+// spmv_row with p formed on the fly from p_old, r and D^{-1}; B3: 3x3 blocks (CG_nomass) or scalar entries. The blobs
+// here have matrices far larger than L2, read past it (__ldcs), and two blocks' loads issue before either's products, in
+// the same order. With one block per trip the time hung on how the compiler placed the loads around whatever else was in
+// registers: ms per step at 76^3 / 80^3 / 96^3 cells 85 / 113 / 201 or 115 / 155 / 274, now 75 / 102 / 196; consistent
+// mass 76^3 1.70 (1.67 to 1.91).
+template <bool B3, class A>
+__device__ __forceinline__ void spmv_row_fly(const A &g, const float *pold, float beta, bool first, int a, int sub,
+                                             bool valid, float &q0, float &q1, float &q2) {
+    q0 = 0.f; q1 = 0.f; q2 = 0.f;
+    const int tpn = g.tpn;
+    if (valid) {
+        const int s = a >> 5, lane = a & 31;
+        const int base = g.slice_ptr[s];
+        const int len = g.rowlen[a];
+        if constexpr (B3) {
+            const float *v = g.val + 9 * (size_t)base + lane;
+            int k = sub;
+#pragma unroll 1
+            for (; k + tpn < len; k += 2 * tpn) {
+                const int ba = __ldg(g.bcol + base + 32 * k + lane), bb = __ldg(g.bcol + base + 32 * (k + tpn) + lane);
+                const float *va = v + (size_t)32 * 9 * k, *vb = v + (size_t)32 * 9 * (k + tpn);
+                float wa[9], wb[9];
+#pragma unroll
+                for (int i = 0; i < 9; ++i) {
+                    wa[i] = __ldcs(va + 32 * i);
+                    wb[i] = __ldcs(vb + 32 * i);
+                }
+                float a0, a1, a2, b0, b1, b2;
+                p_on_the_fly(g, pold, beta, first, ba, a0, a1, a2);
+                p_on_the_fly(g, pold, beta, first, bb, b0, b1, b2);
+                q0 = fmaf(wa[0], a0, q0); q0 = fmaf(wa[1], a1, q0); q0 = fmaf(wa[2], a2, q0);
+                q1 = fmaf(wa[3], a0, q1); q1 = fmaf(wa[4], a1, q1); q1 = fmaf(wa[5], a2, q1);
+                q2 = fmaf(wa[6], a0, q2); q2 = fmaf(wa[7], a1, q2); q2 = fmaf(wa[8], a2, q2);
+                q0 = fmaf(wb[0], b0, q0); q0 = fmaf(wb[1], b1, q0); q0 = fmaf(wb[2], b2, q0);
+                q1 = fmaf(wb[3], b0, q1); q1 = fmaf(wb[4], b1, q1); q1 = fmaf(wb[5], b2, q1);
+                q2 = fmaf(wb[6], b0, q2); q2 = fmaf(wb[7], b1, q2); q2 = fmaf(wb[8], b2, q2);
+            }
+            if (k < len) {
+                const int b = __ldg(g.bcol + base + 32 * k + lane);
+                const float *vk = v + (size_t)32 * 9 * k;
+                float w[9], p0, p1, p2;
+#pragma unroll
+                for (int i = 0; i < 9; ++i) w[i] = __ldcs(vk + 32 * i);
+                p_on_the_fly(g, pold, beta, first, b, p0, p1, p2);
+                q0 = fmaf(w[0], p0, q0); q0 = fmaf(w[1], p1, q0); q0 = fmaf(w[2], p2, q0);
+                q1 = fmaf(w[3], p0, q1); q1 = fmaf(w[4], p1, q1); q1 = fmaf(w[5], p2, q1);
+                q2 = fmaf(w[6], p0, q2); q2 = fmaf(w[7], p1, q2); q2 = fmaf(w[8], p2, q2);
+            }
+        } else {
+            const float *v = g.val + base + lane;
+            for (int k = sub; k < len; k += tpn) {
+                const int b = g.bcol[base + 32 * k + lane];
+                const float m = v[32 * k];
+                float p0, p1, p2;
+                p_on_the_fly(g, pold, beta, first, b, p0, p1, p2);
+                q0 = fmaf(m, p0, q0);
+                q1 = fmaf(m, p1, q1);
+                q2 = fmaf(m, p2, q2);
+            }
+        }
+    }
+    for (int o = 1; o < tpn; o <<= 1) {
+        q0 += __shfl_xor_sync(0xffffffffu, q0, o);
+        q1 += __shfl_xor_sync(0xffffffffu, q1, o);
+        q2 += __shfl_xor_sync(0xffffffffu, q2, o);
+    }
+}
+
+template <class R, bool B3>
 __global__ void __launch_bounds__(1024, 1) cg_mixed_kernel(const __grid_constant__ CgArgs<R> g) {
     __shared__ float smemf[MIXED_A_NP * 32];
     __shared__ double s_sc[MIXED_GATHER_NP];
@@ -329,7 +415,7 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_kernel(const __grid_constant
         {
             FFEA_SPMV_LOOP(g, a, sub, valid) {
                 float q0, q1, q2;
-                spmv_row<true>(g, pold, beta, first, a, sub, valid, q0, q1, q2);
+                spmv_row_fly<B3>(g, pold, beta, first, a, sub, valid, q0, q1, q2);
                 if (!valid || sub != 0) continue;
                 float p0, p1, p2;
                 p_on_the_fly(g, pold, beta, first, a, p0, p1, p2);

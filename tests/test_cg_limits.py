@@ -45,3 +45,27 @@ def test_one_element_blob(gpu, solver):
         b.update(4)
         out[prec] = b.pos()
     assert np.abs(out["mixed"] - out["fp64"]).max() < 1e-5 * np.abs(out["fp64"] - p0).max()
+
+
+# the CG kernels of the largest mixed blobs, each row count leaving the last block and the last slice short: rows on chip
+# with a matrix above 100 MB (and the consistent-mass solve by the same kernel), and the grid-strided kernel beyond its
+# rows, both forms. One step against the FP64 path, the mixed path's bound
+@pytest.mark.gpu
+@pytest.mark.parametrize("cells,solver,kernel", [((55, 54, 53), "CG_nomass", "cg_mixed_own_kernel"),
+                                                 ((55, 54, 53), "CG", "cg_mixed_own_kernel"),
+                                                 ((77, 75, 74), "CG_nomass", "cg_mixed_kernel"),
+                                                 ((77, 75, 74), "CG", "cg_mixed_kernel")])
+def test_largest_mixed_blobs(gpu, cells, solver, kernel):
+    m = kuhn_box(*cells, 5.0, seed=4)
+    kw = dict(solver=solver, dt=1e-13 if solver == "CG_nomass" else 1e-14, kT=4.11e-21, calc_noise=1)
+    p0 = apply_shear(m, 0.001) * (m.scale / 1.7e-10)
+    out = {}
+    for prec in ("fp64", "mixed"):
+        b = lib.Blob(m, precision=prec, **kw)
+        b.set_state(pos=p0)
+        b.update(1)
+        out[prec] = b.pos()
+        if prec == "mixed":
+            assert b.cg_kernel() == kernel
+        b.close()
+    assert np.abs(out["mixed"] - out["fp64"]).max() < 1e-5 * np.abs(out["fp64"] - p0).max()
