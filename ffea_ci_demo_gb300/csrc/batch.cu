@@ -144,6 +144,7 @@ struct ffea_gpu_batch {
         s.inversions = s.cg_fail = s.nonfinite = s.timeout = s.abort = 0;
         s.steps_done = 0;
         s.last_iters = 0;
+        s.beat = 0;
         CK(cudaMemcpyAsync(st, &s, sizeof(DevStatus), cudaMemcpyHostToDevice, stream));
         return FFEA_GPU_OK;
     }
@@ -701,7 +702,7 @@ int ffea_gpu_batch::launch_cg_only() {
     ca.blob_iters = blob_iters;
     ca.imax = p.max_iterations_cg;
     ca.eps2 = p.epsilon2;
-    ca.limit_ns = 2000000000ull;
+    ca.limit_ns = WAIT_LIMIT_NS;
     CK(BatchLaunch::cg(ca, ncta, cg_threads, stream));
     return FFEA_GPU_OK;
 }

@@ -773,7 +773,7 @@ struct BlobImpl final : ffea_gpu_blob {
         ca.gb = gb; ca.st = st;
         ca.imax = p.max_iterations_cg;
         ca.eps2 = p.epsilon2;
-        ca.limit_ns = 2000000000ull;
+        ca.limit_ns = WAIT_LIMIT_NS;
         ca.history = history; ca.hist_cap = hist_cap; ca.tpn = tpn; ca.phase_ns = phase_ns;
         CK(cudaMemsetAsync(comm, 0, comm_bytes, stream));
         ca.halo_ptr = halo_ptr; ca.halo_list = halo_list; ca.lcol = lcol; ca.nhalo = nhalo;
@@ -1233,7 +1233,7 @@ struct BlobImpl final : ffea_gpu_blob {
             ca.gb = sgb; ca.st = sst;
             ca.imax = p.max_iterations_cg;
             ca.eps2 = p.epsilon2;
-            ca.limit_ns = 2000000000ull;
+            ca.limit_ns = WAIT_LIMIT_NS;
             ca.history = nullptr; ca.hist_cap = 0; ca.tpn = ss_tpn; ca.phase_ns = sphase;
             CK(Launch<R>::cg(ca, ss_grid, ss_block, stream));
             DevStatus ds{};

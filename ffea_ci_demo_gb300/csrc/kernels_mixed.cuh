@@ -821,7 +821,7 @@ __device__ __forceinline__ float warp_sum_spread(const float (&v)[NV], int &inde
 // warp, double-float over the block's warps, published as one message per value, and every block adds the blocks'
 // messages in the same order. `tag` counts the launch's reductions from 1. The caller must pass a __syncthreads()
 // before smem (NV x 32 floats) is written again.
-template <int NV, int K, class A>
+template <int NV, int K, bool BEAT, class A>
 __device__ __forceinline__ bool grid_reduce_msg(const A &g, int rank, int nb, const float (&v)[NV], float *smem,
                                                 unsigned int tag, df32 *s_out, DevStatus *st, GridBarrier *gb) {
     const int lane = threadIdx.x & 31, wid = warp_index(), nw = blockDim.x >> 5;
@@ -837,7 +837,7 @@ __device__ __forceinline__ bool grid_reduce_msg(const A &g, int rank, int nb, co
             if (lane == 0) rows[i * g.stride + rank] = make_float2(t.hi, t.lo);
         }
         unsigned int epoch = tag - 1u;
-        if (!barrier_ep(gb, (unsigned)nb, st, 2000000000ull, epoch)) return false;
+        if (!barrier_ep<BEAT>(gb, (unsigned)nb, st, WAIT_LIMIT_NS, epoch)) return false;
         grid_sum_df8<NV>(rows, g.stride, nb, s_out);
         return true;
     }
@@ -1327,7 +1327,7 @@ __device__ __noinline__ bool sr_moments(const A &g, const B &bl, int a0, int nlo
         float v[14];
 #pragma unroll
         for (int i = 0; i < 14; ++i) v[i] = m[14 * half + i];
-        if (!grid_reduce_msg<14, K>(bl, rank, nb, v, smemf, (unsigned)half + 1u, s_scf, g.st, bl.gb)) return false;
+        if (!grid_reduce_msg<14, K, true>(bl, rank, nb, v, smemf, (unsigned)half + 1u, s_scf, g.st, bl.gb)) return false;
         if (threadIdx.x < 14) s_sc[14 * half + threadIdx.x] = df_double(s_scf[threadIdx.x]);
         __syncthreads();
     }
@@ -1575,7 +1575,7 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
             }
         }
         FFEA_MARK(g, tm, 1);
-        if (!(ok = grid_reduce_msg<MIXED_SR_NP, SrForm<RB>::K>(bl, rank, nb, acc, smemf, ++red_ep, s_scf, st, bl.gb))) break;
+        if (!(ok = grid_reduce_msg<MIXED_SR_NP, SrForm<RB>::K, BATCH>(bl, rank, nb, acc, smemf, ++red_ep, s_scf, st, bl.gb))) break;
         FFEA_MARK(g, tm, 3);
         if (warp_index() == 0) {
             // The iteration's scalars, in double-float as the sums arrive: this chain is on every block's critical path
@@ -1624,6 +1624,9 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
                 s_g = gam.hi;
                 s_pq = pq;
             }
+        }
+        if constexpr (BATCH) {  // blocks of other blobs may be waiting for this solve's blocks
+            if (rank == 0 && (k & 63) == 0 && threadIdx.x == blockDim.x - 32) *((volatile unsigned int *)&st->beat) = wait_clock();
         }
         __syncthreads();
         FFEA_MARK(g, tm, 4);

@@ -69,3 +69,16 @@ def test_largest_mixed_blobs(gpu, cells, solver, kernel):
             assert b.cg_kernel() == kernel
         b.close()
     assert np.abs(out["mixed"] - out["fp64"]).max() < 1e-5 * np.abs(out["fp64"] - p0).max()
+
+
+@pytest.mark.gpu
+def test_batch_waits_outlast_another_blobs_solve(gpu):
+    """Two blobs that need 125 of the 152 blocks each: the second's first blocks wait for the rest through the whole of
+    the first's solve, which here never converges (a tolerance of zero) and takes about three seconds, longer than a
+    wait without progress may take. The step ends with the iteration cap, not with a timeout."""
+    m = kuhn_box(39, 39, 39, 5.0, seed=4)
+    bt = lib.Batch([m, m], dt=1e-13, kT=4.11e-21, epsilon=0.0, max_iterations_cg=250_000)
+    with pytest.raises(lib.FFEAError) as e:
+        bt.update(1)
+    assert e.value.code == lib.ECGMAXIT
+    assert list(bt.cg_iterations()[0]) == [250_000, 250_000]
