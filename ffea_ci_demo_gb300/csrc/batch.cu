@@ -144,7 +144,6 @@ struct ffea_gpu_batch {
         s.inversions = s.cg_fail = s.nonfinite = s.timeout = s.abort = 0;
         s.steps_done = 0;
         s.last_iters = 0;
-        s.beat = 0;
         CK(cudaMemcpyAsync(st, &s, sizeof(DevStatus), cudaMemcpyHostToDevice, stream));
         return FFEA_GPU_OK;
     }

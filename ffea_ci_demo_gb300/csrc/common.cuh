@@ -5,7 +5,8 @@
 //  * barrier_ep / grid_sync_ep (the cooperative CG kernels) and group_sync
 //    (the batch kernel's groups): barriers of co-resident blocks whose wait is
 //    bounded by %globaltimer; on timeout they record FFEA_GPU_ETIMEOUT and
-//    every block leaves its loop. Waits for messages (msg_wait_all) likewise.
+//    every block leaves its loop. A wait for messages (msg_wait_all) is
+//    bounded by the number of its polls.
 //  * deterministic block / grid reductions of doubles (fixed shuffle tree,
 //    then every block sums the per-block partials in the same order).
 //  * MRG32k3a in exact 32-bit modular integer arithmetic (the generator of
@@ -28,7 +29,7 @@ struct DevStatus {
     int last_iters;   // CG iterations of the last completed solve
     long long total_iters;
     int steps_done;   // completed steps since the counter was reset
-    unsigned int beat;  // a batch's solve: wait_clock() of the last progress of any blob's solve (0: none)
+    int pad;
 };
 
 struct GridBarrier {
@@ -44,28 +45,9 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
     return t;
 }
 
-// Every wait of a kernel ends after this time without an answer, or, where the blocks waited for may first have another
-// blob's solve to finish (sr_batch_kernel), after this time without progress by any solve of the launch (DevStatus::beat);
-// a solve ends after max_iterations_cg iterations, so a wait always ends.
-constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;
-
-// Units of 2^20 ns, never 0, to be compared by differences.
-__device__ __forceinline__ unsigned int wait_clock() { return (unsigned int)(globaltimer_ns() >> 20) | 1u; }
-
-// One look at a wait that began at `since` (wait_clock): 0 when it is over, by time or because another block has recorded
-// a timeout; else its start, moved on to the last progress. Called every 256th poll, out of line.
-static __device__ __noinline__ unsigned int wait_check(DevStatus *st, unsigned int since, unsigned long long limit_ns) {
-    if (*((volatile int *)&st->timeout)) return 0u;
-    const unsigned int now = wait_clock(), beat = *((volatile unsigned int *)&st->beat);
-    if (since == 0u) since = now;
-    if (beat != 0u && (int)(beat - since) > 0) since = beat;
-    if ((int)(now - since) > (int)(limit_ns >> 20)) {
-        atomicExch(&st->timeout, 1);
-        atomicExch(&st->abort, 1);
-        return 0u;
-    }
-    return since;
-}
+// The limit of a wait: two seconds where the blocks waited for are at the same solve; in a batch's solve on chip they may
+// first have other blobs' solves to finish (a 59,000-row blob's 250,000 iterations take three seconds).
+constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull, WAIT_LIMIT_BATCH_NS = 30000000000ull;
 
 // Bounded barrier of nblk co-resident blocks (the grid of a cooperative launch, or one group of it) sharing
 // *gb, whose count must be zero when the kernel starts (the launch before it on the stream resets it).
@@ -73,9 +55,8 @@ static __device__ __noinline__ unsigned int wait_check(DevStatus *st, unsigned i
 // acquire loads until it reaches (epoch + 1) * nblk, so the last arrival is the only write on the critical
 // path. For the cooperative CG kernels (one block per SM, one counter for the grid); the batch kernel's many
 // small groups keep group_sync. `epoch` counts the barriers this launch has passed on *gb (the same in every block and thread of the
-// barrier; the caller keeps it, starting at 0). BEAT: the wait is wait_check's, which progress elsewhere extends. Returns false if this block gave up waiting or another block
+// barrier; the caller keeps it, starting at 0). Returns false if this block gave up waiting or another block
 // recorded a timeout; the caller then leaves its loop.
-template <bool BEAT = false>
 __device__ __forceinline__ bool barrier_ep(GridBarrier *gb, unsigned int nblk, DevStatus *st,
                                            unsigned long long limit_ns, unsigned int &epoch) {
     ++epoch;
@@ -89,24 +70,20 @@ __device__ __forceinline__ bool barrier_ep(GridBarrier *gb, unsigned int nblk, D
         int ok = 1;
         const unsigned int target = epoch * nblk;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&gb->count) : "memory");
-        const unsigned long long t0 = BEAT ? 0ull : globaltimer_ns();
-        unsigned int polls = 0, since = 0u;
+        const unsigned long long t0 = globaltimer_ns();
+        unsigned int polls = 0;
         for (;;) {
             unsigned int c;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(&gb->count) : "memory");
             if ((int)(c - target) >= 0) break;
             if ((++polls & 255u) == 0u) {
-                if constexpr (BEAT) {
-                    if ((since = wait_check(st, since, limit_ns)) == 0u) { ok = 0; break; }
-                } else {
-                    if (globaltimer_ns() - t0 > limit_ns) {
-                        atomicExch(&st->timeout, 1);
-                        atomicExch(&st->abort, 1);
-                        ok = 0;
-                        break;
-                    }
-                    if (*((volatile int *)&st->timeout)) { ok = 0; break; }
+                if (globaltimer_ns() - t0 > limit_ns) {
+                    atomicExch(&st->timeout, 1);
+                    atomicExch(&st->abort, 1);
+                    ok = 0;
+                    break;
                 }
+                if (*((volatile int *)&st->timeout)) { ok = 0; break; }
             }
         }
         s_ok = ok;
@@ -195,22 +172,30 @@ __device__ __forceinline__ Msg msg_get(const Msg *p) {
     return {(uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32)};
 }
 
+// The same limits in polls, each an L2 round trip (0.6 to 1 us). Polls and not time, and constants: a clock, a progress
+// count or a bound from memory looked at in the loop cost 2 to 10 % of a small blob's step.
+constexpr int MSG_POLLS = 1 << 21, MSG_POLLS_BATCH = 1 << 25;
+
 // m[j] = *p[j] for the K messages with use[j], read again until every one carries `tag`: those still missing are read
 // together, so the wait ends one round trip after the last of them arrives (waited for one after another, each costs
-// its own). False once the wait is over (wait_check).
+// its own). False once `bound` rounds have passed (recorded in st) or another block has recorded that.
 template <int K>
 __device__ __forceinline__ bool msg_wait_all(const Msg *const (&p)[K], const bool (&use)[K], uint32_t tag, Msg (&m)[K],
-                                             DevStatus *st) {
+                                             DevStatus *st, int bound = MSG_POLLS) {
 #pragma unroll
     for (int j = 0; j < K; ++j)
         if (use[j]) m[j] = msg_get(p[j]);
-    unsigned int polls = 0, since = 0u;
-    for (;;) {
+    for (int polls = 0;; ++polls) {
         bool missing = false;
 #pragma unroll
         for (int j = 0; j < K; ++j) missing = missing || (use[j] && m[j].tag != tag);
         if (!missing) return true;
-        if ((++polls & 255u) == 0u && (since = wait_check(st, since, WAIT_LIMIT_NS)) == 0u) return false;
+        if ((polls & 255) == 255 && *((volatile int *)&st->timeout)) return false;
+        if (polls >= bound) {
+            atomicExch(&st->timeout, 1);
+            atomicExch(&st->abort, 1);
+            return false;
+        }
 #pragma unroll
         for (int j = 0; j < K; ++j)
             if (use[j] && m[j].tag != tag) m[j] = msg_get(p[j]);
@@ -230,13 +215,14 @@ constexpr int MSG_SUM_BLOCKS = 32;
 // add(message of block b) for every block b = lane, lane + 32, ... < nb, in that order, once each carries `tag`: one
 // message a lane for up to 32 blocks, else K at a time. False on a timeout.
 template <int K, class F>
-__device__ __forceinline__ bool msg_collect(const Msg *row, int nb, uint32_t tag, DevStatus *st, F add) {
+__device__ __forceinline__ bool msg_collect(const Msg *row, int nb, uint32_t tag, DevStatus *st, F add,
+                                            int bound = MSG_POLLS) {
     const int lane = threadIdx.x & 31;
     if (nb <= 32) {
         const Msg *const at[1] = {row + lane};
         const bool use[1] = {lane < nb};
         Msg m[1];
-        if (!msg_wait_all<1>(at, use, tag, m, st)) return false;
+        if (!msg_wait_all<1>(at, use, tag, m, st, bound)) return false;
         if (use[0]) add(m[0]);
         return true;
     }
@@ -249,7 +235,7 @@ __device__ __forceinline__ bool msg_collect(const Msg *row, int nb, uint32_t tag
             at[j] = row + b0 + 32 * j;
             use[j] = b0 + 32 * j < nb;
         }
-        if (!msg_wait_all<K>(at, use, tag, m, st)) return false;
+        if (!msg_wait_all<K>(at, use, tag, m, st, bound)) return false;
 #pragma unroll
         for (int j = 0; j < K; ++j)
             if (use[j]) add(m[j]);

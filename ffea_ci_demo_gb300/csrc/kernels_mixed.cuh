@@ -762,7 +762,7 @@ struct Staged {
 
 // The halo of this block for publication `tag`: every thread reads its messages (two of them in flight) and puts
 // them, and its own published row, into the staged vector. The first barrier ends the reads of the previous vector.
-template <class A>
+template <bool BATCH, class A>
 __device__ __forceinline__ bool halo_exchange(const A &g, Staged &z, const int (&hx)[2], int h0, int nh,
                                               unsigned int tag, DevStatus *st) {
     __syncthreads();
@@ -778,7 +778,7 @@ __device__ __forceinline__ bool halo_exchange(const A &g, Staged &z, const int (
             const Msg *const at[2] = {m + (t == 0 ? hx[0] : __ldg(g.halo_list + h0 + h)),
                                       m + (!use[1] ? 0 : t == 0 ? hx[1] : __ldg(g.halo_list + h0 + h2))};
             Msg v[2];
-            if (!msg_wait_all<2>(at, use, tag, v, st)) { bad = 1; break; }
+            if (!msg_wait_all<2>(at, use, tag, v, st, BATCH ? MSG_POLLS_BATCH : MSG_POLLS)) { bad = 1; break; }
             zh[h] = make_float4(__uint_as_float(v[0].x), __uint_as_float(v[0].y), __uint_as_float(v[0].z), 0.f);
             if (use[1])
                 zh[h2] = make_float4(__uint_as_float(v[1].x), __uint_as_float(v[1].y), __uint_as_float(v[1].z), 0.f);
@@ -821,7 +821,7 @@ __device__ __forceinline__ float warp_sum_spread(const float (&v)[NV], int &inde
 // warp, double-float over the block's warps, published as one message per value, and every block adds the blocks'
 // messages in the same order. `tag` counts the launch's reductions from 1. The caller must pass a __syncthreads()
 // before smem (NV x 32 floats) is written again.
-template <int NV, int K, bool BEAT, class A>
+template <int NV, int K, bool BATCH, class A>
 __device__ __forceinline__ bool grid_reduce_msg(const A &g, int rank, int nb, const float (&v)[NV], float *smem,
                                                 unsigned int tag, df32 *s_out, DevStatus *st, GridBarrier *gb) {
     const int lane = threadIdx.x & 31, wid = warp_index(), nw = blockDim.x >> 5;
@@ -837,7 +837,7 @@ __device__ __forceinline__ bool grid_reduce_msg(const A &g, int rank, int nb, co
             if (lane == 0) rows[i * g.stride + rank] = make_float2(t.hi, t.lo);
         }
         unsigned int epoch = tag - 1u;
-        if (!barrier_ep<BEAT>(gb, (unsigned)nb, st, WAIT_LIMIT_NS, epoch)) return false;
+        if (!barrier_ep(gb, (unsigned)nb, st, BATCH ? WAIT_LIMIT_BATCH_NS : WAIT_LIMIT_NS, epoch)) return false;
         grid_sum_df8<NV>(rows, g.stride, nb, s_out);
         return true;
     }
@@ -853,7 +853,7 @@ __device__ __forceinline__ bool grid_reduce_msg(const A &g, int rank, int nb, co
             t = df32{0.f, 0.f};
             if (!msg_collect<K>(row, nb, tag, st, [&](const Msg &m) {
                     t = df_add(t, df32{__uint_as_float(m.x), __uint_as_float(m.y)});
-                }))
+                }, BATCH ? MSG_POLLS_BATCH : MSG_POLLS))
                 bad = 1;
             __syncwarp();
             t = warp_sum_df(t);
@@ -1493,7 +1493,7 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
             }
             ++ep;
             FFEA_MARK(g, tm, 6);
-            if (!halo_exchange(g, zs, hx, h0, nh, ep, st)) return false;
+            if (!halo_exchange<BATCH>(g, zs, hx, h0, nh, ep, st)) return false;
             FFEA_MARK(g, tm, 7);
         }
         return true;
@@ -1539,7 +1539,7 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
     if (threadIdx.x == 0) { s_g = 0.f; s_pq = df32{0.f, 0.f}; s_stop = 0; }
     const df32 tol = df_of(g.eps2 * f2);
     const bool small_tol = tol.hi < DF_TEST_MIN;
-    bool ok = halo_exchange(g, zs, hx, h0, nh, ++ep, st);
+    bool ok = halo_exchange<BATCH>(g, zs, hx, h0, nh, ++ep, st);
     if (ok && cheb) ok = cheb_steps();
     FFEA_MARK(g, tm, 0);
     int k = 0;  // updates applied so far
@@ -1625,9 +1625,6 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
                 s_pq = pq;
             }
         }
-        if constexpr (BATCH) {  // blocks of other blobs may be waiting for this solve's blocks
-            if (rank == 0 && (k & 63) == 0 && threadIdx.x == blockDim.x - 32) *((volatile unsigned int *)&st->beat) = wait_clock();
-        }
         __syncthreads();
         FFEA_MARK(g, tm, 4);
         if (s_stop) break;
@@ -1668,7 +1665,7 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
         }
         FFEA_MARK(g, tm, 5);
         ++ep;
-        if (!(ok = halo_exchange(g, zs, hx, h0, nh, ep, st))) break;
+        if (!(ok = halo_exchange<BATCH>(g, zs, hx, h0, nh, ep, st))) break;
         FFEA_MARK(g, tm, 7);
         if (cheb && !(ok = cheb_steps())) break;
     }
