@@ -329,11 +329,14 @@ __device__ __forceinline__ df32 df_of(double v) {
     return {hi, (float)(v - (double)hi)};
 }
 
-__device__ __forceinline__ double df_double(df32 v) { return (double)v.hi + (double)v.lo; }
+// v rounded up to a pair: df_less(t, df_of_up(v)) is t < v for every pair t, also where v leaves FP32's range (a pair there
+// is a multiple of 2^-149, and so is df_of_up(v): 0 is less than it whenever v > 0)
+__device__ __forceinline__ df32 df_of_up(double v) {
+    const float hi = (float)v;
+    return {hi, __double2float_ru(v - (double)hi)};
+}
 
-// The smallest tolerance |r|^2 is tested against as a pair: below it a pair's low part leaves FP32's range, and from 1e-45
-// on the pair is zero and nothing is less, so the tests there are made in FP64 (|r|^2 may round to zero, which is less).
-constexpr float DF_TEST_MIN = 1e-30f;
+__device__ __forceinline__ double df_double(df32 v) { return (double)v.hi + (double)v.lo; }
 
 __device__ __forceinline__ bool df_less(df32 a, df32 b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); }
 

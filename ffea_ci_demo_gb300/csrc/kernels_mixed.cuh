@@ -918,8 +918,7 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_own_kernel(const __grid_cons
         acc0[0] += r0 * z0 + r1 * z1 + r2 * z2;
     }
     if (threadIdx.x < 36) s_A6f[threadIdx.x] = df_of(s_A6[threadIdx.x]);
-    const df32 tol = df_of(g.eps2 * f2);
-    const bool small_tol = tol.hi < DF_TEST_MIN;
+    const df32 tol = df_of_up(g.eps2 * f2);
     const int row0 = MIXED_A_NP + MIXED_B_NP;
     block_reduce_store<1>(acc0, smemf, partials, g.stride, row0);
     unsigned int bar_ep = 0;  // grid barriers passed
@@ -1036,8 +1035,7 @@ __global__ void __launch_bounds__(1024, 1) cg_mixed_own_kernel(const __grid_cons
         FFEA_MARK(g, tm, 7);
         grid_sum_df8<MIXED_B_NP>(partials + MIXED_A_NP * g.stride, g.stride, gridDim.x, s_scf);
         if (threadIdx.x == 0) {
-            s_conv = (g.check_last || it + 1 < g.imax) &&
-                     (f2 == 0.0 || (small_tol ? df_double(s_scf[0]) < g.eps2 * f2 : df_less(s_scf[0], tol)));
+            s_conv = (g.check_last || it + 1 < g.imax) && (f2 == 0.0 || df_less(s_scf[0], tol));
             if (blockIdx.x == 0 && it < g.hist_cap)  // divided by |f|^2 at the end
                 reinterpret_cast<float2 *>(g.history)[it] = make_float2(s_scf[0].hi, s_scf[0].lo);
             s_beta = s_scf[1].hi / s_delta.hi;
@@ -1344,6 +1342,7 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
     __shared__ double s_sc[MIXED_GATHER_NP];
     __shared__ double s_A6[36];
     __shared__ df32 s_scf[14];  // the iteration's sums
+    __shared__ df32 s_tol;      // the stopping tolerance
     __shared__ df32 s_A6f[36];        // A6 times the shift's scale
     __shared__ df32 s_mp[6];          // moments of D p for the current direction
     __shared__ df32 s_pq;             // p.q~ of the previous iteration
@@ -1537,8 +1536,7 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
     if (threadIdx.x < 6) s_mp[threadIdx.x] = df32{0.f, 0.f};
     if (threadIdx.x < 36) s_A6f[threadIdx.x] = df_of(s_A6[threadIdx.x] * s_shift);
     if (threadIdx.x == 0) { s_g = 0.f; s_pq = df32{0.f, 0.f}; s_stop = 0; }
-    const df32 tol = df_of(g.eps2 * f2);
-    const bool small_tol = tol.hi < DF_TEST_MIN;
+    if (threadIdx.x == 0) s_tol = df_of_up(g.eps2 * f2);
     bool ok = halo_exchange<BATCH>(g, zs, hx, h0, nh, ++ep, st);
     if (ok && cheb) ok = cheb_steps();
     FFEA_MARK(g, tm, 0);
@@ -1598,8 +1596,7 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
             }
             const df32 gam = s_scf[0], rr2 = s_scf[1];
             // |r|^2/|f|^2 < epsilon2 after an update, as NoMassCGSolver::solve tests it (a zero force: x = 0 at once)
-            const bool conv = f2 == 0.0 || (k > 0 && (g.check_last || k < g.imax) &&
-                                            (small_tol ? df_double(rr2) < g.eps2 * f2 : df_less(rr2, tol)));
+            const bool conv = f2 == 0.0 || (k > 0 && (g.check_last || k < g.imax) && df_less(rr2, s_tol));
             if (ln == 0 && rank == 0 && k > 0 && k - 1 < g.hist_cap)
                 reinterpret_cast<float2 *>(g.history)[k - 1] = make_float2(rr2.hi, rr2.lo);
             const bool stop = conv || k >= g.imax;
