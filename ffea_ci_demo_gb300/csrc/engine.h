@@ -53,6 +53,7 @@ struct MixedLaunch {
 // launchers of the adjoint kernels (kernels_adjoint.cuh)
 template <class R>
 struct AdjLaunch {
+    // one thread per node in blocks of Launch<R>::gather_threads(a.N), as the step's gather (whose block count `blocks` is)
     static cudaError_t gather(const AdjGatherArgs<R> &a, int blocks, cudaStream_t s);
     static cudaError_t modes(const AdjModesArgs &a, cudaStream_t s);
     static cudaError_t apply(const AdjApplyArgs<R> &a, int blocks, cudaStream_t s);

@@ -256,7 +256,7 @@ cudaError_t Launch<R>::measure(const MeasureArgs<R> &a, int blocks, double *out,
 
 template <class R>
 cudaError_t AdjLaunch<R>::gather(const AdjGatherArgs<R> &a, int blocks, cudaStream_t s) {
-    adj_gather_kernel<R><<<blocks, 256, 0, s>>>(a);
+    adj_gather_kernel<R><<<blocks, Launch<R>::gather_threads(a.N), 0, s>>>(a);
     count_launch();
     return cudaGetLastError();
 }
@@ -270,7 +270,7 @@ cudaError_t AdjLaunch<R>::modes(const AdjModesArgs &a, cudaStream_t s) {
 
 template <class R>
 cudaError_t AdjLaunch<R>::apply(const AdjApplyArgs<R> &a, int blocks, cudaStream_t s) {
-    adj_apply_kernel<R><<<blocks, 256, 0, s>>>(a);
+    adj_apply_kernel<R><<<blocks, Launch<R>::gather_threads(a.N), 0, s>>>(a);
     count_launch();
     return cudaGetLastError();
 }
