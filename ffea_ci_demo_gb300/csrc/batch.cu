@@ -93,7 +93,7 @@ struct ffea_gpu_batch {
     int *sr_task_ptr = nullptr, *sr_halo_ptr = nullptr, *sr_halo_list = nullptr;
     unsigned short *sr_lcol = nullptr;
     Msg *sr_msg = nullptr;
-    double *sr_cheb = nullptr;
+    double *sr_cheb = nullptr, *sr_cheb_keep = nullptr;  // each blob's preconditioner estimate; room to put them aside
     // launch configuration (ffea_gpu_batch_tune)
     int cg_threads = 256, tpn = 4, ncta = 0, ncta_cap = 0;
     // launch shapes of the force phase (ffea_gpu_batch_set_shapes): elements per block of the element kernel,
@@ -505,6 +505,7 @@ int ffea_gpu_batch::plan_solve() {
     sr_msg_bytes = (size_t)msgs * sizeof(Msg);
     CK(mem.alloc(&sr_msg, (size_t)msgs));
     CK(mem.alloc(&sr_cheb, (size_t)CHEB_STATE * nblobs));
+    CK(mem.alloc(&sr_cheb_keep, (size_t)CHEB_STATE * nblobs));
     CK(mem.alloc(&sr_args, (size_t)nblobs));
     for (int b = 0; b < nblobs; ++b) {
         SrBlob &a = sr_host[b];
@@ -1143,6 +1144,21 @@ int ffea_gpu_batch_tune(ffea_gpu_batch *bt, int solves, double *best_ms) {
     if (rc) return rc;
     DevStatus s0{};
     if ((rc = bt->read_status(s0))) return rc;
+    // the timed solves leave estimates of their own: the blobs' are put aside and brought back on every return
+    struct KeepEstimates {
+        ffea_gpu_batch *bt;
+        size_t bytes;
+        ~KeepEstimates() {
+            if (!bytes) return;
+            cudaMemcpyAsync(bt->sr_cheb, bt->sr_cheb_keep, bytes, cudaMemcpyDeviceToDevice, bt->stream);
+            cudaStreamSynchronize(bt->stream);
+        }
+    } keep_estimates{bt, 0};
+    if (bt->sr_ok) {
+        const size_t bytes = (size_t)CHEB_STATE * bt->nblobs * sizeof(double);
+        CK(cudaMemcpyAsync(bt->sr_cheb_keep, bt->sr_cheb, bytes, cudaMemcpyDeviceToDevice, bt->stream));
+        keep_estimates.bytes = bytes;
+    }
     // the force phase's launch shapes, one at a time (coordinate search): elements per block, then the
     // assembly's threads per block and slot split, then the gather's threads per block
     const int keep_threads = bt->cg_threads, keep_tpn = bt->tpn;

@@ -323,7 +323,9 @@ int ffea_gpu_batch_step(ffea_gpu_batch *batch, int nsteps, int *steps_done);
 int ffea_gpu_batch_step_timed(ffea_gpu_batch *batch, int nsteps, long long flush_bytes, int *steps_done,
                               double *step_ms, double *cg_ms);
 
-/* State of one blob in its own node order (as ffea_gpu_blob_get_state / set_state). */
+/* State of one blob in its own node order (as ffea_gpu_blob_get_state / set_state). A blob's preconditioner estimate (see
+ * ffea_gpu_params::cg_poly) outlives set_state and set_states, as a single blob's does: steps from the same state and
+ * stream agree to the solve's tolerance whatever steps went before, and bit for bit after the same calls on a new batch. */
 int ffea_gpu_batch_get_state(ffea_gpu_batch *batch, int blob, double *pos, double *vel);
 int ffea_gpu_batch_set_state(ffea_gpu_batch *batch, int blob, const double *pos, const double *vel);
 /* Every blob's state at once: the blobs' arrays back to back in blob order (sum of the blobs' node
@@ -366,7 +368,7 @@ int ffea_gpu_batch_set_shapes(ffea_gpu_batch *batch, int element_threads, int as
  * `solves` launches per shape and searched one shape at a time: elements per block, then the
  * assembly's threads and split, then the gather's threads. Then `solves` CG solves of the current
  * forces for every CTA size (128..1024) and threads per row (1, 2, 4, 8). Keeps the fastest of each;
- * positions, velocities and RNG states are not changed. *best_ms (may be NULL) gets the best mean solve
+ * positions, velocities, RNG states and the blobs' preconditioner estimates are not changed. *best_ms (may be NULL) gets the best mean solve
  * time. */
 int ffea_gpu_batch_tune(ffea_gpu_batch *batch, int solves, double *best_ms);
 
