@@ -124,6 +124,7 @@ struct ffea_gpu_batch {
     int init();
     int plan_solve();
     int configure(int threads, int tpn_);
+    int set_config(int threads, int tpn_);
     int set_shapes(int em, int at, int as, int gt);
     int time_forces(int reps, double &ms);
     int record_step();
@@ -397,6 +398,13 @@ int ffea_gpu_batch::configure(int threads, int tpn_) {
     tpn = tpn_;
     ncta = grid;
     on_chip = false;
+    return capture();
+}
+
+// ffea_gpu_batch_set_config: the pair that ffea_gpu_batch_config reports for the solve on chip selects that solve
+int ffea_gpu_batch::set_config(int threads, int tpn_) {
+    if (!sr_ok || threads != SR_REG_THREADS || tpn_ != sr_tpn) return configure(threads, tpn_);
+    on_chip = true;
     return capture();
 }
 
@@ -1135,7 +1143,11 @@ int ffea_gpu_batch_set_shapes(ffea_gpu_batch *bt, int element_threads, int assem
 
 int ffea_gpu_batch_set_config(ffea_gpu_batch *bt, int cg_threads, int threads_per_row) {
     if (!bt) return FFEA_GPU_EINPUT;
-    return bt->configure(cg_threads, threads_per_row);
+    return bt->set_config(cg_threads, threads_per_row);
+}
+
+const char *ffea_gpu_batch_cg_kernel(ffea_gpu_batch *bt) {
+    return !bt ? "" : bt->on_chip ? "sr_batch_kernel" : "cg_batch_kernel";
 }
 
 int ffea_gpu_batch_tune(ffea_gpu_batch *bt, int solves, double *best_ms) {

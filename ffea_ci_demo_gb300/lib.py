@@ -132,6 +132,7 @@ def load():
         "ffea_gpu_batch_cg_iterations": (C.c_int, [vp, dp, C.POINTER(C.c_longlong)]),
         "ffea_gpu_batch_config": (C.c_int, [vp, ip, ip, ip]),
         "ffea_gpu_batch_set_config": (C.c_int, [vp, C.c_int, C.c_int]),
+        "ffea_gpu_batch_cg_kernel": (C.c_char_p, [vp]),
         "ffea_gpu_batch_shapes": (C.c_int, [vp, ip, ip, ip, ip]),
         "ffea_gpu_batch_set_shapes": (C.c_int, [vp, C.c_int, C.c_int, C.c_int, C.c_int]),
         "ffea_gpu_batch_tune": (C.c_int, [vp, C.c_int, C.POINTER(C.c_double)]),
@@ -623,7 +624,12 @@ class Batch:
         return {"cg_threads": t.value, "threads_per_row": p.value, "ctas": c.value, "element_threads": e.value,
                 "assembly_threads": a.value, "assembly_split": sp.value, "gather_threads": g.value}
 
+    def cg_kernel(self) -> str:
+        """The CG kernel the batch's steps launch: "sr_batch_kernel" (on chip) or "cg_batch_kernel" (streaming)."""
+        return self._lib.ffea_gpu_batch_cg_kernel(self._h).decode()
+
     def set_config(self, cg_threads: int, threads_per_row: int) -> None:
+        """A shape of the streaming CG kernel; the pair ``config()`` reports on chip selects the solve on chip."""
         _check(self._lib.ffea_gpu_batch_set_config(self._h, int(cg_threads), int(threads_per_row)),
                "batch_set_config")
 

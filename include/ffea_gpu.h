@@ -349,7 +349,14 @@ int ffea_gpu_batch_load_ctforces(ffea_gpu_batch *batch, int blob, const char *ct
 /* CG iterations of each blob's last solve (num_blobs entries, may be NULL) and the total since creation. */
 int ffea_gpu_batch_cg_iterations(ffea_gpu_batch *batch, int *last_per_blob, long long *total);
 
-/* Launch configuration of the batch CG: CTA size, threads per matrix row, CTAs in the grid. */
+/* The batch's CG kernel (static string): "sr_batch_kernel", the solve on chip, wherever the plan made at creation finds
+ * room for every blob, else (or once a shape of it has been set) "cg_batch_kernel", which streams the matrices. */
+const char *ffea_gpu_batch_cg_kernel(ffea_gpu_batch *batch);
+
+/* Launch configuration of the batch CG: CTA size, threads per matrix row, CTAs in the grid. The solve on chip reports
+ * its own (its threads per row are blob 0's; each blob has its own). set_config selects cg_batch_kernel with the shape
+ * given, except that the pair reported by a batch on chip selects, or selects again, the solve on chip: what config
+ * reports can be set. */
 int ffea_gpu_batch_config(ffea_gpu_batch *batch, int *cg_threads, int *threads_per_row, int *ctas);
 int ffea_gpu_batch_set_config(ffea_gpu_batch *batch, int cg_threads, int threads_per_row);
 
@@ -367,9 +374,10 @@ int ffea_gpu_batch_set_shapes(ffea_gpu_batch *batch, int element_threads, int as
 /* Autotuner. First the force phase (node preparation, elements, assembly, node forces), timed over
  * `solves` launches per shape and searched one shape at a time: elements per block, then the
  * assembly's threads and split, then the gather's threads. Then `solves` CG solves of the current
- * forces for every CTA size (128..1024) and threads per row (1, 2, 4, 8). Keeps the fastest of each;
- * positions, velocities, RNG states and the blobs' preconditioner estimates are not changed. *best_ms (may be NULL) gets the best mean solve
- * time. */
+ * forces on chip (where the batch has that solve) and by cg_batch_kernel for every CTA size
+ * (128..1024) and threads per row (1, 2, 4, 8). Keeps the fastest of each; positions, velocities, RNG
+ * states and the blobs' preconditioner estimates are not changed. *best_ms (may be NULL) gets the best
+ * mean solve time. */
 int ffea_gpu_batch_tune(ffea_gpu_batch *batch, int solves, double *best_ms);
 
 /* ---------------------------------------------------------------------------

@@ -26,3 +26,34 @@ def test_tuning_leaves_the_estimates(gpu):
     ref.update(1)
     bt.update(1)
     assert np.abs(ref.cg_iterations()[0] - bt.cg_iterations()[0]).max() <= 2
+
+
+def test_what_config_reports_can_be_set(gpu):
+    """config() and set_config() round-trip on chip and off it; both kernels, the streaming one with groups of several
+    CTAs to a blob, take the blobs along the same trajectory (the mixed path's bound)."""
+    meshes, x0 = batch(((12, 12, 12), (16, 15, 14), (9, 9, 9), (1, 1, 1)))
+    bt = lib.Batch(meshes, **KW)
+    assert bt.cg_kernel() == "sr_batch_kernel"
+    chip = bt.config()
+    bt.set_config(chip["cg_threads"], chip["threads_per_row"])
+    assert bt.cg_kernel() == "sr_batch_kernel" and bt.config() == chip
+    streams = [bt.rng_state(b) for b in range(len(meshes))]
+    ends = []
+    for shape in (None, (256, 4), (128, 1), (1024, 8)):
+        if shape:
+            bt.set_config(*shape)
+            cfg = bt.config()
+            assert bt.cg_kernel() == "cg_batch_kernel" and (cfg["cg_threads"], cfg["threads_per_row"]) == shape
+            assert cfg["ctas"] >= 2 * len(meshes)
+        bt.set_positions(np.concatenate(x0))
+        for b, s in enumerate(streams):
+            bt.set_rng_state(b, s)
+        bt.update(3)
+        ends.append([bt.pos(b) for b in range(len(meshes))])
+    for b, p0 in enumerate(x0):
+        move = np.abs(ends[0][b] - p0).max()
+        for e in ends[1:]:
+            assert np.abs(e[b] - ends[0][b]).max() < 1e-5 * move, b
+    bt.set_config(chip["cg_threads"], chip["threads_per_row"])
+    assert bt.cg_kernel() == "sr_batch_kernel" and bt.config() == chip
+    bt.update(1)
