@@ -356,7 +356,7 @@ struct BlobImpl final : ffea_gpu_blob {
         // step at 8 / 16 / 32 / 64 rows: 343 nodes CG_nomass 772 / 689 / 785 / 844, 2197 nodes 1820 / 1726 / 1803 / 1934;
         // a mass matrix has a third of the products, and 64 nodes are best in one block (CG 127 / 108 / 120 / 96).
         const int want = !b3 && N <= 64 ? 64 : 16;
-        const int grid = std::max(1, std::min(maxg, (N + want - 1) / want)), npb = (N + grid - 1) / grid;
+        const int grid = own_unit_grid(N, want, maxg), npb = (N + grid - 1) / grid;
         int best = 0, best_nc = 0, best_tpu = 0;
         for (int nc : {1, 3})
             for (int t = 1; t <= (nc == 1 ? 8 : 1); t *= 2) {

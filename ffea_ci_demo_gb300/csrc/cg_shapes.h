@@ -28,4 +28,21 @@ FFEA_HD constexpr size_t sr_smem_bytes(int npb, int nhalo, int poly) {
     return poly > 0 && rows < CHEB_SCRATCH_BYTES ? CHEB_SCRATCH_BYTES : rows;
 }
 
+// cg_own_unit_kernel: threads of a block, units of npb rows for nc components to a unit (1 or 3), and the bytes of dynamic
+// shared memory: the staged direction (3 per row of the block and its halo), the units' addends of two sums, and kc matrix
+// blocks per row (values, then local columns; nc = 3 only)
+constexpr int OWN_UNIT_THREADS = 512;
+FFEA_HD inline int own_unit_count(int npb, int nc) { return nc == 3 ? npb : 3 * npb; }
+FFEA_HD inline size_t own_unit_smem(int npb, int nhalo, int nc, int vals, int kc) {
+    return (3 * ((size_t)npb + nhalo) + 2 * (size_t)own_unit_count(npb, nc)) * sizeof(double) +
+           (size_t)kc * npb * (vals * sizeof(double) + sizeof(unsigned short));
+}
+
+// Its blocks for N rows, `rows` to a block while the device's `most` leave room; its sums hold UNIT_SUM_BLOCKS partials.
+constexpr int UNIT_SUM_BLOCKS = 160;
+inline int own_unit_grid(int N, int rows, int most) {
+    const int g = (N + rows - 1) / rows, cap = most < UNIT_SUM_BLOCKS ? most : UNIT_SUM_BLOCKS;
+    return g < 1 ? 1 : g < cap ? g : cap;
+}
+
 }  // namespace ffea

@@ -24,6 +24,7 @@
 //                          slice_ptr[s] + 32*k + lane; block values val[9*slice_ptr[s] + 32*(9*k + c) + lane]
 #pragma once
 
+#include "cg_shapes.h"
 #include "common.cuh"
 
 namespace ffea {
@@ -1433,22 +1434,12 @@ __device__ __forceinline__ void spmv_row_pd(const CgArgs<R> &g, const double2 *p
 // Every value is computed from the same products as in cg_kernel, fused in the same way per component; only the
 // grouping of sums changes.
 // ---------------------------------------------------------------------------
-constexpr int OWN_UNIT_THREADS = 512;
-
 // values per matrix block that a unit multiplies, and blocks of each lane in registers
 template <int NC, bool B3>
 struct UnitBlock {
     static constexpr int V = B3 ? 3 * NC : 1;
     static constexpr int RB = NC == 1 ? (B3 ? 6 : 12) : 0;
 };
-
-// Bytes of dynamic shared memory: the staged direction (3 per row of the block and its halo), the units' addends of
-// two sums, and kc matrix blocks per row (values, then local columns; NC = 3 only)
-__host__ __device__ inline int own_unit_count(int npb, int nc) { return nc == 3 ? npb : 3 * npb; }
-__host__ __device__ inline size_t own_unit_smem(int npb, int nhalo, int nc, int vals, int kc) {
-    return (3 * ((size_t)npb + nhalo) + 2 * (size_t)own_unit_count(npb, nc)) * sizeof(double) +
-           (size_t)kc * npb * (vals * sizeof(double) + sizeof(unsigned short));
-}
 
 // The sum over u < U of NV addends per unit, s[i U + u], in s_out[i] for warp i's lane 0 (other threads: not
 // defined): four warps (one per sub-partition) per value add strided runs, one warp their 128 partials.
@@ -1503,6 +1494,7 @@ __device__ __forceinline__ bool grid_reduce_units(const A &g, double *s, int U, 
         unsigned int epoch = tag - 1u;
         if (!barrier_ep(g.gb, (unsigned)nb, st, g.limit_ns, epoch)) return false;
         if (wid < NV) {
+            static_assert(UNIT_SUM_BLOCKS == 5 * 32, "five partials to a lane");
             double q[5];
 #pragma unroll
             for (int j = 0; j < 5; ++j) q[j] = lane + 32 * j < nb ? __ldcg(rowd + wid * g.stride + lane + 32 * j) : 0.0;

@@ -25,7 +25,6 @@
 // S2 = sum d_a x v_a; D Z c at node a is D_a (tau + Omega x d_a).
 #pragma once
 
-#include "cg_shapes.h"
 #include "kernels.cuh"
 #include "kernels_element_mixed.cuh"
 

@@ -12,6 +12,8 @@ SRC = """
 extern "C" {
 long long smem(int npb, int nhalo, int poly) { return (long long)ffea::sr_smem_bytes(npb, nhalo, poly); }
 int recorded() { return ffea::CHEB_REC; }
+int unit_grid(int n, int rows, int most) { return ffea::own_unit_grid(n, rows, most); }
+int unit_sums() { return ffea::UNIT_SUM_BLOCKS; }
 }
 """
 
@@ -40,3 +42,13 @@ def test_lanczos_scratch_fits_the_smallest_blob(shapes):
                 assert got >= 16 * shapes.recorded()
                 assert got >= 4 * 30 * rows + 16 * (rows + halo)  # and the rows' own fields
             assert shapes.smem(rows, halo, 0) == 4 * 24 * rows + 16 * (rows + halo)  # Jacobi alone records nothing
+
+
+def test_unit_sums_hold_every_block(shapes):
+    """The FP64 solve's sums over blocks hold 160 partials: no device's grid exceeds that, and no row is left out."""
+    for most in (1, 80, 152, 160, 161, 208, 1000):
+        for rows in (16, 64, 512):
+            for n in (1, rows, rows + 1, 2197, 77824, 200000):
+                g = shapes.unit_grid(n, rows, most)
+                assert 1 <= g <= min(most, shapes.unit_sums())
+                assert g == most or g == shapes.unit_sums() or g * rows >= n
