@@ -353,9 +353,11 @@ struct BlobImpl final : ffea_gpu_blob {
         int maxlen = 1;
         for (int a = 0; a < N; ++a) maxlen = std::max(maxlen, h.rowlen[a]);
         // Rows a block is given while the mesh leaves SMs free: more blocks share the FP64 work but lengthen the sums. us per
-        // step at 8 / 16 / 32 / 64 rows: 343 nodes CG_nomass 772 / 689 / 785 / 844, 2197 nodes 1820 / 1726 / 1803 / 1934;
-        // a mass matrix has a third of the products, and 64 nodes are best in one block (CG 127 / 108 / 120 / 96).
-        const int want = !b3 && N <= 64 ? 64 : 16;
+        // step at 8 / 16 / 32 / 64 rows: 343 nodes CG_nomass 772 / 689 / 785 / 844, 2197 nodes 1820 / 1726 / 1803 / 1934.
+        // A mass matrix has a third of the products, and blobs whose components each find a thread in one block stay there
+        // (N <= 170): one block against 16 rows a block 27 nodes 107 / 129, 48 125 / 147, 64 133 / 147, 80 144 / 162, 100
+        // 156 / 170, 125 164 / 176, 150 179 / 194; with a unit per row in one block 180 nodes 199 / 183, 216 205 / 187.
+        const int want = !b3 && own_unit_count(N, 1) <= OWN_UNIT_THREADS ? N : 16;
         const int grid = own_unit_grid(N, want, maxg), npb = (N + grid - 1) / grid;
         int best = 0, best_nc = 0, best_tpu = 0;
         for (int nc : {1, 3})

@@ -82,3 +82,21 @@ def test_batch_waits_outlast_another_blobs_solve(gpu):
         bt.update(1)
     assert e.value.code == lib.ECGMAXIT
     assert list(bt.cg_iterations()[0]) == [250_000, 250_000]
+
+
+# the FP64 consistent-mass solve on both sides of one block's 170 rows, against the oracle's CG
+@pytest.mark.gpu
+@pytest.mark.parametrize("cells", [(1, 4, 16), (2, 2, 18)])
+def test_consistent_mass_one_block_edge(gpu, oracle_built, cells):
+    import pyoracle
+
+    m = kuhn_box(*cells, 5.0, seed=4)
+    kw = dict(solver="CG", dt=1e-14, kT=4.11e-21, calc_noise=1)
+    p0 = apply_shear(m, 0.001) * (m.scale / 1.7e-10)
+    b, o = lib.Blob(m, **kw), pyoracle.OracleBlob(m, threads=1, fast=True, **kw)
+    b.set_state(pos=p0)
+    o.set_pos(p0)
+    b.update(2)
+    assert o.step(2) == 0
+    moved = np.abs(o.pos() - p0).max()
+    assert np.abs(b.pos() - o.pos()).max() < 1e-8 * moved + 1e-15 * np.abs(p0).max()
