@@ -258,6 +258,7 @@ int ffea_gpu_batch::init() {
         CK(mem.upload(&kpos, h.kpos));
         CK(Launch<float>::assemble_init());
     } else {
+        build_sources(h);
         CK(mem.upload(&grp_slice, h.grp_slice));
         CK(mem.upload(&src_ptr, h.src_ptr));
         CK(mem.upload(&src, h.src));

@@ -469,6 +469,7 @@ struct BlobImpl final : ffea_gpu_blob {
             CK(mem.upload(&kpos, h.kpos));
             CK(Launch<R>::assemble_init());
         } else if (p.solver == FFEA_GPU_NOMASS_CG) {
+            build_sources(h);
             CK(mem.upload(&grp_slice, h.grp_slice));
             CK(mem.upload(&src_ptr, h.src_ptr));
             CK(mem.upload(&src, h.src));
@@ -1815,6 +1816,17 @@ int ffea_gpu_blob_get_pattern(ffea_gpu_blob *b, int *key, int *col, double *val,
         int rc = b->get_matrix_values(vals);
         if (rc) return rc;
     }
+    // the sources summed into each slot: one per element of the row that holds the column
+    std::vector<int> sources;
+    if (nsrc) {
+        sources.assign(h.nslots, 0);
+        for (int a = 0; a < h.N; ++a)
+            for (int m = h.inc_ptr[a]; m < h.inc_ptr[a + 1] && !h.pinned[a]; ++m)
+                for (int j = 0; j < 4; ++j) {
+                    const int v = h.tet4[4 * (size_t)(h.inc[m] >> 2) + j];
+                    if (!h.pinned[v]) ++sources[slot_of(h, a, v)];
+                }
+    }
     long long pos = 0;
     for (int i = 0; i < n; ++i)
         for (int c = 0; c < 3; ++c) {
@@ -1825,7 +1837,7 @@ int ffea_gpu_blob_get_pattern(ffea_gpu_blob *b, int *key, int *col, double *val,
                 for (int m = 0; m < h.rowlen[k]; ++m) {
                     const long long slot = (long long)h.slice_ptr[s] + 32 * m + lane;
                     const int bcolv = h.bcol[slot];
-                    const int nsource = h.src_ptr[slot + 1] - h.src_ptr[slot];
+                    const int nsource = nsrc ? sources[slot] : 0;
                     for (int j = 0; j < 3; ++j) {
                         if (col) col[pos] = 3 * h.node_of[bcolv] + j;
                         if (val) val[pos] = vals[9 * (size_t)h.slice_ptr[s] + 32 * (9 * m + 3 * c + j) + lane];

@@ -152,7 +152,7 @@ struct HostModel {
     std::vector<int> slice_ptr, rowlen, bcol, diagk;
     std::vector<int> grp_slice;  // slice of each group of 32 slots
     std::vector<std::vector<int>> nbr;  // sorted neighbours per vertex
-    std::vector<int> src_ptr;
+    std::vector<int> src_ptr;  // build_sources, where the assembly goes by slots
     std::vector<unsigned> src;
     // per incidence entry (inc), the block index in the row of each of the element's four vertices (255: pinned, or a
     // row of more blocks than that, `width` then being 0); width: the most blocks of any slice
@@ -276,6 +276,51 @@ inline void build_cta_lists(const HostModel &h, int cta, CtaLists &o) {
     std::vector<int> fill(o.part_ptr.begin(), o.part_ptr.end() - 1);
     o.perm.resize(o.cta_nodes.size());
     for (size_t q = 0; q < o.cta_nodes.size(); ++q) o.perm[q] = fill[o.cta_nodes[q]]++;
+}
+
+// The matrix slot of the 3x3 block (a, b).
+inline long long slot_of(const HostModel &h, int a, int b) {
+    const auto &v = h.nbr[a];
+    const int k = (int)(std::lower_bound(v.begin(), v.end(), b) - v.begin());
+    return (long long)h.slice_ptr[a >> 5] + 32 * k + (a & 31);
+}
+
+// The assembly sources per slot, in element order (the registration order of NoMassCGSolver::init): for the assembly by
+// slots alone, 90 of 230 ms of a 40^3-cell model.
+inline void build_sources(HostModel &h) {
+    const int N = h.N, T = h.T;
+    h.src_ptr.assign(h.nslots + 1, 0);
+    for (int e = 0; e < T; ++e) {
+        const int *t = &h.tet4[4 * (size_t)e];
+        for (int a = 0; a < 4; ++a) {
+            if (h.pinned[t[a]]) continue;
+            for (int b = 0; b < 4; ++b)
+                if (!h.pinned[t[b]]) h.src_ptr[slot_of(h, t[a], t[b]) + 1]++;
+        }
+    }
+    for (int a = 0; a < N; ++a)
+        if (h.pinned[a]) h.src_ptr[slot_of(h, a, a) + 1]++;
+    for (long long k = 0; k < h.nslots; ++k) h.src_ptr[k + 1] += h.src_ptr[k];
+    h.src.assign(h.src_ptr[h.nslots], 0u);
+    {
+        std::vector<int> fill(h.nslots, 0);
+        for (int a = 0; a < N; ++a)
+            if (h.pinned[a]) {
+                const long long k = slot_of(h, a, a);
+                h.src[h.src_ptr[k] + fill[k]++] = SRC_IDENTITY;
+            }
+        for (int e = 0; e < T; ++e) {
+            const int *t = &h.tet4[4 * (size_t)e];
+            for (int a = 0; a < 4; ++a) {
+                if (h.pinned[t[a]]) continue;
+                for (int b = 0; b < 4; ++b) {
+                    if (h.pinned[t[b]]) continue;
+                    const long long k = slot_of(h, t[a], t[b]);
+                    h.src[h.src_ptr[k] + fill[k]++] = ((unsigned)e << 4) | ((unsigned)a << 2) | (unsigned)b;
+                }
+            }
+        }
+    }
 }
 
 inline int build_model(const ffea_gpu_mesh *mesh, const ffea_gpu_params *p, HostModel &h) {
@@ -423,56 +468,19 @@ inline int build_model(const ffea_gpu_mesh *mesh, const ffea_gpu_params *p, Host
         for (int k = 0; k < w; ++k) h.bcol[h.slice_ptr[s] + 32 * k + lane] = k < (int)v.size() ? v[k] : a;
         h.diagk[a] = (int)(std::lower_bound(v.begin(), v.end(), a) - v.begin());
     }
-    // assembly sources per slot, element order (the registration order of NoMassCGSolver::init)
-    auto slot_of = [&](int a, int b) -> long long {
-        const auto &v = h.nbr[a];
-        const int k = (int)(std::lower_bound(v.begin(), v.end(), b) - v.begin());
-        return (long long)h.slice_ptr[a >> 5] + 32 * k + (a & 31);
-    };
-    h.src_ptr.assign(h.nslots + 1, 0);
-    for (int e = 0; e < T; ++e) {
-        const int *t = &h.tet4[4 * (size_t)e];
-        for (int a = 0; a < 4; ++a) {
-            if (h.pinned[t[a]]) continue;
-            for (int b = 0; b < 4; ++b)
-                if (!h.pinned[t[b]]) h.src_ptr[slot_of(t[a], t[b]) + 1]++;
-        }
-    }
-    for (int a = 0; a < N; ++a)
-        if (h.pinned[a]) h.src_ptr[slot_of(a, a) + 1]++;
-    for (long long k = 0; k < h.nslots; ++k) h.src_ptr[k + 1] += h.src_ptr[k];
-    h.src.assign(h.src_ptr[h.nslots], 0u);
-    {
-        std::vector<int> fill(h.nslots, 0);
-        for (int a = 0; a < N; ++a)
-            if (h.pinned[a]) {
-                const long long k = slot_of(a, a);
-                h.src[h.src_ptr[k] + fill[k]++] = SRC_IDENTITY;
-            }
-        for (int e = 0; e < T; ++e) {
-            const int *t = &h.tet4[4 * (size_t)e];
-            for (int a = 0; a < 4; ++a) {
-                if (h.pinned[t[a]]) continue;
-                for (int b = 0; b < 4; ++b) {
-                    if (h.pinned[t[b]]) continue;
-                    const long long k = slot_of(t[a], t[b]);
-                    h.src[h.src_ptr[k] + fill[k]++] = ((unsigned)e << 4) | ((unsigned)a << 2) | (unsigned)b;
-                }
-            }
-        }
-    }
     if (p->solver == FFEA_GPU_NOMASS_CG) {
         for (int s = 0; s < h.nslices; ++s) h.width = std::max(h.width, (h.slice_ptr[s + 1] - h.slice_ptr[s]) / 32);
         if (h.width >= 255) h.width = 0;
         h.kpos.assign(h.width ? 4 * h.inc.size() : 0, 255);
+        std::vector<unsigned char> at(h.width ? N : 0);  // of the row's neighbours, their block's index in it
         for (int a = 0; a < N && h.width; ++a) {
             if (h.pinned[a]) continue;
             const auto &v = h.nbr[a];
+            for (size_t k = 0; k < v.size(); ++k) at[v[k]] = (unsigned char)k;
             for (int m = h.inc_ptr[a]; m < h.inc_ptr[a + 1]; ++m) {
                 const int *t = &h.tet4[4 * (size_t)(h.inc[m] >> 2)];
                 for (int b = 0; b < 4; ++b)
-                    if (!h.pinned[t[b]])
-                        h.kpos[4 * (size_t)m + b] = (unsigned char)(std::lower_bound(v.begin(), v.end(), t[b]) - v.begin());
+                    if (!h.pinned[t[b]]) h.kpos[4 * (size_t)m + b] = at[t[b]];
             }
         }
     }
@@ -486,11 +494,11 @@ inline int build_model(const ffea_gpu_mesh *mesh, const ffea_gpu_params *p, Host
                 for (int j = 0; j < 4; ++j) {
                     const int ni = t[i], nj = t[j];
                     if (!h.pinned[ni] && !h.pinned[nj]) {
-                        const long long k = slot_of(ni, nj);
+                        const long long k = slot_of(h, ni, nj);
                         if (i == j) h.mass_sell[k] += .1 * h.rho[e] * h.vol0[e];
                         else h.mass_sell[k] += .05 * h.rho[e] * h.vol0[e];
                     } else if (i == j) {
-                        h.mass_sell[slot_of(ni, nj)] = 1;
+                        h.mass_sell[slot_of(h, ni, nj)] = 1;
                     }
                 }
         }
