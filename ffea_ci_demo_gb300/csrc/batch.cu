@@ -878,11 +878,10 @@ int ffea_gpu_batch_create(const ffea_gpu_mesh *meshes, int nblobs, const ffea_gp
                 delete bt;
                 return FFEA_GPU_EINPUT;
             }
+        rc = bt->init();
     } catch (std::bad_alloc &) {
-        delete bt;
-        return FFEA_GPU_ENOMEM;
+        rc = FFEA_GPU_ENOMEM;
     }
-    rc = bt->init();
     if (rc) {
         delete bt;
         return rc;

@@ -1687,10 +1687,10 @@ int ffea_gpu_blob_create(const ffea_gpu_mesh *mesh, const ffea_gpu_params *param
     b->p = *params;
     try {
         rc = build_model(mesh, params, b->h);
+        if (!rc) rc = b->init();
     } catch (std::bad_alloc &) {
         rc = FFEA_GPU_ENOMEM;
     }
-    if (!rc) rc = b->init();
     if (rc) {
         delete b;
         return rc;
@@ -1798,7 +1798,7 @@ int ffea_gpu_blob_sizes(ffea_gpu_blob *b, int *nl, int *ne, long long *nb) {
     return FFEA_GPU_OK;
 }
 
-int ffea_gpu_blob_get_pattern(ffea_gpu_blob *b, int *key, int *col, double *val, int *nsrc, long long *nnz) {
+int ffea_gpu_blob_get_pattern(ffea_gpu_blob *b, int *key, int *col, double *val, int *nsrc, long long *nnz) try {
     if (!b) return FFEA_GPU_EINPUT;
     const HostModel &h = b->h;
     if (b->p.solver != FFEA_GPU_NOMASS_CG) return FFEA_GPU_EINPUT;
@@ -1856,6 +1856,8 @@ int ffea_gpu_blob_get_pattern(ffea_gpu_blob *b, int *key, int *col, double *val,
         }
     if (key) key[3 * (size_t)n] = (int)pos;
     return FFEA_GPU_OK;
+} catch (std::bad_alloc &) {
+    return FFEA_GPU_ENOMEM;
 }
 
 int ffea_gpu_blob_get_connectivity(ffea_gpu_blob *b, int *ptr, int *es, long long *count) {
