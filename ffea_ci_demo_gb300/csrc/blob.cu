@@ -1145,6 +1145,17 @@ struct BlobImpl final : ffea_gpu_blob {
         }
     }
 
+    void kernels(const char *&element, const char *&assembly, const char *&cg, int shape[3]) const override {
+        constexpr bool mixed = std::is_same<R, float>::value;
+        element = mixed ? "element_mixed_kernel" : h.T <= ELEM_SPLIT_MAX ? "element_split_kernel" : "element_kernel";
+        assembly = p.solver != FFEA_GPU_NOMASS_CG ? "none" : kpos ? "assemble_rows_kernel" : "assemble_kernel";
+        cg = cg_unit && p.solver != FFEA_GPU_MASSLUMPED ? "cg_own_unit_kernel" : cg_kernel_name();
+        const bool solves = p.solver != FFEA_GPU_MASSLUMPED;
+        shape[0] = solves ? cg_grid : 0;
+        shape[1] = solves ? cg_block : 0;
+        shape[2] = solves ? cg_npb : 0;
+    }
+
     int get_rhs(double *rhs) override {
         const int N = h.N;
         std::vector<double> hf(4 * (size_t)N);
@@ -1778,6 +1789,18 @@ int ffea_gpu_blob_cg_preconditioner(ffea_gpu_blob *b, int *degree, double *lambd
 }
 
 const char *ffea_gpu_blob_cg_kernel(ffea_gpu_blob *b) { return b ? b->cg_kernel_name() : "none"; }
+
+int ffea_gpu_blob_kernels(ffea_gpu_blob *b, const char **element, const char **assembly, const char **cg, int *cg_shape) {
+    if (!b) return FFEA_GPU_EINPUT;
+    const char *name[3];
+    int shape[3];
+    b->kernels(name[0], name[1], name[2], shape);
+    if (element) *element = name[0];
+    if (assembly) *assembly = name[1];
+    if (cg) *cg = name[2];
+    for (int i = 0; cg_shape && i < 3; ++i) cg_shape[i] = shape[i];
+    return FFEA_GPU_OK;
+}
 
 int ffea_gpu_blob_counts(ffea_gpu_blob *b, int *num_nodes, int *num_elements) {
     if (!b) return FFEA_GPU_EINPUT;

@@ -37,6 +37,8 @@ struct ffea_gpu_blob {
     virtual int cg_profile(double *ns, int n) = 0;
     virtual int cg_preconditioner(int *degree, double *lambda_max) = 0;
     virtual const char *cg_kernel_name() const = 0;
+    // the kernels the steps launch, by their own names; cg: its blocks, threads per block and rows per block (0: shared)
+    virtual void kernels(const char *&element, const char *&assembly, const char *&cg, int shape[3]) const = 0;
     virtual int get_matrix_values(std::vector<double> &val_sell) = 0;
     virtual int solve_static(const double *rhs, double *x, int *iterations) = 0;
     virtual int adj_init(int window, int every) = 0;

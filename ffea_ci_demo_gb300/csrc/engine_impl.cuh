@@ -23,10 +23,7 @@ cudaError_t Launch<R>::element(const ElemArgs<R> &a, cudaStream_t s) {
         return (void)a, (void)s, cudaErrorNotSupported;
     } else {
         if (a.T <= 0) return cudaSuccess;
-        // four lanes to an element while that leaves a sub-partition (608 of them) two warps at most; us at 1296 / 6000 /
-        // 10,368 elements, four lanes against one: inertial 25 / 40 / 56 against 49 / 49 / 50, CG_nomass 14 / 20 / 25
-        // against 23 / 23 / 24
-        if (a.T <= 608 * 2 * 8)
+        if (a.T <= ELEM_SPLIT_MAX)
             element_split_kernel<R><<<(4 * a.T + ELEM_THREADS - 1) / ELEM_THREADS, ELEM_THREADS, 0, s>>>(a);
         else
             element_kernel<R><<<(a.T + ELEM_THREADS - 1) / ELEM_THREADS, ELEM_THREADS, 0, s>>>(a);

@@ -239,6 +239,11 @@ __global__ void __launch_bounds__(128) element_kernel(ElemArgs<R> g) {
     gm[12] = vol;
 }
 
+// element_split_kernel up to this many elements: four lanes to an element while that leaves a sub-partition (608 of them) two
+// warps at most; us at 1296 / 6000 / 10,368 elements, four lanes against one: inertial 25 / 40 / 56 against 49 / 49 / 50,
+// CG_nomass 14 / 20 / 25 against 23 / 23 / 24
+constexpr int ELEM_SPLIT_MAX = 608 * 2 * 8;
+
 // The same element phase with four lanes to an element, lane v working for vertex v (and, for v < 3, row v of the
 // stress). An FP64 instruction holds a sub-partition for 64 cycles whatever lanes it has, and one thread's element is a
 // chain of 750 of them (1,560 with the viscous term of the inertial solvers: 49 us however few elements there are), so

@@ -100,6 +100,7 @@ def load():
         "ffea_gpu_blob_cg_profile": (C.c_int, [vp, dp, C.c_int]),
         "ffea_gpu_blob_cg_preconditioner": (C.c_int, [vp, ip, dp]),
         "ffea_gpu_blob_cg_kernel": (C.c_char_p, [vp]),
+        "ffea_gpu_blob_kernels": (C.c_int, [vp, vp, vp, vp, vp]),
         "ffea_gpu_blob_get_pattern": (C.c_int, [vp, dp, dp, dp, dp, C.POINTER(C.c_longlong)]),
         "ffea_gpu_blob_get_connectivity": (C.c_int, [vp, dp, dp, C.POINTER(C.c_longlong)]),
         "ffea_gpu_blob_get_elements": (C.c_int, [vp, dp, dp, dp]),
@@ -368,6 +369,13 @@ class Blob:
     def cg_kernel(self) -> str:
         """Name of the persistent CG kernel this blob's steps launch ("none" for masslumped)."""
         return self._lib.ffea_gpu_blob_cg_kernel(self._h).decode()
+
+    def kernels(self) -> dict:
+        """The kernels this blob's steps launch by their own names, and the CG's blocks, threads and rows per block."""
+        e, a, g, s = C.c_char_p(), C.c_char_p(), C.c_char_p(), (C.c_int * 3)()
+        _check(self._lib.ffea_gpu_blob_kernels(self._h, C.byref(e), C.byref(a), C.byref(g), s), "kernels")
+        return {"element": e.value.decode(), "assembly": a.value.decode(), "cg": g.value.decode(), "cg_blocks": s[0],
+                "cg_threads": s[1], "cg_rows": s[2]}
 
     def sizes(self) -> tuple[int, int, int]:
         nl, ne, nb = C.c_int(), C.c_int(), C.c_longlong()

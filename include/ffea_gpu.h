@@ -198,10 +198,19 @@ int ffea_gpu_blob_cg_preconditioner(ffea_gpu_blob *blob, int *degree, double *la
 
 /* Name of the persistent CG kernel the blob's steps launch, fixed at creation by the blob's size and
  * precision alone (static string; "none" for masslumped, which solves no system):
- *   FP64: "cg_own_kernel" (each block keeps its rows on chip) or "cg_kernel" (grid-strided, larger blobs);
+ *   FP64: "cg_own_kernel" (each block keeps its rows on chip, by either of two kernels: ffea_gpu_blob_kernels) or
+ *   "cg_kernel" (grid-strided, larger blobs);
  *   mixed: "cg_mixed_sr_kernel" (CG_nomass, one reduction per iteration, FP32 matrix up to 100 MB so that it
  *   stays in L2), "cg_mixed_own_kernel" (two reductions, rows on chip) or "cg_mixed_kernel" (grid-strided). */
 const char *ffea_gpu_blob_cg_kernel(ffea_gpu_blob *blob);
+
+/* The kernels the blob's steps launch, by their own names (static strings; any pointer may be NULL), as the dispatch
+ * rules chose them at creation: *element "element_mixed_kernel", "element_split_kernel" or "element_kernel"; *assembly
+ * "assemble_rows_kernel", "assemble_kernel" or (inertial solvers) "none"; *cg as ffea_gpu_blob_cg_kernel, but
+ * "cg_own_unit_kernel" for that form of the FP64 solve with its rows on chip. cg_shape[3]: the solve's blocks, threads
+ * per block and rows per block (0: the rows are shared among the blocks). */
+int ffea_gpu_blob_kernels(ffea_gpu_blob *blob, const char **element, const char **assembly, const char **cg,
+                          int *cg_shape);
 
 /* Nodes of the reference numbering (vertices and midpoints) and elements of the blob. */
 int ffea_gpu_blob_counts(ffea_gpu_blob *blob, int *num_nodes, int *num_elements);
