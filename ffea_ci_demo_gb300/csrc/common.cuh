@@ -202,44 +202,26 @@ __device__ __forceinline__ bool msg_wait_all(const Msg *const (&p)[K], const boo
     }
 }
 
-// A grid-wide sum's messages are polled by every block: they are published in MSG_COPIES copies on lines of their own
-// (one per lane of the publishing warp), block b reading copy b mod MSG_COPIES, or the polls of all blocks on the same
-// few lines hold up the messages themselves (22 blocks: 213 against 199 us per step).
+// A sum's messages are polled by every block: they are published in MSG_COPIES copies (one per lane of the publishing
+// warp), block b reading copy b mod MSG_COPIES, or the polls of all blocks on the same few lines hold up the messages
+// themselves (22 blocks: 213 against 199 us per step).
 constexpr int MSG_COPIES = 16;
 constexpr int MSG_VALUES = 16;  // values a reduction's buffer holds
-// Sums over more blocks than this go through a counter barrier instead: one poller to a block, where all blocks polling
-// all messages hold one another up (us per step, messages against the barrier: 137 blocks FP64 1728 / 1486, 145 blocks
-// FP64 3588 / 3087, 152 blocks mixed 40^3 2755 / 2575; 22 blocks FP64 646 / 767).
+// Sums over more blocks than this, one message to a lane, go through a counter barrier instead: one poller to a block,
+// where all blocks polling all messages hold one another up (us per step, messages against the barrier: 137 blocks FP64
+// 1728 / 1486, 145 blocks FP64 3588 / 3087, 152 blocks mixed 40^3 2755 / 2575; 22 blocks FP64 646 / 767).
 constexpr int MSG_SUM_BLOCKS = 32;
 
-// add(message of block b) for every block b = lane, lane + 32, ... < nb, in that order, once each carries `tag`: one
-// message a lane for up to 32 blocks, else K at a time. False on a timeout.
-template <int K, class F>
+// add(message of block `lane`) in the lanes below nb <= MSG_SUM_BLOCKS, once each message carries `tag`. False on a timeout.
+template <class F>
 __device__ __forceinline__ bool msg_collect(const Msg *row, int nb, uint32_t tag, DevStatus *st, F add,
                                             int bound = MSG_POLLS) {
     const int lane = threadIdx.x & 31;
-    if (nb <= 32) {
-        const Msg *const at[1] = {row + lane};
-        const bool use[1] = {lane < nb};
-        Msg m[1];
-        if (!msg_wait_all<1>(at, use, tag, m, st, bound)) return false;
-        if (use[0]) add(m[0]);
-        return true;
-    }
-    for (int b0 = lane; b0 - lane < nb; b0 += 32 * K) {
-        const Msg *at[K];
-        bool use[K];
-        Msg m[K];
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            at[j] = row + b0 + 32 * j;
-            use[j] = b0 + 32 * j < nb;
-        }
-        if (!msg_wait_all<K>(at, use, tag, m, st, bound)) return false;
-#pragma unroll
-        for (int j = 0; j < K; ++j)
-            if (use[j]) add(m[j]);
-    }
+    const Msg *const at[1] = {row + lane};
+    const bool use[1] = {lane < nb};
+    Msg m[1];
+    if (!msg_wait_all<1>(at, use, tag, m, st, bound)) return false;
+    if (use[0]) add(m[0]);
     return true;
 }
 

@@ -1520,7 +1520,7 @@ __device__ __forceinline__ bool grid_reduce_units(const A &g, double *s, int U, 
     if (wid < NV) {
         if (nb > 1) {
             t = 0.0;
-            if (!msg_collect<5>(row, nb, tag, st,
+            if (!msg_collect(row, nb, tag, st,
                              [&](const Msg &m) { t += __hiloint2double((int)m.y, (int)m.x); }))
                 bad = 1;
             __syncwarp();

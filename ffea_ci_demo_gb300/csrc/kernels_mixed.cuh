@@ -820,7 +820,7 @@ __device__ __forceinline__ float warp_sum_spread(const float (&v)[NV], int &inde
 // warp, double-float over the block's warps, published as one message per value, and every block adds the blocks'
 // messages in the same order. `tag` counts the launch's reductions from 1. The caller must pass a __syncthreads()
 // before smem (NV x 32 floats) is written again.
-template <int NV, int K, bool BATCH, class A>
+template <int NV, bool BATCH, class A>
 __device__ __forceinline__ bool grid_reduce_msg(const A &g, int rank, int nb, const float (&v)[NV], float *smem,
                                                 unsigned int tag, df32 *s_out, DevStatus *st, GridBarrier *gb) {
     const int lane = threadIdx.x & 31, wid = warp_index(), nw = blockDim.x >> 5;
@@ -828,7 +828,7 @@ __device__ __forceinline__ bool grid_reduce_msg(const A &g, int rank, int nb, co
     const float ws = warp_sum_spread<NV>(v, idx);
     if (idx >= 0) smem[idx * 32 + wid] = ws;
     __syncthreads();
-    if (gb && nb > MSG_SUM_BLOCKS) {
+    if (nb > MSG_SUM_BLOCKS) {
         float2 *const rows = reinterpret_cast<float2 *>(g.rmsg) + (size_t)(tag & 1u) * MSG_VALUES * g.stride;
         for (int i = wid; i < NV; i += nw) {
             df32 t = {lane < nw ? smem[i * 32 + lane] : 0.f, 0.f};
@@ -850,7 +850,7 @@ __device__ __forceinline__ bool grid_reduce_msg(const A &g, int rank, int nb, co
             if (lane < MSG_COPIES)
                 msg_put(rows + (size_t)lane * g.stride + rank, __float_as_uint(t.hi), __float_as_uint(t.lo), 0u, tag);
             t = df32{0.f, 0.f};
-            if (!msg_collect<K>(row, nb, tag, st, [&](const Msg &m) {
+            if (!msg_collect(row, nb, tag, st, [&](const Msg &m) {
                     t = df_add(t, df32{__uint_as_float(m.x), __uint_as_float(m.y)});
                 }, BATCH ? MSG_POLLS_BATCH : MSG_POLLS))
                 bad = 1;
@@ -1173,12 +1173,11 @@ __device__ __forceinline__ void spmv_row_w(const A &g, int tpn, const SrCache &c
 #undef FFEA_W_FMA
 
 // cg_mixed_sr_kernel's forms: up to SR_REG_THREADS lanes a block with RB 3x3 blocks of each lane in registers (4 where a
-// row has four lanes or more, so that they hold all of a usual row; else 6), or 1024 threads without (RB = 0). K is
-// how many of a sum's messages a lane waits for at once: as many as the registers hold without spilling.
+// row has four lanes or more, so that they hold all of a usual row; else 6), or 1024 threads without (RB = 0).
 constexpr int SR_REG_THREADS = 512;
 template <int RB>
 struct SrForm {
-    static constexpr int THREADS = RB > 0 ? SR_REG_THREADS : 1024, K = RB == 4 ? 5 : RB == 6 ? 3 : 2;
+    static constexpr int THREADS = RB > 0 ? SR_REG_THREADS : 1024;
 };
 constexpr int SR_REG_ROWS = 128;  // rows a block is given while the mesh leaves SMs free
 
@@ -1293,7 +1292,7 @@ static __device__ __noinline__ void cheb_coefficients(double *state, int degree)
 // projected right-hand side has no component, so the solution is the same: the one with Z^T D x = 0.
 // A batch's set-up moments of the blob's rows (sums 1 and 2 of the solve), in s_sc for the whole block; a call of its
 // own, so that its 28 values share no registers with the solve.
-template <int K, class A, class B>
+template <class A, class B>
 __device__ __noinline__ bool sr_moments(const A &g, const B &bl, int a0, int nloc, int rank, int nb, float *smemf,
                                         df32 *s_scf, double *s_sc) {
     // f.f, S1_f, S2_f and M = sum Phi^T D Phi (cf. gather_mixed_kernel), half of them per sum
@@ -1324,7 +1323,7 @@ __device__ __noinline__ bool sr_moments(const A &g, const B &bl, int a0, int nlo
         float v[14];
 #pragma unroll
         for (int i = 0; i < 14; ++i) v[i] = m[14 * half + i];
-        if (!grid_reduce_msg<14, K, true>(bl, rank, nb, v, smemf, (unsigned)half + 1u, s_scf, g.st, bl.gb)) return false;
+        if (!grid_reduce_msg<14, true>(bl, rank, nb, v, smemf, (unsigned)half + 1u, s_scf, g.st, bl.gb)) return false;
         if (threadIdx.x < 14) s_sc[14 * half + threadIdx.x] = df_double(s_scf[threadIdx.x]);
         __syncthreads();
     }
@@ -1419,7 +1418,7 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
             return g.dpos[a];
     };
     if constexpr (BATCH) {
-        if (!sr_moments<SrForm<RB>::K>(g, bl, a0, nloc, rank, nb, smemf, s_scf, s_sc)) return false;
+        if (!sr_moments(g, bl, a0, nloc, rank, nb, smemf, s_scf, s_sc)) return false;
         red_ep = 2;
     } else {
         grid_sum_df8<MIXED_GATHER_NP>(reinterpret_cast<const float2 *>(g.init_partials), g.init_stride, g.n_init, s_sc);
@@ -1572,7 +1571,7 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
             }
         }
         FFEA_MARK(g, tm, 1);
-        if (!(ok = grid_reduce_msg<MIXED_SR_NP, SrForm<RB>::K, BATCH>(bl, rank, nb, acc, smemf, ++red_ep, s_scf, st, bl.gb))) break;
+        if (!(ok = grid_reduce_msg<MIXED_SR_NP, BATCH>(bl, rank, nb, acc, smemf, ++red_ep, s_scf, st, bl.gb))) break;
         FFEA_MARK(g, tm, 3);
         if (warp_index() == 0) {
             // The iteration's scalars, in double-float as the sums arrive: this chain is on every block's critical path
