@@ -1330,6 +1330,14 @@ __device__ __noinline__ bool sr_moments(const A &g, const B &bl, int a0, int nlo
     return true;
 }
 
+// Every second iteration of a batch's solve forms q = V p from the matrix, one more pass: carried on by q = w~ + beta q
+// alone, q gathers the rounding of every pass, and the batch's solutions were up to a third further from FP64 than by
+// cg_batch_kernel's q = V p. rms error of the moves, streaming / q carried on / every 4th / 2nd / each direct: blobs of 4 to 8
+// cells 4.9 / 6.5 / 5.9 / 5.3 / 5.2e-7, 9 to 14 8.0 / 8.5 / 8.8 / 8.1 / 8.3e-7, 20 to 30 16.7 / 19.7 / 18.2 / 17.6 / 16.7e-7;
+// ms per step of 32 blobs of 8 to 32 cells 18.9 / 5.80 / 6.01 / 6.18 / 6.50. (In numpy the other vectors held in FP64 change
+// nothing; a pass summed in FP64 would halve the error.)
+constexpr int SR_DIRECT = 2;
+
 // One solve by nb blocks, this one of rank `rank`, with the launch's arguments g and the blob's own bl: the whole grid for a blob (cg_mixed_sr_kernel), or one blob's
 // blocks of a batch (BATCH: kernels_batch.cuh), which also forms the moments that the single blob's gather leaves in
 // g.init_partials. Returns false on a timeout.
@@ -1607,10 +1615,18 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
                 bl.cheb[1 + CHEB_REC + k] = beta;
             }
             __syncwarp();
-            if (ln < 6) {
-                if (ln < 3) s_tau[ln] = c.hi; else s_Om[ln - 3] = c.hi;
-                s_mp[ln] = df_add(mz, df_mul(b1, mp));
+            if (ln < 6) s_mp[ln] = df_add(mz, df_mul(b1, mp));
+            if constexpr (BATCH) {
+                if (k % SR_DIRECT == SR_DIRECT - 1) {  // the coefficients for p in place of z
+                    __syncwarp();
+                    if (defl && ln < 6) {
+                        c = df_mul(s_A6f[6 * ln], s_mp[0]);
+#pragma unroll
+                        for (int qq = 1; qq < 6; ++qq) c = df_add(c, df_mul(s_A6f[6 * ln + qq], s_mp[qq]));
+                    }
+                }
             }
+            if (ln < 3) s_tau[ln] = c.hi; else if (ln < 6) s_Om[ln - 3] = c.hi;
             if (ln == 0) {
                 s_conv = conv;
                 s_stop = stop;
@@ -1625,6 +1641,28 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
         if (s_stop) break;
         const float alpha = s_alpha, beta = s_beta;
         const float t0 = s_tau[0], t1 = s_tau[1], t2 = s_tau[2], O0 = s_Om[0], O1 = s_Om[1], O2 = s_Om[2];
+        bool direct = false;  // q = V p of this iteration from the matrix
+        if constexpr (BATCH) {
+            direct = k % SR_DIRECT == SR_DIRECT - 1;
+            if (direct) {
+                if ((int)threadIdx.x < nloc) {
+                    const int l = threadIdx.x;
+                    float pv[3];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const float zc = cheb ? su[c * npb + l] : sdi[c * npb + l] * sr[c * npb + l];
+                        sp[c * npb + l] = pv[c] = fmaf(beta, sp[c * npb + l], zc);
+                    }
+                    publish(ep + 1, l, pv[0], pv[1], pv[2]);
+                }
+                ++ep;
+                if (!(ok = halo_exchange<BATCH>(g, zs, hx, h0, nh, ep, st))) break;
+                float w0, w1, w2;
+                spmv(w0, w1, w2);
+                if (valid && sub == 0) { sw[l] = w0; sw[npb + l] = w1; sw[2 * npb + l] = w2; }
+                __syncthreads();
+            }
+        }
         // p = z + beta p ; q = w~ + beta q ; x += alpha p ; r -= alpha q ; z = M^{-1} r published (Jacobi), or
         // the Chebyshev iteration's first step (polynomial)
         for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
@@ -1640,8 +1678,8 @@ __device__ __forceinline__ bool sr_solve(const A &g, const B &bl, int rank, int 
             for (int c = 0; c < 3; ++c) {
                 const float r = sr[c * npb + l], di = sdi[c * npb + l];
                 const float zc = cheb ? su[c * npb + l] : di * r;
-                const float pv = fmaf(beta, sp[c * npb + l], zc);
-                const float qv = fmaf(beta, sq[c * npb + l], wv[c]);
+                const float pv = direct ? sp[c * npb + l] : fmaf(beta, sp[c * npb + l], zc);
+                const float qv = direct ? wv[c] : fmaf(beta, sq[c * npb + l], wv[c]);
                 sp[c * npb + l] = pv;
                 sq[c * npb + l] = qv;
                 sx[c * npb + l] += alpha * pv;

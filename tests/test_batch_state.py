@@ -72,3 +72,31 @@ def test_plan_of_the_solve(gpu, cells, kernel):
     bt = lib.Batch([box[c] for c in cells], **KW)
     assert bt.cg_kernel() == kernel
     bt.update(2)
+
+
+def test_accuracy_of_the_solve_on_chip(gpu):
+    """The batch's solutions are as near to FP64 as the streaming kernel's, whose q = V p is formed every iteration: the
+    rms error of the moves over blobs of one block and of several, to a fifth (the spread over such sets)."""
+    cells = [(4, 4, 4), (6, 6, 6), (7, 6, 7), (10, 10, 10), (14, 13, 14), (18, 18, 18)]
+    meshes, x0 = batch(cells)
+    bt = lib.Batch(meshes, **KW)
+    streams = [bt.rng_state(b) for b in range(len(meshes))]
+    exact = []
+    for m, p, s in zip(meshes, x0, streams):
+        f = lib.Blob(m, epsilon=1e-13, rng_state=s, **KW)
+        f.set_state(pos=p)
+        f.update(4)
+        exact.append(f.pos())
+    err = {}
+    for kernel in ("sr_batch_kernel", "cg_batch_kernel"):
+        if kernel == "cg_batch_kernel":
+            bt.set_config(256, 4)
+        assert bt.cg_kernel() == kernel
+        bt.set_positions(np.concatenate(x0))
+        for b, s in enumerate(streams):
+            bt.set_rng_state(b, s)
+        bt.update(4)
+        err[kernel] = np.sqrt(np.mean([((bt.pos(b) - e) ** 2).sum() / ((e - x0[b]) ** 2).sum()
+                                       for b, e in enumerate(exact)]))
+    print(err)
+    assert err["sr_batch_kernel"] <= 1.2 * err["cg_batch_kernel"]
