@@ -154,7 +154,9 @@ namespace {
 constexpr double L2_MATRIX_BYTES = 100e6;
 // how much of a larger matrix cg_mixed_own_kernel asks L2 to keep while the rest streams past it: 64^3 cells (161 MB),
 // ms per step at 0 / 2 / 3 / 4 / 5 eighths 26.0 / 23.8 / 23.3 / 26.0 / 29.5, and 29.8 without the hints (L2 holds about
-// half its size of lines that both dies read)
+// half its size of lines that both dies read). At 0 / 31 / 45 / 62 / 80 MB: 54^3 17.3 / 16.7 / 16.3 / 15.5 / 15.3, 58^3 19.8 /
+// 18.5 / 18.5 / 17.6 / 17.8, 60^3 20.6 / 20.2 / 19.6 / 19.0 / 18.8, 68^3 34.4 / 34.4 / 34.4 / 34.3 / 36.7, 72^3 51.4 / 50.0 /
+// 50.0 / 53.0 / 53.0 (without the hints 59.2)
 constexpr double L2_KEEP_BYTES = 62e6;
 
 template <class R>
@@ -521,7 +523,10 @@ struct BlobImpl final : ffea_gpu_blob {
         // as tagged messages, so a block more costs little, and up to SR_REG_ROWS rows its lanes hold the whole matrix
         // in registers (four lanes of four blocks to a row). us per step at 64 / 128 / 192 / 256 / 320 rows a block:
         // 10^3 cells 499 / 455 / 508 / 509 / 567, 20^3 976 / 879 / 930 / 968 / 1078, 24^3 - / 1117 / 1124 / 1166 / 1321.
-        // Above SR_REG_THREADS rows a block (N > 73,000) the form without register blocks takes over.
+        // Above SR_REG_THREADS rows a block (N > 77,824) the form without register blocks takes over. The mixed
+        // consistent-mass solve (cg_mixed_own_kernel) takes one block up to 512 rows and 64 rows a block from there; us per step
+        // at 32 / 64 / 128 / 256 rows a block, and in one: 343 nodes 199 / 206 / 221 / 218, 180; 512 226 / 230 / 257 / 263, 215;
+        // 1331 227 / 228 / 247 / 245, 367; 9261 244 / 246 / 264 / 267; 24,389 275 / 274 / 275 / 282; 68,921 346 / 346 / 345 / 345.
         const bool sr_able = mixed && p.solver == FFEA_GPU_NOMASS_CG && 40.0 * (double)h.nslots <= L2_MATRIX_BYTES;
         auto pick_grid = [&](bool sr) {
             if (sr) {
@@ -549,7 +554,8 @@ struct BlobImpl final : ffea_gpu_blob {
         int npb = pick_grid(sr_able);
         ss_grid = cg_grid; ss_block = cg_block; ss_tpn = tpn;
         // The CG kernel follows from the blob's size alone (no other input selects it):
-        //  - each block keeps a run of rows in shared memory when they fit (cg_own_kernel, cg_mixed_own_kernel);
+        //  - FP64: the unit kernel while it holds the blob's rows (pick_units);
+        //  - else each block keeps a run of rows in shared memory when they fit (cg_own_kernel, cg_mixed_own_kernel);
         //    the run is a multiple of a warp's rows so that a warp's rows share a SELL slice; else the grid-strided
         //    cg_kernel / cg_mixed_kernel;
         //  - the mixed CG_nomass solve takes one reduction per iteration (cg_mixed_sr_kernel) when its rows fit and
@@ -1185,7 +1191,7 @@ struct BlobImpl final : ffea_gpu_blob {
 
     // Jacobi-PCG solve of the blob's current matrix with every work array in g_solve_scratch, by the
     // grid-strided cg_kernel opened by solve_static_prep_kernel instead of the gather. A step of a blob whose
-    // rows fit in shared memory runs cg_own_kernel instead, whose sums run in another order, so the two agree
+    // rows fit on chip runs cg_own_unit_kernel or cg_own_kernel instead, whose sums run in another order, so the two agree
     // to rounding, not bit for bit. Host copies go through the blob's pinned staging buffer; nothing is
     // allocated. The blob's device is current for the call (the caller's is restored), and once a kernel is
     // queued every return waits for the stream first, so the lock is never released while a kernel of this

@@ -16,9 +16,13 @@
 //
 // Reductions: each node's contribution is formed in FP32, summed over the
 // block and the grid as double-float pairs (two FP32 values, ~48-bit
-// significand) and finished in FP64; GB300 runs FP64 at 1/64 of the FP32
-// rate, so no per-node work touches the FP64 pipe. The scalars alpha, beta
-// and the mode coefficients are computed once per block in FP64.
+// significand); GB300 runs FP64 at 1/64 of the FP32 rate, so no per-node work
+// touches the FP64 pipe. The set-up's mode matrix is formed in FP64, and so are
+// the iteration's scalars of cg_mixed_kernel and cg_batch_kernel; the owned-rows
+// kernels form theirs (p.q, the mode coefficients, the stopping test) in
+// double-float, step lengths in FP32 everywhere. With FP64 scalars in those too,
+// every solution and iteration count of ten meshes of 343 to 166,375 nodes came
+// out the same to the last digit.
 //
 // Z is expressed through per-node offsets d_a from a reference point: the
 // k-th mode is t_k + w_k x d_a. Z^T v needs only S1 = sum v_a and
@@ -1267,7 +1271,7 @@ static __device__ __noinline__ void cheb_coefficients(double *state, int degree)
 // Gear, 1989): the SpMV is applied to the preconditioned residual z = M^{-1} r, w = V z, and the search
 // direction's product follows from q = w~ + beta q_old, p = z + beta p_old, so beta is not needed before the
 // SpMV. One sweep computes w and all the dot products the step needs (r.z, r.r, z.w, z.q_old, p_old.w and the
-// rigid-mode moments of D z); p.q is then formed from them in FP64:
+// rigid-mode moments of D z); p.q is then formed from them in double-float:
 //     p.q = z.w~ + beta (z.q_old + p_old.w~) + beta^2 p_old.q_old,    w~ = w + D Z A6 Z^T D z.
 // Rows are owned as in cg_mixed_own_kernel. With M = D (Jacobi) the iterates are, in exact arithmetic, those of the
 // other mixed CG kernels; in FP32 they agree to rounding and converge in the same number of iterations.

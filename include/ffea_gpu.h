@@ -46,8 +46,8 @@ extern "C" {
 
 /* arithmetic of the step */
 #define FFEA_GPU_FP64 0  /* every operation in FP64, in the reference's evaluation order */
-#define FFEA_GPU_MIXED 1 /* FP32 element stress, noise scaling, matrix and SpMV; FP64 dot products,
-                            residual norms, near-degenerate Jacobians and the position accumulator */
+#define FFEA_GPU_MIXED 1 /* FP32 element stress, noise scaling, matrix and SpMV; double-float (FP32 pairs)
+                            dot products and residual norms; FP64 near-degenerate Jacobians and positions */
 
 /* the hot-path fields of SimulationParams (include/SimulationParams.h:75-211), meso units */
 typedef struct ffea_gpu_params {
@@ -68,9 +68,9 @@ typedef struct ffea_gpu_params {
      * uses Jacobi and estimates the largest eigenvalue of D^-1 V for the later ones. */
     int cg_poly;
     /* Shared-memory copy of the matrix in the mixed-precision single-reduction CG_nomass kernel (not a reference
-     * parameter): each block keeps the first 3x3 blocks of its owned rows on chip for the whole solve.
-     * 0: as many as fit (the default); n > 0: at most n per row; -1: none. The results do not depend on it
-     * (only where the matrix is read from), so it exists for measurements of the cache's effect. */
+     * parameter): each block keeps 3x3 blocks of its owned rows in shared memory for the whole solve, those after
+     * the ones its threads hold in registers. 0: as many as fit (the default); n > 0: at most n per row; -1: none.
+     * The results do not depend on it (only where the matrix is read from), so it exists for measurements. */
     int cg_smem_blocks;
 } ffea_gpu_params;
 #define FFEA_GPU_CG_POLY_DEFAULT 6
@@ -182,11 +182,12 @@ int ffea_gpu_blob_cg_iterations(ffea_gpu_blob *blob, int *last, long long *total
  * NoMassCGSolver::solve tests against epsilon2); *count gets the number written (<= max_entries). */
 int ffea_gpu_blob_cg_history(ffea_gpu_blob *blob, double *res2, int max_entries, int *count);
 
-/* Where the last CG solve spent its time, as seen by one thread block (device timer, ns, summed
- * over iterations): [0] set-up, [1] SpMV, [2] block reduction after the SpMV, [3] grid barrier
- * after the SpMV, [4] cross-block sums and step length, [5] solution/residual update, [6] its block
- * reduction, [7] its grid barrier, [8] its cross-block sums, [9] direction update and its barrier
- * (FP64 path only). n_phases is 10. */
+/* Where the last CG solve spent its time, as seen by one thread block (its SM clock, in ns, summed over iterations):
+ * [0] set-up, with the first preconditioned residual; [1] SpMV; [2] block reduction after the SpMV; [3] the sums
+ * across blocks after it with their wait (where [2] is 0 with the block's part too); [4] cross-block sums and step
+ * length; [5] solution/residual update; [6] its block reduction, or the Chebyshev steps' matrix passes; [7] its sums
+ * across blocks with their wait, or the exchanges with neighbouring blocks; [8] its cross-block sums, or (FP64, rows
+ * on chip) the direction's update; [9] direction update and its exchange (FP64 path only). n_phases is 10. */
 #define FFEA_GPU_CG_PHASES 10
 int ffea_gpu_blob_cg_profile(ffea_gpu_blob *blob, double *phase_ns, int n_phases);
 
