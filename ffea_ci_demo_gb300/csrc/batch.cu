@@ -415,12 +415,8 @@ int ffea_gpu_batch::set_config(int threads, int tpn_) {
 // (10^3 to 40^3 cells; its latencies do not shrink with the rows, so full blocks win as soon as there is work for
 // them all), times 0.17 iterations per row along a side (2 per cell) with the polynomial. Blobs of one block keep the
 // Jacobi preconditioner (3 us an iteration, which the polynomial's passes would cost as well). Left out (sr_ok false:
-// cg_batch_kernel) when a blob's rows do not fit, when there are more than four blobs to a block, or when a block would
-// work for more than three times the longest solve at blobs of up to 64 rows: cg_batch_kernel, which runs four to eight
-// groups on an SM at once, takes 2.9 to 3.4 times that solve's time however many blobs there are. us per solve on chip
-// against streaming, blobs of 8 / 27 / 64 / 125 rows: 456 of them (three to a block) 234 / 416 / 597 / 781 against
-// 222 / 447 / 660 / 1016, 532 (four) 304 / 550 / 790 / 1035 against 220 / 450 / 655 / 1040; 600 of 1 to 3 cells a side
-// 638 against 619.
+// cg_batch_kernel) when a blob's rows do not fit, or when there are so many tiny blobs that a block would run more
+// than four one after another while cg_batch_kernel runs up to eight on an SM at once.
 int ffea_gpu_batch::plan_solve() {
     int sms = 0;
     const size_t limit = BatchLaunch::sr_smem_limit(device, sms);
@@ -465,9 +461,6 @@ int ffea_gpu_batch::plan_solve() {
     }
     if (rows == 0) return FFEA_GPU_OK;
     schedule(rows);
-    int largest = 0;
-    for (int b = 0; b < nblobs; ++b) largest = std::max(largest, row_off[b + 1] - row_off[b]);
-    if (largest <= 64 && best > 3.001 * cost[order[0]]) return FFEA_GPU_OK;
     sr_host.assign(nblobs, SrBlob{});
     Halo hl;
     std::vector<int> first_ptr(nblobs);
