@@ -415,8 +415,11 @@ int ffea_gpu_batch::set_config(int threads, int tpn_) {
 // (10^3 to 40^3 cells; its latencies do not shrink with the rows, so full blocks win as soon as there is work for
 // them all), times 0.17 iterations per row along a side (2 per cell) with the polynomial. Blobs of one block keep the
 // Jacobi preconditioner (3 us an iteration, which the polynomial's passes would cost as well). Left out (sr_ok false:
-// cg_batch_kernel) when a blob's rows do not fit, or when there are so many tiny blobs that a block would run more
-// than four one after another while cg_batch_kernel runs up to eight on an SM at once.
+// cg_batch_kernel) when a blob's rows do not fit, or when there are more than four blobs to a block: cg_batch_kernel runs
+// four to eight groups on an SM at once, and tiny blobs are about even there. us per step on chip against streaming, blobs
+// of 8 / 27 / 64 / 125 rows: 456 of them 265 / 480 / 679 / 910 against 392 / 628 / 849 / 1241, 600 346 / 630 / 896 / 1213
+// against 471 / 708 / 946 / 1372, 608 (every group one CTA) 346 / 630 / 896 / 1213 against 437 / 631 / 850 / 1266. (The
+// solves alone are even from 400 on; the streaming kernel's schedule, one block over all blobs, takes the rest.)
 int ffea_gpu_batch::plan_solve() {
     int sms = 0;
     const size_t limit = BatchLaunch::sr_smem_limit(device, sms);
