@@ -1434,7 +1434,7 @@ __device__ __forceinline__ void spmv_row_pd(const CgArgs<R> &g, const double2 *p
 //    while the sums travel, the convergence test multiplies, and the history is divided at the end;
 //  - x is updated while the residual's sums travel.
 // us per step before (barriers on counters, 256 rows a block, shared-memory state) -> now: 64 nodes consistent mass
-// 288 -> 168, 343 nodes 1905 -> 646, 9261 nodes consistent mass 670 -> 387, 40^3 cells 18.7 -> 15.2 ms (there the SpMV
+// 288 -> 154, 343 nodes 1905 -> 666, 9261 nodes consistent mass 670 -> 399, 40^3 cells 18.7 -> 15.2 ms (there the SpMV
 // issues for 14.2 of its 16.4 us per iteration).
 // Every value is computed from the same products as in cg_kernel, fused in the same way per component; only the
 // grouping of sums changes.

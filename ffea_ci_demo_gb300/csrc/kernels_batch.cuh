@@ -258,8 +258,8 @@ __global__ void __launch_bounds__(BATCH_MAX_THREADS) cg_batch_kernel(const __gri
 // cg_batch_kernel streams every blob's matrix from HBM each iteration, all blobs at once (0.64 of the copy rate, which
 // bounds it); here a blob's matrix is read once per solve and what bounds the solve is its exchanges' latency, so the
 // host gives a block as many rows as the chip holds (plan_solve). 32 blobs of 8 to 32 cells a side, 219,234 nodes:
-// 18.0 -> 5.7 ms per solve (15.8 by the best of cg_batch_kernel's shapes); 8 such blobs 10.1 -> 2.1, 64 34.4 -> 12.7,
-// 40 blobs of 2 to 8 cells 1.71 -> 0.63, 200 of 3 to 6 cells 1.35 -> 0.47.
+// 18.8 -> 5.87 ms per solve; 8 such blobs 10.9 -> 2.14, 64 35.1 -> 12.2, 40 blobs of 2 to 8 cells 1.77 -> 0.71, 200 of 3 to 6
+// cells 1.37 -> 0.52.
 __global__ void __launch_bounds__(SR_REG_THREADS, 1) sr_batch_kernel(const __grid_constant__ SrBatchArgs b) {
     __shared__ SrBlob s_bl;
     if (b.common.st->abort) return;

@@ -1281,8 +1281,8 @@ static __device__ __noinline__ void cheb_coefficients(double *state, int degree)
 // instead of an L2 read per block), and the matrix stays on chip: RB blocks of each lane in registers, the next kc of
 // each row in shared memory, what is left read from L2. 512 threads with 128 registers hold 6 blocks a lane
 // (8 spilled, and the reloads missed the L1 that shared memory leaves: 3.51 against 3.09 ms per 40^3 step).
-// us per step, counters and L2 reads before -> now: 6^3 cells 590 -> 306, 10^3 cells - -> 393, 20^3 1553 -> 765,
-// 30^3 - -> 1283, 40^3 3805 -> 2575, 45^3 (without register blocks) 4624 -> 4018.
+// us per step, counters and L2 reads before -> now: 6^3 cells 590 -> 306, 10^3 cells - -> 399, 20^3 1553 -> 737,
+// 30^3 - -> 1221, 40^3 3805 -> 2483, 45^3 (without register blocks) 4624 -> 3756.
 // Polynomial preconditioning (g.poly = d > 0, once lambda_max of D^{-1} V is known): M^{-1} = P_d(D^{-1} V) D^{-1},
 // with 1 - lambda P_d(lambda) the Chebyshev polynomial of degree d + 1 on [lambda_max / cheb_ratio(d),
 // lambda_max], scaled to 1 at 0. z is built by d steps of the Chebyshev iteration for V z = r from z = 0 (d SpMVs,
